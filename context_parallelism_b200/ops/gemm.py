@@ -56,8 +56,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         assert epi != EPI_F32_ACC, "accumulate needs an output buffer"
     assert out.stride(-1) == 1 and out.dim() == 2 and out.shape[0] == M and out.shape[1] == N
     st = nv.status_for(a.device)
-    nv.call("gemm_bf16", nv.ptr(a), nv.ptr(b), nv.ptr(out), nv.ptr(aux),
-            nv.ptr(bias.float() if bias is not None and bias.dtype != torch.float32 else bias),
+    if bias is not None:
+        bias = bias.float().contiguous()
+        if bias.data_ptr() % 16:
+            bias = bias.clone()
+    nv.call("gemm_bf16", nv.ptr(a), nv.ptr(b), nv.ptr(out), nv.ptr(aux), nv.ptr(bias),
             nv.i(M), nv.i(N), nv.i(K), nv.i(a.stride(0)), nv.i(b.stride(0)), nv.i(out.stride(0)),
             nv.i(aux.stride(0) if aux is not None else 0), nv.i(a_mn), nv.i(b_mn), nv.i(epi),
             st.ptr(), nv.stream_ptr(a.device))

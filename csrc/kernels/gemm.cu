@@ -1,6 +1,6 @@
-// Persistent bf16 GEMM for sm_100a: TMA -> shared memory -> tcgen05.mma -> tensor memory ->
-// registers -> global, warp-specialised, with a double-buffered accumulator so the epilogue of tile
-// i overlaps the main loop of tile i+1.
+// Persistent bf16 GEMM for sm_100a on CTA pairs (tcgen05 cta_group::2): two CTAs of a cluster compute one 256 x BN output
+// tile together, TMA -> shared memory -> tcgen05.mma -> tensor memory -> registers -> shared memory -> TMA, warp-specialised,
+// with a double-buffered accumulator so that the epilogue of one tile overlaps the main loop of the next.
 //
 //   C[M,N] (op)= A * B        A is M x K, B is N x K ("NT": both K-major) by default.
 //   a_mn = 1 : A is stored as [K, M] (M contiguous)   -> weight-gradient GEMM  dW = dY^T X
@@ -10,8 +10,19 @@
 // Replaces the cuBLAS GEMMs behind nn::Linear in the reference trainers
 // (Scripts/Blutrain/bluscriptCP.cpp:212-330, Makefile:129).
 //
-// Warp roles (192 threads): warp 0 = TMA producer, warp 1 = tensor-memory owner + MMA issuer,
-// warps 2..5 = epilogue (warp w reads TMEM lanes 32*(w%4)..+31).
+// Why pairs: with one CTA per tile (128 x 256) every K=16 step of the tensor core reads (128 + 256) x 16 x 2 = 12 KB of
+// operands from shared memory while TMA writes the same 12 KB, i.e. 192 bytes per tensor-core cycle against the 128 bytes
+// per cycle a shared memory delivers.  In a pair each CTA stages its own 128 rows of A and only HALF of the B tile; one MMA
+// instruction issued by the even CTA drives both tensor cores and each of them reads the other CTA's B half through the
+// pair link, so a CTA moves (128 + 128) x 16 x 2 = 8 KB in and 8 KB out per step: 128 bytes per cycle.
+//
+// Protocol (per CTA: warp 0 = TMA producer, warp 1 = tensor-memory owner and, in the even CTA, MMA issuer, warps 2..5 =
+// epilogue).  Every TMA load of either CTA (cta_group::2 form, no multicast) signals the EVEN CTA's `full` barrier, which
+// expects the bytes of both CTAs.  After the MMAs of a stage the issuer commits twice, once to its own `empty` barrier and
+// once to the odd CTA's (a cluster address), and likewise for the accumulator-ready barriers; the odd CTA's epilogue
+// warps release an accumulator by a remote arrival on the even CTA's barrier.  Tensor memory is allocated with the
+// cta_group::2 form by the same warp of both CTAs, so an accumulator has the same address in both; each CTA's epilogue
+// drains its own 128 rows.  All waits are bounded like everywhere else in this library.
 #include "common.cuh"
 #include "gemm_common.cuh"
 #include "host_utils.h"
@@ -19,69 +30,160 @@
 
 namespace cpb {
 
-template <int BN, int STAGES, bool A_MN, bool B_MN>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
-gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p) {
-  using L = GemmSmem<BN, STAGES>;
+template <int BN>
+struct GemmSmem {
+  static constexpr int STAGES = BN == 256 ? 6 : 8;               // 192 KB of operands in flight
+  static constexpr int A_BYTES = GEMM_BM * GEMM_BK * 2;          // 128 rows of A
+  static constexpr int B_BYTES = (BN / 2) * GEMM_BK * 2;         // this CTA's half of B's columns
+  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int STORE_OFFSET = STAGES * STAGE_BYTES;      // 4 epilogue warps x 2 buffers x 4 KB
+  static constexpr int BAR_OFFSET = STORE_OFFSET + 32768;
+  static constexpr int TOTAL = BAR_OFFSET + 256 + 1024;
+};
+
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// TMA load of a CTA pair: the data lands in THIS CTA's shared memory, the bytes are counted on the barrier at `bar_addr`
+// (a cluster address: the even CTA's barrier).  No multicast.
+__device__ __forceinline__ void tma_load_2d_pair(void* smem, const CUtensorMap* m, uint32_t bar_addr, int x, int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(smem_u32(smem)), "l"((uint64_t)m), "r"(bar_addr), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_dst, uint32_t ncols) {      // same warp of both CTAs
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() {
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+template <bool ACC>
+__device__ __forceinline__ void umma_pair_ss_cp(uint32_t leader, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "n"(ACC ? 1 : 0), "r"(leader) : "memory");
+}
+__device__ __forceinline__ void umma_pair_ss_p(uint32_t leader, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
+}
+// Arrive on the barrier at `cluster_addr` (any CTA of the cluster) once every MMA issued so far has completed.
+__device__ __forceinline__ void umma_pair_commit_p(uint32_t leader, uint32_t cluster_addr) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+      ::"r"(cluster_addr), "r"(leader) : "memory");
+}
+
+// Tile order: bands of `band` pair-rows swept along N, rows fastest.  With band = 8 the 74 pairs running at one time
+// share 8 row tiles of A and about 9 column tiles of B, and successive waves keep the band's A rows in L2, so a GEMM
+// whose B operand does not fit in L2 beside A's band (8192^3: 134 MB against 126 MB) streams B once per band instead of
+// once per 2.3 rows of tiles.  band = 1 is the plain order (columns fastest), kept while B stays resident anyway.
+__device__ __forceinline__ void pair_tile_coords(int tile, int num_m_tiles, int num_n_blocks, int band_rows, int& mt, int& nb) {
+  const int per_band = band_rows * num_n_blocks;
+  const int band = tile / per_band, idx = tile - band * per_band;
+  const int rows = min(band_rows, num_m_tiles - band * band_rows);
+  nb = idx / rows;
+  mt = band * band_rows + (idx - nb * rows);
+}
+
+template <int BN, bool A_MN, bool B_MN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
+gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                      const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmX, GemmParams p) {
+  using L = GemmSmem<BN>;
+  constexpr int STAGES = L::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint64_t* full_bar = (uint64_t*)(smem + L::BAR_OFFSET);
+  uint64_t* full_bar = (uint64_t*)(smem + L::BAR_OFFSET);      // used in the even CTA only
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* tfull_bar = empty_bar + STAGES;     // [2]
-  uint64_t* tempty_bar = tfull_bar + 2;         // [2]
+  uint64_t* tempty_bar = tfull_bar + 2;         // [2], used in the even CTA only
   uint32_t* tmem_slot = (uint32_t*)(tempty_bar + 2);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int num_tiles = p.num_m_blocks * p.num_n_blocks;
+  const uint32_t rank = cluster_ctarank();      // 0: even CTA (issues the MMAs), 1: odd CTA
+  const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
+  const int num_tiles = p.num_m_tiles * p.num_n_blocks;
+  const int num_items = num_tiles * p.splits;   // item = split * num_tiles + tile: items of one K range run together
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int s = 0; s < 2; ++s) { mbar_init(&tfull_bar[s], 1); mbar_init(&tempty_bar[s], 4); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&tfull_bar[s], 1); mbar_init(&tempty_bar[s], 8); }      // 4 epilogue warps of each CTA
     *abort_flag = 0;
     fence_mbar_init();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, 2 * BN);
-    tmem_relinquish();
+    tmem_alloc_pair(tmem_slot, 2 * BN);
+    tmem_relinquish_pair();
   }
   tc_fence_before();
   __syncthreads();
+  cluster_sync_all();                           // both CTAs' barriers exist before anything arrives on them remotely
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
+    // ------------------------------------------------------------------ TMA producer (both CTAs)
     if (lane == 0) {
       tma_prefetch_desc(&tmA);
       tma_prefetch_desc(&tmB);
       int stage = 0; uint32_t phase = 0;
-      for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-        const int m0 = (tile / p.num_n_blocks) * GEMM_BM;
-        const int n0 = (tile % p.num_n_blocks) * BN;
-        for (int kb = 0; kb < p.num_k_blocks; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, 100)) break;
+      for (int item = pair; item < num_items; item += num_pairs) {
+        const int split = item / num_tiles;
+        int mt, nb;
+        pair_tile_coords(item - split * num_tiles, p.num_m_tiles, p.num_n_blocks, p.band, mt, nb);
+        const int m0 = mt * (2 * GEMM_BM) + (int)rank * GEMM_BM;      // this CTA's rows
+        const int kb1 = min(p.num_k_blocks, (split + 1) * p.k_per_split);
+        for (int kb = split * p.k_per_split; kb < kb1; ++kb) {
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, 110)) break;
           uint8_t* sa = smem + stage * L::STAGE_BYTES;
           uint8_t* sb = sa + L::A_BYTES;
-          mbar_expect_tx(&full_bar[stage], L::STAGE_BYTES);
+          const uint32_t full_even = map_to_cta(smem_u32(&full_bar[stage]), 0);
+          if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * L::STAGE_BYTES);              // the bytes of both CTAs
           const int k0 = kb * GEMM_BK;
           if (A_MN) {
 #pragma unroll
-            for (int g = 0; g < GEMM_BM / 64; ++g) tma_load_2d(sa + g * 8192, &tmA, &full_bar[stage], m0 + g * 64, k0);
+            for (int g = 0; g < GEMM_BM / 64; ++g) tma_load_2d_pair(sa + g * 8192, &tmA, full_even, m0 + g * 64, k0);
           } else {
-            tma_load_2d(sa, &tmA, &full_bar[stage], k0, m0);
+            tma_load_2d_pair(sa, &tmA, full_even, k0, m0);
           }
           if (p.epi == EPI_BF16_SWIGLU) {
-            // gate rows n0/2.. and up rows F + n0/2.. of the fused [2F, K] weight
-            const int f0 = (tile % p.num_n_blocks) * (BN / 2);
-            tma_load_2d(sb, &tmB, &full_bar[stage], k0, f0);
-            tma_load_2d(sb + (BN / 2) * 128, &tmB, &full_bar[stage], k0, p.swiglu_half + f0);
+            // the even CTA stages the gate rows of features nb*BN/2.., the odd CTA the matching up rows
+            const int f0 = nb * (BN / 2);
+            tma_load_2d_pair(sb, &tmB, full_even, k0, (rank == 0 ? 0 : p.swiglu_half) + f0);
           } else if (B_MN) {
+            const int n0 = nb * BN + (int)rank * (BN / 2);
 #pragma unroll
-            for (int g = 0; g < BN / 64; ++g) tma_load_2d(sb + g * 8192, &tmB, &full_bar[stage], n0 + g * 64, k0);
+            for (int g = 0; g < BN / 2 / 64; ++g) tma_load_2d_pair(sb + g * 8192, &tmB, full_even, n0 + g * 64, k0);
           } else {
-            tma_load_2d(sb, &tmB, &full_bar[stage], k0, n0);
+            tma_load_2d_pair(sb, &tmB, full_even, k0, nb * BN + (int)rank * (BN / 2));
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -89,87 +191,133 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    // The whole warp runs the loop convergently and only the elected lane issues, so that the descriptors stay
-    // warp-uniform and stepping one is a single add: at BN = 128 an MMA lasts 64 cycles, and the scalar work between
-    // two of them must stay well below that.
-    {
+    // ------------------------------------------------------------------ MMA issuer (even CTA only; convergent warp, elected lane)
+    if (rank == 0) {
       const uint32_t leader = elect_one() ? 1u : 0u;
-      constexpr uint32_t idesc = make_idesc_bf16(GEMM_BM, BN, A_MN, B_MN);
+      constexpr uint32_t idesc = make_idesc_bf16(2 * GEMM_BM, BN, A_MN, B_MN);
       const uint32_t s0 = smem_u32(smem);
-      const SDesc da0 = sdesc_split(A_MN ? make_sdesc(s0, 8192, 1024) : sdesc_kmajor(s0));                       // stage 0
+      const SDesc da0 = sdesc_split(A_MN ? make_sdesc(s0, 8192, 1024) : sdesc_kmajor(s0));
       const SDesc db0 = sdesc_split(B_MN ? make_sdesc(s0 + L::A_BYTES, 8192, 1024) : sdesc_kmajor(s0 + L::A_BYTES));
       constexpr uint32_t A_STEP = A_MN ? 2048 : 32, B_STEP = B_MN ? 2048 : 32;
       int stage = 0; uint32_t phase = 0;
       int it = 0;
       bool alive = true;
-      for (int tile = blockIdx.x; tile < num_tiles && alive; tile += gridDim.x, ++it) {
+      for (int item = pair; item < num_items && alive; item += num_pairs, ++it) {
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
-        if (!__all_sync(0xffffffffu, mbar_wait(&tempty_bar[acc], acc_phase ^ 1, abort_flag, p.status, 200))) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(&tempty_bar[acc], acc_phase ^ 1, abort_flag, p.status, 210))) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < p.num_k_blocks; ++kb) {
-          if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, abort_flag, p.status, 201))) { alive = false; break; }
+        const int split = item / num_tiles;
+        const int kb0 = split * p.k_per_split, kb1 = min(p.num_k_blocks, kb0 + p.k_per_split);
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, abort_flag, p.status, 211))) { alive = false; break; }
           tc_fence_after();
           const uint32_t so = (uint32_t)stage * (L::STAGE_BYTES >> 4);
           const SDesc da = SDesc{da0.lo + so, da0.hi}, db = SDesc{db0.lo + so, db0.hi};
-          umma_ss_p(leader, d_tmem, sdesc_at(da, 0), sdesc_at(db, 0), idesc, kb != 0);
+          umma_pair_ss_p(leader, d_tmem, sdesc_at(da, 0), sdesc_at(db, 0), idesc, kb != kb0);
 #pragma unroll
           for (int k = 1; k < GEMM_BK / 16; ++k)
-            umma_ss_cp<true>(leader, d_tmem, sdesc_at(da, k * A_STEP), sdesc_at(db, k * B_STEP), idesc);
-          umma_commit_p(leader, &empty_bar[stage]);
+            umma_pair_ss_cp<true>(leader, d_tmem, sdesc_at(da, k * A_STEP), sdesc_at(db, k * B_STEP), idesc);
+          // the stage is free in both CTAs once these MMAs have read it
+          const uint32_t e_own = smem_u32(&empty_bar[stage]);
+          umma_pair_commit_p(leader, e_own);
+          umma_pair_commit_p(leader, map_to_cta(e_own, 1));
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-        umma_commit_p(leader, &tfull_bar[acc]);
+        const uint32_t t_own = smem_u32(&tfull_bar[acc]);
+        umma_pair_commit_p(leader, t_own);
+        umma_pair_commit_p(leader, map_to_cta(t_own, 1));
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..5)
+    // ------------------------------------------------------------------ epilogue (warps 2..5 of both CTAs: own 128 rows)
     const int quarter = warp & 3;
+    WarpStore ws{smem + L::STORE_OFFSET + quarter * 8192, 0u, lane == 0};
     int it = 0;
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++it) {
+    for (int item = pair; item < num_items; item += num_pairs, ++it) {
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
-      const int m0 = (tile / p.num_n_blocks) * GEMM_BM;
-      const int nb = tile % p.num_n_blocks;
-      bool ok = mbar_wait(&tfull_bar[acc], acc_phase, abort_flag, p.status, 300);
+      int mt, nb;
+      pair_tile_coords(item % num_tiles, p.num_m_tiles, p.num_n_blocks, p.band, mt, nb);
+      const int row0 = mt * (2 * GEMM_BM) + (int)rank * GEMM_BM + quarter * 32;
+      bool ok = mbar_wait(&tfull_bar[acc], acc_phase, abort_flag, p.status, 310);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      const int row = m0 + quarter * 32 + lane;
       const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
-      gemm_epilogue_row<BN>(p, t_row, row, nb);
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&tempty_bar[acc]);
+      gemm_epilogue<BN>(p, &tmC, &tmX, ws, t_row, row0, nb, lane, [&] {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (rank == 0) mbar_arrive(&tempty_bar[acc]);
+          else mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[acc]), 0));
+        }
+      });
     }
+    ws.drain();
   }
 
   tc_fence_before();
   __syncthreads();
+  cluster_sync_all();          // the even CTA's MMAs have finished reading the odd CTA's operands; no remote arrival is in flight
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 2 * BN);
+    tmem_dealloc_pair(tmem_base, 2 * BN);
   }
 }
 
-template <int BN, int STAGES, bool A_MN, bool B_MN>
-static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, cudaStream_t stream) {
-  using L = GemmSmem<BN, STAGES>;
-  auto kern = gemm_bf16_kernel<BN, STAGES, A_MN, B_MN>;
+template <int BN, bool A_MN, bool B_MN>
+static int launch_pair(const CUtensorMap (&tm)[4], const GemmParams& p, cudaStream_t stream) {
+  auto kern = gemm_pair_bf16_kernel<BN, A_MN, B_MN>;
   static bool configured = false;
   if (!configured) {
-    CPB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
+    CPB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<BN>::TOTAL));
     configured = true;
   }
-  const int tiles = p.num_m_blocks * p.num_n_blocks;
-  const int grid = tiles < sm_count() ? tiles : sm_count();
-  kern<<<grid, GEMM_THREADS, L::TOTAL, stream>>>(tmA, tmB, p);
-  return check_launch("gemm_bf16");
+  const int items = p.num_m_tiles * p.num_n_blocks * p.splits;
+  const int max_pairs = sm_count() / 2;
+  const int pairs = items < max_pairs ? items : max_pairs;
+  kern<<<2 * pairs, GEMM_THREADS, GemmSmem<BN>::TOTAL, stream>>>(tm[0], tm[1], tm[2], tm[3], p);
+  return check_launch("gemm_pair_bf16");
 }
 
-int gemm_pair_dispatch(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, int a_mn, int b_mn, cudaStream_t stream);
+template <int BN>
+static int dispatch_pair(const CUtensorMap (&tm)[4], const GemmParams& p, int a_mn, int b_mn, cudaStream_t stream) {
+  if (!a_mn && !b_mn) return launch_pair<BN, false, false>(tm, p, stream);
+  if (!a_mn && b_mn) return launch_pair<BN, false, true>(tm, p, stream);
+  if (a_mn && !b_mn) return launch_pair<BN, true, false>(tm, p, stream);
+  return launch_pair<BN, true, true>(tm, p, stream);
+}
+
+// Tile width and K split.  The work items of a launch (tiles x splits) run on 74 pairs, so the time is that of the pair
+// with the most items: items / 74 rounded up, each the longer of its main loop and its epilogue, plus one epilogue at the
+// end.  Nanoseconds, measured: main loop per 64 of K 370 at 256 columns (8192^3: 694 us) and 240 at 128 columns (892 us),
+// so narrow tiles pay only where they fill a wave (M 4096, N 384, K 50304: 238 us at 256 columns, 182 at 128).  Only the
+// accumulating epilogue is split, because its partial sums are added in L2 by the stores themselves: M 384, N 384, K 8192
+// 47 us unsplit, 14 us in 12 splits; but every further split moves the fp32 matrix once more (M 16384, N 2048, K 8192:
+// 372 us unsplit, 443 us in four), charged at 8 TB/s.
+static void plan_tiles(int M, int N, int K, int epi, int has_aux, int& bn, int& splits) {
+  const long nk = (K + GEMM_BK - 1) / GEMM_BK;
+  const long m_tiles = (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM), pairs = sm_count() > 1 ? sm_count() / 2 : 1;
+  const long per_split = (long)M * N * 8 / 8000;
+  long best = -1;
+  for (int cand = 256; cand >= 128; cand -= 128) {
+    const int per_tile = epi == EPI_BF16_SWIGLU ? cand / 2 : cand;
+    const long tiles = m_tiles * ((N + per_tile - 1) / per_tile);
+    const long ck = cand == 256 ? 370 : 240;
+    long ce = epi == EPI_F32 || epi == EPI_F32_ACC ? 1200 : epi == EPI_BF16_GELU ? (has_aux ? 1600 : 1400) : epi == EPI_BF16_SWIGLU ? (has_aux ? 1300 : 1000) : 650;
+    if (cand == 128) ce = ce / 2 + 50;
+    const long max_split = epi == EPI_F32_ACC ? (nk + 3) / 4 : 1;     // at least four K blocks per item
+    for (long s = 1; s <= max_split && (s == 1 || tiles * s <= pairs * 16); ++s) {
+      const long kps = (nk + s - 1) / s;
+      if ((nk + kps - 1) / kps != s) continue;                       // the same items as a smaller split
+      const long waves = (tiles * s + pairs - 1) / pairs, main = kps * ck;
+      const long t = waves * (main > ce ? main : ce) + (main > ce ? ce : main) + (s - 1) * per_split;
+      if (best < 0 || t < best) { best = t; bn = cand; splits = (int)s; }
+    }
+  }
+}
 
 }  // namespace cpb
 
@@ -187,48 +335,58 @@ extern "C" int cpb_gemm_bf16(const void* A, const void* B, void* C, void* aux, c
   if ((!a_mn || !b_mn) && (K % 8)) return set_error(CPB_ERR_ARG, "gemm: K=%d must be a multiple of 8 for a K-major operand", K);
   if (a_mn && (M % 8)) return set_error(CPB_ERR_ARG, "gemm: M must be a multiple of 8 when A is M-major");
   if (epi == EPI_BF16_SWIGLU && (a_mn || b_mn)) return set_error(CPB_ERR_ARG, "gemm: swiglu epilogue needs K-major operands");
-  const int BN = (epi == EPI_BF16_SWIGLU || N > 128) ? 256 : 128;
-  // CTA pairs (gemm2.cu: 256 x 256 tiles, half the shared-memory traffic per tensor-core step) for everything large
-  // enough to fill pairs; CPB_GEMM_PAIR=0 (read once) keeps the one-CTA kernel.
-  static const bool pair_ok = [] { const char* e = getenv("CPB_GEMM_PAIR"); return e == nullptr || e[0] != '0'; }();
-  const bool use_pair = pair_ok && BN == 256 && M >= 256;
+  if (bias != nullptr && ((uintptr_t)bias & 15)) return set_error(CPB_ERR_ARG, "gemm: bias must be 16-byte aligned");
+  if (epi != EPI_BF16_GELU && epi != EPI_BF16_SWIGLU) aux = nullptr;
+  int bn = 256, splits = 1;
+  plan_tiles(M, N, K, epi, aux != nullptr, bn, splits);
   GemmParams p;
-  p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.ld_aux = ld_aux; p.epi = epi;
-  p.num_m_blocks = (M + GEMM_BM - 1) / GEMM_BM;
+  p.M = M; p.N = N; p.K = K; p.epi = epi;
+  p.num_m_tiles = (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM);
   p.num_k_blocks = (K + GEMM_BK - 1) / GEMM_BK;
+  p.k_per_split = (p.num_k_blocks + splits - 1) / splits;
+  p.splits = splits;
   p.swiglu_half = (epi == EPI_BF16_SWIGLU) ? N : 0;
-  // banded tile order of the pair kernel once B (N x K bf16) reaches 64 MB, half of L2; CPB_GEMM_BAND (read once) overrides
+  // banded tile order once B (N x K bf16) reaches 64 MB, half of L2; CPB_GEMM_BAND (read once) overrides
   static const int band_env = [] { const char* e = getenv("CPB_GEMM_BAND"); return e ? atoi(e) : 0; }();
   p.band = band_env > 0 ? band_env : (((size_t)N * K * 2 >= ((size_t)64 << 20)) ? 8 : 1);
-  p.num_n_blocks = (epi == EPI_BF16_SWIGLU) ? (N + BN / 2 - 1) / (BN / 2) : (N + BN - 1) / BN;
-  p.C = C; p.aux = aux; p.bias = bias; p.status = status;
+  const int per_tile = epi == EPI_BF16_SWIGLU ? bn / 2 : bn;
+  p.num_n_blocks = (N + per_tile - 1) / per_tile;
+  p.has_aux = aux != nullptr; p.bias = bias; p.status = status;
 
-  CUtensorMap tmA, tmB;
+  CUtensorMap tm[4];
   int rc;
   {
     uint64_t dims[2], strides[2]; uint32_t box[2];
     if (a_mn) { dims[0] = (uint64_t)M; dims[1] = (uint64_t)K; box[0] = 64; box[1] = GEMM_BK; }
     else      { dims[0] = (uint64_t)K; dims[1] = (uint64_t)M; box[0] = GEMM_BK; box[1] = GEMM_BM; }
     strides[0] = 0; strides[1] = (uint64_t)lda * 2;
-    if ((rc = encode_tmap(&tmA, A, 2, 2, dims, strides, box, 1)) != CPB_OK) return rc;
+    if ((rc = encode_tmap(&tm[0], A, 2, 2, dims, strides, box, 1)) != CPB_OK) return rc;
   }
   {
     uint64_t dims[2], strides[2]; uint32_t box[2];
     const uint64_t b_rows = (epi == EPI_BF16_SWIGLU) ? (uint64_t)2 * N : (uint64_t)N;
     if (b_mn) { dims[0] = b_rows; dims[1] = (uint64_t)K; box[0] = 64; box[1] = GEMM_BK; }
-    else      { dims[0] = (uint64_t)K; dims[1] = b_rows; box[0] = GEMM_BK; box[1] = (epi == EPI_BF16_SWIGLU || use_pair) ? BN / 2 : BN; }
+    else      { dims[0] = (uint64_t)K; dims[1] = b_rows; box[0] = GEMM_BK; box[1] = bn / 2; }
     strides[0] = 0; strides[1] = (uint64_t)ldb * 2;
-    if ((rc = encode_tmap(&tmB, B, 2, 2, dims, strides, box, 1)) != CPB_OK) return rc;
+    if ((rc = encode_tmap(&tm[1], B, 2, 2, dims, strides, box, 1)) != CPB_OK) return rc;
   }
-  if (use_pair) return gemm_pair_dispatch(tmA, tmB, p, a_mn, b_mn, stream);
-#define CPB_GEMM_DISPATCH(BN_, ST_)                                                      \
-  do {                                                                                   \
-    if (!a_mn && !b_mn) return launch_gemm<BN_, ST_, false, false>(tmA, tmB, p, stream);  \
-    if (!a_mn && b_mn) return launch_gemm<BN_, ST_, false, true>(tmA, tmB, p, stream);    \
-    if (a_mn && !b_mn) return launch_gemm<BN_, ST_, true, false>(tmA, tmB, p, stream);    \
-    return launch_gemm<BN_, ST_, true, true>(tmA, tmB, p, stream);                        \
-  } while (0)
-  if (BN == 256) CPB_GEMM_DISPATCH(256, 4);
-  CPB_GEMM_DISPATCH(128, 6);
-#undef CPB_GEMM_DISPATCH
+  {
+    // one store box = 32 rows x 128 bytes; the map's extents clip the edges of C
+    const int eb = (epi == EPI_F32 || epi == EPI_F32_ACC) ? 4 : 2;
+    uint64_t dims[2] = {(uint64_t)N, (uint64_t)M}, strides[2] = {0, (uint64_t)ldc * eb};
+    uint32_t box[2] = {(uint32_t)(128 / eb), 32};
+    if ((rc = encode_tmap(&tm[2], C, eb, 2, dims, strides, box, 1)) != CPB_OK) return rc;
+  }
+  tm[3] = tm[2];
+  if (aux != nullptr && epi == EPI_BF16_SWIGLU) {      // [g | u] as [M][2][F]: a box never crosses from gate into up
+    uint64_t dims[3] = {(uint64_t)N, 2, (uint64_t)M}, strides[3] = {0, (uint64_t)N * 2, (uint64_t)ld_aux * 2};
+    uint32_t box[3] = {64, 1, 32};
+    if ((rc = encode_tmap(&tm[3], aux, 2, 3, dims, strides, box, 1)) != CPB_OK) return rc;
+  } else if (aux != nullptr) {
+    uint64_t dims[2] = {(uint64_t)N, (uint64_t)M}, strides[2] = {0, (uint64_t)ld_aux * 2};
+    uint32_t box[2] = {64, 32};
+    if ((rc = encode_tmap(&tm[3], aux, 2, 2, dims, strides, box, 1)) != CPB_OK) return rc;
+  }
+  if (bn == 256) return dispatch_pair<256>(tm, p, a_mn, b_mn, stream);
+  return dispatch_pair<128>(tm, p, a_mn, b_mn, stream);
 }

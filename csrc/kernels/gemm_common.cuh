@@ -1,11 +1,18 @@
-// Definitions shared by the one-CTA (gemm.cu) and the CTA-pair (gemm2.cu) bf16 GEMM kernels: parameters, epilogue kinds
-// and the epilogue itself (tensor memory -> registers -> global memory, with bias / GELU / SwiGLU / fp32 accumulate).
+// Epilogues of the bf16 GEMM (gemm.cu): parameters, epilogue kinds, and the way a finished accumulator tile leaves the SM.
+//
+// A thread of an epilogue warp owns one row of the tile (its tensor-memory lane).  Storing its columns straight to global
+// memory puts the 32 lanes of every instruction on 32 different rows: 32 partial sectors per instruction, 4096 load/store
+// cycles per 128 x 256 bf16 tile and 8192 for fp32 or for two bf16 outputs, while the main loop of the tile needs only
+// 512 cycles per 64 of K.  So a warp writes 32 rows x 128 bytes into its own 128-byte-swizzled staging buffer in shared
+// memory (conflict-free 16-byte stores) and one lane hands the buffer to TMA, which writes whole lines, clips the edges of
+// the matrix and, for the accumulating epilogue, adds in L2 without the SM reading C first.  Two buffers per warp: one is
+// drained while the other is filled.
 #pragma once
 #include "common.cuh"
 
 namespace cpb {
 
-constexpr int GEMM_BM = 128;
+constexpr int GEMM_BM = 128;           // rows of A per CTA; a CTA pair computes 256 rows
 constexpr int GEMM_BK = 64;
 constexpr int GEMM_THREADS = 192;
 
@@ -19,133 +26,192 @@ enum : int {
 
 struct GemmParams {
   int M, N, K;
-  int ldc;             // elements
-  int ld_aux;
   int epi;
-  int num_m_blocks, num_n_blocks, num_k_blocks;
+  int num_m_tiles, num_n_blocks, num_k_blocks;
+  int splits, k_per_split;   // split-K (accumulating epilogue only): 64-wide K blocks per work item
   int swiglu_half;     // number of output features F when epi == SWIGLU (B has 2F rows)
-  int band;            // CTA-pair kernel: pair-rows per band of the tile order (1 = rows of tiles, columns fastest)
-  void* C;
-  void* aux;
+  int band;            // pair-rows per band of the tile order (1 = rows of tiles, columns fastest)
+  int has_aux;
   const float* bias;
   int* status;
 };
 
-template <int BN, int STAGES>
-struct GemmSmem {
-  static constexpr int A_BYTES = GEMM_BM * GEMM_BK * 2;
-  static constexpr int B_BYTES = BN * GEMM_BK * 2;
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
-  static constexpr int TOTAL = BAR_OFFSET + 256 + 1024;   // barriers + alignment slack
+// x * sigmoid(2u) with u the argument of the tanh form: the same function as 0.5 x (1 + tanh(u)).  Two values share one
+// reciprocal (1/a = b/(ab)): the special-function unit limits this epilogue, and three operations for two values replace
+// four.  The exponent is clamped so that a product of two denominators stays finite; beyond the clamp the result is
+// below 2^-57 of x, under the smallest change of a bf16 sum.
+__device__ __forceinline__ void gelu_tanh_pair(float& x0, float& x1) {
+  const float k0 = 0.7978845608028654f * -2.f * 1.4426950408889634f, k1 = 0.044715f;
+  const float e0 = ex2f(fminf(k0 * (x0 + k1 * x0 * x0 * x0), 57.f)) + 1.f;
+  const float e1 = ex2f(fminf(k0 * (x1 + k1 * x1 * x1 * x1), 57.f)) + 1.f;
+  const float r = __fdividef(1.f, e0 * e1);
+  x0 = x0 * r * e1;
+  x1 = x1 * r * e0;
+}
+// silu(g) * u for two features, one reciprocal for both (as above).
+__device__ __forceinline__ void silu_mul_pair(float g0, float g1, float u0, float u1, float& o0, float& o1) {
+  const float k = -1.4426950408889634f;
+  const float e0 = ex2f(fminf(g0 * k, 57.f)) + 1.f, e1 = ex2f(fminf(g1 * k, 57.f)) + 1.f;
+  const float r = __fdividef(1.f, e0 * e1);
+  o0 = g0 * u0 * (r * e1);
+  o1 = g1 * u1 * (r * e0);
+}
+
+// One warp's way out: two staging buffers of 32 rows x 128 bytes, used in turn.
+struct WarpStore {
+  uint8_t* buf;        // 2 x 4096 bytes, 1024-byte aligned
+  uint32_t use;        // stores issued so far
+  bool issuer;         // lane 0: issues and waits
+
+  // Claim the next buffer: it is free once at most the newest bulk group is still being read.
+  __device__ __forceinline__ uint8_t* row_ptr(int lane) {
+    if (issuer) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+    __syncwarp();
+    return buf + (use & 1) * 4096 + lane * 128;
+  }
+  // v: this lane's 128 bytes, sixteen bytes to chunk position (chunk ^ row % 8)
+  __device__ __forceinline__ void fill(uint8_t* row, int lane, const uint32_t (&v)[32]) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      *(uint4*)(row + ((c ^ (lane & 7)) << 4)) = make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+    fence_proxy_async_smem();
+    __syncwarp();
+  }
+  __device__ __forceinline__ void store(const CUtensorMap* m, int x, int y) {
+    if (issuer) {
+      asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"
+                   ::"l"((uint64_t)m), "r"(smem_u32(buf + (use & 1) * 4096)), "r"(x), "r"(y) : "memory");
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+    ++use;
+  }
+  __device__ __forceinline__ void store3(const CUtensorMap* m, int x, int y, int z) {
+    if (issuer) {
+      asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
+                   ::"l"((uint64_t)m), "r"(smem_u32(buf + (use & 1) * 4096)), "r"(x), "r"(y), "r"(z) : "memory");
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+    ++use;
+  }
+  __device__ __forceinline__ void add(const CUtensorMap* m, int x, int y) {
+    if (issuer) {
+      asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
+                   ::"l"((uint64_t)m), "r"(smem_u32(buf + (use & 1) * 4096)), "r"(x), "r"(y) : "memory");
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+    ++use;
+  }
+  __device__ __forceinline__ void drain() {
+    if (issuer) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  }
 };
 
-__device__ __forceinline__ float gelu_tanh_f(float x) {
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  float u = k0 * (x + k1 * x * x * x);
-  // tanh(u) = 1 - 2/(exp(2u)+1)
-  float e = __expf(2.f * u);
-  float t = 1.f - 2.f / (e + 1.f);
-  return 0.5f * x * (1.f + t);
+__device__ __forceinline__ void pack_row(const float (&f)[64], uint32_t (&v)[32]) {
+#pragma unroll
+  for (int j = 0; j < 32; ++j) v[j] = pack_bf16(f[2 * j], f[2 * j + 1]);
 }
-__device__ __forceinline__ float silu_f(float x) { return x / (1.f + __expf(-x)); }
 
-// Epilogue of one 128 x BN accumulator tile for one thread: `row` is the thread's output row (tensor-memory lane),
-// `t_row` the tensor-memory address of that lane's first accumulator column, `nb` the tile's index along N.
-template <int BN>
-__device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t t_row, int row, int nb) {
-  const int n0 = nb * BN;
-      if (p.epi == EPI_BF16_SWIGLU) {
-  // accumulator columns [0, BN/2) = gate, [BN/2, BN) = up, for features f0..f0+BN/2
-  const int f0 = nb * (BN / 2);
+// Epilogue of one 32-row slice of a 128 x BN accumulator tile: `t_row` is the tensor-memory address of this warp's lanes at
+// the accumulator's first column, `row0` the slice's first output row, `nb` the tile's index along N.  `release` runs as
+// soon as the accumulator has been read.
+template <int BN, class Release>
+__device__ __forceinline__ void gemm_epilogue(const GemmParams& p, const CUtensorMap* tmC, const CUtensorMap* tmX, WarpStore& ws,
+                                              uint32_t t_row, int row0, int nb, int lane, Release release) {
+  const bool live = row0 < p.M;
+  if (p.epi == EPI_BF16_SWIGLU) {
+    // accumulator columns [0, BN/2) = gate, [BN/2, BN) = up, for features f0 .. f0 + BN/2
 #pragma unroll 1
-  for (int c = 0; c < BN / 2; c += 32) {
-    uint32_t g[32], u[32];
-    tmem_ld32(t_row + c, g);
-    tmem_ld32(t_row + BN / 2 + c, u);
-    tmem_wait_ld();
-    if (row < p.M) {
-      __nv_bfloat16* crow = (__nv_bfloat16*)p.C + (size_t)row * p.ldc + f0 + c;
-      __nv_bfloat16* arow = p.aux ? (__nv_bfloat16*)p.aux + (size_t)row * p.ld_aux : nullptr;
-#pragma unroll
-      for (int j = 0; j < 32; j += 8) {
-        if (f0 + c + j < p.swiglu_half) {
-          uint32_t o[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            float g0 = __uint_as_float(g[j + 2 * q]), g1 = __uint_as_float(g[j + 2 * q + 1]);
-            float u0 = __uint_as_float(u[j + 2 * q]), u1 = __uint_as_float(u[j + 2 * q + 1]);
-            o[q] = pack_bf16(silu_f(g0) * u0, silu_f(g1) * u1);
-          }
-          *(uint4*)(crow + j) = make_uint4(o[0], o[1], o[2], o[3]);
-          if (arow) {
-            uint32_t pg[4], pu[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              pg[q] = pack_bf16(__uint_as_float(g[j + 2 * q]), __uint_as_float(g[j + 2 * q + 1]));
-              pu[q] = pack_bf16(__uint_as_float(u[j + 2 * q]), __uint_as_float(u[j + 2 * q + 1]));
-            }
-            *(uint4*)(arow + f0 + c + j) = make_uint4(pg[0], pg[1], pg[2], pg[3]);
-            *(uint4*)(arow + p.swiglu_half + f0 + c + j) = make_uint4(pu[0], pu[1], pu[2], pu[3]);
-          }
-        }
+    for (int c = 0; c < BN / 2; c += 64) {
+      const int f = nb * (BN / 2) + c;
+      float g[64], u[64];
+      tmem_ld32(t_row + c, *(uint32_t(*)[32])&g[0]);
+      tmem_ld32(t_row + c + 32, *(uint32_t(*)[32])&g[32]);
+      tmem_ld32(t_row + BN / 2 + c, *(uint32_t(*)[32])&u[0]);
+      tmem_ld32(t_row + BN / 2 + c + 32, *(uint32_t(*)[32])&u[32]);
+      tmem_wait_ld();
+      if (c + 64 == BN / 2) release();
+      if (!live || f >= p.swiglu_half) continue;
+      uint32_t v[32];
+      if (p.has_aux) {
+        pack_row(g, v);
+        ws.fill(ws.row_ptr(lane), lane, v);
+        ws.store3(tmX, f, 0, row0);
+        pack_row(u, v);
+        ws.fill(ws.row_ptr(lane), lane, v);
+        ws.store3(tmX, f, 1, row0);
       }
+#pragma unroll
+      for (int j = 0; j < 64; j += 2) {
+        float o0, o1;
+        silu_mul_pair(g[j], g[j + 1], u[j], u[j + 1], o0, o1);
+        v[j >> 1] = pack_bf16(o0, o1);
+      }
+      ws.fill(ws.row_ptr(lane), lane, v);
+      ws.store(tmC, f, row0);
     }
-  }
-} else {
+  } else if (p.epi == EPI_F32 || p.epi == EPI_F32_ACC) {
 #pragma unroll 1
-  for (int c = 0; c < BN; c += 32) {
-    uint32_t v[32];
-    tmem_ld32(t_row + c, v);
-    tmem_wait_ld();
-    const int col = n0 + c;
-    if (row < p.M && col < p.N) {
+    for (int c = 0; c < BN; c += 32) {
+      const int col = nb * BN + c;
+      uint32_t v[32];
+      tmem_ld32(t_row + c, v);
+      tmem_wait_ld();
+      if (c + 32 == BN) release();
+      if (!live || col >= p.N) continue;
       if (p.bias != nullptr) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (col + j < p.N) v[j] = __float_as_uint(__uint_as_float(v[j]) + __ldg(p.bias + col + j));
-      }
-      if (p.epi == EPI_BF16 || p.epi == EPI_BF16_GELU) {
-        __nv_bfloat16* crow = (__nv_bfloat16*)p.C + (size_t)row * p.ldc + col;
-        __nv_bfloat16* arow = (p.epi == EPI_BF16_GELU && p.aux) ? (__nv_bfloat16*)p.aux + (size_t)row * p.ld_aux + col : nullptr;
+        for (int j = 0; j < 32; j += 8)
+          if (col + j < p.N) {                 // N is a multiple of 8
 #pragma unroll
-        for (int j = 0; j < 32; j += 8) {
-          if (col + j < p.N) {       // N is a multiple of 8
-            uint32_t o[4];
-            if (p.epi == EPI_BF16_GELU) {
-              if (arow) {
-                uint32_t a[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) a[q] = pack_bf16(__uint_as_float(v[j + 2 * q]), __uint_as_float(v[j + 2 * q + 1]));
-                *(uint4*)(arow + j) = make_uint4(a[0], a[1], a[2], a[3]);
-              }
-#pragma unroll
-              for (int q = 0; q < 4; ++q)
-                o[q] = pack_bf16(gelu_tanh_f(__uint_as_float(v[j + 2 * q])), gelu_tanh_f(__uint_as_float(v[j + 2 * q + 1])));
-            } else {
-#pragma unroll
-              for (int q = 0; q < 4; ++q) o[q] = pack_bf16(__uint_as_float(v[j + 2 * q]), __uint_as_float(v[j + 2 * q + 1]));
+            for (int q = 0; q < 8; q += 4) {
+              const float4 b = __ldg((const float4*)(p.bias + col + j + q));
+              v[j + q] = __float_as_uint(__uint_as_float(v[j + q]) + b.x);
+              v[j + q + 1] = __float_as_uint(__uint_as_float(v[j + q + 1]) + b.y);
+              v[j + q + 2] = __float_as_uint(__uint_as_float(v[j + q + 2]) + b.z);
+              v[j + q + 3] = __float_as_uint(__uint_as_float(v[j + q + 3]) + b.w);
             }
-            *(uint4*)(crow + j) = make_uint4(o[0], o[1], o[2], o[3]);
           }
-        }
-      } else {
-        float* crow = (float*)p.C + (size_t)row * p.ldc + col;
-#pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-          if (col + j < p.N) {       // N is a multiple of 4 on this path
-            float4 o = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
-            if (p.epi == EPI_F32_ACC) {
-              float4 old = *(float4*)(crow + j);
-              o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-            }
-            *(float4*)(crow + j) = o;
-          }
-        }
       }
+      ws.fill(ws.row_ptr(lane), lane, v);
+      if (p.epi == EPI_F32_ACC) ws.add(tmC, col, row0);
+      else ws.store(tmC, col, row0);
+    }
+  } else {
+#pragma unroll 1
+    for (int c = 0; c < BN; c += 64) {
+      const int col = nb * BN + c;
+      float f[64];
+      tmem_ld32(t_row + c, *(uint32_t(*)[32])&f[0]);
+      tmem_ld32(t_row + c + 32, *(uint32_t(*)[32])&f[32]);
+      tmem_wait_ld();
+      if (c + 64 == BN) release();
+      if (!live || col >= p.N) continue;
+      if (p.bias != nullptr) {
+#pragma unroll
+        for (int j = 0; j < 64; j += 8)
+          if (col + j < p.N) {
+#pragma unroll
+            for (int q = 0; q < 8; q += 4) {
+              const float4 b = __ldg((const float4*)(p.bias + col + j + q));
+              f[j + q] += b.x; f[j + q + 1] += b.y; f[j + q + 2] += b.z; f[j + q + 3] += b.w;
+            }
+          }
+      }
+      uint32_t v[32];
+      if (p.epi == EPI_BF16_GELU) {
+        if (p.has_aux) {
+          pack_row(f, v);
+          ws.fill(ws.row_ptr(lane), lane, v);
+          ws.store(tmX, col, row0);
+        }
+#pragma unroll
+        for (int j = 0; j < 64; j += 2) gelu_tanh_pair(f[j], f[j + 1]);
+      }
+      pack_row(f, v);
+      ws.fill(ws.row_ptr(lane), lane, v);
+      ws.store(tmC, col, row0);
     }
   }
-}
 }
 
 }  // namespace cpb

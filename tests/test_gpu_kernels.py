@@ -77,6 +77,43 @@ def test_gemm_epilogues():
     check_status()
 
 
+# Edges of the tiles (256 x 128 / 256 rows, 64 of K), row counts below one CTA of a pair, and shapes whose weight gradient is
+# split along K.  bf16 outputs: one rounding (2^-9) on top of fp32 sums.  fp32: two summation orders of K products of
+# unit normals differ by about sqrt(K) * 2^-24 * sqrt(K), relative to the result's sqrt(K): 5e-6 at K = 8192.
+@pytest.mark.parametrize("M,N,K", [(8, 264, 64), (136, 768, 776), (129, 8, 72), (257, 120, 64), (384, 384, 8192), (640, 392, 4104), (520, 1288, 136)])
+def test_gemm_tile_edges_every_epilogue(M, N, K):
+    from context_parallelism_b200.ops import gemm as G
+    torch.manual_seed(17)
+    A = torch.randn(M, K, device=dev()).bfloat16()
+    B = torch.randn(N, K, device=dev()).bfloat16()
+    bias = torch.randn(N, device=dev())
+    ref = (A.double() @ B.double().t()).float()
+    rms = K ** 0.5
+    got = G.gemm(A, B, bias=bias)
+    assert_close(got.float(), ref + bias, cos=0.99999, rel=2 ** -8, name="bf16 + bias")
+    assert float((G.gemm(A, B, out_dtype=torch.float32, bias=bias) - ref - bias).abs().max()) < 1e-4 * rms
+    pre = torch.empty(M, N, device=dev(), dtype=torch.bfloat16)
+    act = G.gemm(A, B, bias=bias, epi=G.EPI_BF16_GELU, aux=pre)
+    assert_close(pre.float(), ref + bias, cos=0.99999, rel=2 ** -8, name="gelu pre")
+    want = torch.nn.functional.gelu((ref + bias).double(), approximate="tanh").float()
+    assert_close(act.float(), want, cos=0.99999, rel=2 ** -8, name="gelu")
+    assert torch.equal(G.gemm(A, B, bias=bias, epi=G.EPI_BF16_GELU), act)          # without the pre-activation
+    if N % 16 == 0:
+        F = N // 2
+        gu = torch.empty(M, N, device=dev(), dtype=torch.bfloat16)
+        sw = G.gemm(A, B, epi=G.EPI_BF16_SWIGLU, aux=gu)
+        assert_close(gu.float(), ref, cos=0.99999, rel=2 ** -8, name="swiglu pre")
+        want = torch.nn.functional.silu(ref[:, :F].double()).float() * ref[:, F:]
+        assert_close(sw.float(), want, cos=0.99999, rel=2 ** -8, name="swiglu")
+        assert torch.equal(G.gemm(A, B, epi=G.EPI_BF16_SWIGLU), sw)
+    if M % 8 == 0:
+        acc = torch.randn(M, N, device=dev())
+        want = acc + ref
+        G.gemm(A.t().contiguous(), B.t().contiguous(), a_mn=True, b_mn=True, out=acc, accumulate=True)
+        assert float((acc - want).abs().max()) < 1e-4 * rms
+    check_status()
+
+
 def test_linear_autograd():
     from context_parallelism_b200.ops.gemm import linear, linear_swiglu, linear_gelu
     torch.manual_seed(2)
