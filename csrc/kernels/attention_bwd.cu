@@ -1,4 +1,5 @@
-// Flash-attention backward for sm_100a.  One CTA owns one 128-row K/V tile of one KV head and sweeps
+// Flash-attention backward for sm_100a with query rows in tensor-memory lanes, head_dim 64: the second implementation that
+// attention_bwd64.cu is checked against (CPB_BWD_GENERAL=1); head_dim 128 runs on attention_bwd128.cu.  One CTA owns one 128-row K/V tile of one KV head and sweeps
 // every query tile (of every query head of the GQA group) that can see it, with all five products
 // on tcgen05 tensor cores and every accumulator in tensor memory:
 //
@@ -60,17 +61,17 @@ struct BwdParams {
 
 template <int D>
 struct BwdSmem {
-  static constexpr int STAGES = (D == 64) ? 2 : 1;
+  static constexpr int STAGES = 2;
   static constexpr int TILE = FB_T * D * 2;
   static constexpr int K_OFF = 0;
   static constexpr int V_OFF = TILE;
   static constexpr int Q_OFF = 2 * TILE;
   static constexpr int DO_OFF = Q_OFF + STAGES * TILE;
   static constexpr int PS_OFF = DO_OFF + STAGES * TILE;           // P : 128 queries x 128 keys bf16, 128B-swizzled
-  static constexpr int DS_BUFS = (D == 64) ? 2 : 1;               // head_dim 64: dS double-buffered (pipelined issue order)
+  static constexpr int DS_BUFS = 2;                               // dS double-buffered (pipelined issue order)
   static constexpr int DS_OFF = PS_OFF + FB_T * FB_T * 2;         // dS: same layout
   static constexpr int DQS_OFF = DS_OFF + DS_BUFS * FB_T * FB_T * 2;   // dQ staging: boxes of 128 rows x 32 fp32, 128B-swizzled
-  static constexpr int DQ_BOXES = (D == 64) ? 1 : 2;              // boxes staged per TMA-reduce round
+  static constexpr int DQ_BOXES = 1;              // boxes staged per TMA-reduce round
   static constexpr int VEC_OFF = DQS_OFF + DQ_BOXES * FB_T * 128;        // per stage: lse2[128], delta[128], qpos[128]
   static constexpr int BAR_OFF = VEC_OFF + STAGES * 3 * 512;
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
@@ -93,9 +94,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   constexpr int ST = L::STAGES;
   constexpr int DH = D / 64;
   constexpr uint32_t S_COL = 0, DP_COL = 128, DV_COL = 256, DK_COL = 256 + D;
-  constexpr uint32_t DQ_COL = (D == 64) ? 384 : 0;           // D=128: dQ reuses the S columns
-  constexpr bool DQ_ALIAS = (D != 64);
-  constexpr bool OVERLAP = (D == 64);                         // pipelined issue order (see the MMA issuer)
+  constexpr uint32_t DQ_COL = 384;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = (uint64_t*)(smem + L::BAR_OFF);
@@ -235,8 +234,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         }
       };
       bool ok = __all_sync(0xffffffffu, mbar_wait(kv_full, 0, abort_flag, p.status, 900));
-      if (ok && OVERLAP) {
-        // Pipelined order (head_dim 64).  When the softmax-gradient warps finish tile i the issuer queues
+      if (ok) {
+        // Pipelined order.  When the softmax-gradient warps finish tile i the issuer queues
         //   dV(i) | S(i+1), dP(i+1) | dK(i), dQ(i)
         // so the warps start on tile i+1 as soon as its score products are done while dK(i) and dQ(i), which
         // read the double-buffered dS tile, still run on the tensor cores.  P is single-buffered: dV(i) is
@@ -263,22 +262,6 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           issue_dq(i & 1);
           umma_commit_p(leader, &q_empty[st]);
           umma_commit_p(leader, &ds_empty[i & 1]);
-          umma_commit_p(leader, dq_full);
-        }
-      } else if (ok) {
-        for (int i = 0; i < n_it; ++i) {
-          const int st = i % ST;
-          if (!__all_sync(0xffffffffu, mbar_wait(&q_full[st], (i / ST) & 1, abort_flag, p.status, 901))) break;
-          if (DQ_ALIAS && i > 0 && !__all_sync(0xffffffffu, mbar_wait(dq_empty, (i - 1) & 1, abort_flag, p.status, 902))) break;
-          tc_fence_after();
-          issue_scores(st);
-          if (!__all_sync(0xffffffffu, mbar_wait(p_full, i & 1, abort_flag, p.status, 903))) break;
-          if (!DQ_ALIAS && i > 0 && !__all_sync(0xffffffffu, mbar_wait(dq_empty, (i - 1) & 1, abort_flag, p.status, 904))) break;
-          tc_fence_after();
-          issue_dv(st, i);
-          issue_dk(st, 0, i);
-          issue_dq(0);
-          umma_commit_p(leader, &q_empty[st]);
           umma_commit_p(leader, dq_full);
         }
       }
@@ -311,8 +294,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const bool need_mask = (k0 + FB_T > p.Tk) || (p.causal && (p.k_off + k0 + FB_T - 1 > qpos_min));
       const int kmax = min(p.causal ? qpos_r - p.k_off : 0x7fffffff, p.Tk - 1) - kcol0;   // last visible column of my span
       // 4 chunks of 16 columns; the tensor-memory loads of chunk ch+1 are in flight while chunk ch is processed.
-      uint8_t* ds_row = ds_row0 + (OVERLAP ? (i & 1) * (FB_T * FB_T * 2) : 0);
-      if (OVERLAP) {
+      uint8_t* ds_row = ds_row0 + (i & 1) * (FB_T * FB_T * 2);
+      {
         // this parity's dS buffer was last read by dK/dQ of tile i-2
         bool ok2 = mbar_wait(&ds_empty[i & 1], ((i >> 1) & 1) ^ 1, abort_flag, p.status, 1003);
         ok2 = __all_sync(0xffffffffu, ok2);
@@ -543,7 +526,7 @@ extern "C" int cpb_flash_bwd(const void* q, const void* k, const void* v, const 
                              float scale, int causal, int k_off, const int* q_pos, int dkv_f32_accumulate,
                              const uint64_t* route_k, const uint64_t* route_v, int route_rows, int route_tl,
                              int* status, cudaStream_t stream) {
-  if (D != 64 && D != 128) return set_error(CPB_ERR_ARG, "flash_bwd: head_dim %d not in {64,128}", D);
+  if (D != 64) return set_error(CPB_ERR_ARG, "flash_bwd: head_dim %d is not 64", D);
   if (Hq % Hkv) return set_error(CPB_ERR_ARG, "flash_bwd: Hq %% Hkv != 0");
   if (Tq_pad % FB_T || Tq_pad < Tq) return set_error(CPB_ERR_ARG, "flash_bwd: bad Tq_pad");
   if (q_pos == nullptr) return set_error(CPB_ERR_ARG, "flash_bwd: q_pos is required");
@@ -577,14 +560,8 @@ extern "C" int cpb_flash_bwd(const void* q, const void* k, const void* v, const 
   if (dkv_f32_accumulate == 2 && (route_k == nullptr || route_v == nullptr || route_rows <= 0))
     return set_error(CPB_ERR_ARG, "flash_bwd: routed dK/dV needs route tables");
   dim3 grid((Tk + FB_T - 1) / FB_T, Hkv, B);
-  if (D == 64) {
-    static bool cfg = false;
-    if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_bwd_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<64>::TOTAL)); cfg = true; }
-    flash_bwd_kernel<64><<<grid, FB_THREADS, BwdSmem<64>::TOTAL, stream>>>(tq, tk, tv, tdo, tdq, p);
-  } else {
-    static bool cfg = false;
-    if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_bwd_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<128>::TOTAL)); cfg = true; }
-    flash_bwd_kernel<128><<<grid, FB_THREADS, BwdSmem<128>::TOTAL, stream>>>(tq, tk, tv, tdo, tdq, p);
-  }
+  static bool cfg = false;
+  if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_bwd_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<64>::TOTAL)); cfg = true; }
+  flash_bwd_kernel<64><<<grid, FB_THREADS, BwdSmem<64>::TOTAL, stream>>>(tq, tk, tv, tdo, tdq, p);
   return check_launch("flash_bwd");
 }

@@ -128,6 +128,20 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return mbar_wait_slow(bar, parity, abort_flag, status, site);
 }
 
+// The same wait without a call and without the report: for kernels that move registers between warpgroups (setmaxnreg does
+// not go together with calls).  A few instructions in line; an expired wait leaves its site in `abort_site`, which the
+// kernel reports once all its roles are done.
+__device__ __forceinline__ bool mbar_wait_lean(uint64_t* bar, uint32_t parity, volatile int* abort_site, int site) {
+  if (mbar_try_wait(bar, parity)) return true;
+#pragma unroll 1
+  for (uint32_t it = 0; it < CPB_WAIT_SPINS; ++it) {
+    if (mbar_try_wait_hint(bar, parity, CPB_WAIT_HINT_NS)) return true;
+    if (*abort_site) return false;
+  }
+  *abort_site = site;
+  return false;
+}
+
 // Wait executed by a whole warp that must stay convergent: one lane polls, the result is broadcast.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                                int* status, int site) {

@@ -255,6 +255,37 @@ def test_flash_bwd(D, B, Tq, Tk, Hq, Hkv, causal):
     assert_close(dq.float(), wdq, cos=0.998, rel=5e-2, name="dq")
 
 
+# head_dim 128: one query tile, ragged ends on both sides, several tiles of several grouped heads (both stages of every ring
+# in use), the zig-zag shard of a ring rank, a key block at an offset, rows that see no key.  Same bars as test_flash_bwd.
+@pytest.mark.parametrize("B,Tq,Tk,Hq,Hkv,ring,k_off,accumulate", [
+    (1, 1, 1, 1, 1, 1, 0, False), (2, 129, 127, 2, 1, 1, 0, True), (1, 640, 896, 4, 2, 1, 0, False), (1, 256, 1024, 6, 2, 4, 0, True),
+    (2, 384, 200, 2, 2, 1, 100, False), (1, 130, 300, 3, 1, 1, 64, True)])
+def test_flash_bwd_d128_shapes_and_modes(B, Tq, Tk, Hq, Hkv, ring, k_off, accumulate):
+    from context_parallelism_b200.ops import attention as A, reference as R
+    from context_parallelism_b200.parallel.shard import local_positions
+    torch.manual_seed(21)
+    D = 128
+    q = torch.randn(B, Tq, Hq, D, device=dev()).bfloat16()
+    k, v = (torch.randn(B, Tk, Hkv, D, device=dev()).bfloat16() for _ in range(2))
+    do = torch.randn(B, Tq, Hq, D, device=dev()).bfloat16()
+    pos = local_positions(Tq * ring, ring, 1, True).to(dev()) if ring > 1 else torch.arange(Tq, device=dev())
+    kpos = torch.arange(k_off, k_off + Tk, device=dev())
+    scale = D ** -0.5
+    out, lse = A.flash_fwd(q, k, v, scale, True, pos.int(), k_off)
+    extra = {}
+    if accumulate:
+        extra = dict(dk=torch.ones(B, Tk, Hkv, D, device=dev()), dv=torch.ones(B, Tk, Hkv, D, device=dev()), dkv_accumulate=True)
+    dq, dk, dv = A.flash_bwd(q, k, v, out, lse, do, scale, True, pos.int(), k_off, **extra)
+    check_status()
+    want, wlse = R.attention_dense(q.float(), k.float(), v.float(), scale, q_pos=pos, k_pos=kpos, causal=True)
+    wdq, wdk, wdv = R.attention_dense_bwd(q.float(), k.float(), v.float(), want, wlse, do.float(), scale, q_pos=pos, k_pos=kpos, causal=True)
+    off = 1.0 if accumulate else 0.0
+    for got, ref, name in ((dv.float() - off, wdv, "dv"), (dk.float() - off, wdk, "dk"), (dq.float(), wdq, "dq")):
+        assert torch.isfinite(got).all()
+        if float(ref.abs().max()) > 1e-4:
+            assert_close(got, ref, cos=0.998, rel=5e-2, name=name)
+
+
 @pytest.mark.parametrize("B,Tq,Tk,Hq,Hkv,causal", [(1, 512, 512, 4, 1, True), (2, 300, 712, 2, 2, False), (1, 2048, 2048, 8, 2, True)])
 def test_flash_bwd_d64_kernels_agree(B, Tq, Tk, Hq, Hkv, causal, monkeypatch):
     """The head_dim-64 kernel (transposed, vectors folded into the MMAs) against the general kernel on the same inputs,
