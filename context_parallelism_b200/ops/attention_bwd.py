@@ -67,13 +67,7 @@ def flash_bwd_core(q, k, v, do, lse2, delta, qpos_pad, scale, causal, k_off, dq_
     qs, ks = _strides(q), _strides(k)
     assert v.stride() == k.stride()
     if D == 64 and not _USE_GENERAL_D64:
-        # head_dim 64 kernel (csrc/kernels/attention_bwd64.cu): the per-row vectors enter the tensor-core products as
-        # three-term bf16 splits, produced here from the fp32 vectors (a few tens of microseconds)
-        n = lse2.numel()
-        aug = torch.empty((2, n, 8), dtype=torch.bfloat16, device=q.device)
-        nv.call("flash_bwd64_aug", nv.ptr(lse2), nv.ptr(delta), nv.ptr(aug[0]), nv.ptr(aug[1]), nv.l(n), nv.f(scale),
-                nv.stream_ptr(q.device))
-        nv.call("flash_bwd64", nv.ptr(q), nv.ptr(k), nv.ptr(v), nv.ptr(do), nv.ptr(aug[0]), nv.ptr(aug[1]), nv.ptr(dq_f32),
+        nv.call("flash_bwd64", nv.ptr(q), nv.ptr(k), nv.ptr(v), nv.ptr(do), nv.ptr(lse2), nv.ptr(delta), nv.ptr(dq_f32),
                 nv.ptr(dk), nv.ptr(dv), nv.i(B), nv.i(Tq), nv.i(Tk), nv.i(Hq), nv.i(Hkv), nv.i(lse2.shape[-1]),
                 nv.l(qs[0]), nv.l(qs[1]), nv.l(qs[2]), nv.l(ks[0]), nv.l(ks[1]), nv.l(ks[2]),
                 nv.f(scale), nv.i(causal), nv.i(k_off), nv.ptr(qpos_pad), nv.i(2 if route is not None else int(dkv_accumulate)),

@@ -90,8 +90,6 @@ __device__ __forceinline__ int ld_ahead_s32(const int* ptr) {
   asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(ptr));
   return v;
 }
-template <int R> __device__ __forceinline__ void regs_give() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
-template <int R> __device__ __forceinline__ void regs_take() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
 __device__ __forceinline__ void red_add_v4_128(float* addr, float a, float b, float c, float d) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }

@@ -1,110 +1,93 @@
-// Flash-attention backward specialised for head_dim 64 (the flagship 1B shape and GPT-2).
+// Flash-attention backward specialised for head_dim 64.
 //
-// At head_dim 64 the general kernel (attention_bwd.cu) is bound by shared-memory bandwidth: three of its
-// five products read a 128x128 bf16 A tile from shared memory for only 64 output columns.  This kernel
-// keeps the K/V rows in tensor-memory lanes instead (S^T = K Q^T, dP^T = V dO^T), so P^T and dS^T are
-// tensor-memory A operands of the dV / dK products, and removes every per-column vector from the inner loop
-// by folding them into the tensor-core products:
+// One CTA owns one 128-row K/V tile of one KV head and sweeps the query tiles (of every query head of the GQA group) that
+// see it, with the K/V rows in tensor-memory lanes.  A 128 x 128 tile is worked on as two halves of 64 queries, each by
+// eight warps of its own and with barriers of its own:
 //
-//     S'^T  = K Q^T   - 1 (x) L^T        L[q]     = LSE[q] / scale   (three bf16 terms: hi + mid + lo)
-//     dP'^T = V dO^T  - 1 (x) Delta^T    Delta[q] = rowsum(dO o O)   (three bf16 terms)
+//     S^T  = K Q^T            (tmem x smem)      P^T  = exp2(S^T c - LSE)        (registers -> tensor memory, bf16)
+//     dP^T = V dO^T           (tmem x smem)      dS^T = P^T o (dP^T - Delta)     (registers -> tensor memory and smem, bf16)
+//     dV  += P^T dO           (tmem x smem)      dK  += dS^T Q                   (tmem x smem)
+//     dQ   = dS K             (smem x smem, dS^T read M-major, both halves at once) -> staging -> TMA reduce-add (fp32)
 //
-// as one extra K=16 UMMA each, whose A operand is a constant tile of ones and whose B operand is a
-// [128 queries x 8] bf16 tile produced by `bwd64_aug_kernel` and loaded with one bulk copy.  Then
-//     P^T = exp2(S'^T * scale*log2e)        dS^T = P^T o dP'^T            (no loads, no subtraction)
-//     dV += P^T dO  (A in tensor memory)    dK += dS^T Q  (A in tensor memory)
-//     dQ  = dS K    (A = dS^T staged M-major in shared memory) -> TMA reduce-add into the fp32 dQ buffer.
+// What bounds it: the exponentials (16 per clock: 1024 cycles for 16384) if they never pause, then shared memory.  With all
+// sixteen warps on one tile the exponential unit idles while they form dS and wait for each other (3150 cycles per tile);
+// here one half can take its exponentials while the other forms dS.  N = 64 score products would read
+// 192 bytes of operands per tensor-core cycle from shared memory, so K and V are copied into tensor memory once and only Q
+// and dO are streamed.  Shared memory then moves about 270 KB per tile (64 KB for four products, 48 KB for dQ, 32 KB of dS^T,
+// 64 KB of dQ staging, 33 KB of TMA fills and the LSE / Delta vectors): 2100 cycles at 128 bytes per cycle.
 //
-// Issue order of the MMA warp (tile i = one 128x128 query/key tile pair):
-//     S'(i+1) as soon as the warps have read S'(i);   then after the warps finish tile i:
-//     dK(i), dP'(i+1), dV(i), dQ(i)
-// so the exponentials of tile i+1 overlap the gradient products of tile i, and dP'(i+1) is ready long before the
-// warps want it.  The warps keep P^T and dS^T in registers until dQ(i-1) has finished and store them at the end of
-// the tile: two barrier waits in the middle of a tile, one at its end.  Tensor memory (512 columns):
-// S'^T 128 | dP'^T 128 (dS^T bf16 written back into it) | dV 64 | dK 64 | dQ 64 | P^T 64.
+// Tensor memory (512 columns): S^T / P^T 128 | dP^T / dS^T 128 | dV 64 | dK 64 | dQ 64 | K 32 | V 32.  P^T overwrites the
+// part of S^T its thread has read and dS^T that of dP^T.  Issue order of the MMA warp for tile i (halves A and B):
+//     dK_B(i-1), dP_B(i), dQ(i-1)    when dS_B(i-1) is stored        dV_A(i), S_A(i+1)     when P_A(i) is stored
+//     dK_A(i), dP_A(i+1)             when dS_A(i) is stored          dV_B(i), S_B(i+1)     when P_B(i) is stored
+// so every product a half needs next is issued a whole phase before it is wanted.  dS^T has two buffers in shared memory:
+// the commit behind dP of either half for tile i covers dQ(i-2), so no barrier of its own guards them.
 //
-// Same interface, masking rules, dK/dV output modes and bounded waits as the general kernel.
+// Measured against the kernel this one replaces (all sixteen warps on one tile, K and V read from shared memory, LSE and Delta
+// as extra K = 16 products; same GPU, cold L2, us): T 32768, 32/8 heads 12886 -> 12244 (898 TFLOP/s); T 16384 2997 -> 2948;
+// 2 x 4096, 6/2 heads 194 -> 181; 2 x 1000, 6/2 heads 64.5 -> 56.3 (the vectors' own launch is gone); 4 x 1024, 6/6 50.2 -> 48.2.
+//
+// Masking is on global positions, dK/dV output modes and bounded waits are those of the head_dim-128 kernel.  Replaces
+// mem_efficient_bwd_unified_kernel_exp11 (context_parallel/AttentionBackward.cu:300-541) and gqa_fused_rope_bwd_dQ / _dKdV
+// (context_parallel/GQA_fused_bwd_sm103_cp.cu:135-565).
+//
+// Warp roles (768 threads): 0 = TMA loader, 1 = MMA issuer, 2, 3 idle, 4..11 = softmax-gradient warps of half A, 12..19 of
+// half B (thread = key row, 32 queries), 20..23 = dQ drain warps (thread = query row).
 #include "common.cuh"
 #include "host_utils.h"
 
-#include <stdio.h>
 #include <stdlib.h>
 
 namespace cpb {
 
-// Diagnostics (cycle counters and an event timeline of CTA (0,0,0), tiles 64..71) are compiled in only with
-// -DCPB_BWD64_PROF; without it the predicates below are constant false and the code disappears.
-#ifdef CPB_BWD64_PROF
-#define B64_PROF_ON(x) (x)
-#else
-#define B64_PROF_ON(x) false
-#endif
-// diagnostic timeline: CTA (0,0,0), tiles 64..71: event e of tile t -> prof[16 + (t-64)*32 + e]
-#define B64_STAMP(cond, t, e) do { if ((cond) && (t) >= 64 && (t) < 72) p.prof[16 + ((t) - 64) * 32 + (e)] = clock64(); } while (0)
-
 constexpr int B64_T = 128;
 constexpr int B64_D = 64;
-// Warps: 0 = TMA loader, 1 = MMA issuer, then 4*NG softmax-gradient warps (NG column groups of 128/NG queries; a warp
-// can only touch the 32 tensor-memory lanes of its quarter, so every group has four warps), then 4 dQ drain warps.
-constexpr int b64_threads(int ng) { return 64 + 128 * ng + 128; }
-constexpr int B64_NG = 4;          // column groups of the softmax-gradient warps (2: 64 queries per thread, 4: 32)
-constexpr int B64_POLY = 0;        // share (of 8) of the exponentials computed on the FMA pipe: measured neutral (846 to 855 TFLOP/s for 0..4), kept off
-
-static __device__ long long g_bwd64_prof[16 + 32 * 8];
+constexpr int B64_CW = 32;                              // query columns per softmax-gradient thread
+constexpr int B64_THREADS = 6 * 128;                     // six warpgroups
+// Registers per thread and warpgroup: the launch gives every thread 80 (768 x 80); the loader / issuer warpgroup hands back
+// what the drain warps need to hold a whole dQ row.  48 + 4 x 80 + 112 = 6 x 80.
+constexpr int B64_REGS_ISSUE = 48, B64_REGS_DRAIN = 112;
+constexpr int B64_POLY = 0;        // share (of 8) of the exponentials computed on the FMA pipe
 
 struct Bwd64Params {
   int B, Tq, Tk, Hq, Hkv, Tq_pad;
+  const __nv_bfloat16* k;       // K and V rows are also read with plain loads, once, into tensor memory
+  const __nv_bfloat16* v;
+  long k_sh, k_st, k_sb;
   int causal, k_off;
   float scale, scale_log2;
-  const __nv_bfloat16* aug_l;   // [B,Hq,Tq_pad,8]  (-L_hi, -L_mid, -L_lo, 0...)
-  const __nv_bfloat16* aug_d;   // [B,Hq,Tq_pad,8]  (-Delta_hi, -Delta_mid, -Delta_lo, 0...)
-  const int* q_pos;             // [Tq_pad]
-  void* dk; void* dv;
+  const float* lse2;            // [B,Hq,Tq_pad] LSE * log2(e), +inf in the padding
+  const float* delta;           // [B,Hq,Tq_pad] rowsum(dO o O), 0 in the padding
+  const int* q_pos;             // [Tq_pad] global positions, INT_MAX in the padding
+  void* dk; void* dv;           // [B,Tk,Hkv,D] bf16 (store) or fp32 (accumulate)
   int dkv_mode;                 // 0 bf16 store, 1 fp32 accumulate, 2 routed red.add (fused ring)
-  const uint64_t* route_k;
+  const uint64_t* route_k;      // mode 2: per chunk of route_rows K/V rows the address of its owner's fp32 accumulator
   const uint64_t* route_v;
   int route_rows, route_tl;
-  int debug_skip_dq;
-  long long* prof;              // diagnostic: CTA (0,0,0) writes cycle breakdowns here (16 counters)
+  int debug_skip_dq;            // diagnostic: do not add dQ tiles to global memory (timing experiments only)
   int* status;
 };
 
 struct Bwd64Smem {
-  static constexpr int TILE = B64_T * B64_D * 2;          // 16 KB
-  static constexpr int K_OFF = 0;
-  static constexpr int V_OFF = TILE;
-  static constexpr int NST = 3;                           // Q / dO ring depth: a stage is released only when dQ of its tile
-                                                          // has finished, and S' of the tile after next wants to start then
-  static constexpr int Q_OFF = 2 * TILE;
+  static constexpr int TILE = B64_T * B64_D * 2;         // 16 KB: 128 rows x 128 bytes
+  static constexpr int NST = 3;                          // Q and dO ring depth
+  static constexpr int K_OFF = 0;                        // K once more, as the B operand of dQ
+  static constexpr int Q_OFF = TILE;
   static constexpr int DO_OFF = Q_OFF + NST * TILE;
-  static constexpr int DS_OFF = DO_OFF + NST * TILE;      // dS^T 128 keys x 128 queries bf16 (32 KB)
-  static constexpr int DQS_OFF = DS_OFF + 32768;          // dQ staging: per drain warp two boxes of 32 rows x 32 fp32 (4 x 8 KB)
-  static constexpr int ONES_OFF = DQS_OFF + 32768;        // [128 x 8] bf16 (1,1,1,0,...)           2 KB
-  static constexpr int AUGL_OFF = ONES_OFF + 2048;        // NST x 2 KB
-  static constexpr int AUGD_OFF = AUGL_OFF + NST * 2048;  // NST x 2 KB
-  static constexpr int ZERO_OFF = AUGD_OFF + NST * 2048;        // zero block: second K chunk of every augmenting tile (after them: offsets > 0)
-  static constexpr int QPOS_OFF = ZERO_OFF + 2048;        // NST x 512 B
-  static constexpr int BAR_OFF = QPOS_OFF + NST * 512;
-  static constexpr int TOTAL = BAR_OFF + 256 + 1024;
+  static constexpr int DS_BYTES = B64_T * B64_T * 2;     // dS^T: two 64-query halves of 128 key rows x 128 bytes
+  static constexpr int DS_OFF = DO_OFF + NST * TILE;     // two buffers
+  static constexpr int DQS_OFF = DS_OFF + 2 * DS_BYTES;  // per drain warp two boxes of 32 rows x 32 fp32
+  static constexpr int VEC_OFF = DQS_OFF + 32768;        // NST x (-lse2[128], -delta[128])
+  static constexpr int BAR_OFF = VEC_OFF + NST * 1024;
+  static constexpr int TOTAL = BAR_OFF + 256;            // 216,320 bytes; the base must be 1024-byte aligned as it is
 };
-
-// K-major operand without swizzle: core matrices of 8 rows x 16 bytes; the two 16-byte K chunks of a K=16 step are
-// `lbo` bytes apart, successive 8-row groups `sbo` bytes apart.
-__device__ __forceinline__ uint64_t make_sdesc_noswz(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFF) << 32;
-  d |= (uint64_t)1 << 46;       // version
-  return d;                     // layout type 0: no swizzle
-}
 
 __device__ __forceinline__ void bulk_load_1d_64(void* smem, const void* gmem, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(smem_u32(smem)), "l"((uint64_t)gmem), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 // A global load that stays where it is written (the compiler would otherwise sink it to its first use, one tile later).
-__device__ __forceinline__ int ld_pinned_s32(const int* ptr) {
+__device__ __forceinline__ int ld_ahead_s32(const int* ptr) {
   int v;
   asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(ptr));
   return v;
@@ -113,33 +96,29 @@ __device__ __forceinline__ void red_add_v4_64(float* addr, float a, float b, flo
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
-// POLY: of the 8 column pairs of every 16-column group of an unmasked tile, the last POLY take their exponentials from
-// exp2_poly_f32x2 (FMA pipe) and the others from ex2.approx (special-function unit).
-template <int POLY, int NG>
-__global__ void __launch_bounds__(b64_threads(NG), 1)
+template <int POLY>
+__global__ void __launch_bounds__(B64_THREADS, 1)
 flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                   const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                   const __grid_constant__ CUtensorMap tmDQ, Bwd64Params p) {
+                   const __grid_constant__ CUtensorMap tmDO, const __grid_constant__ CUtensorMap tmDQ, Bwd64Params p) {
   using L = Bwd64Smem;
-  constexpr int D = B64_D;
-  constexpr int CW = B64_T / NG;            // query columns per softmax-gradient thread
-  constexpr int NCH = CW / 16;              // 16-column groups per thread
-  constexpr uint32_t ST_COL = 0, DPT_COL = 128, DV_COL = 256, DK_COL = 320, DQ_COL = 384, PT_COL = 448;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  constexpr int D = B64_D, CW = B64_CW, NST = L::NST;
+  constexpr uint32_t ST_COL = 0, DPT_COL = 128, DV_COL = 256, DK_COL = 320, DQ_COL = 384, K_COL = 448, V_COL = 480;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  if (smem_u32(smem) & 1023) { report(p.status, ST_BAD_INDEX, 870, (int)smem_u32(smem)); return; }
   uint64_t* bars = (uint64_t*)(smem + L::BAR_OFF);
   uint64_t* kv_full = bars + 0;
-  constexpr int NST = L::NST;
   uint64_t* q_full = bars + 1;        // [NST]
   uint64_t* q_empty = bars + 4;       // [NST]
-  uint64_t* s_ready = bars + 7;
-  uint64_t* s_consumed = bars + 8;
-  uint64_t* dp_ready = bars + 9;
-  uint64_t* p_full = bars + 11;
-  uint64_t* dq_full = bars + 12;
-  uint64_t* dq_empty = bars + 13;
-  uint64_t* acc_done = bars + 14;
-  uint32_t* tmem_slot = (uint32_t*)(bars + 16);
+  uint64_t* do_full = bars + 7;       // [NST]
+  uint64_t* do_empty = bars + 10;     // [NST]
+  uint64_t* s_ready = bars + 13;      // [2 halves], like the three below
+  uint64_t* p_ready = bars + 15;
+  uint64_t* dp_ready = bars + 17;
+  uint64_t* ds_ready = bars + 19;
+  uint64_t* dq_full = bars + 21;
+  uint64_t* dq_empty = bars + 22;
+  uint64_t* acc_done = bars + 23;
+  uint32_t* tmem_slot = (uint32_t*)(bars + 24);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
   int* qt_start_s = (int*)(tmem_slot + 2);
 
@@ -151,26 +130,20 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
-    for (int s = 0; s < NST; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 1); }
-    mbar_init(s_ready, 1); mbar_init(s_consumed, 4 * NG); mbar_init(dp_ready, 1);
-    mbar_init(p_full, 4 * NG); mbar_init(dq_full, 1); mbar_init(dq_empty, 4); mbar_init(acc_done, 1);
+    for (int s = 0; s < NST; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 1); mbar_init(&do_full[s], 1); mbar_init(&do_empty[s], 1); }
+    for (int h = 0; h < 2; ++h) { mbar_init(&s_ready[h], 1); mbar_init(&p_ready[h], 8); mbar_init(&dp_ready[h], 1); mbar_init(&ds_ready[h], 8); }
+    mbar_init(dq_full, 1); mbar_init(dq_empty, 4); mbar_init(acc_done, 1);
     *abort_flag = 0;
     *qt_start_s = num_q_tiles;
     fence_mbar_init();
   }
-  // constant augmenting operands: ones tile (first three of eight K elements) and the zero block
-  for (int i = threadIdx.x; i < 128; i += blockDim.x) {
-    uint32_t one2 = 0x3F803F80u;      // (1.0bf16, 1.0bf16)
-    *(uint4*)(smem + L::ONES_OFF + i * 16) = make_uint4(one2, 0x00003F80u, 0u, 0u);
-    *(uint4*)(smem + L::ZERO_OFF + i * 16) = make_uint4(0u, 0u, 0u, 0u);
-  }
-  fence_proxy_async_smem();
   if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
+  // first query tile that can see this K/V tile (q_pos is non-decreasing)
   if (p.causal) {
     const int kpos_min = p.k_off + k0;
     for (int t = threadIdx.x; t < num_q_tiles; t += blockDim.x) {
@@ -180,31 +153,47 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   } else if (threadIdx.x == 0) {
     *qt_start_s = 0;
   }
+  // K and V rows into tensor memory as bf16 A operands (warps 4..7 K, 8..11 V; rows past the end are zero)
+  if (warp >= 4 && warp < 12) {
+    const int row = k0 + (warp & 3) * 32 + lane;
+    const __nv_bfloat16* src = (warp < 8 ? p.k : p.v) + (size_t)b * p.k_sb + (size_t)hkv * p.k_sh + (size_t)(row < p.Tk ? row : 0) * p.k_st;
+    uint32_t w[32];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const uint4 x = row < p.Tk ? *(const uint4*)(src + 8 * c) : make_uint4(0, 0, 0, 0);
+      w[4 * c] = x.x; w[4 * c + 1] = x.y; w[4 * c + 2] = x.z; w[4 * c + 3] = x.w;
+    }
+    tmem_st32(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (warp < 8 ? K_COL : V_COL), w);
+    tmem_wait_st();
+    tc_fence_before();
+  }
   __syncthreads();
   const int qt_start = *qt_start_s;
   const int n_qt = num_q_tiles - qt_start;
   const int n_it = n_qt * G;
 
+  if (warp < 4) {
+  regs_give<B64_REGS_ISSUE>();
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA loader
     if (lane == 0 && n_it > 0) {
-      tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmDO);
-      mbar_expect_tx(kv_full, 2 * L::TILE);
+      tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmDO);
+      mbar_expect_tx(kv_full, L::TILE);
       tma_load_4d(smem + L::K_OFF, &tmK, kv_full, 0, hkv, k0, b);
-      tma_load_4d(smem + L::V_OFF, &tmV, kv_full, 0, hkv, k0, b);
+      int st = 0, ph = 1, hq = hkv * G, t = 0;
       for (int i = 0; i < n_it; ++i) {
-        const int st = i % NST;
-        const uint32_t ph = (i / NST) & 1;
-        if (!mbar_wait(&q_empty[st], ph ^ 1, abort_flag, p.status, 800)) break;
-        const int hq = hkv * G + i / n_qt;
-        const int q0 = (qt_start + i % n_qt) * B64_T;
-        mbar_expect_tx(&q_full[st], 2 * L::TILE + 2 * 2048 + 512);
+        const int q0 = (qt_start + t) * B64_T;
+        if (!mbar_wait_lean(&q_empty[st], ph, abort_flag, 800)) break;
+        mbar_expect_tx(&q_full[st], L::TILE + 1024);
         tma_load_4d(smem + L::Q_OFF + st * L::TILE, &tmQ, &q_full[st], 0, hq, q0, b);
-        tma_load_4d(smem + L::DO_OFF + st * L::TILE, &tmDO, &q_full[st], 0, hq, q0, b);
         const size_t row_off = ((size_t)b * p.Hq + hq) * p.Tq_pad + q0;
-        bulk_load_1d_64(smem + L::AUGL_OFF + st * 2048, p.aug_l + row_off * 8, 2048, &q_full[st]);
-        bulk_load_1d_64(smem + L::AUGD_OFF + st * 2048, p.aug_d + row_off * 8, 2048, &q_full[st]);
-        bulk_load_1d_64(smem + L::QPOS_OFF + st * 512, p.q_pos + q0, 512, &q_full[st]);
+        bulk_load_1d_64(smem + L::VEC_OFF + st * 1024, p.lse2 + row_off, 512, &q_full[st]);
+        bulk_load_1d_64(smem + L::VEC_OFF + st * 1024 + 512, p.delta + row_off, 512, &q_full[st]);
+        if (!mbar_wait_lean(&do_empty[st], ph, abort_flag, 801)) break;
+        mbar_expect_tx(&do_full[st], L::TILE);
+        tma_load_4d(smem + L::DO_OFF + st * L::TILE, &tmDO, &do_full[st], 0, hq, q0, b);
+        if (++st == NST) { st = 0; ph ^= 1; }
+        if (++t == n_qt) { t = 0; ++hq; }
       }
     }
   } else if (warp == 1) {
@@ -212,212 +201,194 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     // The whole warp runs this code convergently; only the elected lane issues the MMAs and commits.
     if (n_it > 0) {
       const uint32_t leader = elect_one() ? 1u : 0u;
-      constexpr uint32_t idesc_s = make_idesc_bf16(B64_T, B64_T, false, false);    // S'^T, dP'^T (and their augmenting steps)
-      constexpr uint32_t idesc_acc = make_idesc_bf16(B64_T, D, false, true);       // dV, dK: A in tensor memory, B N-major
-      constexpr uint32_t idesc_dq = make_idesc_bf16(B64_T, D, true, true);         // dQ: A M-major smem, B N-major
-      // descriptor bases, built once; per MMA only the start-address field is stepped
-      const uint32_t sOnes = smem_u32(smem + L::ONES_OFF), sZero = smem_u32(smem + L::ZERO_OFF);
-      const uint32_t sAL = smem_u32(smem + L::AUGL_OFF), sAD = smem_u32(smem + L::AUGD_OFF);
-      const SDesc dK_k = sdesc_split(sdesc_kmajor(smem_u32(smem + L::K_OFF)));                       // K as K-major A (scores)
-      const SDesc dV_k = sdesc_split(sdesc_kmajor(smem_u32(smem + L::V_OFF)));
-      const SDesc dQ_k = sdesc_split(sdesc_kmajor(smem_u32(smem + L::Q_OFF)));                       // stage 0; stage st: + st * TILE
-      const SDesc dDO_k = sdesc_split(sdesc_kmajor(smem_u32(smem + L::DO_OFF)));
-      const SDesc dQ_n = sdesc_split(make_sdesc(smem_u32(smem + L::Q_OFF), B64_T * 128, 1024));      // Q / dO / K as N-major B
+      constexpr uint32_t idesc_s = make_idesc_bf16(B64_T, 64, false, false);        // one half of S^T, dP^T
+      constexpr uint32_t idesc_acc = make_idesc_bf16(B64_T, D, false, true);        // dV, dK: A in tensor memory, B N-major
+      constexpr uint32_t idesc_dq = make_idesc_bf16(B64_T, D, true, true);          // dQ: A M-major smem, B N-major
+      const SDesc dQ_k = sdesc_split(sdesc_kmajor(smem_u32(smem + L::Q_OFF))), dDO_k = sdesc_split(sdesc_kmajor(smem_u32(smem + L::DO_OFF)));
+      const SDesc dQ_n = sdesc_split(make_sdesc(smem_u32(smem + L::Q_OFF), B64_T * 128, 1024));
       const SDesc dDO_n = sdesc_split(make_sdesc(smem_u32(smem + L::DO_OFF), B64_T * 128, 1024));
       const SDesc dK_n = sdesc_split(make_sdesc(smem_u32(smem + L::K_OFF), B64_T * 128, 1024));
-      const SDesc dDS_m = sdesc_split(make_sdesc(smem_u32(smem + L::DS_OFF), B64_T * 128, 1024));    // dS^T as M-major A
-      const uint64_t d_ones = make_sdesc_noswz(sOnes, sZero - sOnes, 128);
-      // augmenting tiles: the zero block lies NST * 2048 (lse) resp. fewer bytes behind stage 0; stepping the stage moves
-      // the start address forward and the leading offset back by the same amount
+      const SDesc dDS_m = sdesc_split(make_sdesc(smem_u32(smem + L::DS_OFF), B64_T * 128, 1024));
       const uint32_t t_s = tmem_base + ST_COL, t_dp = tmem_base + DPT_COL, t_dv = tmem_base + DV_COL, t_dk = tmem_base + DK_COL,
-                     t_dq = tmem_base + DQ_COL, t_pt = tmem_base + PT_COL;
-      auto issue_s = [&](int st) {          // S'^T = K Q^T - 1 (x) L^T
-        const SDesc q = SDesc{dQ_k.lo + st * (L::TILE >> 4), dQ_k.hi};
-        const uint32_t sA = sAL + st * 2048;
-        umma_ss_cp<false>(leader, t_s, sdesc_at(dK_k, 0), sdesc_at(q, 0), idesc_s);
-        umma_ss_cp<true>(leader, t_s, sdesc_at(dK_k, 32), sdesc_at(q, 32), idesc_s);
-        umma_ss_cp<true>(leader, t_s, sdesc_at(dK_k, 64), sdesc_at(q, 64), idesc_s);
-        umma_ss_cp<true>(leader, t_s, sdesc_at(dK_k, 96), sdesc_at(q, 96), idesc_s);
-        umma_ss_cp<true>(leader, t_s, d_ones, make_sdesc_noswz(sA, sZero - sA, 128), idesc_s);
-        umma_commit_p(leader, s_ready);
+                     t_dq = tmem_base + DQ_COL, t_k = tmem_base + K_COL, t_v = tmem_base + V_COL;
+      auto stage = [](const SDesc& d, int st) { return SDesc{d.lo + (uint32_t)st * (L::TILE >> 4), d.hi}; };
+      // one half of S^T = K Q^T (resp. dP^T = V dO^T): 64 query rows of the stage are 8 KB
+      auto issue_half = [&](uint32_t t_out, uint32_t t_a, const SDesc& d, int h, uint64_t* ready) {
+        umma_ts_cp<false>(leader, t_out + 64 * h, t_a, sdesc_at(d, 8192 * h), idesc_s);
+#pragma unroll
+        for (int k = 1; k < D / 16; ++k) umma_ts_cp<true>(leader, t_out + 64 * h, t_a + 8 * k, sdesc_at(d, 8192 * h + 32 * k), idesc_s);
+        umma_commit_p(leader, &ready[h]);
       };
-      auto issue_dp = [&](int st) {         // dP'^T = V dO^T - 1 (x) Delta^T
-        const SDesc g = SDesc{dDO_k.lo + st * (L::TILE >> 4), dDO_k.hi};
-        const uint32_t sA = sAD + st * 2048;
-        umma_ss_cp<false>(leader, t_dp, sdesc_at(dV_k, 0), sdesc_at(g, 0), idesc_s);
-        umma_ss_cp<true>(leader, t_dp, sdesc_at(dV_k, 32), sdesc_at(g, 32), idesc_s);
-        umma_ss_cp<true>(leader, t_dp, sdesc_at(dV_k, 64), sdesc_at(g, 64), idesc_s);
-        umma_ss_cp<true>(leader, t_dp, sdesc_at(dV_k, 96), sdesc_at(g, 96), idesc_s);
-        umma_ss_cp<true>(leader, t_dp, d_ones, make_sdesc_noswz(sA, sZero - sA, 128), idesc_s);
-        umma_commit_p(leader, dp_ready);
+      // dV += P^T dO (resp. dK += dS^T Q) over the 64 queries of one half; the bf16 operand of 16 queries is 8 columns and
+      // sits in the front half of its writer's 32-column span
+      auto issue_acc = [&](uint32_t t_out, uint32_t t_a, const SDesc& d, int h, uint32_t acc) {
+        umma_ts_p(leader, t_out, t_a + 64 * h, sdesc_at(d, 8192 * h), idesc_acc, acc);
+        umma_ts_cp<true>(leader, t_out, t_a + 64 * h + 8, sdesc_at(d, 8192 * h + 2048), idesc_acc);
+        umma_ts_cp<true>(leader, t_out, t_a + 64 * h + 32, sdesc_at(d, 8192 * h + 4096), idesc_acc);
+        umma_ts_cp<true>(leader, t_out, t_a + 64 * h + 40, sdesc_at(d, 8192 * h + 6144), idesc_acc);
       };
-      const bool wr_prof = B64_PROF_ON(p.prof != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && lane == 0);
-      bool ok = __all_sync(0xffffffffu, mbar_wait(kv_full, 0, abort_flag, p.status, 900) && mbar_wait(&q_full[0], 0, abort_flag, p.status, 901));
+      bool ok = __all_sync(0xffffffffu, mbar_wait_lean(kv_full, 0, abort_flag, 900) && mbar_wait_lean(&q_full[0], 0, abort_flag, 901) &&
+                                            mbar_wait_lean(&do_full[0], 0, abort_flag, 902));
       if (ok) {
         tc_fence_after();
-        issue_s(0);
-        issue_dp(0);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) issue_half(t_s, t_k, dQ_k, h, s_ready);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) issue_half(t_dp, t_v, dDO_k, h, dp_ready);
       }
-      for (int i = 0; ok && i < n_it; ++i) {
-        const int st = i % NST;
-        const SDesc qn = SDesc{dQ_n.lo + st * (L::TILE >> 4), dQ_n.hi}, gn = SDesc{dDO_n.lo + st * (L::TILE >> 4), dDO_n.hi};
-        if (i + 1 < n_it) {
-          // the warps have read S'(i): the next score tile can be produced while they work on tile i
-          if (!__all_sync(0xffffffffu, mbar_wait(s_consumed, i & 1, abort_flag, p.status, 902))) break;
-          B64_STAMP(wr_prof, i, 0);
-          if (!__all_sync(0xffffffffu, mbar_wait(&q_full[(i + 1) % NST], ((i + 1) / NST) & 1, abort_flag, p.status, 903))) break;
+      int st = 0, ph = 0;                      // stage of tile i and the parity of its fill
+      int sp = 0;                              // stage of tile i - 1
+      for (int i = 0; ok && i <= n_it; ++i) {
+        int sn = st + 1, pn = ph;              // stage and parity of tile i + 1
+        if (sn == NST) { sn = 0; pn ^= 1; }
+        const bool more = i + 1 < n_it;
+        if (i > 0) {
+          if (!__all_sync(0xffffffffu, mbar_wait_lean(&ds_ready[1], (i - 1) & 1, abort_flag, 903))) break;
           tc_fence_after();
-          B64_STAMP(wr_prof, i, 1);
-          issue_s((i + 1) % NST);
-          B64_STAMP(wr_prof, i, 2);
+          issue_acc(t_dk, t_dp, stage(dQ_n, sp), 1, 1);
+          umma_commit_p(leader, &q_empty[sp]);
+          if (i < n_it) issue_half(t_dp, t_v, stage(dDO_k, st), 1, dp_ready);       // dO(i) has arrived: dP_A(i) waited for it
+          if (i > 1 && !__all_sync(0xffffffffu, mbar_wait_lean(dq_empty, i & 1, abort_flag, 904))) break;
+          tc_fence_after();
+          const SDesc ds = SDesc{dDS_m.lo + (uint32_t)((i - 1) & 1) * (L::DS_BYTES >> 4), dDS_m.hi};
+          umma_ss_cp<false>(leader, t_dq, sdesc_at(ds, 0), sdesc_at(dK_n, 0), idesc_dq);
+#pragma unroll
+          for (int k = 1; k < B64_T / 16; ++k) umma_ss_cp<true>(leader, t_dq, sdesc_at(ds, k * 2048), sdesc_at(dK_n, k * 2048), idesc_dq);
+          umma_commit_p(leader, dq_full);
+          if (i == n_it) break;
         }
-        if (!__all_sync(0xffffffffu, mbar_wait(p_full, i & 1, abort_flag, p.status, 904))) break;
+        if (!__all_sync(0xffffffffu, mbar_wait_lean(&p_ready[0], i & 1, abort_flag, 905))) break;
         tc_fence_after();
-        B64_STAMP(wr_prof, i, 3);
-        umma_ts_p(leader, t_dk, t_dp, sdesc_at(qn, 0), idesc_acc, i != 0);            // dK += dS^T Q  (frees the dS^T alias)
-#pragma unroll
-        for (int k = 1; k < B64_T / 16; ++k)
-          umma_ts_cp<true>(leader, t_dk, t_dp + ((16 * k) / CW) * CW + (((16 * k) % CW) / 16) * 8, sdesc_at(qn, k * 2048), idesc_acc);
-        B64_STAMP(wr_prof, i, 4);
-        if (i + 1 < n_it) issue_dp((i + 1) % NST);                                     // dP'(i+1): early, off the warps' critical path
-        B64_STAMP(wr_prof, i, 5);
-        umma_ts_p(leader, t_dv, t_pt, sdesc_at(gn, 0), idesc_acc, i != 0);            // dV += P^T dO
-#pragma unroll
-        for (int k = 1; k < B64_T / 16; ++k)
-          umma_ts_cp<true>(leader, t_dv, t_pt + k * 8, sdesc_at(gn, k * 2048), idesc_acc);
-        umma_commit_p(leader, &q_empty[st]);    // Q(i), dO(i) and their vectors are free
-        B64_STAMP(wr_prof, i, 6);
-        if (i > 0 && !__all_sync(0xffffffffu, mbar_wait(dq_empty, (i - 1) & 1, abort_flag, p.status, 905))) break;
+        issue_acc(t_dv, t_s, stage(dDO_n, st), 0, i != 0);
+        if (more) {
+          if (!__all_sync(0xffffffffu, mbar_wait_lean(&q_full[sn], pn, abort_flag, 906))) break;
+          tc_fence_after();
+          issue_half(t_s, t_k, stage(dQ_k, sn), 0, s_ready);                        // over P_A(i), which dV has read
+        }
+        if (!__all_sync(0xffffffffu, mbar_wait_lean(&ds_ready[0], i & 1, abort_flag, 907))) break;
         tc_fence_after();
-        B64_STAMP(wr_prof, i, 7);
-        umma_ss_cp<false>(leader, t_dq, sdesc_at(dDS_m, 0), sdesc_at(dK_n, 0), idesc_dq);      // dQ = dS K
-#pragma unroll
-        for (int k = 1; k < B64_T / 16; ++k)
-          umma_ss_cp<true>(leader, t_dq, sdesc_at(dDS_m, k * 2048), sdesc_at(dK_n, k * 2048), idesc_dq);
-        umma_commit_p(leader, dq_full);         // also: dV(i) has read P^T, dQ(i) the shared-memory dS^T
-        B64_STAMP(wr_prof, i, 8);
+        issue_acc(t_dk, t_dp, stage(dQ_n, st), 0, i != 0);
+        if (more) {
+          if (!__all_sync(0xffffffffu, mbar_wait_lean(&do_full[sn], pn, abort_flag, 908))) break;
+          tc_fence_after();
+          issue_half(t_dp, t_v, stage(dDO_k, sn), 0, dp_ready);                     // over dS_A(i), which dK has read
+        }
+        if (!__all_sync(0xffffffffu, mbar_wait_lean(&p_ready[1], i & 1, abort_flag, 909))) break;
+        tc_fence_after();
+        issue_acc(t_dv, t_s, stage(dDO_n, st), 1, 1);
+        umma_commit_p(leader, &do_empty[st]);
+        if (more) issue_half(t_s, t_k, stage(dQ_k, sn), 1, s_ready);
+        sp = st; st = sn; ph = pn;
       }
       umma_commit_p(leader, acc_done);
-#ifdef CPB_BWD64_PROF
-      if (wr_prof) p.prof[15] = n_it;
-#endif
     }
-  } else if (warp >= 2 && warp < 2 + 4 * NG) {
-    // ------------------------------------------------------------------ softmax-gradient warps (thread = key row, CW queries)
+  }
+  } else if (warp < 20) {
+    // ------------------------------------------------------------------ softmax-gradient warps (thread = key row, 32 queries)
     const int quarter = warp & 3;
-    const int grp = (warp - 2) >> 2;                    // which CW query columns of the tile this thread owns
+    const int grp = (warp - 4) >> 2;                    // which 32 query columns of the tile this thread owns
+    const int half = grp >> 1;
     const int cbase = grp * CW;
     const int r = quarter * 32 + lane;                  // key row inside the tile
     const int kidx = k0 + r;
     const bool k_valid = kidx < p.Tk;
     const int kpos = p.k_off + kidx;
     const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16);
-    // dS^T in shared memory: two [128 keys x 64 queries] halves, 128-byte swizzled rows; this thread's queries start at
-    // 16-byte chunk `chunk0` of its row in half cbase / 64
-    uint8_t* ds_row = smem + L::DS_OFF + (cbase / 64) * (B64_T * 128) + r * 128;
-    constexpr int DS_CHUNKS = CW / 8;
+    uint8_t* ds_row = smem + L::DS_OFF + half * (B64_T * 128) + r * 128;
     const int chunk0 = (cbase % 64) / 8;
     bool alive = true;
-    const bool wprof = B64_PROF_ON(p.prof != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 64);
-    // first query position of a tile decides whether it needs masking; read one tile ahead, straight from global memory
-    int qmin_next = n_it > 0 ? ld_pinned_s32(p.q_pos + qt_start * B64_T) : 0;
+    // first query position of a half tile decides whether it needs masking; read one tile ahead, straight from global memory
+    const int* qp0 = p.q_pos + qt_start * B64_T + 64 * half;
+    int qmin_next = n_it > 0 ? ld_ahead_s32(qp0) : 0;
+    int st = 0, ph = 0, t = 0;
     for (int i = 0; i < n_it && alive; ++i) {
-      const int st = i % NST;
       const int qmin = qmin_next;
-      if (i + 1 < n_it) qmin_next = ld_pinned_s32(p.q_pos + (qt_start + (i + 1) % n_qt) * B64_T);
+      const int t_cur = t;
+      if (++t == n_qt) t = 0;
+      if (i + 1 < n_it) qmin_next = ld_ahead_s32(qp0 + t * B64_T);
       // slow path only for tiles that touch the causal diagonal or the end of the key sequence
       const bool need_mask = (k0 + B64_T > p.Tk) || (p.causal && (p.k_off + k0 + B64_T - 1 > qmin));
-      B64_STAMP(wprof, i, 16);
-      bool ok = mbar_wait(s_ready, i & 1, abort_flag, p.status, 1001);
-      B64_STAMP(wprof, i, 17);
-      if (need_mask) ok = ok && mbar_wait(&q_full[st], (i / NST) & 1, abort_flag, p.status, 1000);   // query positions in shared memory
+      const float* vec = (const float*)(smem + L::VEC_OFF + st * 1024) + cbase;
+      bool ok = mbar_wait_lean(&q_full[st], ph, abort_flag, 1000) && mbar_wait_lean(&s_ready[half], i & 1, abort_flag, 1001);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) { alive = false; break; }
       tc_fence_after();
-      B64_STAMP(wprof, i, 9);
-      const int* qpos = (const int*)(smem + L::QPOS_OFF + st * 512);
-      uint32_t sv[NCH][16];
-#pragma unroll
-      for (int ch = 0; ch < NCH; ++ch) tmem_ld16(t_lane + ST_COL + cbase + 16 * ch, sv[ch]);
+      uint32_t sv[CW];
+      tmem_ld32(t_lane + ST_COL + cbase, sv);
       tmem_wait_ld();
-      tc_fence_before();
-      mbar_arrive_warp(s_consumed);                         // the next score tile may overwrite S'^T
-      uint32_t pk[CW / 2];                              // P^T of this thread's queries, bf16 pairs
       if (!need_mask) {
         const uint64_t c2 = pack_f32x2(p.scale_log2, p.scale_log2);
 #pragma unroll
-        for (int ch = 0; ch < NCH; ++ch)
+        for (int j = 0; j < CW; j += 4) {
+          const float4 l = *(const float4*)(vec + j);
 #pragma unroll
-          for (int j = 0; j < 16; j += 2) {
-            if ((j >> 1) >= 8 - POLY) {                 // resolved at compile time (the loops are unrolled)
-              float p0, p1;
-              unpack_f32x2(exp2_poly_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(sv[ch][j]), __uint_as_float(sv[ch][j + 1])), c2)), p0, p1);
-              pk[ch * 8 + (j >> 1)] = pack_bf16(p0, p1);
+          for (int e = 0; e < 4; e += 2) {
+            const uint64_t x = fma_f32x2(pack_f32x2(__uint_as_float(sv[j + e]), __uint_as_float(sv[j + e + 1])), c2, e ? pack_f32x2(-l.z, -l.w) : pack_f32x2(-l.x, -l.y));
+            float x0, x1;
+            if ((((j + e) % 16) >> 1) >= 8 - POLY) {            // resolved at compile time (the loops are unrolled)
+              unpack_f32x2(exp2_poly_f32x2(x), x0, x1);
             } else {
-              pk[ch * 8 + (j >> 1)] = pack_bf16(ex2f(__uint_as_float(sv[ch][j]) * p.scale_log2), ex2f(__uint_as_float(sv[ch][j + 1]) * p.scale_log2));
+              unpack_f32x2(x, x0, x1);
+              x0 = ex2f(x0); x1 = ex2f(x1);
             }
+            sv[j + e] = __float_as_uint(x0); sv[j + e + 1] = __float_as_uint(x1);
           }
+        }
       } else {
+        const int lim = (p.causal ? kpos : -0x7fffffff - 1);               // visible: lim <= q position
+        const int4* qp = (const int4*)(p.q_pos + (qt_start + t_cur) * B64_T + cbase);
 #pragma unroll
-        for (int ch = 0; ch < NCH; ++ch)
-#pragma unroll
-          for (int j = 0; j < 16; j += 2) {
-            const int c = cbase + ch * 16 + j;
-            const bool v0 = k_valid && (!p.causal || kpos <= qpos[c]), v1 = k_valid && (!p.causal || kpos <= qpos[c + 1]);
-            const float p0 = v0 ? ex2f(__uint_as_float(sv[ch][j]) * p.scale_log2) : 0.f;
-            const float p1 = v1 ? ex2f(__uint_as_float(sv[ch][j + 1]) * p.scale_log2) : 0.f;
-            pk[ch * 8 + (j >> 1)] = pack_bf16(p0, p1);
-          }
-      }
-      // dp_ready(i): dP'(i) is complete, and so is dK(i-1), which read the previous dS^T alias inside the dP'^T columns
-      bool ok3 = mbar_wait(dp_ready, i & 1, abort_flag, p.status, 1004);
-      ok3 = __all_sync(0xffffffffu, ok3);
-      if (!ok3) { alive = false; break; }
-      tc_fence_after();
-      B64_STAMP(wprof, i, 12);
-      // dS^T = P^T o dP'^T with the bf16-rounded P (the value dV is computed from), kept packed in registers
-      uint32_t dsk[CW / 2];
-      {
-        uint32_t dpv[2][16];
-        tmem_ld16(t_lane + DPT_COL + cbase, dpv[0]);
-        tmem_wait_ld();
-#pragma unroll
-        for (int ch = 0; ch < NCH; ++ch) {
-          if (ch < NCH - 1) tmem_ld16(t_lane + DPT_COL + cbase + 16 * (ch + 1), dpv[(ch + 1) & 1]);
-#pragma unroll
-          for (int j = 0; j < 16; j += 2) {
-            const uint32_t pp = pk[ch * 8 + (j >> 1)];
-            dsk[ch * 8 + (j >> 1)] = pack_bf16(bf16_lo(pp) * __uint_as_float(dpv[ch & 1][j]), bf16_hi(pp) * __uint_as_float(dpv[ch & 1][j + 1]));
-          }
-          if (ch < NCH - 1) tmem_wait_ld();
+        for (int j = 0; j < CW; j += 4) {
+          const float4 l = *(const float4*)(vec + j);
+          const int4 q = __ldg(qp + (j >> 2));
+          sv[j] = (k_valid && lim <= q.x) ? __float_as_uint(ex2f(fmaf(__uint_as_float(sv[j]), p.scale_log2, -l.x))) : 0u;
+          sv[j + 1] = (k_valid && lim <= q.y) ? __float_as_uint(ex2f(fmaf(__uint_as_float(sv[j + 1]), p.scale_log2, -l.y))) : 0u;
+          sv[j + 2] = (k_valid && lim <= q.z) ? __float_as_uint(ex2f(fmaf(__uint_as_float(sv[j + 2]), p.scale_log2, -l.z))) : 0u;
+          sv[j + 3] = (k_valid && lim <= q.w) ? __float_as_uint(ex2f(fmaf(__uint_as_float(sv[j + 3]), p.scale_log2, -l.w))) : 0u;
         }
       }
-      // dq_full(i-1): dV(i-1) has read the previous P^T and dQ(i-1) the previous dS^T in shared memory
-      if (i > 0) {
-        bool ok4 = mbar_wait(dq_full, (i - 1) & 1, abort_flag, p.status, 1005);
-        ok4 = __all_sync(0xffffffffu, ok4);
-        if (!ok4) { alive = false; break; }
-        tc_fence_after();
-      }
-      // P^T -> its own columns (A operand of dV); dS^T -> the front half of this thread's dP'^T span (A operand of dK: the
-      // k-step of queries 16k.. sits at columns (16k / CW) * CW + ((16k % CW) / 16) * 8) and -> shared memory (row = key,
-      // 64 queries per 128-byte swizzled row; M-major A of dQ)
-      B64_STAMP(wprof, i, 14);
-      if constexpr (CW == 64) {
-        tmem_st32(t_lane + PT_COL + cbase / 2, pk);
-        tmem_st32(t_lane + DPT_COL + cbase, dsk);
-      } else {
-        tmem_st16(t_lane + PT_COL + cbase / 2, pk);
-        tmem_st16(t_lane + DPT_COL + cbase, dsk);
-      }
+      {
+        uint32_t pk[CW / 2];                            // P^T of this thread's queries as bf16 pairs, over its own scores
 #pragma unroll
-      for (int c8 = 0; c8 < DS_CHUNKS; ++c8)
-        *(uint4*)(ds_row + (((chunk0 + c8) ^ (r & 7)) << 4)) = make_uint4(dsk[4 * c8], dsk[4 * c8 + 1], dsk[4 * c8 + 2], dsk[4 * c8 + 3]);
+        for (int j = 0; j < CW; j += 2) pk[j >> 1] = pack_bf16(__uint_as_float(sv[j]), __uint_as_float(sv[j + 1]));
+        tmem_st16(t_lane + ST_COL + cbase, pk);
+      }
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive_warp(&p_ready[half]);
+      // dp_ready(i): dP(i) of this half is complete, and so is dQ(i-2), which read the dS^T buffer written below
+      ok = mbar_wait_lean(&dp_ready[half], i & 1, abort_flag, 1002);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) { alive = false; break; }
+      tc_fence_after();
+      uint32_t dsk[CW / 2];                             // dS^T = P^T o (dP^T - Delta) with P in fp32
+#pragma unroll
+      for (int ch = 0; ch < CW; ch += 16) {
+        uint32_t dpv[16];
+        tmem_ld16(t_lane + DPT_COL + cbase + ch, dpv);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 16; j += 4) {
+          const float4 dl = *(const float4*)(vec + 128 + ch + j);
+          float e0, e1, e2, e3;
+          unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(sv[ch + j]), __uint_as_float(sv[ch + j + 1])),
+                                 add_f32x2(pack_f32x2(__uint_as_float(dpv[j]), __uint_as_float(dpv[j + 1])), pack_f32x2(-dl.x, -dl.y))), e0, e1);
+          unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(sv[ch + j + 2]), __uint_as_float(sv[ch + j + 3])),
+                                 add_f32x2(pack_f32x2(__uint_as_float(dpv[j + 2]), __uint_as_float(dpv[j + 3])), pack_f32x2(-dl.z, -dl.w))), e2, e3);
+          dsk[(ch + j) >> 1] = pack_bf16(e0, e1);
+          dsk[((ch + j) >> 1) + 1] = pack_bf16(e2, e3);
+        }
+      }
+      tmem_st16(t_lane + DPT_COL + cbase, dsk);
+      uint8_t* dsb = ds_row + (i & 1) * L::DS_BYTES;
+#pragma unroll
+      for (int c8 = 0; c8 < CW / 8; ++c8)
+        *(uint4*)(dsb + (((chunk0 + c8) ^ (r & 7)) << 4)) = make_uint4(dsk[4 * c8], dsk[4 * c8 + 1], dsk[4 * c8 + 2], dsk[4 * c8 + 3]);
       tmem_wait_st();
       fence_proxy_async_smem();
       tc_fence_before();
-      mbar_arrive_warp(p_full);
-      B64_STAMP(wprof, i, 15);
+      mbar_arrive_warp(&ds_ready[half]);
+      if (++st == NST) { st = 0; ph ^= 1; }
     }
     // final: dK, dV -> global
     if (n_it == 0) {
@@ -428,21 +399,18 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         for (int c = 0; c < D; c += 8) { *(uint4*)(dkr + c) = make_uint4(0, 0, 0, 0); *(uint4*)(dvr + c) = make_uint4(0, 0, 0, 0); }
       }
     } else if (alive) {
-      bool ok = mbar_wait(acc_done, 0, abort_flag, p.status, 1002);
+      bool ok = mbar_wait_lean(acc_done, 0, abort_flag, 1003);
       ok = __all_sync(0xffffffffu, ok);
       if (ok) {
         tc_fence_after();
         const size_t off = (((size_t)b * p.Tk + (k_valid ? kidx : 0)) * p.Hkv + hkv) * D;
-        const int which = grp >= NG / 2;                 // the first half of the warp groups drains dK, the second dV
-        constexpr int DCOLS = D / (NG / 2);              // accumulator columns per warp group
-        const int c_lo = (grp % (NG / 2)) * DCOLS;
-        const uint32_t col = which ? DV_COL : DK_COL;
+        const int which = grp >> 1;                      // groups 0, 1 drain dK, groups 2, 3 dV: 32 columns each
+        const int c = (grp & 1) * 32;
         void* base = which ? p.dv : p.dk;
         const float osc = which ? 1.f : p.scale;         // dS^T was accumulated without the softmax scale
-#pragma unroll 1
-        for (int c = c_lo; c < c_lo + DCOLS; c += 32) {
+        {
           uint32_t v[32];
-          tmem_ld32(t_lane + col + c, v);
+          tmem_ld32(t_lane + (which ? DV_COL : DK_COL) + c, v);
           tmem_wait_ld();
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * osc);
@@ -479,40 +447,36 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
     }
   } else {
-    // ------------------------------------------------------------------ dQ drain warps (the last four)
-    // tensor memory -> registers -> 128B-swizzled fp32 staging -> TMA reduce-add into the global fp32 dQ (rows past the
-    // end of the sequence are clipped by the tensor map).  Every warp drains its own 32 query rows through its own
-    // staging slice with its own bulk group, so the four warps never wait for one another; the reduce of tile i is read
-    // out of the slice while the warp waits for tile i+1.
+    // ------------------------------------------------------------------ dQ drain warps (20..23)
+    regs_take<B64_REGS_DRAIN>();
+    // tensor memory -> registers -> 128B-swizzled fp32 staging -> TMA reduce-add into the global fp32 dQ (rows past the end
+    // of the sequence are clipped by the tensor map).  Every warp drains its own 32 query rows through its own two boxes
+    // with its own bulk group, so the four warps never wait for one another.
     const int quarter = warp & 3;
-    const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16);
-    uint8_t* stage = smem + L::DQS_OFF + quarter * 8192;      // [2 column halves][32 rows][128 B]
+    const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16) + DQ_COL;
+    uint8_t* stage = smem + L::DQS_OFF + quarter * 8192;      // [2 boxes][32 rows][128 B]
     const bool issuer = (lane == 0);
     if (issuer) tma_prefetch_desc(&tmDQ);
+    int hq = hkv * G, t = 0;
     for (int i = 0; i < n_it; ++i) {
-      const bool dprof = B64_PROF_ON(p.prof != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && warp == 2 + 4 * NG && issuer);
-      const bool dprof_all = B64_PROF_ON(p.prof != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && lane == 0 && i >= 64 && i < 72);
-      bool ok = mbar_wait(dq_full, i & 1, abort_flag, p.status, 1100);
+      bool ok = mbar_wait_lean(dq_full, i & 1, abort_flag, 1100);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      if (dprof_all) atomicMax((unsigned long long*)&p.prof[16 + (i - 64) * 32 + 10], (unsigned long long)clock64());
-      const int hq = hkv * G + i / n_qt;
-      const int q0 = (qt_start + i % n_qt) * B64_T;
+      const int q0 = (qt_start + t) * B64_T;
       uint32_t v[2][32];
-      tmem_ld32(t_lane + DQ_COL, v[0]);
-      tmem_ld32(t_lane + DQ_COL + 32, v[1]);
+      tmem_ld32(t_lane, v[0]);
+      tmem_ld32(t_lane + 32, v[1]);
       tmem_wait_ld();
       tc_fence_before();
-      mbar_arrive_warp(dq_empty);                          // tensor-memory dQ is free again
-      if (dprof_all) atomicMax((unsigned long long*)&p.prof[16 + (i - 64) * 32 + 11], (unsigned long long)clock64());
-      if (issuer) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the previous tile has left the slice
+      mbar_arrive_warp(dq_empty);                           // tensor-memory dQ is free again
+      if (issuer) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the boxes have been read out
       __syncwarp();
 #pragma unroll
-      for (int h = 0; h < D / 32; ++h) {
+      for (int h = 0; h < 2; ++h) {
         uint8_t* rowp = stage + h * 4096 + lane * 128;
 #pragma unroll
-        for (int c4 = 0; c4 < 8; ++c4)                  // dS was formed without the softmax scale: apply it here
+        for (int c4 = 0; c4 < 8; ++c4)                      // dS was formed without the softmax scale: apply it here
           *(float4*)(rowp + ((c4 ^ (lane & 7)) << 4)) = make_float4(__uint_as_float(v[h][4 * c4]) * p.scale, __uint_as_float(v[h][4 * c4 + 1]) * p.scale,
                                                                     __uint_as_float(v[h][4 * c4 + 2]) * p.scale, __uint_as_float(v[h][4 * c4 + 3]) * p.scale);
       }
@@ -520,13 +484,13 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       __syncwarp();
       if (issuer && !p.debug_skip_dq) {
 #pragma unroll
-        for (int h = 0; h < D / 32; ++h)
+        for (int h = 0; h < 2; ++h)
           asm volatile("cp.reduce.async.bulk.tensor.4d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
                        ::"l"((uint64_t)&tmDQ), "r"(smem_u32(stage + h * 4096)), "r"(h * 32), "r"(hq), "r"(q0 + quarter * 32), "r"(b)
                        : "memory");
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
       }
-      B64_STAMP(dprof, i, 13);
+      if (++t == n_qt) { t = 0; ++hq; }
     }
     if (issuer) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
@@ -534,32 +498,7 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   tc_fence_before();
   __syncthreads();
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
-}
-
-// aug_l[row] = -(hi, mid, lo) of lse2[row] / scale_log2 and aug_d[row] = -(hi, mid, lo) of delta[row], each padded to
-// eight bf16 (16 bytes per query row).  Rows whose lse2 is +inf (padding, fully masked) get a large finite magnitude so
-// that their probabilities underflow to exactly zero.
-__global__ void bwd64_aug_kernel(const float* __restrict__ lse2, const float* __restrict__ delta,
-                                 uint4* __restrict__ aug_l, uint4* __restrict__ aug_d, size_t n, float inv_scale_log2) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const float src[2] = {lse2[i], delta[i]};
-    uint4 out[2];
-#pragma unroll
-    for (int w = 0; w < 2; ++w) {
-      float x = src[w];
-      if (w == 0) x = (x > 1e37f) ? 1e30f : x * inv_scale_log2;
-      x = -x;
-      const __nv_bfloat16 h = __float2bfloat16_rn(x);
-      const float r1 = x - __bfloat162float(h);
-      const __nv_bfloat16 m = __float2bfloat16_rn(r1);
-      const float r2 = r1 - __bfloat162float(m);
-      const __nv_bfloat16 l = __float2bfloat16_rn(r2);
-      out[w] = make_uint4((uint32_t)__bfloat16_as_ushort(h) | ((uint32_t)__bfloat16_as_ushort(m) << 16),
-                          (uint32_t)__bfloat16_as_ushort(l), 0u, 0u);
-    }
-    aug_l[i] = out[0];
-    aug_d[i] = out[1];
-  }
+  if (threadIdx.x == 0 && *abort_flag) report(p.status, ST_TIMEOUT_MBAR, *abort_flag, 0);
 }
 
 static int make_tmap4_64(CUtensorMap* m, const void* ptr, int H, int T, int B, long s_head, long s_tok, long s_batch) {
@@ -573,36 +512,27 @@ static int make_tmap4_64(CUtensorMap* m, const void* ptr, int H, int T, int B, l
 
 using namespace cpb;
 
-// lse2 / delta: fp32 [B,Hq,Tq_pad] as produced by cpb_flash_bwd_prep; aug_l / aug_d: bf16 [B,Hq,Tq_pad,8].
-extern "C" int cpb_flash_bwd64_aug(const float* lse2, const float* delta, void* aug_l, void* aug_d, long n, float scale,
-                                   cudaStream_t stream) {
-  if (n <= 0) return CPB_OK;
-  size_t g = ((size_t)n + 255) / 256;
-  const size_t cap = (size_t)sm_count() * 8;
-  if (g > cap) g = cap;
-  bwd64_aug_kernel<<<(int)g, 256, 0, stream>>>(lse2, delta, (uint4*)aug_l, (uint4*)aug_d, (size_t)n, 1.f / (scale * 1.4426950408889634f));
-  return check_launch("flash_bwd64_aug");
-}
-
-// Same contract as cpb_flash_bwd for head_dim 64, with the per-row vectors passed in their augmented bf16 form.
-extern "C" int cpb_flash_bwd64(const void* q, const void* k, const void* v, const void* dout, const void* aug_l,
-                               const void* aug_d, float* dq, void* dk, void* dv,
-                               int B, int Tq, int Tk, int Hq, int Hkv, int Tq_pad,
-                               long q_sh, long q_st, long q_sb, long k_sh, long k_st, long k_sb,
-                               float scale, int causal, int k_off, const int* q_pos, int dkv_mode,
-                               const uint64_t* route_k, const uint64_t* route_v, int route_rows, int route_tl,
-                               int* status, cudaStream_t stream) {
+// q, k, v: strided views (element strides: head, token, batch); dout contiguous [B,Tq,Hq,D].
+// dq: fp32 [B,Tq,Hq,D] (accumulated; caller zeroes).  dk/dv: [B,Tk,Hkv,D] bf16 (written) or fp32 (+=).
+// lse2 / delta: fp32 [B,Hq,Tq_pad] as produced by cpb_flash_bwd_prep; q_pos: int32 [Tq_pad] (INT_MAX padding), required.
+extern "C" int cpb_flash_bwd64(const void* q, const void* k, const void* v, const void* dout, const float* lse2,
+                                const float* delta, float* dq, void* dk, void* dv,
+                                int B, int Tq, int Tk, int Hq, int Hkv, int Tq_pad,
+                                long q_sh, long q_st, long q_sb, long k_sh, long k_st, long k_sb,
+                                float scale, int causal, int k_off, const int* q_pos, int dkv_mode,
+                                const uint64_t* route_k, const uint64_t* route_v, int route_rows, int route_tl,
+                                int* status, cudaStream_t stream) {
   if (Hq % Hkv) return set_error(CPB_ERR_ARG, "flash_bwd64: Hq %% Hkv != 0");
   if (Tq_pad % B64_T || Tq_pad < Tq) return set_error(CPB_ERR_ARG, "flash_bwd64: bad Tq_pad");
-  if (q_pos == nullptr || aug_l == nullptr || aug_d == nullptr) return set_error(CPB_ERR_ARG, "flash_bwd64: q_pos and the augmented vectors are required");
-  if (((uintptr_t)aug_l | (uintptr_t)aug_d | (uintptr_t)q_pos) & 15) return set_error(CPB_ERR_ARG, "flash_bwd64: vectors must be 16-byte aligned");
+  if (q_pos == nullptr) return set_error(CPB_ERR_ARG, "flash_bwd64: q_pos is required");
+  if (((uintptr_t)k | (uintptr_t)v) & 15 || (k_sh | k_st | k_sb) & 7) return set_error(CPB_ERR_ARG, "flash_bwd64: K/V rows must be 16-byte aligned");
+  if (((uintptr_t)lse2 | (uintptr_t)delta | (uintptr_t)q_pos) & 15) return set_error(CPB_ERR_ARG, "flash_bwd64: vectors must be 16-byte aligned");
   if (dkv_mode == 2 && (route_k == nullptr || route_v == nullptr || route_rows <= 0))
     return set_error(CPB_ERR_ARG, "flash_bwd64: routed dK/dV needs route tables");
-  CUtensorMap tq, tk, tv, tdo, tdq;
+  CUtensorMap tq, tk, tdo, tdq;
   int rc;
   if ((rc = make_tmap4_64(&tq, q, Hq, Tq, B, q_sh, q_st, q_sb)) != CPB_OK) return rc;
   if ((rc = make_tmap4_64(&tk, k, Hkv, Tk, B, k_sh, k_st, k_sb)) != CPB_OK) return rc;
-  if ((rc = make_tmap4_64(&tv, v, Hkv, Tk, B, k_sh, k_st, k_sb)) != CPB_OK) return rc;
   if ((rc = make_tmap4_64(&tdo, dout, Hq, Tq, B, B64_D, (long)Hq * B64_D, (long)Tq * Hq * B64_D)) != CPB_OK) return rc;
   {
     uint64_t dims[4] = {(uint64_t)B64_D, (uint64_t)Hq, (uint64_t)Tq, (uint64_t)B};
@@ -613,67 +543,19 @@ extern "C" int cpb_flash_bwd64(const void* q, const void* k, const void* v, cons
   Bwd64Params p;
   p.B = B; p.Tq = Tq; p.Tk = Tk; p.Hq = Hq; p.Hkv = Hkv; p.Tq_pad = Tq_pad; p.causal = causal; p.k_off = k_off;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
-  p.aug_l = (const __nv_bfloat16*)aug_l; p.aug_d = (const __nv_bfloat16*)aug_d; p.q_pos = q_pos;
-  p.dk = dk; p.dv = dv; p.dkv_mode = dkv_mode; p.status = status;
+  p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v; p.k_sh = k_sh; p.k_st = k_st; p.k_sb = k_sb;
+  p.lse2 = lse2; p.delta = delta; p.q_pos = q_pos; p.dk = dk; p.dv = dv; p.dkv_mode = dkv_mode; p.status = status;
   p.route_k = route_k; p.route_v = route_v; p.route_rows = route_rows; p.route_tl = route_tl;
-  // diagnostic switches and the tuning knob are read once per process, not per launch
   static const bool skip_dq = [] {
     const char* e = getenv("CPB_BWD_SKIP_DQ");
     const bool on = e != nullptr && e[0] == '1';
     if (on) fprintf(stderr, "CPB_BWD_SKIP_DQ=1: the attention backward does NOT produce dQ (timing experiment only)\n");
     return on;
   }();
-  static const bool want_prof = [] { const char* e = getenv("CPB_BWD_PROF"); return e != nullptr && e[0] == '1'; }();
-  static const int poly = [] { const char* e = getenv("CPB_BWD64_POLY"); return e ? atoi(e) : B64_POLY; }();
   p.debug_skip_dq = skip_dq;
-  p.prof = nullptr;
-  if (want_prof) {
-    void* sym = nullptr;
-    if (cudaGetSymbolAddress(&sym, g_bwd64_prof) == cudaSuccess) { p.prof = (long long*)sym; cudaMemsetAsync(sym, 0, sizeof(long long) * (16 + 32 * 8), stream); }
-  }
   dim3 grid((Tk + B64_T - 1) / B64_T, Hkv, B);
-#define CPB_BWD64_LAUNCH(PP, GG)                                                                                        \
-  do {                                                                                                                  \
-    static bool cfg = false;                                                                                            \
-    if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_bwd64_kernel<PP, GG>, cudaFuncAttributeMaxDynamicSharedMemorySize, Bwd64Smem::TOTAL)); cfg = true; } \
-    flash_bwd64_kernel<PP, GG><<<grid, b64_threads(GG), Bwd64Smem::TOTAL, stream>>>(tq, tk, tv, tdo, tdq, p);           \
-  } while (0)
-  static const int ng = [] { const char* e = getenv("CPB_BWD64_NG"); return e ? atoi(e) : B64_NG; }();
-  if (ng == 2) {
-    switch (poly) {
-      case 3: CPB_BWD64_LAUNCH(3, 2); break;
-      default: CPB_BWD64_LAUNCH(0, 2); break;
-    }
-  } else {
-    switch (poly) {
-      case 2: CPB_BWD64_LAUNCH(2, 4); break;
-      case 3: CPB_BWD64_LAUNCH(3, 4); break;
-      case 4: CPB_BWD64_LAUNCH(4, 4); break;
-      default: CPB_BWD64_LAUNCH(0, 4); break;
-    }
-  }
-#undef CPB_BWD64_LAUNCH
-  if (p.prof != nullptr) {
-    long long h[16 + 32 * 8];
-    cudaStreamSynchronize(stream);
-    if (cudaMemcpy(h, p.prof, sizeof(h), cudaMemcpyDeviceToHost) == cudaSuccess && h[15] > 0)
-      fprintf(stderr, "[flash_bwd64 prof] tiles=%lld cycles/tile of the MMA warp: wait_s_consumed+issue_S=%lld wait_p_full=%lld wait_dq_empty=%lld issue_grads=%lld\n",
-              h[15], h[0] / h[15], h[1] / h[15], h[2] / h[15], h[3] / h[15]);
-    if (cudaMemcpy(h, p.prof, sizeof(h), cudaMemcpyDeviceToHost) == cudaSuccess && h[15] > 72) {
-      const long long base = h[16 + 9];
-      const int NE = 18;
-      static const char* names[18] = {"M:s_consumed", "M:q_full", "M:S'issued", "M:p_full", "M:dK issued", "M:dP' issued", "M:dV issued", "M:dq_empty",
-                                      "M:dQ issued", "W:s_ready", "D:dq_full seen(last warp)", "D:dq_empty arrive(last warp)", "W:dp_ready", "D:staged", "W:dq_full", "W:p_full arrive", "W:tile top", "W:s_ready try ok"};
-      for (int t = 0; t < 4; ++t) {
-        fprintf(stderr, "  tile %d:", 64 + t);
-        // chronological order
-        int order[18]; for (int e = 0; e < NE; ++e) order[e] = e;
-        for (int a2 = 0; a2 < NE; ++a2) for (int b2 = a2 + 1; b2 < NE; ++b2) if (h[16 + t * 32 + order[b2]] < h[16 + t * 32 + order[a2]]) { int x = order[a2]; order[a2] = order[b2]; order[b2] = x; }
-        for (int e = 0; e < NE; ++e) fprintf(stderr, " %s@%lld", names[order[e]], h[16 + t * 32 + order[e]] - base);
-        fprintf(stderr, " [dq_empty polls: %lld]", h[16 + t * 32 + 20]);
-        fprintf(stderr, "\n");
-      }
-    }
-  }
+  static bool cfg = false;
+  if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_bwd64_kernel<B64_POLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, Bwd64Smem::TOTAL)); cfg = true; }
+  flash_bwd64_kernel<B64_POLY><<<grid, B64_THREADS, Bwd64Smem::TOTAL, stream>>>(tq, tk, tdo, tdq, p);
   return check_launch("flash_bwd64");
 }

@@ -142,6 +142,10 @@ __device__ __forceinline__ bool mbar_wait_lean(uint64_t* bar, uint32_t parity, v
   return false;
 }
 
+// Registers moved between warpgroups (setmaxnreg, all four warps of the warpgroup).
+template <int R> __device__ __forceinline__ void regs_give() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
+template <int R> __device__ __forceinline__ void regs_take() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
+
 // Wait executed by a whole warp that must stay convergent: one lane polls, the result is broadcast.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                                int* status, int site) {

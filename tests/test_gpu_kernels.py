@@ -255,16 +255,16 @@ def test_flash_bwd(D, B, Tq, Tk, Hq, Hkv, causal):
     assert_close(dq.float(), wdq, cos=0.998, rel=5e-2, name="dq")
 
 
-# head_dim 128: one query tile, ragged ends on both sides, several tiles of several grouped heads (both stages of every ring
+# Both head widths: one query tile, ragged ends on both sides, several tiles of several grouped heads (both stages of every ring
 # in use), the zig-zag shard of a ring rank, a key block at an offset, rows that see no key.  Same bars as test_flash_bwd.
+@pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("B,Tq,Tk,Hq,Hkv,ring,k_off,accumulate", [
     (1, 1, 1, 1, 1, 1, 0, False), (2, 129, 127, 2, 1, 1, 0, True), (1, 640, 896, 4, 2, 1, 0, False), (1, 256, 1024, 6, 2, 4, 0, True),
     (2, 384, 200, 2, 2, 1, 100, False), (1, 130, 300, 3, 1, 1, 64, True)])
-def test_flash_bwd_d128_shapes_and_modes(B, Tq, Tk, Hq, Hkv, ring, k_off, accumulate):
+def test_flash_bwd_shapes_and_modes(D, B, Tq, Tk, Hq, Hkv, ring, k_off, accumulate):
     from context_parallelism_b200.ops import attention as A, reference as R
     from context_parallelism_b200.parallel.shard import local_positions
     torch.manual_seed(21)
-    D = 128
     q = torch.randn(B, Tq, Hq, D, device=dev()).bfloat16()
     k, v = (torch.randn(B, Tk, Hkv, D, device=dev()).bfloat16() for _ in range(2))
     do = torch.randn(B, Tq, Hq, D, device=dev()).bfloat16()
