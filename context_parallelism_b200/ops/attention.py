@@ -100,6 +100,27 @@ class _FlashAttnFn(torch.autograd.Function):
         return dq, dk, dv, None, None, None, None
 
 
+class _FlashAttnPackedFn(torch.autograd.Function):
+    """Attention on packed projections ``[B,T,(Hq+2·Hkv)·D]`` whose gradient is written packed as well."""
+
+    @staticmethod
+    def forward(ctx, qkv, Hq, Hkv, D, scale, causal):
+        B, T = qkv.shape[:2]
+        x = qkv.view(B, T, Hq + 2 * Hkv, D)
+        out, lse = flash_fwd(x[:, :, :Hq], x[:, :, Hq:Hq + Hkv], x[:, :, Hq + Hkv:], scale, causal)
+        ctx.save_for_backward(x, out, lse)
+        ctx.meta = (Hq, Hkv, scale, causal)
+        return out.view(B, T, Hq * D)
+
+    @staticmethod
+    def backward(ctx, dout):
+        from .attention_bwd import flash_bwd_packed
+        x, out, lse = ctx.saved_tensors
+        Hq, Hkv, scale, causal = ctx.meta
+        dqkv = flash_bwd_packed(x, Hq, Hkv, out, lse, dout.reshape(out.shape), scale, causal)
+        return dqkv.view(*dqkv.shape[:2], -1), None, None, None, None, None
+
+
 # ATTN_FP32=1: differentiable attention goes through the fp32-accurate CUDA-core kernels (parity runs); set by the engine.
 FP32_ACCURATE = False
 
@@ -159,3 +180,13 @@ def flash_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: Op
     Tk = k.shape[1]
     kp = torch.arange(k_off, k_off + Tk)
     return ref.attention_dense(q, k, v, scale, q_pos, kp, causal)
+
+
+def flash_attention_packed(qkv: torch.Tensor, Hq: int, Hkv: int, D: int, scale: float, causal: bool = True) -> torch.Tensor:
+    """Differentiable attention over packed projections ``[B,T,(Hq+2·Hkv)·D]`` -> ``[B,T,Hq·D]``."""
+    if qkv.is_cuda and not FP32_ACCURATE:
+        return _FlashAttnPackedFn.apply(qkv, Hq, Hkv, D, scale, causal)
+    B, T = qkv.shape[:2]
+    x = qkv.view(B, T, Hq + 2 * Hkv, D)
+    o, _ = flash_attention(x[:, :, :Hq], x[:, :, Hq:Hq + Hkv], x[:, :, Hq + Hkv:], scale, causal)
+    return o.reshape(B, T, Hq * D)

@@ -24,14 +24,16 @@ def padded_q_pos(Tq: int, device, q_pos: Optional[torch.Tensor]) -> torch.Tensor
     return out
 
 
-def flash_bwd_prep(o: torch.Tensor, do: torch.Tensor, lse: torch.Tensor):
-    """``delta = rowsum(dO∘O)`` and ``lse·log2(e)`` padded to a multiple of 128 rows."""
+def flash_bwd_prep(o: torch.Tensor, do: torch.Tensor, lse: torch.Tensor, dq: Optional[torch.Tensor] = None,
+                   q_pos: Optional[torch.Tensor] = None, qpos_pad: Optional[torch.Tensor] = None):
+    """``delta = rowsum(dO∘O)`` and ``lse·log2(e)`` padded to a multiple of 128 rows.  The same launch clears the fp32
+    accumulator ``dq`` (shaped like ``o``) and fills ``qpos_pad`` as :func:`padded_q_pos` does, when they are given."""
     B, Tq, Hq, D = o.shape
     tq_pad = (Tq + 127) // 128 * 128
     delta = torch.empty((B, Hq, tq_pad), dtype=torch.float32, device=o.device)
     lse2 = torch.empty_like(delta)
-    nv.call("flash_bwd_prep", nv.ptr(o), nv.ptr(do), nv.ptr(lse), nv.ptr(delta), nv.ptr(lse2),
-            nv.i(B), nv.i(Tq), nv.i(Hq), nv.i(D), nv.i(tq_pad), nv.stream_ptr(o.device))
+    nv.call("flash_bwd_prep", nv.ptr(o), nv.ptr(do), nv.ptr(lse), nv.ptr(delta), nv.ptr(lse2), nv.ptr(dq), nv.ptr(q_pos),
+            nv.ptr(qpos_pad), nv.i(B), nv.i(Tq), nv.i(Hq), nv.i(D), nv.i(tq_pad), nv.stream_ptr(o.device))
     return delta, lse2
 
 
@@ -40,7 +42,7 @@ def flash_bwd_delta(o: torch.Tensor, do: torch.Tensor) -> torch.Tensor:
     B, Tq, Hq, D = o.shape
     tq_pad = (Tq + 127) // 128 * 128
     delta = torch.empty((B, Hq, tq_pad), dtype=torch.float32, device=o.device)
-    nv.call("flash_bwd_prep", nv.ptr(o), nv.ptr(do), nv.ptr(None), nv.ptr(delta), nv.ptr(None),
+    nv.call("flash_bwd_prep", nv.ptr(o), nv.ptr(do), nv.ptr(None), nv.ptr(delta), nv.ptr(None), nv.ptr(None), nv.ptr(None), nv.ptr(None),
             nv.i(B), nv.i(Tq), nv.i(Hq), nv.i(D), nv.i(tq_pad), nv.stream_ptr(o.device))
     return delta
 
@@ -50,17 +52,18 @@ def flash_bwd_lse2(lse: torch.Tensor, D: int) -> torch.Tensor:
     B, Hq, Tq = lse.shape
     tq_pad = (Tq + 127) // 128 * 128
     lse2 = torch.empty((B, Hq, tq_pad), dtype=torch.float32, device=lse.device)
-    nv.call("flash_bwd_prep", nv.ptr(None), nv.ptr(None), nv.ptr(lse), nv.ptr(None), nv.ptr(lse2),
+    nv.call("flash_bwd_prep", nv.ptr(None), nv.ptr(None), nv.ptr(lse), nv.ptr(None), nv.ptr(lse2), nv.ptr(None), nv.ptr(None), nv.ptr(None),
             nv.i(B), nv.i(Tq), nv.i(Hq), nv.i(D), nv.i(tq_pad), nv.stream_ptr(lse.device))
     return lse2
 
 
 def flash_bwd_core(q, k, v, do, lse2, delta, qpos_pad, scale, causal, k_off, dq_f32, dk, dv, dkv_accumulate,
-                   route=None):
+                   route=None, dkv_st: int = 0):
     """One launch of the backward kernel: ``dq_f32`` (fp32) is accumulated with atomics; ``dk``/``dv`` are
     written as bf16, or accumulated in fp32 when ``dkv_accumulate``.  ``route = (route_k, route_v, rows, tl)``
     (int64 device tables of per-chunk owner addresses) makes the epilogue add each dK/dV tile into its owner's
-    fp32 accumulator over NVLink instead."""
+    fp32 accumulator over NVLink instead.  ``dkv_st`` is the distance between two tokens of ``dk`` / ``dv`` in elements
+    (default: dense)."""
     B, Tq, Hq, D = q.shape
     Tk, Hkv = k.shape[1], k.shape[2]
     st = nv.status_for(q.device)
@@ -70,7 +73,7 @@ def flash_bwd_core(q, k, v, do, lse2, delta, qpos_pad, scale, causal, k_off, dq_
         nv.call("flash_bwd64", nv.ptr(q), nv.ptr(k), nv.ptr(v), nv.ptr(do), nv.ptr(lse2), nv.ptr(delta), nv.ptr(dq_f32),
                 nv.ptr(dk), nv.ptr(dv), nv.i(B), nv.i(Tq), nv.i(Tk), nv.i(Hq), nv.i(Hkv), nv.i(lse2.shape[-1]),
                 nv.l(qs[0]), nv.l(qs[1]), nv.l(qs[2]), nv.l(ks[0]), nv.l(ks[1]), nv.l(ks[2]),
-                nv.f(scale), nv.i(causal), nv.i(k_off), nv.ptr(qpos_pad), nv.i(2 if route is not None else int(dkv_accumulate)),
+                nv.f(scale), nv.i(causal), nv.i(k_off), nv.ptr(qpos_pad), nv.i(2 if route is not None else int(dkv_accumulate)), nv.l(dkv_st or Hkv * D),
                 nv.ptr(route[0] if route else None), nv.ptr(route[1] if route else None),
                 nv.i(route[2] if route else 0), nv.i(route[3] if route else 0), st.ptr(), nv.stream_ptr(q.device))
         return
@@ -78,10 +81,11 @@ def flash_bwd_core(q, k, v, do, lse2, delta, qpos_pad, scale, causal, k_off, dq_
         nv.call("flash_bwd128", nv.ptr(q), nv.ptr(k), nv.ptr(v), nv.ptr(do), nv.ptr(lse2), nv.ptr(delta), nv.ptr(dq_f32),
                 nv.ptr(dk), nv.ptr(dv), nv.i(B), nv.i(Tq), nv.i(Tk), nv.i(Hq), nv.i(Hkv), nv.i(lse2.shape[-1]),
                 nv.l(qs[0]), nv.l(qs[1]), nv.l(qs[2]), nv.l(ks[0]), nv.l(ks[1]), nv.l(ks[2]),
-                nv.f(scale), nv.i(causal), nv.i(k_off), nv.ptr(qpos_pad), nv.i(2 if route is not None else int(dkv_accumulate)),
+                nv.f(scale), nv.i(causal), nv.i(k_off), nv.ptr(qpos_pad), nv.i(2 if route is not None else int(dkv_accumulate)), nv.l(dkv_st or Hkv * D),
                 nv.ptr(route[0] if route else None), nv.ptr(route[1] if route else None),
                 nv.i(route[2] if route else 0), nv.i(route[3] if route else 0), st.ptr(), nv.stream_ptr(q.device))
         return
+    assert dkv_st in (0, Hkv * D), "the general kernel writes dense dK/dV"
     nv.call("flash_bwd", nv.ptr(q), nv.ptr(k), nv.ptr(v), nv.ptr(do), nv.ptr(lse2), nv.ptr(delta), nv.ptr(dq_f32),
             nv.ptr(dk), nv.ptr(dv), nv.i(B), nv.i(Tq), nv.i(Tk), nv.i(Hq), nv.i(Hkv), nv.i(D), nv.i(lse2.shape[-1]),
             nv.l(qs[0]), nv.l(qs[1]), nv.l(qs[2]), nv.l(ks[0]), nv.l(ks[1]), nv.l(ks[2]),
@@ -96,10 +100,7 @@ def cast_to_bf16(x_f32: torch.Tensor, scale: float = 1.0) -> torch.Tensor:
     return out
 
 
-def flash_bwd_cuda(q, k, v, o, lse, do, scale, causal=True, q_pos=None, k_off=0,
-                   dq=None, dk=None, dv=None, dkv_accumulate=False):
-    B, Tq, Hq, D = q.shape
-    Tk, Hkv = k.shape[1], k.shape[2]
+def _launch_ready(q, k, v):
     if not _ok_layout(q):
         q = q.contiguous()
     if not _ok_layout(k):
@@ -108,11 +109,23 @@ def flash_bwd_cuda(q, k, v, o, lse, do, scale, causal=True, q_pos=None, k_off=0,
         v = v.contiguous()
         if v.stride() != k.stride():
             k = k.contiguous()
-    do = do.contiguous()
-    o = o.contiguous()
-    delta, lse2 = flash_bwd_prep(o, do, lse)
-    qpos_pad = padded_q_pos(Tq, q.device, q_pos)
-    dq_f32 = torch.zeros((B, Tq, Hq, D), dtype=torch.float32, device=q.device) if dq is None else dq
+    return q, k, v
+
+
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+def flash_bwd_cuda(q, k, v, o, lse, do, scale, causal=True, q_pos=None, k_off=0,
+                   dq=None, dk=None, dv=None, dkv_accumulate=False):
+    B, Tq, Hq, D = q.shape
+    Tk, Hkv = k.shape[1], k.shape[2]
+    q, k, v = _launch_ready(q, k, v)
+    do, o = _aligned(do), _aligned(o)
+    dq_f32 = torch.empty((B, Tq, Hq, D), dtype=torch.float32, device=q.device) if dq is None else dq
+    qpos_pad = torch.empty((Tq + 127) // 128 * 128, dtype=torch.int32, device=q.device)
+    delta, lse2 = flash_bwd_prep(o, do, lse, dq_f32 if dq is None else None, None if q_pos is None else q_pos.to(torch.int32).contiguous(), qpos_pad)
     if dkv_accumulate:
         assert dk is not None and dv is not None and dk.dtype == torch.float32
     else:
@@ -122,3 +135,26 @@ def flash_bwd_cuda(q, k, v, o, lse, do, scale, causal=True, q_pos=None, k_off=0,
     if dq is None:
         return cast_to_bf16(dq_f32), dk, dv
     return dq_f32, dk, dv
+
+
+def flash_bwd_packed(qkv: torch.Tensor, Hq: int, Hkv: int, o, lse, do, scale: float, causal: bool = True) -> torch.Tensor:
+    """Gradient of packed projections ``qkv [B,T,Hq+2·Hkv,D]`` (query heads, then key heads, then value heads), every part
+    written where it belongs: three separate gradients cost autograd a zero-filled full-size tensor and a copy each, and
+    two full-size additions."""
+    B, T, H, D = qkv.shape
+    q, k, v = qkv[:, :, :Hq], qkv[:, :, Hq:Hq + Hkv], qkv[:, :, Hq + Hkv:]
+    dqkv = torch.empty((B, T, H, D), dtype=torch.bfloat16, device=qkv.device)
+    if D == 64 and _USE_GENERAL_D64:
+        for part, g in zip((dqkv[:, :, :Hq], dqkv[:, :, Hq:Hq + Hkv], dqkv[:, :, Hq + Hkv:]),
+                           flash_bwd_cuda(q, k, v, o, lse, do, scale, causal)):
+            part.copy_(g)
+        return dqkv
+    q, k, v = _launch_ready(q, k, v)
+    do, o = _aligned(do), _aligned(o)
+    dq_f32 = torch.empty((B, T, Hq, D), dtype=torch.float32, device=qkv.device)
+    qpos_pad = torch.empty((T + 127) // 128 * 128, dtype=torch.int32, device=qkv.device)
+    delta, lse2 = flash_bwd_prep(o, do, lse, dq_f32, None, qpos_pad)
+    flash_bwd_core(q, k, v, do, lse2, delta, qpos_pad, scale, causal, 0, dq_f32, dqkv[:, :, Hq:Hq + Hkv], dqkv[:, :, Hq + Hkv:], False,
+                   dkv_st=H * D)
+    nv.call("cast_f32_bf16_rows", nv.ptr(dq_f32), nv.ptr(dqkv), nv.l(B * T), nv.i(Hq * D), nv.l(H * D), nv.f(1.0), nv.stream_ptr(qkv.device))
+    return dqkv

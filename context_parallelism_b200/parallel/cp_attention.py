@@ -163,6 +163,8 @@ class CPAttention:
         cfg = self.cfg
         B, Tl = qkv.shape[:2]
         Hq, Hkv, D = cfg.n_head, cfg.n_kv_head, cfg.head_dim
+        if self.ctx.cp_size == 1:
+            return A.flash_attention_packed(qkv, Hq, Hkv, D, self.scale, True)
         x = qkv.view(B, Tl, Hq + 2 * Hkv, D)
         q, k, v = x[:, :, :Hq], x[:, :, Hq:Hq + Hkv], x[:, :, Hq + Hkv:]
         return self._attend(q, k, v).reshape(B, Tl, Hq * D)

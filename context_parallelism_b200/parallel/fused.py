@@ -461,9 +461,9 @@ def ring_bwd_compute(fc: FusedComm, rb: _RingBuffers, slot: int, q, out, lse, do
     B, Tl, Hq, D = q.shape
     segs = rb.segs(fc, slot)
     nv.call("ring_gather", nv.ptr(segs), nv.i(segs.shape[0]), nv.ptr(rb.ready_bwd), nv.i(_gather_ctas(dev)), nv.stream_ptr(dev))
-    delta, lse2 = AB.flash_bwd_prep(out, do, lse)
-    qpos_pad = AB.padded_q_pos(Tl, dev, pos32)
-    dq = torch.zeros((B, Tl, Hq, D), dtype=torch.float32, device=dev)
+    dq = torch.empty((B, Tl, Hq, D), dtype=torch.float32, device=dev)
+    qpos_pad = torch.empty((Tl + 127) // 128 * 128, dtype=torch.int32, device=dev)
+    delta, lse2 = AB.flash_bwd_prep(out, do, lse, dq, pos32, qpos_pad)
     if fc.dkv_mode == "pull":
         AB.flash_bwd_core(q, rb.gathered[0], rb.gathered[1], do, lse2, delta, qpos_pad, scale, True, 0, dq,
                           rb.dkv_full[0], rb.dkv_full[1], True)

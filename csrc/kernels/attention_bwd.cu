@@ -456,36 +456,49 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
 }
 
-// delta[b,h,t] = sum_d dO*O ; lse2 = lse*log2(e) ; padding rows get delta 0 / lse2 +inf.  One warp per row.
+// delta[b,h,t] = sum_d dO*O ; lse2 = lse*log2(e) ; padding rows get delta 0 / lse2 +inf.  Rows are taken in the order of o and
+// dout, D / 8 lanes with one 16-byte load each per row, so a warp reads 512 contiguous bytes of both.  The same pass
+// clears the fp32 dQ accumulator and pads the query positions, which were four launches of their own.
 template <int D>
 __global__ void bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
                                 const float* __restrict__ lse, float* __restrict__ delta, float* __restrict__ lse2,
+                                float* __restrict__ dq, const int* __restrict__ q_pos, int* __restrict__ q_pos_pad,
                                 int B, int Tq, int Hq, int Tq_pad) {
-  const int lane = threadIdx.x & 31;
+  constexpr int LPR = D / 8;                                 // lanes per row
+  const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (q_pos_pad != nullptr)
+    for (size_t t = tid; t < (size_t)Tq_pad; t += (size_t)gridDim.x * blockDim.x)
+      q_pos_pad[t] = t < (size_t)Tq ? (q_pos != nullptr ? q_pos[t] : (int)t) : 0x7fffffff;
+  const int sub = threadIdx.x % LPR;
   const size_t nrow = (size_t)B * Hq * Tq_pad;
-  for (size_t w = blockIdx.x * (size_t)(blockDim.x >> 5) + (threadIdx.x >> 5); w < nrow; w += (size_t)gridDim.x * (blockDim.x >> 5)) {
-    const int t = (int)(w % Tq_pad);
-    const int h = (int)((w / Tq_pad) % Hq);
-    const int b = (int)(w / ((size_t)Tq_pad * Hq));
+  for (size_t w = tid / LPR; w < nrow; w += (size_t)gridDim.x * blockDim.x / LPR) {   // LPR lanes share a row
+    const int h = (int)(w % Hq);
+    const size_t bt = w / Hq;
+    const int t = (int)(bt % Tq_pad), b = (int)(bt / Tq_pad);
+    const size_t out = ((size_t)b * Hq + h) * Tq_pad + t;
     if (t >= Tq) {
-      if (lane == 0) { if (delta) delta[w] = 0.f; if (lse2) lse2[w] = INFINITY; }
+      if (sub == 0) { if (delta) delta[out] = 0.f; if (lse2) lse2[out] = INFINITY; }
       continue;
     }
+    const size_t off = (((size_t)b * Tq + t) * Hq + h) * D + sub * 8;
     if (delta) {
-      const size_t off = (((size_t)b * Tq + t) * Hq + h) * D;
-      float s = 0.f;
+      const uint4 x = *(const uint4*)(o + off), g = *(const uint4*)(dout + off);
+      float s = bf16_lo(x.x) * bf16_lo(g.x) + bf16_hi(x.x) * bf16_hi(g.x);
+      s += bf16_lo(x.y) * bf16_lo(g.y) + bf16_hi(x.y) * bf16_hi(g.y);
+      s += bf16_lo(x.z) * bf16_lo(g.z) + bf16_hi(x.z) * bf16_hi(g.z);
+      s += bf16_lo(x.w) * bf16_lo(g.w) + bf16_hi(x.w) * bf16_hi(g.w);
+      const uint32_t lanes = (LPR == 32 ? 0xffffffffu : ((1u << LPR) - 1)) << ((threadIdx.x & 31) / LPR * LPR);
 #pragma unroll
-      for (int e = lane * 2; e < D; e += 64) {
-        const uint32_t a = *(const uint32_t*)(o + off + e), g = *(const uint32_t*)(dout + off + e);
-        s += bf16_lo(a) * bf16_lo(g) + bf16_hi(a) * bf16_hi(g);
-      }
-#pragma unroll
-      for (int m = 16; m > 0; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
-      if (lane == 0) delta[w] = s;
+      for (int m = LPR / 2; m > 0; m >>= 1) s += __shfl_xor_sync(lanes, s, m);
+      if (sub == 0) delta[out] = s;
     }
-    if (lse2 && lane == 0) {
+    if (lse2 && sub == 0) {
       const float l = lse[((size_t)b * Hq + h) * Tq + t];
-      lse2[w] = (l == -INFINITY) ? INFINITY : l * 1.4426950408889634f;
+      lse2[out] = (l == -INFINITY) ? INFINITY : l * 1.4426950408889634f;
+    }
+    if (dq) {
+      *(float4*)(dq + off) = make_float4(0.f, 0.f, 0.f, 0.f);
+      *(float4*)(dq + off + 4) = make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
 }
@@ -503,16 +516,20 @@ using namespace cpb;
 
 // o and dout are contiguous [B,Tq,Hq,D]; delta/lse2 are [B,Hq,Tq_pad] with Tq_pad = ceil(Tq/128)*128.
 // Either output may be null (then its inputs are not read): the Ulysses backward computes delta where the
-// tokens live and lse2 where the heads live.
-extern "C" int cpb_flash_bwd_prep(const void* o, const void* dout, const float* lse, float* delta, float* lse2,
-                                  int B, int Tq, int Hq, int D, int Tq_pad, cudaStream_t stream) {
+// tokens live and lse2 where the heads live.  dq (fp32, shaped like o), when given, is set to zero; q_pos_pad [Tq_pad], when
+// given, receives q_pos (int32 [Tq], or 0 .. Tq-1 when null) followed by INT_MAX.
+extern "C" int cpb_flash_bwd_prep(const void* o, const void* dout, const float* lse, float* delta, float* lse2, float* dq,
+                                  const int* q_pos, int* q_pos_pad, int B, int Tq, int Hq, int D, int Tq_pad, cudaStream_t stream) {
+  if (D != 64 && D != 128) return set_error(CPB_ERR_ARG, "flash_bwd_prep: head_dim %d not in {64,128}", D);
+  if ((delta != nullptr && (((uintptr_t)o | (uintptr_t)dout) & 15)) || ((uintptr_t)dq & 15))
+    return set_error(CPB_ERR_ARG, "flash_bwd_prep: tensors must be 16-byte aligned");
+  const size_t rows_per_block = 256 / (D / 8);
   const size_t nrow = (size_t)B * Hq * Tq_pad;
-  size_t g = (nrow + 7) / 8;
-  const size_t cap = (size_t)sm_count() * 16;
+  size_t g = (nrow + rows_per_block - 1) / rows_per_block;
+  const size_t cap = (size_t)sm_count() * 32;
   if (g > cap) g = cap;
-  if (D == 64) bwd_prep_kernel<64><<<(int)g, 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, lse, delta, lse2, B, Tq, Hq, Tq_pad);
-  else if (D == 128) bwd_prep_kernel<128><<<(int)g, 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, lse, delta, lse2, B, Tq, Hq, Tq_pad);
-  else return set_error(CPB_ERR_ARG, "flash_bwd_prep: head_dim %d not in {64,128}", D);
+  auto kern = D == 64 ? bwd_prep_kernel<64> : bwd_prep_kernel<128>;
+  kern<<<(int)g, 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, lse, delta, lse2, dq, q_pos, q_pos_pad, B, Tq, Hq, Tq_pad);
   return check_launch("flash_bwd_prep");
 }
 

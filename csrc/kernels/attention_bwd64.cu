@@ -60,6 +60,7 @@ struct Bwd64Params {
   const float* delta;           // [B,Hq,Tq_pad] rowsum(dO o O), 0 in the padding
   const int* q_pos;             // [Tq_pad] global positions, INT_MAX in the padding
   void* dk; void* dv;           // [B,Tk,Hkv,D] bf16 (store) or fp32 (accumulate)
+  long dkv_st;                  // elements from one token of dk / dv to the next (heads adjacent, batches dense)
   int dkv_mode;                 // 0 bf16 store, 1 fp32 accumulate, 2 routed red.add (fused ring)
   const uint64_t* route_k;      // mode 2: per chunk of route_rows K/V rows the address of its owner's fp32 accumulator
   const uint64_t* route_v;
@@ -393,8 +394,8 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     // final: dK, dV -> global
     if (n_it == 0) {
       if (p.dkv_mode == 0 && k_valid && grp == 0) {
-        __nv_bfloat16* dkr = (__nv_bfloat16*)p.dk + (((size_t)b * p.Tk + kidx) * p.Hkv + hkv) * D;
-        __nv_bfloat16* dvr = (__nv_bfloat16*)p.dv + (((size_t)b * p.Tk + kidx) * p.Hkv + hkv) * D;
+        __nv_bfloat16* dkr = (__nv_bfloat16*)p.dk + ((size_t)b * p.Tk + kidx) * p.dkv_st + hkv * D;
+        __nv_bfloat16* dvr = (__nv_bfloat16*)p.dv + ((size_t)b * p.Tk + kidx) * p.dkv_st + hkv * D;
 #pragma unroll
         for (int c = 0; c < D; c += 8) { *(uint4*)(dkr + c) = make_uint4(0, 0, 0, 0); *(uint4*)(dvr + c) = make_uint4(0, 0, 0, 0); }
       }
@@ -403,7 +404,7 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       ok = __all_sync(0xffffffffu, ok);
       if (ok) {
         tc_fence_after();
-        const size_t off = (((size_t)b * p.Tk + (k_valid ? kidx : 0)) * p.Hkv + hkv) * D;
+        const size_t off = ((size_t)b * p.Tk + (k_valid ? kidx : 0)) * p.dkv_st + hkv * D;
         const int which = grp >> 1;                      // groups 0, 1 drain dK, groups 2, 3 dV: 32 columns each
         const int c = (grp & 1) * 32;
         void* base = which ? p.dv : p.dk;
@@ -513,13 +514,13 @@ static int make_tmap4_64(CUtensorMap* m, const void* ptr, int H, int T, int B, l
 using namespace cpb;
 
 // q, k, v: strided views (element strides: head, token, batch); dout contiguous [B,Tq,Hq,D].
-// dq: fp32 [B,Tq,Hq,D] (accumulated; caller zeroes).  dk/dv: [B,Tk,Hkv,D] bf16 (written) or fp32 (+=).
+// dq: fp32 [B,Tq,Hq,D] (accumulated; caller zeroes).  dk/dv: [B,Tk,Hkv,D] bf16 (written) or fp32 (+=), tokens dkv_st elements apart.
 // lse2 / delta: fp32 [B,Hq,Tq_pad] as produced by cpb_flash_bwd_prep; q_pos: int32 [Tq_pad] (INT_MAX padding), required.
 extern "C" int cpb_flash_bwd64(const void* q, const void* k, const void* v, const void* dout, const float* lse2,
                                 const float* delta, float* dq, void* dk, void* dv,
                                 int B, int Tq, int Tk, int Hq, int Hkv, int Tq_pad,
                                 long q_sh, long q_st, long q_sb, long k_sh, long k_st, long k_sb,
-                                float scale, int causal, int k_off, const int* q_pos, int dkv_mode,
+                                float scale, int causal, int k_off, const int* q_pos, int dkv_mode, long dkv_st,
                                 const uint64_t* route_k, const uint64_t* route_v, int route_rows, int route_tl,
                                 int* status, cudaStream_t stream) {
   if (Hq % Hkv) return set_error(CPB_ERR_ARG, "flash_bwd64: Hq %% Hkv != 0");
@@ -527,6 +528,8 @@ extern "C" int cpb_flash_bwd64(const void* q, const void* k, const void* v, cons
   if (q_pos == nullptr) return set_error(CPB_ERR_ARG, "flash_bwd64: q_pos is required");
   if (((uintptr_t)k | (uintptr_t)v) & 15 || (k_sh | k_st | k_sb) & 7) return set_error(CPB_ERR_ARG, "flash_bwd64: K/V rows must be 16-byte aligned");
   if (((uintptr_t)lse2 | (uintptr_t)delta | (uintptr_t)q_pos) & 15) return set_error(CPB_ERR_ARG, "flash_bwd64: vectors must be 16-byte aligned");
+  if (dkv_mode != 2 && (dkv_st < (long)Hkv * B64_D || (dkv_st & 7) || (((uintptr_t)dk | (uintptr_t)dv) & 15)))
+    return set_error(CPB_ERR_ARG, "flash_bwd64: dK/dV rows must be 16-byte aligned");
   if (dkv_mode == 2 && (route_k == nullptr || route_v == nullptr || route_rows <= 0))
     return set_error(CPB_ERR_ARG, "flash_bwd64: routed dK/dV needs route tables");
   CUtensorMap tq, tk, tdo, tdq;
@@ -544,7 +547,7 @@ extern "C" int cpb_flash_bwd64(const void* q, const void* k, const void* v, cons
   p.B = B; p.Tq = Tq; p.Tk = Tk; p.Hq = Hq; p.Hkv = Hkv; p.Tq_pad = Tq_pad; p.causal = causal; p.k_off = k_off;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v; p.k_sh = k_sh; p.k_st = k_st; p.k_sb = k_sb;
-  p.lse2 = lse2; p.delta = delta; p.q_pos = q_pos; p.dk = dk; p.dv = dv; p.dkv_mode = dkv_mode; p.status = status;
+  p.lse2 = lse2; p.delta = delta; p.q_pos = q_pos; p.dk = dk; p.dv = dv; p.dkv_mode = dkv_mode; p.dkv_st = dkv_st; p.status = status;
   p.route_k = route_k; p.route_v = route_v; p.route_rows = route_rows; p.route_tl = route_tl;
   static const bool skip_dq = [] {
     const char* e = getenv("CPB_BWD_SKIP_DQ");

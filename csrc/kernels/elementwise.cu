@@ -747,6 +747,15 @@ __global__ void cast_f32_bf16_kernel(const float* __restrict__ in, __nv_bfloat16
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     out[i] = __float2bfloat16(in[i] * scale);
 }
+// rows x (8 c8) fp32, dense, into bf16 rows `out_stride` elements apart; eight elements per thread (32 bytes in, 16 out).
+__global__ void cast_f32_bf16_rows_kernel(const float* __restrict__ in, __nv_bfloat16* __restrict__ out, size_t n8, int c8, long out_stride, float scale) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n8; i += (size_t)gridDim.x * blockDim.x) {
+    const size_t r = i / c8;
+    const float4 a = *(const float4*)(in + i * 8), b = *(const float4*)(in + i * 8 + 4);
+    *(uint4*)(out + r * out_stride + (i - r * c8) * 8) =
+        make_uint4(pack_bf16(a.x * scale, a.y * scale), pack_bf16(a.z * scale, a.w * scale), pack_bf16(b.x * scale, b.y * scale), pack_bf16(b.z * scale, b.w * scale));
+  }
+}
 __global__ void cast_bf16_f32_kernel(const __nv_bfloat16* __restrict__ in, float* __restrict__ out, size_t n, float scale, int accumulate) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const float v = __bfloat162float(in[i]) * scale;
@@ -945,8 +954,18 @@ extern "C" int cpb_adamw(float* p, const float* g, float* m, float* v, void* p16
   adamw_kernel<<<grid_for((size_t)n, 256), 256, 0, stream>>>(p, g, m, v, (__nv_bfloat16*)p16, (size_t)n, lr, b1, b2, eps, wd, bc1, bc2, grad_prescale, clip, sumsq, flag);
   return check_launch("adamw");
 }
+extern "C" int cpb_cast_f32_bf16_rows(const float* in, void* out, long rows, int cols, long out_stride, float scale, cudaStream_t stream) {
+  if (rows <= 0 || cols <= 0) return CPB_OK;
+  if (cols % 8 || out_stride % 8 || (((uintptr_t)in | (uintptr_t)out) & 15))
+    return set_error(CPB_ERR_ARG, "cast_f32_bf16_rows: rows must be 16-byte aligned multiples of eight elements");
+  const size_t n8 = (size_t)rows * (cols / 8);
+  cast_f32_bf16_rows_kernel<<<grid_for(n8, 256, 32), 256, 0, stream>>>(in, (__nv_bfloat16*)out, n8, cols / 8, out_stride, scale);
+  return check_launch("cast_f32_bf16_rows");
+}
 extern "C" int cpb_cast_f32_bf16(const float* in, void* out, long n, float scale, cudaStream_t stream) {
   if (n <= 0) return CPB_OK;
+  if (n % 8 == 0 && (((uintptr_t)in | (uintptr_t)out) & 15) == 0)
+    return cpb_cast_f32_bf16_rows(in, out, n / 8, 8, 8, scale, stream);
   cast_f32_bf16_kernel<<<grid_for((size_t)n, 256), 256, 0, stream>>>(in, (__nv_bfloat16*)out, (size_t)n, scale);
   return check_launch("cast_f32_bf16");
 }

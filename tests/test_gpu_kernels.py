@@ -362,3 +362,48 @@ def test_attention_fp32_accurate_variant(D, Hq, Hkv):
     assert_close(lse, lse_ref, cos=0.999999, rel=1e-4, name="fp32 attn lse")
     for got, want, nm in zip((qi.grad, ki.grad, vi.grad), g_ref, ("dq", "dk", "dv")):
         assert_close(got.float(), want, cos=0.9999, rel=2e-2, name="fp32 attn " + nm)
+
+
+# packed projections: every layout the packed gradient is written in (one and several KV heads, an odd number of rows, one row)
+@pytest.mark.parametrize("B,T,Hq,Hkv,D", [(2, 200, 6, 2, 64), (1, 1, 2, 1, 64), (1, 129, 4, 4, 128), (2, 384, 3, 1, 128)])
+def test_packed_attention_matches_separate(B, T, Hq, Hkv, D):
+    """The same kernels either way: the output is equal, gradients differ by the order of the dQ additions only."""
+    from context_parallelism_b200.ops import attention as A
+    torch.manual_seed(5)
+    qkv = torch.randn(B, T, (Hq + 2 * Hkv) * D, device=dev()).bfloat16()
+    do = torch.randn(B, T, Hq * D, device=dev()).bfloat16()
+    a, b = qkv.clone().requires_grad_(), qkv.clone().requires_grad_()
+    out = A.flash_attention_packed(a, Hq, Hkv, D, D ** -0.5)
+    x = b.view(B, T, Hq + 2 * Hkv, D)
+    want, _ = A.flash_attention(x[:, :, :Hq], x[:, :, Hq:Hq + Hkv], x[:, :, Hq + Hkv:], D ** -0.5)
+    out.backward(do)
+    want.backward(do.view(B, T, Hq, D))
+    check_status()
+    assert torch.equal(out, want.view(B, T, Hq * D))
+    nq = Hq * D
+    assert torch.equal(a.grad[..., nq:], b.grad[..., nq:])                      # dK, dV: one writer, fixed order
+    assert_close(a.grad[..., :nq].float(), b.grad[..., :nq].float(), cos=0.99999, rel=4e-3, name="dq")
+
+
+@pytest.mark.parametrize("B,T,H,D,with_pos", [(2, 130, 3, 64, True), (1, 128, 2, 128, False), (1, 1, 1, 64, False)])
+def test_flash_bwd_prep_outputs(B, T, H, D, with_pos):
+    from context_parallelism_b200.ops import attention_bwd as AB
+    torch.manual_seed(6)
+    o, do = (torch.randn(B, T, H, D, device=dev()).bfloat16() for _ in range(2))
+    lse = torch.randn(B, H, T, device=dev())
+    lse[0, 0, T // 2] = -math.inf
+    dq = torch.full((B, T, H, D), 7.0, device=dev())
+    pos = torch.arange(T, device=dev(), dtype=torch.int32) * 3 if with_pos else None
+    pad = (T + 127) // 128 * 128
+    qp = torch.zeros(pad, dtype=torch.int32, device=dev())
+    delta, lse2 = AB.flash_bwd_prep(o, do, lse, dq, pos, qp)
+    assert float(dq.abs().max()) == 0.0
+    assert torch.equal(qp, AB.padded_q_pos(T, dev(), pos))
+    want = (o.double() * do.double()).sum(-1).transpose(1, 2)
+    # fp32 sum of D products of bf16 values: D rounding errors of 2^-24 of the sum of magnitudes
+    bound = (o.double() * do.double()).abs().sum(-1).transpose(1, 2) * D * 2.0 ** -24
+    assert bool(((delta[..., :T].double() - want).abs() <= bound).all())
+    assert bool((delta[..., T:] == 0).all()) and bool((lse2[..., T:] == math.inf).all())
+    finite = lse != -math.inf
+    assert torch.allclose(lse2[..., :T][finite], lse[finite] * 1.4426950408889634, rtol=1e-6)
+    assert bool((lse2[..., :T][~finite] == math.inf).all())
