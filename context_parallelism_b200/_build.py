@@ -12,6 +12,7 @@ from __future__ import annotations
 import concurrent.futures as cf
 import hashlib
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -82,8 +83,42 @@ def _compile_one(src: Path, verbose: bool, ptxas_v: bool) -> Path:
     return obj
 
 
+_CODES = {"int": "i", "int32_t": "i", "long": "l", "int64_t": "l", "float": "f", "double": "d", "size_t": "z",
+          "uint64_t": "z", "cudaStream_t": "p"}
+
+
+def signatures(text: str) -> dict:
+    """``{"cpb_name": "ppiilf..."}`` for every ``extern "C" int cpb_name(...)`` definition in C++ source: one letter per
+    argument (p pointer or stream, i int, l long, f float, d double, z size_t).  The binding declares these to ctypes,
+    which then converts plain Python numbers in C; an argument object of its own for each of the 20 arguments of a
+    launcher cost more host time than the launch."""
+    out = {}
+    for name, args in re.findall(r'extern "C"\s+int\s+(cpb_\w+)\(([^)]*)\)\s*\{', re.sub(r"//[^\n]*", "", text)):
+        code = ""
+        for a in (x.strip() for x in args.split(",")):
+            if a in ("", "void"):
+                continue
+            kind = "p" if "*" in a or "[" in a else _CODES.get(re.sub(r"\bconst\b", "", a).split()[0])
+            if kind is None:
+                raise RuntimeError(f"{name}: no code for argument '{a}'")
+            code += kind
+        out[name] = code
+    return out
+
+
+def _write_signatures(srcs: List[Path]) -> Path:
+    sig = {}
+    for s in srcs:
+        sig.update(signatures(s.read_text()))
+    text = 'extern "C" const char* cpb_signatures() {\n  return "' + " ".join(f"{k}:{v}" for k, v in sorted(sig.items())) + '";\n}\n'
+    out = OBJ_DIR / "signatures.cpp"
+    if not out.exists() or out.read_text() != text:
+        out.write_text(text)
+    return out
+
+
 def sources() -> List[Path]:
-    return sorted(p for p in CSRC.rglob("*") if p.suffix in (".cu", ".cpp") and "build" not in p.parts)
+    return sorted(p for p in CSRC.rglob("*") if p.suffix in (".cu", ".cpp") and "build" not in p.relative_to(CSRC).parts)
 
 
 def build(verbose: bool = False, ptxas_v: bool = False, force: bool = False) -> Path:
@@ -94,6 +129,7 @@ def build(verbose: bool = False, ptxas_v: bool = False, force: bool = False) -> 
         for o in OBJ_DIR.glob("*.o"):
             o.unlink()
     srcs = sources()
+    srcs.append(_write_signatures(srcs))
     with cf.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 4)) as ex:
         objs = list(ex.map(lambda s: _compile_one(s, verbose, ptxas_v), srcs))
     if LIB_PATH.exists() and all(LIB_PATH.stat().st_mtime > o.stat().st_mtime for o in objs):

@@ -11,13 +11,14 @@ from __future__ import annotations
 
 import ctypes
 import os
-from ctypes import c_char_p, c_float, c_int, c_long, c_void_p
+from ctypes import c_char_p, c_double, c_float, c_int, c_long, c_size_t, c_void_p
 from pathlib import Path
 from typing import Optional
 
 import torch
 
 _LIB: Optional[ctypes.CDLL] = None
+_CTYPES = {"p": c_void_p, "i": c_int, "l": c_long, "f": c_float, "d": c_double, "z": c_size_t}
 _LIB_PATH = Path(__file__).resolve().parent / "lib" / "libcpb.so"
 
 
@@ -45,6 +46,11 @@ def lib() -> ctypes.CDLL:
         # libnccl / libcudart are provided by the already-imported torch; load with global symbols visible
         _LIB = ctypes.CDLL(str(_LIB_PATH), mode=ctypes.RTLD_GLOBAL)
         _LIB.cpb_last_error.restype = c_char_p
+        # declared argument types: launchers take plain Python numbers, converted by ctypes in C
+        _LIB.cpb_signatures.restype = c_char_p
+        for entry in _LIB.cpb_signatures().decode().split():
+            name, codes = entry.split(":")
+            getattr(_LIB, name).argtypes = [_CTYPES[c] for c in codes]
     return _LIB
 
 
@@ -54,12 +60,14 @@ def check(rc: int, what: str = "") -> None:
         raise NativeError(f"{what} failed (code {rc}): {msg}")
 
 
-def stream_ptr(device=None) -> c_void_p:
-    return c_void_p(torch.cuda.current_stream(device).cuda_stream)
+def stream_ptr(device=None) -> int:
+    """The calling thread's current stream on ``device`` as an address (no ``torch.cuda.Stream`` object is made)."""
+    idx = None if device is None else (device if isinstance(device, torch.device) else torch.device(device)).index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if idx is None else idx)
 
 
-def ptr(t: Optional[torch.Tensor]) -> c_void_p:
-    return c_void_p(0) if t is None else c_void_p(t.data_ptr())
+def ptr(t: Optional[torch.Tensor]) -> int:
+    return 0 if t is None else t.data_ptr()
 
 
 LAUNCHES = [0]          # number of kernel launchers invoked (each launches exactly one of our kernels)
@@ -68,7 +76,7 @@ _PROFILE = None         # name -> list of (start event, end event) while a per-k
 
 
 def call(name: str, *args) -> None:
-    """Invoke ``cpb_<name>`` with already-converted ctypes arguments and raise on error."""
+    """Invoke ``cpb_<name>`` (argument types as declared by its definition) and raise on error."""
     fn = _FN_CACHE.get(name)
     if fn is None:
         fn = getattr(lib(), "cpb_" + name)
@@ -114,8 +122,8 @@ class KernelStatus:
     def __init__(self, device):
         self.buf = torch.zeros(4, dtype=torch.int32, device=device)
 
-    def ptr(self) -> c_void_p:
-        return c_void_p(self.buf.data_ptr())
+    def ptr(self) -> int:
+        return self.buf.data_ptr()
 
     def check(self, what: str = "kernel") -> None:
         code, site, block, aux = self.buf.tolist()
@@ -129,20 +137,12 @@ _status_cache = {}
 
 
 def status_for(device) -> KernelStatus:
-    key = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
+    dev = device if isinstance(device, torch.device) else torch.device(device)
+    key = dev.index if dev.index is not None else torch.cuda.current_device()
     st = _status_cache.get(key)
     if st is None:
         st = _status_cache[key] = KernelStatus(torch.device("cuda", key))
     return st
 
 
-def f(x) -> c_float:
-    return c_float(float(x))
-
-
-def i(x) -> c_int:
-    return c_int(int(x))
-
-
-def l(x) -> c_long:
-    return c_long(int(x))
+f, i, l = float, int, int

@@ -300,3 +300,22 @@ def test_pair_gemm_band_order_visits_every_tile_once(m_tiles, n_blocks, band):
     # consecutive tiles of a full band share a column of B (rows fastest)
     if m_tiles >= band > 1:
         assert [c[1] for c in got[:band]] == [0] * band and [c[0] for c in got[:band]] == list(range(band))
+
+
+def test_native_signatures_cover_every_launcher():
+    """Argument codes parsed from C definitions, and the table the library was built with covers its launchers."""
+    import ctypes
+    from pathlib import Path
+    from context_parallelism_b200 import _build, _native as nv
+    text = ('// extern "C" int cpb_no(int a) {\nextern "C" int cpb_a(const void* q, int n, long s,\n  const float* x, float f, // t\n  double d,'
+            ' size_t z, const int* p, cudaStream_t st) {')
+    assert _build.signatures(text) == {"cpb_a": "pilpfdzpp"}
+    with pytest.raises(RuntimeError):
+        _build.signatures('extern "C" int cpb_b(short n) {')
+    table = {}
+    for src in _build.sources():
+        table.update(_build.signatures(src.read_text()))
+    lib = nv.lib()
+    built = dict(e.split(":") for e in lib.cpb_signatures().decode().split())
+    assert built == table and "cpb_gemm_bf16" in built
+    assert lib.cpb_gemm_bf16.argtypes[5] is ctypes.c_int and lib.cpb_gemm_bf16.argtypes[0] is ctypes.c_void_p
