@@ -23,46 +23,15 @@
 #include "common.cuh"
 #include <stdio.h>
 #include <stdlib.h>
-#include "host_utils.h"
-#include "ring_copy.cuh"
+#include "attention_fwd.cuh"
 
 namespace cpb {
 
-constexpr int FA_BQ = 128;
-constexpr int FA_BK = 128;
 constexpr int FA_THREADS = 320;
 constexpr int FA_KSTAGES = 3;      // K is wanted one tile ahead of V (the next score tile overlaps the softmax of this one)
 constexpr int FA_VSTAGES = 2;
 constexpr int FA_POLY_D64 = 0;     // default share (of 8) of the exponentials taken off the special-function unit
 constexpr int FA_POLY_D128 = 2;
-
-struct FwdParams {
-  int B, Tq, Tk, Hq, Hkv;
-  int causal;
-  int k_off;                 // global position of K row 0
-  float scale_log2;          // softmax scale * log2(e)
-  const int* q_pos;          // [Tq] global position of each query row, or null (= row index)
-  __nv_bfloat16* O;          // [B,Tq,Hq,D]
-  float* lse;                // [B,Hq,Tq]
-  // fused-ring readiness flags: K/V rows [c*block_rows, (c+1)*block_rows) may be read once
-  // ready[c] >= ready_epoch.  null -> everything is ready.
-  int* ready;
-  int ready_epoch;
-  int block_rows;
-  // fused ring: the first n_copy CTAs (blockIdx.x < n_copy, y = z = 0) pull the K/V blocks listed in segs into
-  // the local position-ordered buffer and bump ready[]; the compute CTAs start on the chunk that holds
-  // their own diagonal (local data) and wrap around while remote chunks land.
-  const CopySeg* segs;
-  int n_segs;
-  int n_copy;
-  // Ulysses: when o_peers != null the epilogue stores each output row straight into the arena of the rank
-  // that owns the token: row qi -> peer qi / o_rows_per_peer, local row qi % o_rows_per_peer, layout
-  // [B, o_rows_per_peer, o_heads_total, D] at byte offset o_off, head slot o_head_off + hq.
-  const uint64_t* o_peers;
-  long o_off;
-  int o_rows_per_peer, o_head_off, o_heads_total;
-  int* status;
-};
 
 // Diagnostics: with -DCPB_FWD_PROF the CTA that owns the last query tile of (head 0, batch 0) records an event
 // timeline of K/V tiles 32..35 into a static device array that the launcher prints.
@@ -83,20 +52,6 @@ struct FwdSmem {
   static constexpr int XCH_OFF = BAR_OFF + 256;            // [2 tiles][2 halves][128 rows] fp32 row-max exchange
   static constexpr int TOTAL = XCH_OFF + 2048 + 1024;
 };
-
-// Bounded acquire-spin on a readiness flag in global memory (written by a copy kernel or a peer).
-__device__ __forceinline__ bool wait_flag_ge(const int* flag, int value, volatile int* abort_flag, int* status, int site) {
-  for (uint32_t it = 0; it < (1u << 22); ++it) {
-    int v;
-    asm volatile("ld.acquire.sys.global.s32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
-    if (v >= value) return true;
-    if (*abort_flag) return false;
-    __nanosleep(200);
-  }
-  *abort_flag = 1;
-  report(status, ST_TIMEOUT_FLAG, site, value);
-  return false;
-}
 
 // POLY: of the 8 column pairs of every 16-column group, the last POLY take exp2_poly_f32x2 and the others ex2.approx.
 template <int D, int POLY>
@@ -505,6 +460,11 @@ extern "C" int cpb_flash_fwd(const void* q, const void* k, const void* v, void* 
   p.o_peers = o_peers; p.o_off = o_off; p.o_rows_per_peer = o_rows_per_peer; p.o_head_off = o_head_off;
   p.o_heads_total = o_heads_total;
   if (p.n_copy > 0 && ready == nullptr) return set_error(CPB_ERR_ARG, "flash_fwd: copy CTAs need ready flags");
+  // Two query tiles per CTA pay when the sweep over the keys is long (one CTA per SM: its start and end are not hidden; 4096
+  // keys, 32/8 heads: 187 us with one tile, 189 to 205 with two; 8192 keys: 646 and 591) and when there are enough CTAs for
+  // their unequal lengths to even out (8192 keys, 8 heads, 256 CTAs: 171 and 163; 12000 keys, 4 heads, 188 CTAs: 191 and 228).
+  const long pairs = (long)((Tq + 2 * FA_BQ - 1) / (2 * FA_BQ)) * Hq * B;
+  if (D == 128 && Tk >= 8192 && Tq > FA_BQ && 2 * pairs >= 3 * sm_count()) return launch_flash_fwd128_pair(tq, tk, tv, p, stream);
   const int G = Hq / Hkv;
   dim3 grid(p.n_copy + ((Tq + FA_BQ - 1) / FA_BQ) * G, Hkv, B);
   // Share of the exponentials computed on the FMA pipe (column pairs out of 8); CPB_FWD_POLY overrides the tuned

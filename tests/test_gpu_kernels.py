@@ -407,3 +407,28 @@ def test_flash_bwd_prep_outputs(B, T, H, D, with_pos):
     finite = lse != -math.inf
     assert torch.allclose(lse2[..., :T][finite], lse[finite] * 1.4426950408889634, rtol=1e-6)
     assert bool((lse2[..., :T][~finite] == math.inf).all())
+
+
+# two query tiles per CTA (long key sequences, many CTAs): ragged query tiles, a zig-zag shard whose tiles see
+# very different spans, an odd key count, and the wrapped sweep with readiness flags
+@pytest.mark.parametrize("Tq,Tk,Hq,Hkv,causal,ring,flags", [
+    (300, 8292, 120, 8, True, 0, False), (129, 8192, 240, 2, False, 0, False), (512, 8192, 120, 4, True, 16, False),
+    (512, 8192, 120, 4, True, 16, True), (1000, 8199, 60, 1, True, 0, False)])
+def test_flash_fwd_d128_pair_kernel(Tq, Tk, Hq, Hkv, causal, ring, flags):
+    from context_parallelism_b200.ops import attention as A, reference as R
+    from context_parallelism_b200.parallel.shard import local_positions
+    torch.manual_seed(12)
+    D = 128
+    q = torch.randn(1, Tq, Hq, D, device=dev()).bfloat16()
+    k, v = (torch.randn(1, Tk, Hkv, D, device=dev()).bfloat16() for _ in range(2))
+    pos = local_positions(Tk, ring, 3, True).to(dev()) if ring else torch.arange(Tk - Tq, Tk, device=dev())
+    extra = {}
+    if flags:
+        rows = Tk // (2 * ring)
+        extra = dict(ready=torch.full((2 * ring,), 5, dtype=torch.int32, device=dev()), ready_epoch=5, block_rows=rows)
+    out, lse = A.flash_fwd(q, k, v, D ** -0.5, causal, pos.int(), **extra)
+    check_status()
+    assert Hq * ((Tq + 255) // 256) * 2 >= 3 * torch.cuda.get_device_properties(0).multi_processor_count      # the rule's side
+    want, wlse = R.attention_dense(q.float(), k.float(), v.float(), D ** -0.5, q_pos=pos, causal=causal)
+    assert_close(out.float(), want, cos=0.9995, rel=3e-2, name="out")
+    assert_close(lse, wlse, cos=0.99999, rel=1e-3, name="lse")
