@@ -6,8 +6,10 @@
 // backward pass; two more GEMMs then produce dX and accumulate dW.  Replaces the reference's
 // materialised logits + sparse_cross_entropy_loss (Scripts/Blutrain/bluscriptCP.cpp:452-459,1712).
 //
-// One CTA per row: pass 1 computes max and sum(exp) online, pass 2 re-reads the row (L2 resident) and
-// writes dlogits.  Rows whose target is negative are ignored (zero gradient, no loss).
+// With gradients the row is read from memory once: a cluster of CTAs keeps it in shared memory between the two passes
+// (xent_smem_kernel).  Without gradients, or when a row does not fit, one CTA per row computes max and sum(exp) online and,
+// if asked to, re-reads the row for dlogits (xent_kernel).  Rows whose target is negative are ignored (zero gradient, no
+// loss).
 #include "common.cuh"
 #include "host_utils.h"
 
@@ -83,6 +85,122 @@ xent_kernel(const float* __restrict__ logits, const int64_t* __restrict__ target
   }
 }
 
+// Bytes of a row that one CTA of a cluster keeps: two such CTAs fit an SM, so one computes while the other's row arrives (four
+// CTAs of half the size and clusters of twice as many: 300 and 805 us at the sizes below).
+constexpr int XE_SEG_BYTES = 104 * 1024;
+constexpr int XE_PARTS = 4;            // bulk copies per segment: the first pass starts when a quarter has arrived
+constexpr int XE_THREADS = 512;
+
+// x, m, s: online softmax over four values at once
+__device__ __forceinline__ void xe_online4(const float4 v, float& m, float& s) {
+  const float mx = fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w));
+  if (mx > m) { s *= __expf(m - mx); m = mx; }
+  s += __expf(v.x - m) + __expf(v.y - m) + __expf(v.z - m) + __expf(v.w - m);
+}
+__device__ __forceinline__ void xe_merge(float& m, float& s, float m2, float s2) {
+  const float mn = fmaxf(m, m2);
+  s = (m == -INFINITY ? 0.f : s * __expf(m - mn)) + (m2 == -INFINITY ? 0.f : s2 * __expf(m2 - mn));
+  m = mn;
+}
+
+// Bound by memory: 4 bytes in and 2 out per logit.  One CTA per row that re-reads the row for the second pass moved 10 bytes
+// instead of 6, because the rows in flight (four per SM, 119 MB at 50304 columns) do not stay in L2.  Here cluster rank r
+// loads columns [r seg, (r+1) seg) with bulk copies, the ranks exchange (max, sum) through distributed shared memory, and
+// the second pass reads shared memory.  Measured, cold L2, one CTA per
+// row -> cluster: 4096 x 50304 323 -> 274 us, 4096 x 128256 808 -> 746, 1000 x 50304 94 -> 78.
+__global__ void __launch_bounds__(XE_THREADS)
+xent_smem_kernel(const float* __restrict__ logits, const int64_t* __restrict__ targets, __nv_bfloat16* __restrict__ dlogits,
+                 float* __restrict__ loss_sum, float* __restrict__ row_loss, int V, int Vcols, int seg, int ranks,
+                 long ld_logits, long ld_dlogits, float grad_scale, int* status) {
+  extern __shared__ __align__(16) float xs[];
+  __shared__ __align__(8) uint64_t bars[XE_PARTS];
+  __shared__ float red_m[XE_THREADS / 32], red_s[XE_THREADS / 32];
+  __shared__ float2 mine;                                          // this rank's (max, sum)
+  __shared__ int abort_flag;
+  const int rank = (int)(blockIdx.x % ranks), row = (int)(blockIdx.x / ranks);
+  const int c0 = rank * seg, n = min(seg, Vcols - c0);             // columns of this rank (a multiple of four)
+  const int part = (n / 4 + XE_PARTS - 1) / XE_PARTS * 4;
+  const float* x = logits + (size_t)row * ld_logits;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < XE_PARTS; ++i) mbar_init(&bars[i], 1);
+    abort_flag = 0;
+    fence_mbar_init();
+    for (int i = 0; i < XE_PARTS; ++i) {
+      const int len = min(part, n - i * part);
+      if (len <= 0) break;
+      mbar_expect_tx(&bars[i], len * 4);
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                   ::"r"(smem_u32(xs + i * part)), "l"((uint64_t)(x + c0 + i * part)), "r"(len * 4), "r"(smem_u32(&bars[i])) : "memory");
+    }
+  }
+  const int64_t tgt = targets[row];
+  __syncthreads();
+  float m = -INFINITY, s = 0.f;
+  bool ok = true;
+  for (int i = 0; i < XE_PARTS && i * part < n; ++i) {
+    ok = ok && mbar_wait(&bars[i], 0, &abort_flag, status, 1210);
+    if (!ok) break;
+    const int end = min((i + 1) * part, n);
+    for (int c = i * part + 4 * (int)threadIdx.x; c < end; c += 4 * XE_THREADS) {
+      const float4 v = *(const float4*)(xs + c);
+      if (c0 + c + 3 < V) {
+        xe_online4(v, m, s);
+      } else {
+        const float e[4] = {v.x, v.y, v.z, v.w};
+        for (int k = 0; k < 4; ++k)
+          if (c0 + c + k < V) {
+            if (e[k] > m) { s *= __expf(m - e[k]); m = e[k]; }
+            s += __expf(e[k] - m);
+          }
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) xe_merge(m, s, __shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, s, o));
+  if (lane == 0) { red_m[warp] = m; red_s[warp] = s; }
+  __syncthreads();
+  if (warp == 0) {
+    m = lane < XE_THREADS / 32 ? red_m[lane] : -INFINITY;
+    s = lane < XE_THREADS / 32 ? red_s[lane] : 0.f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) xe_merge(m, s, __shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, s, o));
+    if (lane == 0) mine = make_float2(m, s);
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  m = -INFINITY; s = 0.f;
+  for (int r = 0; r < ranks; ++r) {
+    uint32_t addr;
+    float m2, s2;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(&mine)), "r"(r));
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(m2), "=f"(s2) : "r"(addr) : "memory");
+    xe_merge(m, s, m2, s2);
+  }
+  asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");    // this thread has read every rank's pair
+  const bool ignore = tgt < 0 || tgt >= V;
+  if (rank == 0 && threadIdx.x == 0) {
+    if (tgt >= V) report(status, ST_BAD_INDEX, 1200, (int)tgt);
+    const float l = ignore ? 0.f : (m + __logf(s) - x[tgt]);
+    if (row_loss) row_loss[row] = l;
+    if (loss_sum && !ignore) atomicAdd(loss_sum, l);
+  }
+  if (ok) {
+    __nv_bfloat16* d = dlogits + (size_t)row * ld_dlogits + c0;
+    const float inv = ignore ? 0.f : grad_scale / s;
+    const int t = ignore || tgt < c0 || tgt >= c0 + n ? -1 : (int)(tgt - c0);
+    for (int c = 4 * (int)threadIdx.x; c < n; c += 4 * XE_THREADS) {
+      const float4 v = *(const float4*)(xs + c);
+      float p0 = c0 + c < V ? __expf(v.x - m) * inv : 0.f, p1 = c0 + c + 1 < V ? __expf(v.y - m) * inv : 0.f;
+      float p2 = c0 + c + 2 < V ? __expf(v.z - m) * inv : 0.f, p3 = c0 + c + 3 < V ? __expf(v.w - m) * inv : 0.f;
+      if ((t & ~3) == c) {
+        if (t == c) p0 -= grad_scale; else if (t == c + 1) p1 -= grad_scale; else if (t == c + 2) p2 -= grad_scale; else p3 -= grad_scale;
+      }
+      *(uint2*)(d + c) = make_uint2(pack_bf16(p0, p1), pack_bf16(p2, p3));
+    }
+  }
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");      // no rank leaves while another may still read its pair
+}
+
 }  // namespace cpb
 
 using namespace cpb;
@@ -94,6 +212,25 @@ extern "C" int cpb_xent(const float* logits, const int64_t* targets, void* dlogi
   if (rows <= 0) return CPB_OK;
   if (Vcols < V || (Vcols % 4)) return set_error(CPB_ERR_ARG, "xent: Vcols must be >= V and a multiple of 4");
   if ((ld_logits % 4) || (dlogits && (ld_dlogits % 4))) return set_error(CPB_ERR_ARG, "xent: row strides must be multiples of 4");
+  // A cluster of up to eight CTAs (the portable limit) holds rows of up to 213000 columns.  Rows that fit one CTA stay with the
+  // kernel below: they are in L2 when it re-reads them (4096 x 8192: 55 us there, 63 us here).
+  const int ranks = (int)(((long)Vcols * 4 + XE_SEG_BYTES - 1) / XE_SEG_BYTES);
+  if (dlogits != nullptr && ranks > 1 && ranks <= 8 && ((uintptr_t)logits & 15) == 0 && ((uintptr_t)dlogits & 7) == 0) {
+    const int seg = (Vcols / 4 + ranks - 1) / ranks * 4;
+    if (seg * (ranks - 1) < Vcols && (long)rows * ranks <= 0x7fffffffL) {
+      static bool cfg = false;
+      if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(xent_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, XE_SEG_BYTES + 64)); cfg = true; }
+      cudaLaunchConfig_t lc = {};
+      lc.gridDim = dim3((unsigned)(rows * ranks)); lc.blockDim = dim3(XE_THREADS); lc.dynamicSmemBytes = (size_t)seg * 4; lc.stream = stream;
+      cudaLaunchAttribute at;
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim.x = ranks; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+      lc.attrs = &at; lc.numAttrs = 1;
+      CPB_CUDA_OK(cudaLaunchKernelEx(&lc, xent_smem_kernel, logits, targets, (__nv_bfloat16*)dlogits, loss_sum, row_loss, V, Vcols, seg, ranks,
+                                     ld_logits, ld_dlogits, grad_scale, status));
+      return check_launch("xent");
+    }
+  }
   xent_kernel<<<rows, 512, 0, stream>>>(logits, targets, (__nv_bfloat16*)dlogits, loss_sum, row_loss, rows, V, Vcols, ld_logits, ld_dlogits, grad_scale, status);
   return check_launch("xent");
 }

@@ -432,3 +432,27 @@ def test_flash_fwd_d128_pair_kernel(Tq, Tk, Hq, Hkv, causal, ring, flags):
     want, wlse = R.attention_dense(q.float(), k.float(), v.float(), D ** -0.5, q_pos=pos, causal=causal)
     assert_close(out.float(), want, cos=0.9995, rel=3e-2, name="out")
     assert_close(lse, wlse, cos=0.99999, rel=1e-3, name="lse")
+
+
+# rows held by one, two, five and eight CTAs, padded columns, an ignored row, a row too wide for a cluster (the other kernel)
+@pytest.mark.parametrize("rows,V,Vc", [(5, 17, 64), (3, 26621, 26624), (2, 50257, 50304), (2, 128256, 128256), (2, 212000, 212992), (2, 220000, 220032)])
+def test_xent_row_widths(rows, V, Vc):
+    from context_parallelism_b200.ops import xent as X
+    torch.manual_seed(3)
+    lg = torch.randn(rows, Vc, device=dev()) * 4
+    tg = torch.randint(0, V, (rows,), device=dev())
+    tg[0], tg[1] = V - 1, -100
+    loss, row_loss = torch.zeros(1, device=dev()), torch.empty(rows, device=dev())
+    d = X.xent_chunk(lg, tg, loss, 0.25, True, row_loss, V)
+    check_status()
+    x = lg[:, :V].double().requires_grad_()
+    want = torch.nn.functional.cross_entropy(x, tg, ignore_index=-100, reduction="none")
+    want.sum().backward()
+    # fp32 exponentials and sums: 2^-21 relative in the sum, absolute in the loss (values up to 30)
+    assert float((row_loss.double() - want).abs().max()) < 2e-5
+    assert abs(float(loss) - float(want.sum())) < 2e-5 * rows
+    g = torch.zeros(rows, Vc, device=dev(), dtype=torch.float64)
+    g[:, :V] = x.grad * 0.25
+    assert float((d.double() - g).abs().max()) <= 0.25 * 2.0 ** -8               # one rounding to bf16 of a value below 0.25
+    assert float((d.double() - g).norm() / g.norm()) < 2.0 ** -8
+    assert bool((d[1] == 0).all()) and bool((d[:, V:] == 0).all())
