@@ -456,3 +456,28 @@ def test_xent_row_widths(rows, V, Vc):
     assert float((d.double() - g).abs().max()) <= 0.25 * 2.0 ** -8               # one rounding to bf16 of a value below 0.25
     assert float((d.double() - g).norm() / g.norm()) < 2.0 ** -8
     assert bool((d[1] == 0).all()) and bool((d[:, V:] == 0).all())
+
+
+# widths around the sizes at which a row changes hands (32, 64, 128, 256, 512 threads), rows that leave a turn of four unfinished
+@pytest.mark.parametrize("layer", [0, 1])
+@pytest.mark.parametrize("rows,d", [(1, 8), (5, 256), (1001, 264), (37, 512), (6, 520), (3, 1024), (2, 1032), (700, 2048), (9, 2056), (4, 4096)])
+def test_norm_bwd_widths(layer, rows, d):
+    from context_parallelism_b200 import _native as nv
+    torch.manual_seed(4)
+    x, dy, dr = (torch.randn(rows, d, device=dev()).bfloat16() for _ in range(3))
+    w = torch.randn(d, device=dev())
+    mean = x.float().mean(1) if layer else torch.zeros(rows, device=dev())
+    rstd = torch.rsqrt(((x.float() - mean[:, None]) ** 2).mean(1) + 1e-5)
+    stats, dx = torch.stack([mean, rstd], 1).contiguous(), torch.empty_like(x)
+    dw, db = torch.ones(d, device=dev()), torch.ones(d, device=dev())
+    nv.call("norm_bwd", nv.ptr(x), nv.ptr(dy), nv.ptr(dr), nv.ptr(w), nv.ptr(stats), nv.ptr(dx), nv.ptr(dw), nv.ptr(db if layer else None),
+            nv.i(rows), nv.i(d), nv.i(layer), nv.stream_ptr(dev()))
+    check_status()
+    xh = (x.double() - mean.double()[:, None]) * rstd.double()[:, None]
+    g = dy.double() * w.double()
+    want = rstd.double()[:, None] * (g - xh * (g * xh).mean(1, keepdim=True) - (g.mean(1, keepdim=True) if layer else 0)) + dr.double()
+    assert float((dx.double() - want).norm() / want.norm()) < 2.0 ** -8            # one rounding to bf16
+    # fp32 sums over the rows: rows + 4 roundings of 2^-24 of the sum of magnitudes
+    for got, term in ((dw, dy.double() * xh), (db, dy.double())) if layer else ((dw, dy.double() * xh),):
+        bound = (term.abs().sum(0) + 1) * (rows + 8) * 2.0 ** -24 + 1e-12
+        assert bool(((got.double() - 1 - term.sum(0)).abs() <= bound).all())
