@@ -288,7 +288,7 @@ def test_flash_bwd_shapes_and_modes(D, B, Tq, Tk, Hq, Hkv, ring, k_off, accumula
 
 @pytest.mark.parametrize("B,Tq,Tk,Hq,Hkv,causal", [(1, 512, 512, 4, 1, True), (2, 300, 712, 2, 2, False), (1, 2048, 2048, 8, 2, True)])
 def test_flash_bwd_d64_kernels_agree(B, Tq, Tk, Hq, Hkv, causal, monkeypatch):
-    """The head_dim-64 kernel (transposed, vectors folded into the MMAs) against the general kernel on the same inputs,
+    """The head_dim-64 kernel (transposed, in two query halves) against the general kernel on the same inputs,
     including the fp32-accumulating dK/dV mode; query positions of a zig-zag shard when causal."""
     from context_parallelism_b200.ops import attention as A, attention_bwd as AB
     from context_parallelism_b200.parallel.shard import local_positions
