@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 from ctypes import c_char_p, c_double, c_float, c_int, c_long, c_size_t, c_void_p
 from pathlib import Path
 from typing import Optional
@@ -18,6 +19,7 @@ from typing import Optional
 import torch
 
 _LIB: Optional[ctypes.CDLL] = None
+_LOAD_LOCK = threading.Lock()
 _CTYPES = {"p": c_void_p, "i": c_int, "l": c_long, "f": c_float, "d": c_double, "z": c_size_t}
 _LIB_PATH = Path(__file__).resolve().parent / "lib" / "libcpb.so"
 
@@ -34,23 +36,36 @@ def available() -> bool:
     return _LIB_PATH.exists()
 
 
+def _declare(handle) -> None:
+    """Declare every launcher's argument types: launchers take plain Python numbers, converted by ctypes in C.  Without the
+    declaration ctypes passes a Python integer as a C ``int``, which cuts a device pointer to 32 bits."""
+    try:
+        handle.cpb_signatures.restype = c_char_p
+    except AttributeError:
+        raise NativeError(f"{_LIB_PATH} was built from other sources (it lacks cpb_signatures); "
+                          "rebuild it: `python -m context_parallelism_b200._build`") from None
+    for entry in handle.cpb_signatures().decode().split():
+        name, codes = entry.split(":")
+        getattr(handle, name).argtypes = [_CTYPES[c] for c in codes]
+    handle.cpb_last_error.restype = c_char_p
+
+
 def lib() -> ctypes.CDLL:
-    """Load (once) and return the native library."""
+    """Load (once) and return the native library.  It is published only when every argument type is declared, so neither a
+    failed load nor a second thread can get at a library whose launchers would take truncated pointers."""
     global _LIB
     if _LIB is None:
-        if not _LIB_PATH.exists():
-            if os.environ.get("CPB_NO_AUTOBUILD", "0") == "1":
-                raise NativeError(f"{_LIB_PATH} is missing; run `python -m context_parallelism_b200._build`")
-            from . import _build
-            _build.build()
-        # libnccl / libcudart are provided by the already-imported torch; load with global symbols visible
-        _LIB = ctypes.CDLL(str(_LIB_PATH), mode=ctypes.RTLD_GLOBAL)
-        _LIB.cpb_last_error.restype = c_char_p
-        # declared argument types: launchers take plain Python numbers, converted by ctypes in C
-        _LIB.cpb_signatures.restype = c_char_p
-        for entry in _LIB.cpb_signatures().decode().split():
-            name, codes = entry.split(":")
-            getattr(_LIB, name).argtypes = [_CTYPES[c] for c in codes]
+        with _LOAD_LOCK:
+            if _LIB is None:
+                if not _LIB_PATH.exists():
+                    if os.environ.get("CPB_NO_AUTOBUILD", "0") == "1":
+                        raise NativeError(f"{_LIB_PATH} is missing; run `python -m context_parallelism_b200._build`")
+                    from . import _build
+                    _build.build()
+                # libnccl / libcudart are provided by the already-imported torch; load with global symbols visible
+                handle = ctypes.CDLL(str(_LIB_PATH), mode=ctypes.RTLD_GLOBAL)
+                _declare(handle)
+                _LIB = handle
     return _LIB
 
 

@@ -319,3 +319,50 @@ def test_native_signatures_cover_every_launcher():
     built = dict(e.split(":") for e in lib.cpb_signatures().decode().split())
     assert built == table and "cpb_gemm_bf16" in built
     assert lib.cpb_gemm_bf16.argtypes[5] is ctypes.c_int and lib.cpb_gemm_bf16.argtypes[0] is ctypes.c_void_p
+
+
+class _StandInLibrary:
+    """The three things ``lib()`` touches; ``cpb_signatures`` may be missing (a library built from older sources) or slow."""
+
+    class _Fn:
+        argtypes = None
+        restype = None
+
+        def __init__(self, result=None, slow=0.0):
+            self.result, self.slow = result, slow
+
+        def __call__(self, *args):
+            import time
+            time.sleep(self.slow)
+            return self.result
+
+    def __init__(self, signatures=True):
+        if signatures:
+            self.cpb_signatures = self._Fn(b"cpb_launch:ppi", 0.05)
+        self.cpb_last_error = self._Fn(b"")
+        self.cpb_launch = self._Fn(0)
+
+
+def test_library_without_signatures_is_never_handed_out(monkeypatch):
+    import ctypes
+    from context_parallelism_b200 import _native as nv
+    monkeypatch.setattr(nv, "_LIB", None)
+    monkeypatch.setattr(ctypes, "CDLL", lambda *a, **k: _StandInLibrary(signatures=False))
+    for _ in range(2):                                  # the second call, too
+        with pytest.raises(nv.NativeError, match="rebuild"):
+            nv.lib()
+
+
+def test_every_thread_gets_a_declared_library(monkeypatch):
+    import ctypes
+    import threading
+    from context_parallelism_b200 import _native as nv
+    loads, seen = [], []
+    monkeypatch.setattr(nv, "_LIB", None)
+    monkeypatch.setattr(ctypes, "CDLL", lambda *a, **k: loads.append(1) or _StandInLibrary())
+    threads = [threading.Thread(target=lambda: seen.append(nv.lib().cpb_launch.argtypes)) for _ in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(loads) == 1 and seen == [[ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int]] * 8
