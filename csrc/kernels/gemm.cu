@@ -246,7 +246,7 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       if (!ok) break;
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
-      gemm_epilogue<BN>(p, &tmC, &tmX, ws, t_row, row0, nb, lane, [&] {
+      gemm_epilogue<BN>(p, &tmC, &tmX, ws, t_row, row0, nb, lane, item < num_tiles ? p.bias : nullptr, [&] {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {

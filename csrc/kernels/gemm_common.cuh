@@ -19,7 +19,7 @@ constexpr int GEMM_THREADS = 192;
 enum : int {
   EPI_BF16 = 0,        // C(bf16) = acc (+bias)
   EPI_F32 = 1,         // C(f32)  = acc (+bias)
-  EPI_F32_ACC = 2,     // C(f32) += acc
+  EPI_F32_ACC = 2,     // C(f32) += acc (+bias)
   EPI_BF16_GELU = 3,   // C(bf16) = gelu_tanh(acc + bias); aux(bf16) = acc + bias (pre-activation) when aux != null
   EPI_BF16_SWIGLU = 4, // B tile = [gate rows | up rows]; C(bf16)[:, n] = silu(g)*u ; aux gets [g | u] when aux != null
 };
@@ -112,11 +112,12 @@ __device__ __forceinline__ void pack_row(const float (&f)[64], uint32_t (&v)[32]
 }
 
 // Epilogue of one 32-row slice of a 128 x BN accumulator tile: `t_row` is the tensor-memory address of this warp's lanes at
-// the accumulator's first column, `row0` the slice's first output row, `nb` the tile's index along N.  `release` runs as
-// soon as the accumulator has been read.
+// the accumulator's first column, `row0` the slice's first output row, `nb` the tile's index along N, `bias` what to add (null
+// for every split along K but the first: the splits of a tile are summed).  `release` runs as soon as the accumulator has
+// been read.
 template <int BN, class Release>
 __device__ __forceinline__ void gemm_epilogue(const GemmParams& p, const CUtensorMap* tmC, const CUtensorMap* tmX, WarpStore& ws,
-                                              uint32_t t_row, int row0, int nb, int lane, Release release) {
+                                              uint32_t t_row, int row0, int nb, int lane, const float* bias, Release release) {
   const bool live = row0 < p.M;
   if (p.epi == EPI_BF16_SWIGLU) {
     // accumulator columns [0, BN/2) = gate, [BN/2, BN) = up, for features f0 .. f0 + BN/2
@@ -158,13 +159,13 @@ __device__ __forceinline__ void gemm_epilogue(const GemmParams& p, const CUtenso
       tmem_wait_ld();
       if (c + 32 == BN) release();
       if (!live || col >= p.N) continue;
-      if (p.bias != nullptr) {
+      if (bias != nullptr) {
 #pragma unroll
         for (int j = 0; j < 32; j += 8)
           if (col + j < p.N) {                 // N is a multiple of 8
 #pragma unroll
             for (int q = 0; q < 8; q += 4) {
-              const float4 b = __ldg((const float4*)(p.bias + col + j + q));
+              const float4 b = __ldg((const float4*)(bias + col + j + q));
               v[j + q] = __float_as_uint(__uint_as_float(v[j + q]) + b.x);
               v[j + q + 1] = __float_as_uint(__uint_as_float(v[j + q + 1]) + b.y);
               v[j + q + 2] = __float_as_uint(__uint_as_float(v[j + q + 2]) + b.z);
@@ -186,13 +187,13 @@ __device__ __forceinline__ void gemm_epilogue(const GemmParams& p, const CUtenso
       tmem_wait_ld();
       if (c + 64 == BN) release();
       if (!live || col >= p.N) continue;
-      if (p.bias != nullptr) {
+      if (bias != nullptr) {
 #pragma unroll
         for (int j = 0; j < 64; j += 8)
           if (col + j < p.N) {
 #pragma unroll
             for (int q = 0; q < 8; q += 4) {
-              const float4 b = __ldg((const float4*)(p.bias + col + j + q));
+              const float4 b = __ldg((const float4*)(bias + col + j + q));
               f[j + q] += b.x; f[j + q + 1] += b.y; f[j + q + 2] += b.z; f[j + q + 3] += b.w;
             }
           }

@@ -114,6 +114,19 @@ def test_gemm_tile_edges_every_epilogue(M, N, K):
     check_status()
 
 
+@pytest.mark.parametrize("M,N,K", [(384, 384, 8192), (512, 768, 384), (2048, 1024, 64)])      # split along K, split in two, not split
+def test_gemm_accumulate_adds_the_bias_once(M, N, K):
+    from context_parallelism_b200.ops import gemm as G
+    torch.manual_seed(18)
+    A, B = torch.randn(M, K, device=dev()).bfloat16(), torch.randn(N, K, device=dev()).bfloat16()
+    bias, acc = 100 * torch.randn(N, device=dev()), torch.randn(M, N, device=dev())
+    want = acc.double() + A.double() @ B.double().t() + bias.double()
+    G.gemm(A, B, out=acc, accumulate=True, bias=bias)
+    check_status()
+    # K products of unit normals in fp32: about sqrt(K) * 2^-24 * sqrt(K); two more roundings of values up to 500
+    assert float((acc.double() - want).abs().max()) < 1e-6 * K + 2e-4
+
+
 def test_linear_autograd():
     from context_parallelism_b200.ops.gemm import linear, linear_swiglu, linear_gelu
     torch.manual_seed(2)
