@@ -13,6 +13,7 @@ On CPU tensors the same functions run plain PyTorch (oracle path).
 """
 from __future__ import annotations
 
+import functools
 from typing import Optional
 
 import torch
@@ -32,13 +33,19 @@ def _rowmajor2d(t: torch.Tensor) -> torch.Tensor:
     return t
 
 
+@functools.lru_cache(maxsize=4096)
+def acc_splits(M: int, N: int, K: int) -> int:
+    """Into how many ranges of K the kernel's plan splits an accumulating GEMM of this shape."""
+    return nv.lib().cpb_gemm_splits(M, N, K)
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
          out: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torch.bfloat16,
          accumulate: bool = False, bias: Optional[torch.Tensor] = None, epi: Optional[int] = None,
          aux: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``C[M,N] (+)= A·B``.  ``a`` is ``[M,K]`` (or ``[K,M]`` when ``a_mn``), ``b`` is ``[N,K]``
     (or ``[K,N]`` when ``b_mn``); both bf16.  For ``epi == EPI_BF16_SWIGLU`` ``b`` is the fused
-    ``[2F,K]`` weight and the result has ``F`` columns."""
+    ``[2F,K]`` weight and the result has ``F`` columns.  The result of every call repeats bit for bit."""
     assert a.is_cuda and a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
     a = _rowmajor2d(a)
     b = _rowmajor2d(b)
@@ -60,10 +67,15 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         bias = bias.float().contiguous()
         if bias.data_ptr() % 16:
             bias = bias.clone()
+    # A split accumulation adds its partial tiles in a fixed order in a launch of its own, from a workspace of this call.
+    splits, part = (acc_splits(M, N, K) if epi == EPI_F32_ACC else 1), None
+    if splits > 1:
+        part = torch.empty((splits - 1) * M * N, dtype=torch.float32, device=a.device)
+        nv.LAUNCHES[0] += 1
     nv.call("gemm_bf16", nv.ptr(a), nv.ptr(b), nv.ptr(out), nv.ptr(aux), nv.ptr(bias),
             nv.i(M), nv.i(N), nv.i(K), nv.i(a.stride(0)), nv.i(b.stride(0)), nv.i(out.stride(0)),
             nv.i(aux.stride(0) if aux is not None else 0), nv.i(a_mn), nv.i(b_mn), nv.i(epi),
-            st.ptr(), nv.stream_ptr(a.device))
+            nv.ptr(part), splits, st.ptr(), nv.stream_ptr(a.device))
     return out
 
 

@@ -246,7 +246,7 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       if (!ok) break;
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
-      gemm_epilogue<BN>(p, &tmC, &tmX, ws, t_row, row0, nb, lane, item < num_tiles ? p.bias : nullptr, [&] {
+      gemm_epilogue<BN>(p, &tmC, &tmX, ws, t_row, row0, nb, lane, item / num_tiles, [&] {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
@@ -290,30 +290,59 @@ static int dispatch_pair(const CUtensorMap (&tm)[4], const GemmParams& p, int a_
   return launch_pair<BN, true, true>(tm, p, stream);
 }
 
+// C += partials[0] + partials[1] + ..., always in that order and after the first split has been added, so that a weight gradient
+// repeats bit for bit (all splits adding to C in L2 as they finish, in one launch, do not).  Launched while the GEMM drains
+// (programmatic dependent launch); griddepcontrol.wait returns once the GEMM is complete and its writes are visible.
+__global__ void __launch_bounds__(256)
+gemm_add_partials_kernel(float* __restrict__ C, const float4* __restrict__ partials, unsigned n4, unsigned total4, long ldc, int count) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total4; i += gridDim.x * blockDim.x) {
+    const unsigned r = i / n4;
+    float4* dst = (float4*)(C + r * ldc) + (i - r * n4);
+    const float4 c = *dst;
+    float4 a = partials[i];
+#pragma unroll 4
+    for (int s = 1; s < count; ++s) {
+      const float4 v = partials[(size_t)s * total4 + i];
+      a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+    }
+    *dst = make_float4(c.x + a.x, c.y + a.y, c.z + a.z, c.w + a.w);
+  }
+}
+
 // Tile width and K split.  The work items of a launch (tiles x splits) run on 74 pairs, so the time is that of the pair
 // with the most items: items / 74 rounded up, each the longer of its main loop and its epilogue, plus one epilogue at the
 // end.  Nanoseconds, measured: main loop per 64 of K 370 at 256 columns (8192^3: 694 us) and 240 at 128 columns (892 us),
-// so narrow tiles pay only where they fill a wave (M 4096, N 384, K 50304: 238 us at 256 columns, 182 at 128).  Only the
-// accumulating epilogue is split, because its partial sums are added in L2 by the stores themselves: M 384, N 384, K 8192
-// 47 us unsplit, 14 us in 12 splits; but every further split moves the fp32 matrix once more (M 16384, N 2048, K 8192:
-// 372 us unsplit, 443 us in four), charged at 8 TB/s.
-static void plan_tiles(int M, int N, int K, int epi, int has_aux, int& bn, int& splits) {
+// so narrow tiles pay only where they fill a wave (M 4096, N 384, K 50304: 238 us at 256 columns, 182 at 128).
+//
+// Only the accumulating epilogue is split: all splits but the first go through a workspace of at most 128 MB, and a second
+// launch adds them in a fixed order.  On the GPU that costs 1.4 us and, per split, a write and a read of the fp32 matrix in L2 at
+// about 16 TB/s (M 3072, N 2048, K 8192: 106 us unsplit, 86 in two; M 384, N 384, K 8192: 36.6 unsplit, 22.6 in two, 11.7 in
+// twelve; M 2048, N 2048, K 8192: 50 unsplit, 57 in two); the host pays 4 us for the launch and the workspace.  So a split has to
+// save 8 us: with 1.4 us as the bar the small training steps, which wait for the host, were 1 to 3 % slower, and without any
+// split 1 to 2 %.  All splits adding to C in L2 from one launch took 9.0 us in twelve and 75.7 in two, but in the order in
+// which they finished: weight gradients did not repeat.
+// With all pairs on narrow tiles their operands come to 15 TB/s out of L2 and 64 of K takes 290 instead of 240 (M 3072, N 768,
+// K 4096: 24 us, against 22 in two splits of wide tiles).
+// `want` > 0 asks for the best width at that many splits, 0 for the best of both.
+static void plan_tiles(int M, int N, int K, int epi, int has_aux, int want, int& bn, int& splits) {
   const long nk = (K + GEMM_BK - 1) / GEMM_BK;
   const long m_tiles = (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM), pairs = sm_count() > 1 ? sm_count() / 2 : 1;
-  const long per_split = (long)M * N * 8 / 8000;
+  const long pass = (long)M * N * 8 / 16000;
   long best = -1;
   for (int cand = 256; cand >= 128; cand -= 128) {
     const int per_tile = epi == EPI_BF16_SWIGLU ? cand / 2 : cand;
     const long tiles = m_tiles * ((N + per_tile - 1) / per_tile);
-    const long ck = cand == 256 ? 370 : 240;
     long ce = epi == EPI_F32 || epi == EPI_F32_ACC ? 1200 : epi == EPI_BF16_GELU ? (has_aux ? 1600 : 1400) : epi == EPI_BF16_SWIGLU ? (has_aux ? 1300 : 1000) : 650;
     if (cand == 128) ce = ce / 2 + 50;
-    const long max_split = epi == EPI_F32_ACC ? (nk + 3) / 4 : 1;     // at least four K blocks per item
-    for (long s = 1; s <= max_split && (s == 1 || tiles * s <= pairs * 16); ++s) {
+    const long max_split = want > 0 ? want : epi == EPI_F32_ACC ? (nk + 3) / 4 : 1;     // at least four K blocks per item
+    for (long s = want > 0 ? want : 1; s <= max_split && (s == 1 || want > 0 || (s - 1) * (long)M * N <= (32L << 20)); ++s) {
       const long kps = (nk + s - 1) / s;
       if ((nk + kps - 1) / kps != s) continue;                       // the same items as a smaller split
-      const long waves = (tiles * s + pairs - 1) / pairs, main = kps * ck;
-      const long t = waves * (main > ce ? main : ce) + (main > ce ? ce : main) + (s - 1) * per_split;
+      const long waves = (tiles * s + pairs - 1) / pairs, busy = tiles * s < pairs ? tiles * s : pairs;
+      const long main = kps * (cand == 256 ? 370 : epi == EPI_F32_ACC ? 240 + 50 * busy / pairs : 240);
+      long t = waves * (main > ce ? main : ce) + (main > ce ? ce : main);
+      if (s > 1) t += 8000 + (s + 1) * pass;                         // 1.4 us and what a split has to save
       if (best < 0 || t < best) { best = t; bn = cand; splits = (int)s; }
     }
   }
@@ -326,9 +355,11 @@ using namespace cpb;
 // A: bf16, [M,K] row stride lda (a_mn=0) or [K,M] row stride lda (a_mn=1).
 // B: bf16, [N,K] row stride ldb (b_mn=0) or [K,N] row stride ldb (b_mn=1).
 // epi: see EPI_* above.  For EPI_BF16_SWIGLU B is the fused [2F, K] weight, N = F output features.
+// splits > 1 (accumulating epilogue only, see cpb_gemm_splits): K is split that often; partials is a workspace of
+// (splits - 1) * M * N floats, 16-byte aligned, and a second launch adds it to C.
 extern "C" int cpb_gemm_bf16(const void* A, const void* B, void* C, void* aux, const float* bias,
                              int M, int N, int K, int lda, int ldb, int ldc, int ld_aux,
-                             int a_mn, int b_mn, int epi, int* status, cudaStream_t stream) {
+                             int a_mn, int b_mn, int epi, float* partials, int splits, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return set_error(CPB_ERR_ARG, "gemm: empty problem %dx%dx%d", M, N, K);
   // the contiguous dimension of every operand and every row stride must be a multiple of 8 elements (16 bytes)
   if ((N % 8) || (lda % 8) || (ldb % 8)) return set_error(CPB_ERR_ARG, "gemm: N,lda,ldb must be multiples of 8 (got N=%d lda=%d ldb=%d)", N, lda, ldb);
@@ -337,8 +368,16 @@ extern "C" int cpb_gemm_bf16(const void* A, const void* B, void* C, void* aux, c
   if (epi == EPI_BF16_SWIGLU && (a_mn || b_mn)) return set_error(CPB_ERR_ARG, "gemm: swiglu epilogue needs K-major operands");
   if (bias != nullptr && ((uintptr_t)bias & 15)) return set_error(CPB_ERR_ARG, "gemm: bias must be 16-byte aligned");
   if (epi != EPI_BF16_GELU && epi != EPI_BF16_SWIGLU) aux = nullptr;
-  int bn = 256, splits = 1;
-  plan_tiles(M, N, K, epi, aux != nullptr, bn, splits);
+  if (splits < 1) splits = 1;
+  {
+    const int nk = (K + GEMM_BK - 1) / GEMM_BK, kps = (nk + splits - 1) / splits;
+    if (splits > 1 && (epi != EPI_F32_ACC || partials == nullptr || ((uintptr_t)partials & 15) || (nk + kps - 1) / kps != splits))
+      return set_error(CPB_ERR_ARG, "gemm: %d splits of K=%d need the accumulating epilogue and a 16-byte aligned workspace", splits, K);
+    if (splits > 1 && (((uintptr_t)C & 15) || (ldc & 3) || (long)M * N >= (1L << 32)))
+      return set_error(CPB_ERR_ARG, "gemm: a split C must have 16-byte aligned rows and less than 2^32 elements");
+  }
+  int bn = 256;
+  plan_tiles(M, N, K, epi, aux != nullptr, splits, bn, splits);
   GemmParams p;
   p.M = M; p.N = N; p.K = K; p.epi = epi;
   p.num_m_tiles = (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM);
@@ -387,6 +426,28 @@ extern "C" int cpb_gemm_bf16(const void* A, const void* B, void* C, void* aux, c
     uint32_t box[2] = {64, 32};
     if ((rc = encode_tmap(&tm[3], aux, 2, 2, dims, strides, box, 1)) != CPB_OK) return rc;
   }
-  if (bn == 256) return dispatch_pair<256>(tm, p, a_mn, b_mn, stream);
-  return dispatch_pair<128>(tm, p, a_mn, b_mn, stream);
+  if (splits > 1) {
+    uint64_t dims[3] = {(uint64_t)N, (uint64_t)M, (uint64_t)(splits - 1)}, strides[3] = {0, (uint64_t)N * 4, (uint64_t)M * N * 4};
+    uint32_t box[3] = {32, 32, 1};
+    if ((rc = encode_tmap(&tm[3], partials, 4, 3, dims, strides, box, 1)) != CPB_OK) return rc;
+  }
+  rc = bn == 256 ? dispatch_pair<256>(tm, p, a_mn, b_mn, stream) : dispatch_pair<128>(tm, p, a_mn, b_mn, stream);
+  if (rc != CPB_OK || splits == 1) return rc;
+  const unsigned total4 = (unsigned)((long)M * N / 4);
+  const unsigned blocks = (total4 + 255) / 256, cap = (unsigned)sm_count() * 8;
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(blocks < cap ? blocks : cap); lc.blockDim = dim3(256); lc.stream = stream;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = &at; lc.numAttrs = 1;
+  CPB_CUDA_OK(cudaLaunchKernelEx(&lc, gemm_add_partials_kernel, (float*)C, (const float4*)partials, (unsigned)N / 4, total4, (long)ldc, splits - 1));
+  return check_launch("gemm_add_partials");
+}
+
+// How often the accumulating GEMM of this shape should split K (at least 1): the caller brings the workspace.
+extern "C" int cpb_gemm_splits(int M, int N, int K) {
+  int bn = 256, splits = 1;
+  if (M > 0 && N > 0 && K > 0) plan_tiles(M, N, K, EPI_F32_ACC, 0, 0, bn, splits);
+  return splits;
 }

@@ -28,7 +28,8 @@ struct GemmParams {
   int M, N, K;
   int epi;
   int num_m_tiles, num_n_blocks, num_k_blocks;
-  int splits, k_per_split;   // split-K (accumulating epilogue only): 64-wide K blocks per work item
+  int splits, k_per_split;   // split-K (accumulating epilogue only): 64-wide K blocks per work item.  The first split
+                             // adds to C, the others go to a workspace [splits - 1][M][N] for gemm_add_partials_kernel
   int swiglu_half;     // number of output features F when epi == SWIGLU (B has 2F rows)
   int band;            // pair-rows per band of the tile order (1 = rows of tiles, columns fastest)
   int has_aux;
@@ -112,13 +113,13 @@ __device__ __forceinline__ void pack_row(const float (&f)[64], uint32_t (&v)[32]
 }
 
 // Epilogue of one 32-row slice of a 128 x BN accumulator tile: `t_row` is the tensor-memory address of this warp's lanes at
-// the accumulator's first column, `row0` the slice's first output row, `nb` the tile's index along N, `bias` what to add (null
-// for every split along K but the first: the splits of a tile are summed).  `release` runs as soon as the accumulator has
-// been read.
+// the accumulator's first column, `row0` the slice's first output row, `nb` the tile's index along N, `split` its range of K (the
+// first one brings the bias).  `release` runs as soon as the accumulator has been read.
 template <int BN, class Release>
 __device__ __forceinline__ void gemm_epilogue(const GemmParams& p, const CUtensorMap* tmC, const CUtensorMap* tmX, WarpStore& ws,
-                                              uint32_t t_row, int row0, int nb, int lane, const float* bias, Release release) {
+                                              uint32_t t_row, int row0, int nb, int lane, int split, Release release) {
   const bool live = row0 < p.M;
+  const float* bias = split == 0 ? p.bias : nullptr;
   if (p.epi == EPI_BF16_SWIGLU) {
     // accumulator columns [0, BN/2) = gate, [BN/2, BN) = up, for features f0 .. f0 + BN/2
 #pragma unroll 1
@@ -174,7 +175,8 @@ __device__ __forceinline__ void gemm_epilogue(const GemmParams& p, const CUtenso
           }
       }
       ws.fill(ws.row_ptr(lane), lane, v);
-      if (p.epi == EPI_F32_ACC) ws.add(tmC, col, row0);
+      if (split > 0) ws.store3(tmX, col, row0, split - 1);
+      else if (p.epi == EPI_F32_ACC) ws.add(tmC, col, row0);
       else ws.store(tmC, col, row0);
     }
   } else {

@@ -321,6 +321,18 @@ def test_native_signatures_cover_every_launcher():
     assert lib.cpb_gemm_bf16.argtypes[5] is ctypes.c_int and lib.cpb_gemm_bf16.argtypes[0] is ctypes.c_void_p
 
 
+@pytest.mark.parametrize("seed", range(4))
+def test_split_plan_of_the_accumulating_gemm(seed):
+    """Every split the plan names is one the launcher accepts (no empty range of K) and its workspace stays within 128 MB."""
+    import random
+    from context_parallelism_b200.ops.gemm import acc_splits
+    rng = random.Random(seed)
+    shapes = [(8, 8, 8), (8, 8, 1 << 20), (128256, 4096, 64)] + [tuple(8 * rng.randint(1, 1 << rng.randint(1, 13)) for _ in range(3)) for _ in range(200)]
+    for M, N, K in shapes:
+        s, nk = acc_splits(M, N, K), -(-K // 64)
+        assert s >= 1 and -(-nk // -(-nk // s)) == s and (s == 1 or nk >= 4 * (s - 1)) and 4 * (s - 1) * M * N <= 128 << 20
+
+
 class _StandInLibrary:
     """The three things ``lib()`` touches; ``cpb_signatures`` may be missing (a library built from older sources) or slow."""
 

@@ -114,7 +114,7 @@ def test_gemm_tile_edges_every_epilogue(M, N, K):
     check_status()
 
 
-@pytest.mark.parametrize("M,N,K", [(384, 384, 8192), (512, 768, 384), (2048, 1024, 64)])      # split along K, split in two, not split
+@pytest.mark.parametrize("M,N,K", [(384, 384, 8192), (768, 768, 4096), (2048, 1024, 64)])      # twelve splits along K, four, none
 def test_gemm_accumulate_adds_the_bias_once(M, N, K):
     from context_parallelism_b200.ops import gemm as G
     torch.manual_seed(18)
@@ -125,6 +125,21 @@ def test_gemm_accumulate_adds_the_bias_once(M, N, K):
     check_status()
     # K products of unit normals in fp32: about sqrt(K) * 2^-24 * sqrt(K); two more roundings of values up to 500
     assert float((acc.double() - want).abs().max()) < 1e-6 * K + 2e-4
+
+
+@pytest.mark.parametrize("M,N,K", [(384, 384, 8192), (1152, 384, 4096), (640, 392, 4104)])
+def test_gemm_accumulate_repeats_bit_for_bit(M, N, K):
+    """Weight gradients whose K range is split are added in a fixed order."""
+    from context_parallelism_b200.ops import gemm as G
+    torch.manual_seed(19)
+    A, B = torch.randn(K, M, device=dev()).bfloat16(), torch.randn(K, N, device=dev()).bfloat16()
+    start, runs = torch.randn(M, N, device=dev()), []
+    for _ in range(20):
+        acc = start.clone()
+        G.gemm(A, B, a_mn=True, b_mn=True, out=acc, accumulate=True)
+        runs.append(acc)
+    check_status()
+    assert all(torch.equal(r, runs[0]) for r in runs)
 
 
 def test_linear_autograd():
