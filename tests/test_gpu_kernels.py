@@ -142,6 +142,26 @@ def test_gemm_accumulate_repeats_bit_for_bit(M, N, K):
     assert all(torch.equal(r, runs[0]) for r in runs)
 
 
+def test_gemm_activation_epilogues_over_the_range():
+    """SwiGLU and GELU of single values from -80 to 80: one column of A times a row of ones gives every value exactly.  The bound
+    is one rounding to bf16 (half a step of 8 significant bits, 2^-8) and a hundred fp32 ones (the exponential of 80); GELU is taken as 0.5 x (1 + tanh) in fp32, so its negative side
+    is good to a few 2^-24 of x only."""
+    from context_parallelism_b200.ops import gemm as G
+    x = torch.linspace(-80, 80, 2048, device=dev()).bfloat16()
+    A = torch.zeros(2048, 64, device=dev()).bfloat16()
+    A[:, 0], A[:, 1] = x, 1.0
+    W = torch.zeros(32, 64, device=dev()).bfloat16()
+    W[:16, 0], W[16:, 1] = 1.0, 1.0                                    # gate = x, up = 1
+    xd = x.double()
+    sw = G.gemm(A, W, epi=G.EPI_BF16_SWIGLU)[:, 3].double()
+    want = xd * torch.sigmoid(xd)
+    assert bool(((sw - want).abs() <= want.abs() * (2.0 ** -8 + 2.0 ** -16)).all())
+    ge = G.gemm(A, W[:16], epi=G.EPI_BF16_GELU)[:, 3].double()
+    want = torch.nn.functional.gelu(xd, approximate="tanh")
+    assert bool(((ge - want).abs() <= want.abs() * (2.0 ** -8 + 2.0 ** -16) + xd.abs() * 2.0 ** -21).all())
+    check_status()
+
+
 def test_linear_autograd():
     from context_parallelism_b200.ops.gemm import linear, linear_swiglu, linear_gelu
     torch.manual_seed(2)
