@@ -460,16 +460,17 @@ extern "C" int cpb_flash_fwd(const void* q, const void* k, const void* v, void* 
   p.o_peers = o_peers; p.o_off = o_off; p.o_rows_per_peer = o_rows_per_peer; p.o_head_off = o_head_off;
   p.o_heads_total = o_heads_total;
   if (p.n_copy > 0 && ready == nullptr) return set_error(CPB_ERR_ARG, "flash_fwd: copy CTAs need ready flags");
+  // Share of the exponentials computed on the FMA pipe (column pairs out of 8); CPB_FWD_POLY overrides the tuned
+  // default and is read once.
+  static const int poly_env = [] { const char* e = getenv("CPB_FWD_POLY"); return e ? atoi(e) : -1; }();
+  const int poly = poly_env < 0 ? (D == 64 ? FA_POLY_D64 : FA_POLY_D128) : poly_env;
   // Two query tiles per CTA pay when the sweep over the keys is long (one CTA per SM: its start and end are not hidden; 4096
   // keys, 32/8 heads: 187 us with one tile, 189 to 205 with two; 8192 keys: 646 and 591) and when there are enough CTAs for
   // their unequal lengths to even out (8192 keys, 8 heads, 256 CTAs: 171 and 163; 12000 keys, 4 heads, 188 CTAs: 191 and 228).
   const long pairs = (long)((Tq + 2 * FA_BQ - 1) / (2 * FA_BQ)) * Hq * B;
-  if (D == 128 && Tk >= 8192 && Tq > FA_BQ && 2 * pairs >= 3 * sm_count()) return launch_flash_fwd128_pair(tq, tk, tv, p, stream);
+  if (D == 128 && Tk >= 8192 && Tq > FA_BQ && 2 * pairs >= 3 * sm_count()) return launch_flash_fwd128_pair(poly, tq, tk, tv, p, stream);
   const int G = Hq / Hkv;
   dim3 grid(p.n_copy + ((Tq + FA_BQ - 1) / FA_BQ) * G, Hkv, B);
-  // Share of the exponentials computed on the FMA pipe (column pairs out of 8); CPB_FWD_POLY overrides the tuned
-  // default and is read once.
-  static const int poly = [] { const char* e = getenv("CPB_FWD_POLY"); return e ? atoi(e) : -1; }();
 #define CPB_FWD_LAUNCH(DD, PP)                                                                                         \
   do {                                                                                                                 \
     static bool cfg = false;                                                                                           \
@@ -477,7 +478,7 @@ extern "C" int cpb_flash_fwd(const void* q, const void* k, const void* v, void* 
     flash_fwd_kernel<DD, PP><<<grid, FA_THREADS, FwdSmem<DD>::TOTAL, stream>>>(tq, tk, tv, p);                         \
   } while (0)
   if (D == 64) {
-    switch (poly < 0 ? FA_POLY_D64 : poly) {
+    switch (poly) {
       case 0: CPB_FWD_LAUNCH(64, 0); break;
       case 1: CPB_FWD_LAUNCH(64, 1); break;
       case 2: CPB_FWD_LAUNCH(64, 2); break;
@@ -486,7 +487,7 @@ extern "C" int cpb_flash_fwd(const void* q, const void* k, const void* v, void* 
       default: CPB_FWD_LAUNCH(64, 3); break;
     }
   } else {
-    switch (poly < 0 ? FA_POLY_D128 : poly) {
+    switch (poly) {
       case 0: CPB_FWD_LAUNCH(128, 0); break;
       case 1: CPB_FWD_LAUNCH(128, 1); break;
       case 3: CPB_FWD_LAUNCH(128, 3); break;

@@ -51,7 +51,7 @@ __device__ __forceinline__ bool wait_flag_ge(const int* flag, int value, volatil
   return false;
 }
 
-// attention_fwd128.cu: head_dim 128, two query tiles per CTA
-int launch_flash_fwd128_pair(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p, cudaStream_t stream);
+// attention_fwd128.cu: head_dim 128, two query tiles per CTA; poly = share (of 8) of polynomial exponentials, 0 to 4
+int launch_flash_fwd128_pair(int poly, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p, cudaStream_t stream);
 
 }  // namespace cpb

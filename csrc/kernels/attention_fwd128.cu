@@ -10,13 +10,13 @@
 // What bounds it: the chain of one tile, about 3450 cycles for two tiles of 2 x 1024 tensor-core cycles: of it 1650 from the
 // store of P until the next scores are in registers.  Measured against one tile per CTA (attention_fwd.cu), same GPU, cold L2,
 // us: 32768 keys, 32/8 heads 8921 -> 8025; 4/1 heads 996 -> 938 (1172 TFLOP/s; 994 -> 873 on another GPU); 16384, 16/4 heads
-// 1068 -> 942; 8192, 32/8 heads 656 -> 599.  Share of polynomial exponentials 0, 1, 3 of 8: 992, 925, 906 us at 16384 keys.
-// Making the two tiles' warps take turns on the exponentials: 966.
+// 1068 -> 942; 8192, 32/8 heads 656 -> 599 (all with three of eight exponentials from the polynomial; it is two of eight, as in
+// the other kernel, because three gave up accuracy).  Share of polynomial exponentials 0, 1, 3 of 8: 992, 925, 906 us at 16384
+// keys.  Making the two tiles' warps take turns on the exponentials: 966.
 #include "attention_fwd.cuh"
 
 namespace cpb {
 
-constexpr int FP_POLY = 3;         // share (of 8) of the exponentials taken off the special-function unit
 constexpr int FP_THREADS = 384;    // warpgroup 0: loader, MMA issuer, two idle warps; 1 and 2: softmax of one query tile each
 constexpr int FP_REGS_ISSUE = 56, FP_REGS_SOFTMAX = 224;      // 56 + 2 x 224 = 3 x 168
 
@@ -30,12 +30,13 @@ struct FpSmem {
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
 };
 
-// Of the 8 column pairs of every 16-column group the last FP_POLY take exp2_poly_f32x2 and the others ex2.approx.
+// POLY: of the 8 column pairs of every 16-column group, the last POLY take exp2_poly_f32x2 and the others ex2.approx.
+template <int POLY>
 __global__ void __launch_bounds__(FP_THREADS, 1)
 flash_fwd128_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, FwdParams p) {
   using L = FpSmem;
-  constexpr int D = L::D, POLY = FP_POLY;
+  constexpr int D = L::D;
   if (p.n_copy > 0 && blockIdx.x < (unsigned)p.n_copy) {
     if (blockIdx.y == 0 && blockIdx.z == 0) ring_copy_cta(p.segs, p.n_segs, p.n_copy, blockIdx.x, p.ready);
     return;
@@ -383,12 +384,23 @@ flash_fwd128_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   if (threadIdx.x == 0 && *abort_flag) report(p.status, ST_TIMEOUT_MBAR, *abort_flag, 0);
 }
 
-int launch_flash_fwd128_pair(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p, cudaStream_t stream) {
+template <int POLY>
+static int launch_pair(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p, cudaStream_t stream) {
   static bool cfg = false;
-  if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_fwd128_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FpSmem::TOTAL)); cfg = true; }
+  if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_fwd128_pair_kernel<POLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, FpSmem::TOTAL)); cfg = true; }
   const dim3 grid(p.n_copy + (p.Tq + 2 * FA_BQ - 1) / (2 * FA_BQ) * (p.Hq / p.Hkv), p.Hkv, p.B);
-  flash_fwd128_pair_kernel<<<grid, FP_THREADS, FpSmem::TOTAL, stream>>>(tq, tk, tv, p);
+  flash_fwd128_pair_kernel<POLY><<<grid, FP_THREADS, FpSmem::TOTAL, stream>>>(tq, tk, tv, p);
   return check_launch("flash_fwd");
+}
+
+int launch_flash_fwd128_pair(int poly, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p, cudaStream_t stream) {
+  switch (poly) {
+    case 0: return launch_pair<0>(tq, tk, tv, p, stream);
+    case 1: return launch_pair<1>(tq, tk, tv, p, stream);
+    case 3: return launch_pair<3>(tq, tk, tv, p, stream);
+    case 4: return launch_pair<4>(tq, tk, tv, p, stream);
+    default: return launch_pair<2>(tq, tk, tv, p, stream);
+  }
 }
 
 }  // namespace cpb

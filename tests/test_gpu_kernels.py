@@ -482,6 +482,28 @@ def test_flash_fwd_d128_pair_kernel(Tq, Tk, Hq, Hkv, causal, ring, flags):
     assert_close(lse, wlse, cos=0.99999, rel=1e-3, name="lse")
 
 
+@pytest.mark.parametrize("poly,share", [(None, 2 / 8), ("0", 0.0), ("3", 3 / 8)])
+def test_flash_fwd_d128_share_of_polynomial_exponentials(poly, share):
+    """With all scores zero every exponential is 1, where the polynomial gives 1 - 7.24e-5: the LSE shows the share of columns that
+    took it, for one query tile per CTA and for two, and CPB_FWD_POLY (read once per process) sets it for both."""
+    import os
+    import subprocess
+    import sys
+    code = ("import torch, math\nfrom context_parallelism_b200.ops import attention as A\n"
+            "for Tq, Tk, H in ((256, 1024, 2), (512, 8192, 120)):\n"
+            "    q, k = torch.zeros(1, Tq, H, 128, device='cuda').bfloat16(), torch.zeros(1, Tk, 1, 128, device='cuda').bfloat16()\n"
+            "    lse = A.flash_fwd(q, k, k, 1.0, False)[1].double()\n"
+            "    print(float((lse - math.log(Tk)).min()), float((lse - math.log(Tk)).max()))\n")
+    env = {k: v for k, v in os.environ.items() if k != "CPB_FWD_POLY"}
+    env.update({} if poly is None else {"CPB_FWD_POLY": poly}, PYTHONPATH=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    values = [float(x) for x in r.stdout.split()]
+    assert len(values) == 4
+    for v in values:                                        # LSE up to 9.01: fp32 steps of 1e-6, log2 and the sum a few of them
+        assert abs(v + share * 7.24e-5) < 4e-6, values
+
+
 # rows held by one, two, five and eight CTAs, padded columns, an ignored row, a row too wide for a cluster (the other kernel)
 @pytest.mark.parametrize("rows,V,Vc", [(5, 17, 64), (3, 26621, 26624), (2, 50257, 50304), (2, 128256, 128256), (2, 212000, 212992), (2, 220000, 220032)])
 def test_xent_row_widths(rows, V, Vc):
