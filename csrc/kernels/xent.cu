@@ -213,9 +213,12 @@ extern "C" int cpb_xent(const float* logits, const int64_t* targets, void* dlogi
   if (Vcols < V || (Vcols % 4)) return set_error(CPB_ERR_ARG, "xent: Vcols must be >= V and a multiple of 4");
   if ((ld_logits % 4) || (dlogits && (ld_dlogits % 4))) return set_error(CPB_ERR_ARG, "xent: row strides must be multiples of 4");
   // A cluster of up to eight CTAs (the portable limit) holds rows of up to 213000 columns.  Rows that fit one CTA stay with the
-  // kernel below: they are in L2 when it re-reads them (4096 x 8192: 55 us there, 63 us here).
+  // kernel below: they are in L2 when it re-reads them (4096 x 8192: 55 us there, 63 us here).  So do rows in great number of
+  // which four per SM, those in flight there, come to 80 MB at most (us there and here: 4096 x 26752 130 and 144, 2400 x 32000 101
+  // and 106; but 4096 x 36096 194 and 183, and with few rows, 64 x 32000, 7.8 and 6.4, 600 x 26752 30 and 27).
   const int ranks = (int)(((long)Vcols * 4 + XE_SEG_BYTES - 1) / XE_SEG_BYTES);
-  if (dlogits != nullptr && ranks > 1 && ranks <= 8 && ((uintptr_t)logits & 15) == 0 && ((uintptr_t)dlogits & 7) == 0) {
+  const bool resident = rows > 8 * sm_count() && (long)Vcols * 4 * 4 * sm_count() <= 80000000L;
+  if (dlogits != nullptr && !resident && ranks > 1 && ranks <= 8 && ((uintptr_t)logits & 15) == 0 && ((uintptr_t)dlogits & 7) == 0) {
     const int seg = (Vcols / 4 + ranks - 1) / ranks * 4;
     if (seg * (ranks - 1) < Vcols && (long)rows * ranks <= 0x7fffffffL) {
       static bool cfg = false;

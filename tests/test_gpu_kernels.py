@@ -504,8 +504,9 @@ def test_flash_fwd_d128_share_of_polynomial_exponentials(poly, share):
         assert abs(v + share * 7.24e-5) < 4e-6, values
 
 
-# rows held by one, two, five and eight CTAs, padded columns, an ignored row, a row too wide for a cluster (the other kernel)
-@pytest.mark.parametrize("rows,V,Vc", [(5, 17, 64), (3, 26621, 26624), (2, 50257, 50304), (2, 128256, 128256), (2, 212000, 212992), (2, 220000, 220032)])
+# rows held by one, two, five and eight CTAs, padded columns, an ignored row; the other kernel: a row too wide for a cluster, and
+# many rows that L2 holds
+@pytest.mark.parametrize("rows,V,Vc", [(5, 17, 64), (3, 26621, 26624), (2, 50257, 50304), (2, 128256, 128256), (2, 212000, 212992), (2, 220000, 220032), (1200, 27001, 27008)])
 def test_xent_row_widths(rows, V, Vc):
     from context_parallelism_b200.ops import xent as X
     torch.manual_seed(3)
