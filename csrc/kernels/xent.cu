@@ -167,6 +167,7 @@ xent_smem_kernel(const float* __restrict__ logits, const int64_t* __restrict__ t
     for (int o = 16; o > 0; o >>= 1) xe_merge(m, s, __shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, s, o));
     if (lane == 0) mine = make_float2(m, s);
   }
+  __syncwarp();                                                    // the aligned forms want the whole warp at the same instruction
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   m = -INFINITY; s = 0.f;
   for (int r = 0; r < ranks; ++r) {
@@ -176,6 +177,7 @@ xent_smem_kernel(const float* __restrict__ logits, const int64_t* __restrict__ t
     asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(m2), "=f"(s2) : "r"(addr) : "memory");
     xe_merge(m, s, m2, s2);
   }
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");    // this thread has read every rank's pair
   const bool ignore = tgt < 0 || tgt >= V;
   if (rank == 0 && threadIdx.x == 0) {
@@ -198,6 +200,7 @@ xent_smem_kernel(const float* __restrict__ logits, const int64_t* __restrict__ t
       *(uint2*)(d + c) = make_uint2(pack_bf16(p0, p1), pack_bf16(p2, p3));
     }
   }
+  __syncwarp();
   asm volatile("barrier.cluster.wait.aligned;" ::: "memory");      // no rank leaves while another may still read its pair
 }
 
