@@ -118,8 +118,11 @@ __global__ void norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_
 // Bound by memory (x, dy, dres in, dx out).  A group of G threads owns the d columns, eight each, and takes four rows at a time:
 // all loads are issued before the first use, the rows share one reduction, and dw / db stay in registers until the end.
 // One warp per row, with dw / db added to shared memory, spent its time in those additions (compare-and-swap loops).
-// Cold L2, one warp per row -> this, us: 32768 x 4096 761 -> 213 (5.0 TB/s); 131072 x 2048 729 -> 377 (5.7); 8192 x 2048
-// 70 -> 53; 8192 x 384 20.5 -> 16.4; layer norm 4096 x 768 20.5 -> 16.3, 4096 x 384 16.4 -> 12.3.
+// Cold L2, one warp per row -> this, us: 32768 x 4096 757 -> 206 (5.2 TB/s); 131072 x 2048 732 -> 367 (5.9); 8192 x 2048
+// 71 -> 36; 8192 x 384 20.5 -> 16.4; layer norm 4096 x 768 20.5 -> 16.3, 4096 x 384 16.4 -> 12.3.
+__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
 template <bool LAYER, int G>
 __global__ void __launch_bounds__(G > 256 ? 512 : 256, G > 256 ? 1 : 2)
 norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
@@ -128,7 +131,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
                 float* __restrict__ dw, float* __restrict__ db, int rows, int d) {
   constexpr int TB = G > 256 ? 512 : 256, NG = TB / G, W = G / 32, R = 4;
   __shared__ float4 red[2][NG][W][LAYER ? 2 : 1];            // per warp: four rows' sums; two buffers, one barrier per turn
-  __shared__ float part[NG > 1 ? TB * 8 : 1];
+  __shared__ float part[NG > 1 ? TB * 8 : 1];                // used only when a block holds several groups
   const int g = threadIdx.x / G, c = threadIdx.x % G, lane = threadIdx.x & 31, warp = c >> 5;
   const bool on = c < (d >> 3);
   float wv[8], aw[8], ab[8];
@@ -203,14 +206,24 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
       ((uint4*)(dx + (size_t)(row0 + r) * d))[c] = pack8(o);
     }
   }
-  // the groups of a block are added in shared memory, the blocks in global memory
+  // the groups of a block are added in shared memory, the blocks in global memory.  One group: four columns per addition (one
+  // column at a time, 32 bytes from lane to lane, takes 33 us at 2048 x 1032, where 256 blocks meet on every column).
   for (int pass = 0; pass < (LAYER ? 2 : 1); ++pass) {
     float* dst = pass ? db : dw;
     if (dst == nullptr) continue;
     if (NG == 1) {
-      if (on)
+      if (on) {
+        float v[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) atomicAdd(&dst[c * 8 + j], pass ? ab[j] : aw[j]);
+        for (int j = 0; j < 8; ++j) v[j] = pass ? ab[j] : aw[j];
+        if (((uintptr_t)dst & 15) == 0) {
+          red_add_v4(dst + c * 8, v[0], v[1], v[2], v[3]);
+          red_add_v4(dst + c * 8 + 4, v[4], v[5], v[6], v[7]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) atomicAdd(&dst[c * 8 + j], v[j]);
+        }
+      }
     } else {
       __syncthreads();
 #pragma unroll

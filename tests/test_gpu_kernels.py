@@ -552,3 +552,25 @@ def test_norm_bwd_widths(layer, rows, d):
     for got, term in ((dw, dy.double() * xh), (db, dy.double())) if layer else ((dw, dy.double() * xh),):
         bound = (term.abs().sum(0) + 1) * (rows + 8) * 2.0 ** -24 + 1e-12
         assert bool(((got.double() - 1 - term.sum(0)).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("layer", [0, 1])
+@pytest.mark.parametrize("offset", [0, 1, 4])
+def test_norm_bwd_gradient_buffers_at_any_address(layer, offset):
+    """Weight gradients of wide rows are added four columns at a time where the buffer is 16-byte aligned, else one at a time."""
+    from context_parallelism_b200 import _native as nv
+    torch.manual_seed(6)
+    rows, d = 70, 1032
+    x, dy = (torch.randn(rows, d, device=dev()).bfloat16() for _ in range(2))
+    w, stats, dx = torch.randn(d, device=dev()), torch.rand(rows, 2, device=dev()), torch.empty_like(x)
+    buf = torch.zeros(2, d + 8, device=dev())
+    dw, db = buf[0, offset:], buf[1, offset:]
+    nv.call("norm_bwd", nv.ptr(x), nv.ptr(dy), nv.ptr(None), nv.ptr(w), nv.ptr(stats), nv.ptr(dx), nv.ptr(dw), nv.ptr(db if layer else None),
+            nv.i(rows), nv.i(d), nv.i(layer), nv.stream_ptr(dev()))
+    check_status()
+    xh = (x.double() - (stats[:, :1].double() if layer else 0)) * stats[:, 1:].double()
+    for got, term in ((dw, dy.double() * xh), (db, dy.double())) if layer else ((dw, dy.double() * xh),):
+        # fp32 sums over the rows: rows + 8 roundings of 2^-24 of the sum of magnitudes; nothing beside the d columns is touched
+        assert bool(((got[:d].double() - term.sum(0)).abs() <= term.abs().sum(0) * (rows + 8) * 2.0 ** -24 + 1e-12).all())
+        assert not bool(got[d:].any())
+    assert not bool(buf[:, :offset].any())
