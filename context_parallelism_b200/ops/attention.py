@@ -107,17 +107,20 @@ class _FlashAttnPackedFn(torch.autograd.Function):
     def forward(ctx, qkv, Hq, Hkv, D, scale, causal):
         B, T = qkv.shape[:2]
         x = qkv.view(B, T, Hq + 2 * Hkv, D)
-        out, lse = flash_fwd(x[:, :, :Hq], x[:, :, Hq:Hq + Hkv], x[:, :, Hq + Hkv:], scale, causal)
+        # allocated in the shape it is returned in: autograd refuses in-place operations on a view made in here
+        out = torch.empty((B, T, Hq * D), dtype=torch.bfloat16, device=qkv.device)
+        _, lse = flash_fwd(x[:, :, :Hq], x[:, :, Hq:Hq + Hkv], x[:, :, Hq + Hkv:], scale, causal, out=out.view(B, T, Hq, D))
         ctx.save_for_backward(x, out, lse)
         ctx.meta = (Hq, Hkv, scale, causal)
-        return out.view(B, T, Hq * D)
+        return out
 
     @staticmethod
     def backward(ctx, dout):
         from .attention_bwd import flash_bwd_packed
         x, out, lse = ctx.saved_tensors
         Hq, Hkv, scale, causal = ctx.meta
-        dqkv = flash_bwd_packed(x, Hq, Hkv, out, lse, dout.reshape(out.shape), scale, causal)
+        heads = (*out.shape[:2], Hq, -1)
+        dqkv = flash_bwd_packed(x, Hq, Hkv, out.view(heads), lse, dout.reshape(heads), scale, causal)
         return dqkv.view(*dqkv.shape[:2], -1), None, None, None, None, None
 
 

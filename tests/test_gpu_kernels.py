@@ -433,6 +433,15 @@ def test_packed_attention_matches_separate(B, T, Hq, Hkv, D):
     assert_close(a.grad[..., :nq].float(), b.grad[..., :nq].float(), cos=0.99999, rel=4e-3, name="dq")
 
 
+def test_packed_attention_output_can_be_changed_in_place():
+    from context_parallelism_b200.ops import attention as A
+    qkv = torch.randn(1, 128, 4 * 64, device=dev()).bfloat16().requires_grad_()
+    out = A.flash_attention_packed(qkv, 2, 1, 64, 0.125)
+    want = out.detach() + 1
+    out += 1                                    # a view made inside the autograd function would refuse this
+    assert torch.equal(out.detach(), want)
+
+
 @pytest.mark.parametrize("B,T,H,D,with_pos", [(2, 130, 3, 64, True), (1, 128, 2, 128, False), (1, 1, 1, 64, False)])
 def test_flash_bwd_prep_outputs(B, T, H, D, with_pos):
     from context_parallelism_b200.ops import attention_bwd as AB
