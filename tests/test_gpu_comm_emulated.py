@@ -167,6 +167,63 @@ def test_fused_ulysses_emulated(n, hq, hkv):
         assert_close(dv.float(), loc(dv_ref, r), cos=0.998, rel=5e-2, name=f"ulysses dv rank {r}")
 
 
+# ------------------------------------------------------------------- long sequences: two query tiles per CTA (head_dim 128)
+@pytest.mark.parametrize("n,chunk,hq", [(8, 640, 48), (8, 1024, 32), (4, 1032, 32)])
+def test_fused_ring_emulated_two_query_tiles(n, chunk, hq):
+    """The forward with copy CTAs, flags and the wrapped sweep where ``cpb_flash_fwd`` takes the kernel with two query tiles per
+    CTA: one emulated rank at a time against its rows of the dense result.  Chunks of five, eight and 8 1/16 tiles: in the first
+    the two tiles of a CTA lie in different chunks, in the last a tile straddles the chunks' border."""
+    from context_parallelism_b200.ops import reference as R
+    from context_parallelism_b200.parallel import fused as F
+    from context_parallelism_b200.parallel import shard
+    torch.manual_seed(n + chunk)
+    B, T, D, hkv = 1, 2 * n * chunk, 128, 2
+    Tl, scale = T // n, D ** -0.5
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert T >= 8192 and 2 * ((Tl + 255) // 256) * hq >= 3 * sms              # the rule's side
+    cfg, fcs = make_comms(n, "ring", heap_mb=64)
+    q, k, v = (torch.randn(B, T, h, D, device=dev()).bfloat16() for h in (hq, hkv, hkv))
+    pos = [shard.local_positions(T, n, r, True).to(dev()) for r in range(n)]
+    loc = lambda t, r: t.index_select(1, pos[r]).contiguous()        # noqa: E731
+    st = [F.ring_fwd_publish(fcs[r], loc(k, r), loc(v, r)) for r in range(n)]
+    for r in (0, 1, n - 1):
+        o, lse = F.ring_fwd_compute(fcs[r], st[r][0], st[r][1], loc(q, r), pos[r].int(), scale)
+        status_ok()
+        assert torch.equal(st[r][0].gathered[0].view_as(k), k) and torch.equal(st[r][0].gathered[1].view_as(v), v)
+        o2, lse2 = F.ring_fwd_settled(fcs[r], st[r][0], loc(q, r), pos[r].int(), scale)
+        assert torch.equal(o, o2) and torch.equal(lse, lse2)
+        for h in range(0, hq, 8):                                     # the dense result a few heads at a time
+            kv = slice(h * hkv // hq, h * hkv // hq + 1)
+            want, wlse = R.attention_dense(loc(q, r)[:, :, h:h + 1].float(), k[:, :, kv].float(), v[:, :, kv].float(), scale, q_pos=pos[r], causal=True)
+            assert_close(o[:, :, h:h + 1].float(), want, cos=0.9995, rel=3e-2, name=f"ring out rank {r} head {h}")
+            assert_close(lse[:, h:h + 1], wlse, cos=0.99999, rel=1e-3, name=f"ring lse rank {r} head {h}")
+
+
+@pytest.mark.parametrize("B,T,hq,hkv", [(1, 8200, 28, 2), (2, 8192, 16, 4)])
+def test_fused_ulysses_emulated_two_query_tiles(B, T, hq, hkv):
+    """The scatter epilogue of the kernel with two query tiles per CTA, a batch of two and rows of one tile in two owners' arenas."""
+    from context_parallelism_b200.ops import reference as R
+    from context_parallelism_b200.parallel import fused as F
+    torch.manual_seed(T + hq)
+    n, D = 2, 128
+    Tl, scale = T // n, D ** -0.5
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert 2 * ((T + 255) // 256) * (hq // n) * B >= 3 * sms                  # the rule's side
+    cfg, fcs = make_comms(n, "ulysses", heap_mb=512)
+    q, k, v = (torch.randn(B, T, h, D, device=dev()).bfloat16() for h in (hq, hkv, hkv))
+    loc = lambda t, r: t[:, r * Tl:(r + 1) * Tl].clone(memory_format=torch.contiguous_format)        # noqa: E731
+    st = [F.uly_fwd_push(fcs[r], loc(q, r), loc(k, r), loc(v, r)) for r in range(n)]
+    lses = [F.uly_fwd_compute(fcs[r], st[r][0], st[r][1], scale) for r in range(n)]
+    status_ok()
+    out = torch.cat([st[r][0].o_view(fcs[r], st[r][1]) for r in range(n)], 1)
+    lse = torch.cat(lses, 1)
+    for h in range(0, hq, 6):
+        kv = slice(h * hkv // hq, h * hkv // hq + 1)
+        want, wlse = R.attention_dense(q[:, :, h:h + 1].float(), k[:, :, kv].float(), v[:, :, kv].float(), scale, causal=True)
+        assert_close(out[:, :, h:h + 1].float(), want, cos=0.9995, rel=3e-2, name=f"ulysses out head {h}")
+        assert_close(lse[:, h:h + 1], wlse, cos=0.99999, rel=1e-3, name=f"ulysses lse head {h}")
+
+
 # ----------------------------------------------------------------------------------------------------- gradient transport
 def _tiny_params(seed):
     g = torch.Generator().manual_seed(seed)
