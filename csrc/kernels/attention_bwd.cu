@@ -1,7 +1,8 @@
 // Flash-attention backward for sm_100a with query rows in tensor-memory lanes, head_dim 64: the second implementation that
-// attention_bwd64.cu is checked against (CPB_BWD_GENERAL=1); head_dim 128 runs on attention_bwd128.cu.  One CTA owns one 128-row K/V tile of one KV head and sweeps
-// every query tile (of every query head of the GQA group) that can see it, with all five products
-// on tcgen05 tensor cores and every accumulator in tensor memory:
+// attention_bwd64.cu is checked against (CPB_BWD_GENERAL=1), and the preparation kernel of all three backward kernels
+// (bwd_prep_kernel); head_dim 128 runs on attention_bwd128.cu.  One CTA owns one 128-row K/V tile of one KV head and
+// sweeps every query tile (of every query head of the GQA group) that can see it, with all five products on tcgen05 tensor
+// cores and every accumulator in tensor memory:
 //
 //   S  = Q K^T              (smem x smem)          P  = exp2(S*c - LSE)             (registers -> smem, bf16)
 //   dP = dO V^T             (smem x smem)          dS = P o (dP - Delta)            (registers -> smem, bf16)
@@ -36,6 +37,7 @@ namespace cpb {
 
 
 constexpr int FB_T = 128;            // tile edge (queries and keys)
+constexpr int FB_D = 64;
 constexpr int FB_THREADS = 448;
 
 struct BwdParams {
@@ -59,10 +61,9 @@ struct BwdParams {
   int* status;
 };
 
-template <int D>
 struct BwdSmem {
   static constexpr int STAGES = 2;
-  static constexpr int TILE = FB_T * D * 2;
+  static constexpr int TILE = FB_T * FB_D * 2;
   static constexpr int K_OFF = 0;
   static constexpr int V_OFF = TILE;
   static constexpr int Q_OFF = 2 * TILE;
@@ -71,26 +72,19 @@ struct BwdSmem {
   static constexpr int DS_BUFS = 2;                               // dS double-buffered (pipelined issue order)
   static constexpr int DS_OFF = PS_OFF + FB_T * FB_T * 2;         // dS: same layout
   static constexpr int DQS_OFF = DS_OFF + DS_BUFS * FB_T * FB_T * 2;   // dQ staging: boxes of 128 rows x 32 fp32, 128B-swizzled
-  static constexpr int DQ_BOXES = 1;              // boxes staged per TMA-reduce round
+  static constexpr int DQ_BOXES = 1;                              // boxes staged per TMA-reduce round
   static constexpr int VEC_OFF = DQS_OFF + DQ_BOXES * FB_T * 128;        // per stage: lse2[128], delta[128], qpos[128]
   static constexpr int BAR_OFF = VEC_OFF + STAGES * 3 * 512;
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
 };
 
-__device__ __forceinline__ void bulk_load_1d(void* smem, const void* gmem, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_u32(smem)), "l"((uint64_t)gmem), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
 
-template <int D>
 __global__ void __launch_bounds__(FB_THREADS, 1)
 flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
                  const __grid_constant__ CUtensorMap tmDQ, BwdParams p) {
-  using L = BwdSmem<D>;
+  using L = BwdSmem;
+  constexpr int D = FB_D;
   constexpr int ST = L::STAGES;
   constexpr int DH = D / 64;
   constexpr uint32_t S_COL = 0, DP_COL = 128, DV_COL = 256, DK_COL = 256 + D;
@@ -578,7 +572,7 @@ extern "C" int cpb_flash_bwd(const void* q, const void* k, const void* v, const 
     return set_error(CPB_ERR_ARG, "flash_bwd: routed dK/dV needs route tables");
   dim3 grid((Tk + FB_T - 1) / FB_T, Hkv, B);
   static bool cfg = false;
-  if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_bwd_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<64>::TOTAL)); cfg = true; }
-  flash_bwd_kernel<64><<<grid, FB_THREADS, BwdSmem<64>::TOTAL, stream>>>(tq, tk, tv, tdo, tdq, p);
+  if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem::TOTAL)); cfg = true; }
+  flash_bwd_kernel<<<grid, FB_THREADS, BwdSmem::TOTAL, stream>>>(tq, tk, tv, tdo, tdq, p);
   return check_launch("flash_bwd");
 }

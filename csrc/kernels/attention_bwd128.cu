@@ -19,8 +19,8 @@
 //     dV(i), S(i+1)      when the warps have stored P(i): both run while the warps form dS(i)
 //     dK(i), dQ(i)       when dS(i) is stored: both run while the warps take the exponentials of tile i+1
 //     dP(i+1)            when dQ(i) has been read out of tensor memory
-// The drain warps take half of dQ through the staging buffer and the other half into registers, so that tensor memory is
-// free after two loads.  Shared memory: K 32 KB, V 32, Q two stages 64, dO one stage 32 (dO(i) is done with dV(i), long
+// The drain warps load a whole dQ row (128 columns) into registers and release tensor memory at once, then pass it through the
+// staging buffer in two rounds of 64 columns.  Shared memory: K 32 KB, V 32, Q two stages 64, dO one stage 32 (dO(i) is done with dV(i), long
 // before dP(i+1) wants the next one), dS^T 32, dQ staging 32, LSE and Delta of two stages 2: all of it.
 //
 // Measured (T 32768, 32/8 heads, causal): 33.8 ms = 650 TFLOP/s for the kernel this one replaces (query rows in lanes, P and
@@ -81,19 +81,6 @@ struct Bwd128Smem {
   static constexpr int TOTAL = BAR_OFF + 256;            // 231,680 bytes; the base must be 1024-byte aligned as it is
 };
 
-__device__ __forceinline__ void bulk_load_1d_128(void* smem, const void* gmem, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_u32(smem)), "l"((uint64_t)gmem), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
-// A global load that stays where it is written (the compiler would otherwise sink it to its first use, one tile later).
-__device__ __forceinline__ int ld_ahead_s32(const int* ptr) {
-  int v;
-  asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(ptr));
-  return v;
-}
-__device__ __forceinline__ void red_add_v4_128(float* addr, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
 
 __global__ void __launch_bounds__(B128_THREADS, 1)
 flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -179,8 +166,8 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll
         for (int h = 0; h < 2; ++h) tma_load_4d(smem + L::Q_OFF + st * L::TILE + h * L::HALF, &tmQ, &q_full[st], h * 64, hq, q0, b);
         const size_t row_off = ((size_t)b * p.Hq + hq) * p.Tq_pad + q0;
-        bulk_load_1d_128(smem + L::VEC_OFF + st * 1024, p.lse2 + row_off, 512, &q_full[st]);
-        bulk_load_1d_128(smem + L::VEC_OFF + st * 1024 + 512, p.delta + row_off, 512, &q_full[st]);
+        bulk_load_1d(smem + L::VEC_OFF + st * 1024, p.lse2 + row_off, 512, &q_full[st]);
+        bulk_load_1d(smem + L::VEC_OFF + st * 1024 + 512, p.delta + row_off, 512, &q_full[st]);
         if (!mbar_wait_lean(do_empty, (i & 1) ^ 1, abort_flag, 801)) break;
         mbar_expect_tx(do_full, L::TILE);
 #pragma unroll
@@ -391,7 +378,7 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
               float* dst = (float*)(which ? p.route_v[ch] : p.route_k[ch]) + (((size_t)b * p.route_tl + lrow) * p.Hkv + hkv) * D + c;
 #pragma unroll
               for (int j = 0; j < 32; j += 4)
-                red_add_v4_128(dst + j, __uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+                red_add_v4(dst + j, __uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
             } else if (p.dkv_mode == 1) {
               float* dst = (float*)base + off + c;
 #pragma unroll

@@ -47,7 +47,6 @@ constexpr int B64_THREADS = 6 * 128;                     // six warpgroups
 // Registers per thread and warpgroup: the launch gives every thread 80 (768 x 80); the loader / issuer warpgroup hands back
 // what the drain warps need to hold a whole dQ row.  48 + 4 x 80 + 112 = 6 x 80.
 constexpr int B64_REGS_ISSUE = 48, B64_REGS_DRAIN = 112;
-constexpr int B64_POLY = 0;        // share (of 8) of the exponentials computed on the FMA pipe
 
 struct Bwd64Params {
   int B, Tq, Tk, Hq, Hkv, Tq_pad;
@@ -78,26 +77,12 @@ struct Bwd64Smem {
   static constexpr int DS_BYTES = B64_T * B64_T * 2;     // dS^T: two 64-query halves of 128 key rows x 128 bytes
   static constexpr int DS_OFF = DO_OFF + NST * TILE;     // two buffers
   static constexpr int DQS_OFF = DS_OFF + 2 * DS_BYTES;  // per drain warp two boxes of 32 rows x 32 fp32
-  static constexpr int VEC_OFF = DQS_OFF + 32768;        // NST x (-lse2[128], -delta[128])
+  static constexpr int VEC_OFF = DQS_OFF + 32768;        // NST x (lse2[128], delta[128])
   static constexpr int BAR_OFF = VEC_OFF + NST * 1024;
   static constexpr int TOTAL = BAR_OFF + 256;            // 216,320 bytes; the base must be 1024-byte aligned as it is
 };
 
-__device__ __forceinline__ void bulk_load_1d_64(void* smem, const void* gmem, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_u32(smem)), "l"((uint64_t)gmem), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
-// A global load that stays where it is written (the compiler would otherwise sink it to its first use, one tile later).
-__device__ __forceinline__ int ld_ahead_s32(const int* ptr) {
-  int v;
-  asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(ptr));
-  return v;
-}
-__device__ __forceinline__ void red_add_v4_64(float* addr, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
 
-template <int POLY>
 __global__ void __launch_bounds__(B64_THREADS, 1)
 flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmDO, const __grid_constant__ CUtensorMap tmDQ, Bwd64Params p) {
@@ -188,8 +173,8 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         mbar_expect_tx(&q_full[st], L::TILE + 1024);
         tma_load_4d(smem + L::Q_OFF + st * L::TILE, &tmQ, &q_full[st], 0, hq, q0, b);
         const size_t row_off = ((size_t)b * p.Hq + hq) * p.Tq_pad + q0;
-        bulk_load_1d_64(smem + L::VEC_OFF + st * 1024, p.lse2 + row_off, 512, &q_full[st]);
-        bulk_load_1d_64(smem + L::VEC_OFF + st * 1024 + 512, p.delta + row_off, 512, &q_full[st]);
+        bulk_load_1d(smem + L::VEC_OFF + st * 1024, p.lse2 + row_off, 512, &q_full[st]);
+        bulk_load_1d(smem + L::VEC_OFF + st * 1024 + 512, p.delta + row_off, 512, &q_full[st]);
         if (!mbar_wait_lean(&do_empty[st], ph, abort_flag, 801)) break;
         mbar_expect_tx(&do_full[st], L::TILE);
         tma_load_4d(smem + L::DO_OFF + st * L::TILE, &tmDO, &do_full[st], 0, hq, q0, b);
@@ -326,13 +311,8 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           for (int e = 0; e < 4; e += 2) {
             const uint64_t x = fma_f32x2(pack_f32x2(__uint_as_float(sv[j + e]), __uint_as_float(sv[j + e + 1])), c2, e ? pack_f32x2(-l.z, -l.w) : pack_f32x2(-l.x, -l.y));
             float x0, x1;
-            if ((((j + e) % 16) >> 1) >= 8 - POLY) {            // resolved at compile time (the loops are unrolled)
-              unpack_f32x2(exp2_poly_f32x2(x), x0, x1);
-            } else {
-              unpack_f32x2(x, x0, x1);
-              x0 = ex2f(x0); x1 = ex2f(x1);
-            }
-            sv[j + e] = __float_as_uint(x0); sv[j + e + 1] = __float_as_uint(x1);
+            unpack_f32x2(x, x0, x1);
+            sv[j + e] = __float_as_uint(ex2f(x0)); sv[j + e + 1] = __float_as_uint(ex2f(x1));
           }
         }
       } else {
@@ -421,7 +401,7 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
               float* dst = (float*)(which ? p.route_v[ch] : p.route_k[ch]) + (((size_t)b * p.route_tl + lrow) * p.Hkv + hkv) * D + c;
 #pragma unroll
               for (int j = 0; j < 32; j += 4)
-                red_add_v4_64(dst + j, __uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+                red_add_v4(dst + j, __uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
             } else if (p.dkv_mode == 1) {
               float* dst = (float*)base + off + c;
 #pragma unroll
@@ -558,7 +538,7 @@ extern "C" int cpb_flash_bwd64(const void* q, const void* k, const void* v, cons
   p.debug_skip_dq = skip_dq;
   dim3 grid((Tk + B64_T - 1) / B64_T, Hkv, B);
   static bool cfg = false;
-  if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_bwd64_kernel<B64_POLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, Bwd64Smem::TOTAL)); cfg = true; }
-  flash_bwd64_kernel<B64_POLY><<<grid, B64_THREADS, Bwd64Smem::TOTAL, stream>>>(tq, tk, tdo, tdq, p);
+  if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_bwd64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Bwd64Smem::TOTAL)); cfg = true; }
+  flash_bwd64_kernel<<<grid, B64_THREADS, Bwd64Smem::TOTAL, stream>>>(tq, tk, tdo, tdq, p);
   return check_launch("flash_bwd64");
 }

@@ -120,9 +120,6 @@ __global__ void norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_
 // One warp per row, with dw / db added to shared memory, spent its time in those additions (compare-and-swap loops).
 // Cold L2, one warp per row -> this, us: 32768 x 4096 757 -> 206 (5.2 TB/s); 131072 x 2048 732 -> 367 (5.9); 8192 x 2048
 // 71 -> 36; 8192 x 384 20.5 -> 16.4; layer norm 4096 x 768 20.5 -> 16.3, 4096 x 384 16.4 -> 12.3.
-__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
 template <bool LAYER, int G>
 __global__ void __launch_bounds__(G > 256 ? 512 : 256, G > 256 ? 1 : 2)
 norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,

@@ -130,8 +130,7 @@ xent_smem_kernel(const float* __restrict__ logits, const int64_t* __restrict__ t
       const int len = min(part, n - i * part);
       if (len <= 0) break;
       mbar_expect_tx(&bars[i], len * 4);
-      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                   ::"r"(smem_u32(xs + i * part)), "l"((uint64_t)(x + c0 + i * part)), "r"(len * 4), "r"(smem_u32(&bars[i])) : "memory");
+      bulk_load_1d(xs + i * part, x + c0 + i * part, len * 4, &bars[i]);
     }
   }
   const int64_t tgt = targets[row];

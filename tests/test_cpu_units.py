@@ -286,7 +286,7 @@ def test_ring_chunk_tables_are_inverse(N, lb):
 
 @pytest.mark.parametrize("m_tiles,n_blocks,band", [(1, 1, 8), (11, 32, 8), (64, 8, 8), (5, 3, 1), (9, 7, 4), (32, 32, 8)])
 def test_pair_gemm_band_order_visits_every_tile_once(m_tiles, n_blocks, band):
-    """The tile order of the CTA-pair GEMM (csrc/kernels/gemm2.cu, pair_tile_coords): bands of ``band`` pair-rows swept along
+    """The tile order of the CTA-pair GEMM (csrc/kernels/gemm.cu, pair_tile_coords): bands of ``band`` pair-rows swept along
     N with rows fastest, the last band possibly shorter.  Restated here; the device code is checked against cuBLAS-free fp32
     matmul on a ragged shape in tests/test_gpu_kernels.py::test_gemm_pair_banded_order."""
     def coords(tile):
