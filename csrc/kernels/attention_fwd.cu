@@ -465,10 +465,11 @@ extern "C" int cpb_flash_fwd(const void* q, const void* k, const void* v, void* 
   static const int poly_env = [] { const char* e = getenv("CPB_FWD_POLY"); return e ? atoi(e) : -1; }();
   const int poly = poly_env < 0 ? (D == 64 ? FA_POLY_D64 : FA_POLY_D128) : poly_env;
   // Two query tiles per CTA pay when the sweep over the keys is long (one CTA per SM: its start and end are not hidden; 4096
-  // keys, 32/8 heads: 187 us with one tile, 189 to 205 with two; 8192 keys: 646 and 591) and when there are enough CTAs for
-  // their unequal lengths to even out (8192 keys, 8 heads, 256 CTAs: 171 and 163; 12000 keys, 4 heads, 188 CTAs: 191 and 228).
+  // keys, 32/8 heads: 187 us with one tile, 189 to 205 with two; 8192 keys: 615 and 552) and when there are enough CTAs for
+  // their unequal lengths to even out (us with one tile and with two: 12000 keys, 188 CTAs 191 and 228; 14336, 224 CTAs 231 and
+  // 236; 8192, 224 CTAs 154 and 153; 8192, 256 CTAs 163 and 153; 32768 keys, 256 CTAs 528 and 507).
   const long pairs = (long)((Tq + 2 * FA_BQ - 1) / (2 * FA_BQ)) * Hq * B;
-  if (D == 128 && Tk >= 8192 && Tq > FA_BQ && 2 * pairs >= 3 * sm_count()) return launch_flash_fwd128_pair(poly, tq, tk, tv, p, stream);
+  if (D == 128 && Tk >= 8192 && Tq > FA_BQ && 5 * pairs >= 8 * sm_count()) return launch_flash_fwd128_pair(poly, tq, tk, tv, p, stream);
   const int G = Hq / Hkv;
   dim3 grid(p.n_copy + ((Tq + FA_BQ - 1) / FA_BQ) * G, Hkv, B);
 #define CPB_FWD_LAUNCH(DD, PP)                                                                                         \
