@@ -23,11 +23,12 @@
 // staging buffer in two rounds of 64 columns.  Shared memory: K 32 KB, V 32, Q two stages 64, dO one stage 32 (dO(i) is done with dV(i), long
 // before dP(i+1) wants the next one), dS^T 32, dQ staging 32, LSE and Delta of two stages 2: all of it.
 //
-// Measured (T 32768, 32/8 heads, causal): 33.8 ms = 650 TFLOP/s for the kernel this one replaces (query rows in lanes, P and
-// dS through shared memory, dQ over S: fully serialised), 23.0 ms = 956 with the drain warps storing dQ before they release
-// tensor memory, 20.3 ms = 1084 now:
-// about 3950 cycles per tile, of which shared memory needs 3840.  The second tile half of dP^T is loaded after the first is
-// used: loading both at once spills in the 72 registers of these warps (24.4 ms).
+// Measured (T 32768, 32/8 heads, causal, the kernel alone): 33.8 ms = 650 TFLOP/s for the kernel this one replaces (query rows in
+// lanes, P and dS through shared memory, dQ over S: fully serialised), 23.0 ms = 956 with the drain warps storing dQ before they
+// release tensor memory, 20.3 ms = 1084 now.  With the clock beside it, on another GPU: back to back for two seconds 20.7 ms at 1.47
+// GHz and 1002 W, which is 4280 cycles per tile, of which shared memory needs 3840; one launch at a time 18.1 ms.  So on long runs
+// the power cap sets the clock and shared memory nine tenths of the cycles.  The second tile half of dP^T is loaded after
+// the first is used: loading both at once spills in the 72 registers of these warps (24.4 ms).
 //
 // Masking is on global positions, dK/dV output modes and bounded waits are those of the head_dim-64 kernel.  Replaces
 // mem_efficient_bwd_unified_kernel_exp11 (context_parallel/AttentionBackward.cu:300-541) and gqa_fused_rope_bwd_dQ / _dKdV

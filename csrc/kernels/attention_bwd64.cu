@@ -26,6 +26,9 @@
 // Measured against the kernel this one replaces (all sixteen warps on one tile, K and V read from shared memory, LSE and Delta
 // as extra K = 16 products; same GPU, cold L2, us): T 32768, 32/8 heads 12886 -> 12244 (898 TFLOP/s); T 16384 2997 -> 2948;
 // 2 x 4096, 6/2 heads 194 -> 181; 2 x 1000, 6/2 heads 64.5 -> 56.3 (the vectors' own launch is gone); 4 x 1024, 6/6 50.2 -> 48.2.
+// Of the whole gradient (preparation and cast included) 1 to 18 %: 8192, 32/8 heads 1019 -> 924; 4096 queries, 32768 keys, 8/8, not
+// causal 786 -> 771.  With the clock beside it: T 32768, 32/8 heads, back to back for two seconds, 12.8 ms at 1.59 GHz and 1004 W,
+// 2860 cycles per tile; one launch at a time 11.2 ms (980 TFLOP/s).
 //
 // Masking is on global positions, dK/dV output modes and bounded waits are those of the head_dim-128 kernel.  Replaces
 // mem_efficient_bwd_unified_kernel_exp11 (context_parallel/AttentionBackward.cu:300-541) and gqa_fused_rope_bwd_dQ / _dKdV

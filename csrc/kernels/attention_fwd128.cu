@@ -7,12 +7,14 @@
 // S(j+1) of a tile are issued together, and S(j+1) ready implies that P V(j) has finished: the warps wait for one barrier per
 // tile, need no exchange of row maxima, and can rescale O (rarely) without another.
 //
-// What bounds it: the chain of one tile, about 3450 cycles for two tiles of 2 x 1024 tensor-core cycles: of it 1650 from the
-// store of P until the next scores are in registers.  Measured against one tile per CTA (attention_fwd.cu), same GPU, cold L2,
-// us: 32768 keys, 32/8 heads 8921 -> 8025; 4/1 heads 996 -> 938 (1172 TFLOP/s; 994 -> 873 on another GPU); 16384, 16/4 heads
-// 1068 -> 942; 8192, 32/8 heads 656 -> 599 (all with three of eight exponentials from the polynomial; it is two of eight, as in
-// the other kernel, because three gave up accuracy).  Share of polynomial exponentials 0, 1, 3 of 8: 992, 925, 906 us at 16384
-// keys.  Making the two tiles' warps take turns on the exponentials: 966.
+// What bounds it: the chain of one tile (clock counters in the kernel: about 3450 cycles for two tiles of 2 x 1024 tensor-core
+// cycles, 1650 of them from the store of P until the next scores are in registers), and on long runs the power cap: T 32768, 32/8
+// heads, back to back for two seconds, 8.0 ms at an SM clock of 1.64 GHz (1104 TFLOP/s, 3680 cycles per pair of tiles, 1005 W); one
+// launch at a time 7.1 ms.
+// Measured against one tile per CTA (attention_fwd.cu), same GPU, cold L2, us: 32768 keys, 32/8 heads 8740 -> 7760; 4/1 heads
+// 1110 -> 1026; 16384, 16/4 heads 1131 -> 1017; 8192, 32/8 heads 615 -> 552.  Share of polynomial exponentials 0, 1, 3 of 8: 992,
+// 925, 906 us at 16384 keys (another GPU); two, as in the other kernel, because three gave up accuracy.  Making the two tiles'
+// warps take turns on the exponentials: 966.
 #include "attention_fwd.cuh"
 
 namespace cpb {
