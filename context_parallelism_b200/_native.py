@@ -2,7 +2,7 @@
 
 The library has a plain C ABI: every launcher takes raw device pointers, sizes and a CUDA stream
 and returns 0 or a negative error code whose text is available from ``cpb_last_error``.  Python
-passes ``tensor.data_ptr()`` and ``torch.cuda.current_stream().cuda_stream``.
+passes ``tensor.data_ptr()`` and the stream as plain integers; :func:`lib` declares every argument's type.
 
 On a machine with a GPU a missing or unloadable library is a hard error: the CUDA ops never fall
 back to PyTorch silently.

@@ -1,4 +1,5 @@
-"""Flash attention on tcgen05 tensor cores (``csrc/kernels/attention_fwd.cu`` / ``attention_bwd.cu``).
+"""Flash attention on tcgen05 tensor cores (``csrc/kernels/attention_fwd.cu``, ``attention_fwd128.cu``, ``attention_bwd64.cu``,
+``attention_bwd128.cu``).
 
 ``flash_attention(q, k, v, ...)`` takes token-major tensors ``q [B,Tq,Hq,D]`` and ``k``/``v``
 ``[B,Tk,Hkv,D]`` (any 16-byte aligned strides: views into a packed QKV buffer are consumed in place),
