@@ -10,15 +10,17 @@ vocabulary would be 64 GB.
 """
 from __future__ import annotations
 
-from typing import Tuple
+from typing import Optional
 
 import torch
 import torch.nn.functional as F
 
 from .. import _native as nv
-from .gemm import gemm
+from .gemm import _rowmajor2d, gemm
 
 CHUNK_ROWS = 4096
+# Up to this width of the hidden states the gradient pass computes the logits a second time instead of reading them back.
+RECOMPUTE_WIDTH = 1024
 
 
 def xent_chunk(logits: torch.Tensor, targets: torch.Tensor, loss_sum: torch.Tensor, grad_scale: float,
@@ -30,6 +32,32 @@ def xent_chunk(logits: torch.Tensor, targets: torch.Tensor, loss_sum: torch.Tens
     nv.call("xent", nv.ptr(logits), nv.ptr(targets), nv.ptr(dlog), nv.ptr(loss_sum), nv.ptr(row_loss), nv.i(rows), nv.i(V), nv.i(Vc),
             nv.l(logits.stride(0)), nv.l(dlog.stride(0) if dlog is not None else 0), nv.f(grad_scale), st.ptr(),
             nv.stream_ptr(logits.device))
+    return dlog
+
+
+HEAD_TILE = 256          # columns per tile of the head's GEMM
+
+
+def _head_rows(xc: torch.Tensor, w: torch.Tensor, tg: torch.Tensor, n_valid: int, grad_scale: float, loss_sum: Optional[torch.Tensor],
+               row_loss: Optional[torch.Tensor], want_coef: bool) -> Optional[torch.Tensor]:
+    """Loss of the rows ``xc`` without their logits (``loss_sum`` += , ``row_loss`` =); returns the rows' gradient coefficients."""
+    rows, V = xc.shape[0], w.shape[0]
+    tiles = (V + HEAD_TILE - 1) // HEAD_TILE
+    stats = torch.empty((tiles, rows, 2), dtype=torch.float32, device=xc.device)
+    tlogit = torch.empty(rows, dtype=torch.float32, device=xc.device)
+    coef = torch.empty((rows, 2), dtype=torch.float32, device=xc.device) if want_coef else None
+    st, stream = nv.status_for(xc.device).ptr(), nv.stream_ptr(xc.device)
+    nv.call("gemm_head", xc.data_ptr(), w.data_ptr(), 0, tg.data_ptr(), stats.data_ptr(), tlogit.data_ptr(), 0, rows, V, xc.shape[1],
+            xc.stride(0), w.stride(0), 0, n_valid, grad_scale, st, stream)
+    nv.call("xent_rows", stats.data_ptr(), tlogit.data_ptr(), tg.data_ptr(), nv.ptr(coef), nv.ptr(row_loss), nv.ptr(loss_sum), rows, tiles,
+            n_valid, grad_scale, st, stream)
+    return coef
+
+
+def _head_dlogits(xc: torch.Tensor, w: torch.Tensor, tg: torch.Tensor, coef: torch.Tensor, n_valid: int, grad_scale: float) -> torch.Tensor:
+    dlog = torch.empty((xc.shape[0], w.shape[0]), dtype=torch.bfloat16, device=xc.device)
+    nv.call("gemm_head", xc.data_ptr(), w.data_ptr(), dlog.data_ptr(), tg.data_ptr(), 0, 0, coef.data_ptr(), xc.shape[0], w.shape[0], xc.shape[1],
+            xc.stride(0), w.stride(0), dlog.stride(0), n_valid, grad_scale, nv.status_for(xc.device).ptr(), nv.stream_ptr(xc.device))
     return dlog
 
 
@@ -47,15 +75,21 @@ class _LinearCEFn(torch.autograd.Function):
         dw_own = None
         if need_grad and mg is None:
             dw_own = torch.zeros((V, d), dtype=torch.float32, device=x.device)
-        logits = torch.empty((min(CHUNK_ROWS, N), V), dtype=torch.float32, device=x.device)
+        x2, wm = _rowmajor2d(x2), _rowmajor2d(w)
+        stored = need_grad and d > RECOMPUTE_WIDTH
+        logits = torch.empty((min(CHUNK_ROWS, N), V), dtype=torch.float32, device=x.device) if stored else None
         for r0 in range(0, N, CHUNK_ROWS):
             r1 = min(N, r0 + CHUNK_ROWS)
-            xc = x2[r0:r1]
-            lg = logits[: r1 - r0]
-            gemm(xc, w, out=lg, epi=1)
-            dlog = xent_chunk(lg, tg[r0:r1], loss_sum, grad_scale, need_grad, None, n_valid)
+            xc, tc = x2[r0:r1], tg[r0:r1]
+            if stored:
+                lg = logits[: r1 - r0]
+                gemm(xc, wm, out=lg, epi=1)
+                dlog = xent_chunk(lg, tc, loss_sum, grad_scale, True, None, n_valid)
+            else:
+                coef = _head_rows(xc, wm, tc, n_valid or V, grad_scale, loss_sum, None, need_grad)
+                dlog = _head_dlogits(xc, wm, tc, coef, n_valid or V, grad_scale) if need_grad else None
             if need_grad:
-                gemm(dlog, w, b_mn=True, out=dx[r0:r1])
+                gemm(dlog, wm, b_mn=True, out=dx[r0:r1])
                 gemm(dlog, xc, a_mn=True, b_mn=True, out=(mg if mg is not None else dw_own).view(V, d), accumulate=True)
         if need_grad and mg is not None:
             hook = getattr(w, "_grad_ready", None)
@@ -107,12 +141,10 @@ def per_token_nll(x: torch.Tensor, w: torch.Tensor, targets: torch.Tensor, n_val
         return F.cross_entropy(logits, tg, reduction="none")
     N, V = x2.shape[0], w.shape[0]
     out = torch.empty(N, dtype=torch.float32, device=x.device)
-    logits = torch.empty((min(CHUNK_ROWS, N), V), dtype=torch.float32, device=x.device)
+    x2, wm = _rowmajor2d(x2), _rowmajor2d(w)
     for r0 in range(0, N, CHUNK_ROWS):
         r1 = min(N, r0 + CHUNK_ROWS)
-        lg = logits[: r1 - r0]
-        gemm(x2[r0:r1], w, out=lg, epi=1)
-        xent_chunk(lg, tg[r0:r1], None, 1.0, False, out[r0:r1], n_valid)
+        _head_rows(x2[r0:r1], wm, tg[r0:r1], n_valid or V, 1.0, None, out[r0:r1], False)
     return out
 
 

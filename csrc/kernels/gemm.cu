@@ -242,19 +242,22 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       int mt, nb;
       pair_tile_coords(item % num_tiles, p.num_m_tiles, p.num_n_blocks, p.band, mt, nb);
       const int row0 = mt * (2 * GEMM_BM) + (int)rank * GEMM_BM + quarter * 32;
+      const HeadRow head = head_row(p, row0 + lane);
       bool ok = mbar_wait(&tfull_bar[acc], acc_phase, abort_flag, p.status, 310);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
-      gemm_epilogue<BN>(p, &tmC, &tmX, ws, t_row, row0, nb, lane, item / num_tiles, [&] {
+      const auto release = [&] {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
           if (rank == 0) mbar_arrive(&tempty_bar[acc]);
           else mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[acc]), 0));
         }
-      });
+      };
+      if (p.epi >= EPI_HEAD_STATS) head_epilogue<BN>(p, &tmC, ws, t_row, row0, nb, lane, head, release);
+      else gemm_epilogue<BN>(p, &tmC, &tmX, ws, t_row, row0, nb, lane, item / num_tiles, release);
     }
     ws.drain();
   }
@@ -349,6 +352,23 @@ static void plan_tiles(int M, int N, int K, int epi, int has_aux, int want, int&
   }
 }
 
+// banded tile order once B (N x K bf16) reaches 64 MB, half of L2; CPB_GEMM_BAND (read once) overrides
+static int tile_band(int N, int K) {
+  static const int band_env = [] { const char* e = getenv("CPB_GEMM_BAND"); return e ? atoi(e) : 0; }();
+  return band_env > 0 ? band_env : (((size_t)N * K * 2 >= ((size_t)64 << 20)) ? 8 : 1);
+}
+
+static int kmajor_tmap(CUtensorMap* m, const void* ptr, int rows, int K, int ld, int box_rows) {
+  uint64_t dims[2] = {(uint64_t)K, (uint64_t)rows}, strides[2] = {0, (uint64_t)ld * 2};
+  uint32_t box[2] = {GEMM_BK, (uint32_t)box_rows};
+  return encode_tmap(m, ptr, 2, 2, dims, strides, box, 1);
+}
+static int mnmajor_tmap(CUtensorMap* m, const void* ptr, int rows, int K, int ld) {
+  uint64_t dims[2] = {(uint64_t)rows, (uint64_t)K}, strides[2] = {0, (uint64_t)ld * 2};
+  uint32_t box[2] = {64, GEMM_BK};
+  return encode_tmap(m, ptr, 2, 2, dims, strides, box, 1);
+}
+
 }  // namespace cpb
 
 using namespace cpb;
@@ -379,37 +399,23 @@ extern "C" int cpb_gemm_bf16(const void* A, const void* B, void* C, void* aux, c
   }
   int bn = 256;
   plan_tiles(M, N, K, epi, aux != nullptr, splits, bn, splits);
-  GemmParams p;
+  GemmParams p{};
   p.M = M; p.N = N; p.K = K; p.epi = epi;
   p.num_m_tiles = (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM);
   p.num_k_blocks = (K + GEMM_BK - 1) / GEMM_BK;
   p.k_per_split = (p.num_k_blocks + splits - 1) / splits;
   p.splits = splits;
   p.swiglu_half = (epi == EPI_BF16_SWIGLU) ? N : 0;
-  // banded tile order once B (N x K bf16) reaches 64 MB, half of L2; CPB_GEMM_BAND (read once) overrides
-  static const int band_env = [] { const char* e = getenv("CPB_GEMM_BAND"); return e ? atoi(e) : 0; }();
-  p.band = band_env > 0 ? band_env : (((size_t)N * K * 2 >= ((size_t)64 << 20)) ? 8 : 1);
+  p.band = tile_band(N, K);
   const int per_tile = epi == EPI_BF16_SWIGLU ? bn / 2 : bn;
   p.num_n_blocks = (N + per_tile - 1) / per_tile;
   p.has_aux = aux != nullptr; p.bias = bias; p.status = status;
 
   CUtensorMap tm[4];
   int rc;
-  {
-    uint64_t dims[2], strides[2]; uint32_t box[2];
-    if (a_mn) { dims[0] = (uint64_t)M; dims[1] = (uint64_t)K; box[0] = 64; box[1] = GEMM_BK; }
-    else      { dims[0] = (uint64_t)K; dims[1] = (uint64_t)M; box[0] = GEMM_BK; box[1] = GEMM_BM; }
-    strides[0] = 0; strides[1] = (uint64_t)lda * 2;
-    if ((rc = encode_tmap(&tm[0], A, 2, 2, dims, strides, box, 1)) != CPB_OK) return rc;
-  }
-  {
-    uint64_t dims[2], strides[2]; uint32_t box[2];
-    const uint64_t b_rows = (epi == EPI_BF16_SWIGLU) ? (uint64_t)2 * N : (uint64_t)N;
-    if (b_mn) { dims[0] = b_rows; dims[1] = (uint64_t)K; box[0] = 64; box[1] = GEMM_BK; }
-    else      { dims[0] = (uint64_t)K; dims[1] = b_rows; box[0] = GEMM_BK; box[1] = bn / 2; }
-    strides[0] = 0; strides[1] = (uint64_t)ldb * 2;
-    if ((rc = encode_tmap(&tm[1], B, 2, 2, dims, strides, box, 1)) != CPB_OK) return rc;
-  }
+  const int b_rows = epi == EPI_BF16_SWIGLU ? 2 * N : N;
+  if ((rc = a_mn ? mnmajor_tmap(&tm[0], A, M, K, lda) : kmajor_tmap(&tm[0], A, M, K, lda, GEMM_BM)) != CPB_OK) return rc;
+  if ((rc = b_mn ? mnmajor_tmap(&tm[1], B, b_rows, K, ldb) : kmajor_tmap(&tm[1], B, b_rows, K, ldb, bn / 2)) != CPB_OK) return rc;
   {
     // one store box = 32 rows x 128 bytes; the map's extents clip the edges of C
     const int eb = (epi == EPI_F32 || epi == EPI_F32_ACC) ? 4 : 2;
@@ -444,6 +450,43 @@ extern "C" int cpb_gemm_bf16(const void* A, const void* B, void* C, void* aux, c
   lc.attrs = &at; lc.numAttrs = 1;
   CPB_CUDA_OK(cudaLaunchKernelEx(&lc, gemm_add_partials_kernel, (float*)C, (const float4*)partials, (unsigned)N / 4, total4, (long)ldc, splits - 1));
   return check_launch("gemm_add_partials");
+}
+
+// Cross entropy of the language-model head without its logits: logits = x w^T (x [M,K], w [N,K], both K-major) stay in tensor memory.
+// dlogits == null: per row and 256-wide tile (max, sum of exponentials) to stats [ceil(N / 256)][M] and the target's logit; otherwise
+// dlogits (bf16 [M,N], row stride ldc) = (softmax - onehot) * grad_scale from row_coef (cpb_xent_rows).
+//
+// The second pass computes the logits again, 2 K operations for each, where storing them in fp32 moves 4 bytes for the GEMM and 4
+// more for the kernel that turns them into dlogits.
+extern "C" int cpb_gemm_head(const void* x, const void* w, void* dlogits, const int64_t* targets, float* stats, float* target_logit,
+                             const float* row_coef, int M, int N, int K, int ldx, int ldw, int ldc, int n_valid, float grad_scale,
+                             int* status, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return set_error(CPB_ERR_ARG, "gemm_head: empty problem %dx%dx%d", M, N, K);
+  if ((N % 8) || (K % 8) || (ldx % 8) || (ldw % 8) || (dlogits && (ldc % 8)))
+    return set_error(CPB_ERR_ARG, "gemm_head: N,K,ldx,ldw,ldc must be multiples of 8 (got N=%d K=%d ldx=%d ldw=%d ldc=%d)", N, K, ldx, ldw, ldc);
+  if (n_valid <= 0 || n_valid > N) return set_error(CPB_ERR_ARG, "gemm_head: n_valid=%d outside 1..%d", n_valid, N);
+  if (dlogits ? row_coef == nullptr : (stats == nullptr || target_logit == nullptr)) return set_error(CPB_ERR_ARG, "gemm_head: missing buffers");
+  GemmParams p{};
+  p.M = M; p.N = N; p.K = K; p.epi = dlogits ? EPI_HEAD_GRAD : EPI_HEAD_STATS;
+  p.num_m_tiles = (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM);
+  p.num_n_blocks = (N + 255) / 256;
+  p.num_k_blocks = p.k_per_split = (K + GEMM_BK - 1) / GEMM_BK;
+  p.splits = 1;
+  p.band = tile_band(N, K);
+  p.head = HeadParams{targets, (float2*)stats, target_logit, (const float2*)row_coef, n_valid, grad_scale};
+  p.status = status;
+  CUtensorMap tm[4];
+  int rc;
+  if ((rc = kmajor_tmap(&tm[0], x, M, K, ldx, GEMM_BM)) != CPB_OK) return rc;
+  if ((rc = kmajor_tmap(&tm[1], w, N, K, ldw, 128)) != CPB_OK) return rc;
+  tm[2] = tm[0];
+  if (dlogits) {
+    uint64_t dims[2] = {(uint64_t)N, (uint64_t)M}, strides[2] = {0, (uint64_t)ldc * 2};
+    uint32_t box[2] = {64, 32};
+    if ((rc = encode_tmap(&tm[2], dlogits, 2, 2, dims, strides, box, 1)) != CPB_OK) return rc;
+  }
+  tm[3] = tm[2];
+  return launch_pair<256, false, false>(tm, p, stream);
 }
 
 // How often the accumulating GEMM of this shape should split K (at least 1): the caller brings the workspace.

@@ -22,6 +22,18 @@ enum : int {
   EPI_F32_ACC = 2,     // C(f32) += acc (+bias)
   EPI_BF16_GELU = 3,   // C(bf16) = gelu_tanh(acc + bias); aux(bf16) = acc + bias (pre-activation) when aux != null
   EPI_BF16_SWIGLU = 4, // B tile = [gate rows | up rows]; C(bf16)[:, n] = silu(g)*u ; aux gets [g | u] when aux != null
+  EPI_HEAD_STATS = 5,  // language-model head: (max, sum of exponentials) of the tile's columns per row, no C
+  EPI_HEAD_GRAD = 6,   // C(bf16) = (softmax - onehot(target)) * grad_scale from the rows' (max, grad_scale / sum)
+};
+
+// Cross entropy in the epilogue of the head's GEMM (xent.cu has the kernel between the two passes).
+struct HeadParams {
+  const int64_t* targets;    // [M]; a row whose target is outside [0, n_valid) has neither loss nor gradient
+  float2* stats;             // [tiles along N][M] (max, sum of exp(x - max))
+  float* target_logit;       // [M], written where the target is in range
+  const float2* row_coef;    // [M] (max, grad_scale / sum), (max, 0) for ignored rows
+  int n_valid;               // columns from here on are padding
+  float grad_scale;
 };
 
 struct GemmParams {
@@ -34,6 +46,7 @@ struct GemmParams {
   int band;            // pair-rows per band of the tile order (1 = rows of tiles, columns fastest)
   int has_aux;
   const float* bias;
+  HeadParams head;
   int* status;
 };
 
@@ -101,6 +114,105 @@ struct WarpStore {
 __device__ __forceinline__ void pack_row(const float (&f)[64], uint32_t (&v)[32]) {
 #pragma unroll
   for (int j = 0; j < 32; ++j) v[j] = pack_bf16(f[2 * j], f[2 * j + 1]);
+}
+
+__device__ __forceinline__ float head_exp(float x, float m) { return ex2f((x - m) * 1.4426950408889634f); }
+
+// f[at] without dynamic register indexing (at in [0, 64))
+__device__ __forceinline__ float pick64(const float (&f)[64], int at) {
+  float r = 0.f;
+#pragma unroll
+  for (int j = 0; j < 64; ++j) r = j == at ? f[j] : r;
+  return r;
+}
+
+// What a thread needs of its row, read before the accumulator is waited for.
+struct HeadRow {
+  int target;                // column, or negative
+  float2 coef;
+};
+__device__ __forceinline__ HeadRow head_row(const GemmParams& p, int row) {
+  HeadRow h{-1, {0.f, 0.f}};
+  if (p.epi >= EPI_HEAD_STATS && row < p.M) {
+    const int64_t t = __ldg(p.head.targets + row);
+    h.target = t >= 0 && t < p.head.n_valid ? (int)t : -1;
+    if (p.epi == EPI_HEAD_GRAD) h.coef = __ldg(p.head.row_coef + row);
+  }
+  return h;
+}
+
+// Bound by the main loop from a K of about 300 on: a tile's 256 exponentials per thread take the special-function unit 2048 cycles,
+// 64 of K take 370 ns.
+template <int BN, class Release>
+__device__ __forceinline__ void head_epilogue(const GemmParams& p, const CUtensorMap* tmC, WarpStore& ws, uint32_t t_row, int row0, int nb,
+                                              int lane, const HeadRow& h, Release release) {
+  const int row = row0 + lane;
+  const bool live = row0 < p.M;
+  float m = -INFINITY, s = 0.f;
+#pragma unroll 1
+  for (int c = 0; c < BN; c += 64) {
+    const int col = nb * BN + c;
+    float f[64];
+    tmem_ld32(t_row + c, *(uint32_t(*)[32])&f[0]);
+    tmem_ld32(t_row + c + 32, *(uint32_t(*)[32])&f[32]);
+    tmem_wait_ld();
+    if (c + 64 == BN) release();
+    if (!live || col >= p.N) continue;
+    const int at = h.target - col;
+    const bool hit = at >= 0 && at < 64;
+    if (p.epi == EPI_HEAD_STATS) {
+      if (col >= p.head.n_valid) continue;
+      if (hit) p.head.target_logit[row] = pick64(f, at);
+      if (col + 64 > p.head.n_valid) {
+#pragma unroll
+        for (int j = 0; j < 64; ++j) if (col + j >= p.head.n_valid) f[j] = -INFINITY;
+      }
+      float mx[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        mx[q] = fmaxf(f[q], f[q + 4]);
+#pragma unroll
+        for (int j = 8; j < 64; j += 8) mx[q] = fmax3(mx[q], f[j + q], f[j + q + 4]);
+      }
+      const float mt = fmax3(fmaxf(mx[0], mx[1]), mx[2], mx[3]);
+      if (mt > m) { s = m == -INFINITY ? s : s * head_exp(m, mt); m = mt; }
+      // a row of nothing but -inf so far adds nothing; NaN gets into the sum, whatever the maximum says
+      const float ref = m == -INFINITY ? 0.f : m;
+      const uint64_t nm = pack_f32x2(-ref, -ref), l2e = pack_f32x2(1.4426950408889634f, 1.4426950408889634f);
+      uint64_t acc[2] = {pack_f32x2(0.f, 0.f), pack_f32x2(0.f, 0.f)};
+#pragma unroll
+      for (int j = 0; j < 64; j += 2) {
+        float x0, x1;
+        unpack_f32x2(mul_f32x2(add_f32x2(pack_f32x2(f[j], f[j + 1]), nm), l2e), x0, x1);
+        acc[(j >> 1) & 1] = add_f32x2(acc[(j >> 1) & 1], pack_f32x2(ex2f(x0), ex2f(x1)));
+      }
+      float a, b;
+      unpack_f32x2(add_f32x2(acc[0], acc[1]), a, b);
+      s += a + b;
+    } else {
+      const uint64_t nm = pack_f32x2(-h.coef.x, -h.coef.x), l2e = pack_f32x2(1.4426950408889634f, 1.4426950408889634f);
+      const uint64_t inv = pack_f32x2(h.coef.y, h.coef.y);
+#pragma unroll
+      for (int j = 0; j < 64; j += 2) {
+        float x0, x1;
+        unpack_f32x2(mul_f32x2(add_f32x2(pack_f32x2(f[j], f[j + 1]), nm), l2e), x0, x1);
+        unpack_f32x2(mul_f32x2(pack_f32x2(ex2f(x0), ex2f(x1)), inv), f[j], f[j + 1]);
+      }
+      if (col + 64 > p.head.n_valid) {
+#pragma unroll
+        for (int j = 0; j < 64; ++j) if (col + j >= p.head.n_valid) f[j] = 0.f;
+      }
+      if (hit) {
+#pragma unroll
+        for (int j = 0; j < 64; ++j) f[j] = j == at ? f[j] - p.head.grad_scale : f[j];
+      }
+      uint32_t v[32];
+      pack_row(f, v);
+      ws.fill(ws.row_ptr(lane), lane, v);
+      ws.store(tmC, col, row0);
+    }
+  }
+  if (p.epi == EPI_HEAD_STATS && row < p.M) p.head.stats[(size_t)nb * p.M + row] = make_float2(m, s);
 }
 
 // Epilogue of one 32-row slice of a 128 x BN accumulator tile: `t_row` is the tensor-memory address of this warp's lanes at

@@ -203,9 +203,68 @@ xent_smem_kernel(const float* __restrict__ logits, const int64_t* __restrict__ t
   asm volatile("barrier.cluster.wait.aligned;" ::: "memory");      // no rank leaves while another may still read its pair
 }
 
+// Between the two passes of the head's GEMM (cpb_gemm_head): per row the maximum and the sum of exponentials over all column tiles,
+// the loss, and the coefficients of the gradient.  A block takes 32 rows, a warp every eighth tile of them (the lanes' pairs are
+// adjacent in memory), and warp 0 adds the eight parts, always in the same order.
+constexpr int XR_WARPS = 8;
+__global__ void __launch_bounds__(XR_WARPS * 32)
+xent_rows_kernel(const float2* __restrict__ stats, const float* __restrict__ target_logit, const int64_t* __restrict__ targets,
+                 float2* __restrict__ row_coef, float* __restrict__ row_loss, float* __restrict__ loss_sum, int rows, int tiles, int V,
+                 float grad_scale, int* status) {
+  __shared__ float2 part[XR_WARPS][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int row = blockIdx.x * 32 + lane;
+  float m = -INFINITY, s = 0.f;
+  // a part without a finite maximum contributes its sum as it is: zero, or NaN
+  const auto add = [&](float2 v) {
+    const float mn = fmaxf(m, v.x);
+    s = (m == -INFINITY ? s : s * __expf(m - mn)) + (v.x == -INFINITY ? v.y : v.y * __expf(v.x - mn));
+    m = mn;
+  };
+  if (row < rows) {
+    int t = warp;
+    for (; t + 3 * XR_WARPS < tiles; t += 4 * XR_WARPS) {
+      float2 v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = stats[(size_t)(t + k * XR_WARPS) * rows + row];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) add(v[k]);
+    }
+    for (; t < tiles; t += XR_WARPS) add(stats[(size_t)t * rows + row]);
+  }
+  part[warp][lane] = make_float2(m, s);
+  __syncthreads();
+  if (warp != 0) return;
+  for (int k = 1; k < XR_WARPS; ++k) add(part[k][lane]);
+  float l = 0.f;
+  if (row < rows) {
+    const int64_t tgt = targets[row];
+    if (tgt >= V) report(status, ST_BAD_INDEX, 1200, (int)tgt);
+    const bool ignore = tgt < 0 || tgt >= V;
+    if (!ignore) l = m + __logf(s) - target_logit[row];
+    if (row_loss) row_loss[row] = l;
+    if (row_coef) row_coef[row] = make_float2(m, ignore ? 0.f : grad_scale / s);
+  }
+  if (loss_sum) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    if (lane == 0) atomicAdd(loss_sum, l);
+  }
+}
+
 }  // namespace cpb
 
 using namespace cpb;
+
+// stats [tiles][rows] (max, sum) pairs and target_logit [rows] of cpb_gemm_head; row_coef [rows] pairs, row_loss [rows] and
+// loss_sum (fp32 scalar, +=) are optional.  V: columns that are real vocabulary.
+extern "C" int cpb_xent_rows(const float* stats, const float* target_logit, const int64_t* targets, float* row_coef, float* row_loss,
+                             float* loss_sum, int rows, int tiles, int V, float grad_scale, int* status, cudaStream_t stream) {
+  if (rows <= 0) return CPB_OK;
+  xent_rows_kernel<<<(rows + 31) / 32, XR_WARPS * 32, 0, stream>>>((const float2*)stats, target_logit, targets, (float2*)row_coef, row_loss,
+                                                                    loss_sum, rows, tiles, V, grad_scale, status);
+  return check_launch("xent_rows");
+}
 
 // logits fp32 [rows, Vcols] (row stride ld_logits, multiple of 4) of which the first V columns are real vocabulary;
 // dlogits bf16 [rows, Vcols] (row stride multiple of 4) or null; loss_sum (fp32 scalar, +=) and row_loss [rows] optional.
