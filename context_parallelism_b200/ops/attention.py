@@ -106,23 +106,27 @@ class _FlashAttnPackedFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, qkv, Hq, Hkv, D, scale, causal):
-        B, T = qkv.shape[:2]
-        x = qkv.view(B, T, Hq + 2 * Hkv, D)
+        B, T, W = qkv.shape
+        dev = qkv.device
         # allocated in the shape it is returned in: autograd refuses in-place operations on a view made in here
-        out = torch.empty((B, T, Hq * D), dtype=torch.bfloat16, device=qkv.device)
-        _, lse = flash_fwd(x[:, :, :Hq], x[:, :, Hq:Hq + Hkv], x[:, :, Hq + Hkv:], scale, causal, out=out.view(B, T, Hq, D))
-        ctx.save_for_backward(x, out, lse)
+        out = torch.empty((B, T, Hq * D), dtype=torch.bfloat16, device=dev)
+        if qkv.is_contiguous() and qkv.data_ptr() % 16 == 0 and qkv.dtype == torch.bfloat16 and W == (Hq + 2 * Hkv) * D:
+            lse, x = torch.empty((B, Hq, T), dtype=torch.float32, device=dev), qkv.data_ptr()
+            nv.call("flash_fwd", x, x + 2 * Hq * D, x + 2 * (Hq + Hkv) * D, out.data_ptr(), lse.data_ptr(), B, T, T, Hq, Hkv, D, D, W, T * W, D, W,
+                    T * W, scale, int(causal), 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, nv.status_for(dev).ptr(), nv.stream_ptr(dev))
+        else:
+            x = qkv.view(B, T, Hq + 2 * Hkv, D)
+            _, lse = flash_fwd(x[:, :, :Hq], x[:, :, Hq:Hq + Hkv], x[:, :, Hq + Hkv:], scale, causal, out=out.view(B, T, Hq, D))
+        ctx.save_for_backward(qkv, out, lse)
         ctx.meta = (Hq, Hkv, scale, causal)
         return out
 
     @staticmethod
     def backward(ctx, dout):
         from .attention_bwd import flash_bwd_packed
-        x, out, lse = ctx.saved_tensors
+        qkv, out, lse = ctx.saved_tensors
         Hq, Hkv, scale, causal = ctx.meta
-        heads = (*out.shape[:2], Hq, -1)
-        dqkv = flash_bwd_packed(x, Hq, Hkv, out.view(heads), lse, dout.reshape(heads), scale, causal)
-        return dqkv.view(*dqkv.shape[:2], -1), None, None, None, None, None
+        return flash_bwd_packed(qkv, Hq, Hkv, out, lse, dout, scale, causal), None, None, None, None, None
 
 
 # ATTN_FP32=1: differentiable attention goes through the fp32-accurate CUDA-core kernels (parity runs); set by the engine.

@@ -1,6 +1,7 @@
 """Host wrapper of the tcgen05 flash-attention backward (``csrc/kernels/attention_bwd.cu``)."""
 from __future__ import annotations
 
+import functools
 import os
 from typing import Optional
 
@@ -24,16 +25,21 @@ def padded_q_pos(Tq: int, device, q_pos: Optional[torch.Tensor]) -> torch.Tensor
     return out
 
 
+def bwd_chunk(B: int, Tq: int, Tk: int, Hq: int, Hkv: int, D: int, causal: bool, k_off: int, local: bool) -> int:
+    """Pairs of (query head, query tile) per CTA of the backward kernel, 0 for whole sweeps (the library's rule)."""
+    return nv.lib().cpb_flash_bwd_chunk(B, Tq, Tk, Hq, Hkv, D, int(causal), k_off, int(local))
+
+
 def flash_bwd_prep(o: torch.Tensor, do: torch.Tensor, lse: torch.Tensor, dq: Optional[torch.Tensor] = None,
                    q_pos: Optional[torch.Tensor] = None, qpos_pad: Optional[torch.Tensor] = None):
     """``delta = rowsum(dO∘O)`` and ``lse·log2(e)`` padded to a multiple of 128 rows.  The same launch clears the fp32
-    accumulator ``dq`` (shaped like ``o``) and fills ``qpos_pad`` as :func:`padded_q_pos` does, when they are given."""
+    accumulator ``dq`` (any contiguous tensor of a multiple of four values) and fills ``qpos_pad`` as :func:`padded_q_pos` does, when they are given."""
     B, Tq, Hq, D = o.shape
     tq_pad = (Tq + 127) // 128 * 128
     delta = torch.empty((B, Hq, tq_pad), dtype=torch.float32, device=o.device)
     lse2 = torch.empty_like(delta)
-    nv.call("flash_bwd_prep", nv.ptr(o), nv.ptr(do), nv.ptr(lse), nv.ptr(delta), nv.ptr(lse2), nv.ptr(dq), nv.ptr(q_pos),
-            nv.ptr(qpos_pad), nv.i(B), nv.i(Tq), nv.i(Hq), nv.i(D), nv.i(tq_pad), nv.stream_ptr(o.device))
+    nv.call("flash_bwd_prep", nv.ptr(o), nv.ptr(do), nv.ptr(lse), nv.ptr(delta), nv.ptr(lse2), nv.ptr(dq),
+            0 if dq is None else dq.numel(), nv.ptr(q_pos), nv.ptr(qpos_pad), nv.i(B), nv.i(Tq), nv.i(Hq), nv.i(D), nv.i(tq_pad), nv.stream_ptr(o.device))
     return delta, lse2
 
 
@@ -42,7 +48,7 @@ def flash_bwd_delta(o: torch.Tensor, do: torch.Tensor) -> torch.Tensor:
     B, Tq, Hq, D = o.shape
     tq_pad = (Tq + 127) // 128 * 128
     delta = torch.empty((B, Hq, tq_pad), dtype=torch.float32, device=o.device)
-    nv.call("flash_bwd_prep", nv.ptr(o), nv.ptr(do), nv.ptr(None), nv.ptr(delta), nv.ptr(None), nv.ptr(None), nv.ptr(None), nv.ptr(None),
+    nv.call("flash_bwd_prep", nv.ptr(o), nv.ptr(do), nv.ptr(None), nv.ptr(delta), nv.ptr(None), nv.ptr(None), 0, nv.ptr(None), nv.ptr(None),
             nv.i(B), nv.i(Tq), nv.i(Hq), nv.i(D), nv.i(tq_pad), nv.stream_ptr(o.device))
     return delta
 
@@ -52,7 +58,7 @@ def flash_bwd_lse2(lse: torch.Tensor, D: int) -> torch.Tensor:
     B, Hq, Tq = lse.shape
     tq_pad = (Tq + 127) // 128 * 128
     lse2 = torch.empty((B, Hq, tq_pad), dtype=torch.float32, device=lse.device)
-    nv.call("flash_bwd_prep", nv.ptr(None), nv.ptr(None), nv.ptr(lse), nv.ptr(None), nv.ptr(lse2), nv.ptr(None), nv.ptr(None), nv.ptr(None),
+    nv.call("flash_bwd_prep", nv.ptr(None), nv.ptr(None), nv.ptr(lse), nv.ptr(None), nv.ptr(lse2), nv.ptr(None), 0, nv.ptr(None), nv.ptr(None),
             nv.i(B), nv.i(Tq), nv.i(Hq), nv.i(D), nv.i(tq_pad), nv.stream_ptr(lse.device))
     return lse2
 
@@ -75,7 +81,7 @@ def flash_bwd_core(q, k, v, do, lse2, delta, qpos_pad, scale, causal, k_off, dq_
                 nv.l(qs[0]), nv.l(qs[1]), nv.l(qs[2]), nv.l(ks[0]), nv.l(ks[1]), nv.l(ks[2]),
                 nv.f(scale), nv.i(causal), nv.i(k_off), nv.ptr(qpos_pad), nv.i(2 if route is not None else int(dkv_accumulate)), nv.l(dkv_st or Hkv * D),
                 nv.ptr(route[0] if route else None), nv.ptr(route[1] if route else None),
-                nv.i(route[2] if route else 0), nv.i(route[3] if route else 0), st.ptr(), nv.stream_ptr(q.device))
+                nv.i(route[2] if route else 0), nv.i(route[3] if route else 0), 0, 0, st.ptr(), nv.stream_ptr(q.device))
         return
     if D == 128:
         nv.call("flash_bwd128", nv.ptr(q), nv.ptr(k), nv.ptr(v), nv.ptr(do), nv.ptr(lse2), nv.ptr(delta), nv.ptr(dq_f32),
@@ -83,7 +89,7 @@ def flash_bwd_core(q, k, v, do, lse2, delta, qpos_pad, scale, causal, k_off, dq_
                 nv.l(qs[0]), nv.l(qs[1]), nv.l(qs[2]), nv.l(ks[0]), nv.l(ks[1]), nv.l(ks[2]),
                 nv.f(scale), nv.i(causal), nv.i(k_off), nv.ptr(qpos_pad), nv.i(2 if route is not None else int(dkv_accumulate)), nv.l(dkv_st or Hkv * D),
                 nv.ptr(route[0] if route else None), nv.ptr(route[1] if route else None),
-                nv.i(route[2] if route else 0), nv.i(route[3] if route else 0), st.ptr(), nv.stream_ptr(q.device))
+                nv.i(route[2] if route else 0), nv.i(route[3] if route else 0), 0, 0, st.ptr(), nv.stream_ptr(q.device))
         return
     assert dkv_st in (0, Hkv * D), "the general kernel writes dense dK/dV"
     nv.call("flash_bwd", nv.ptr(q), nv.ptr(k), nv.ptr(v), nv.ptr(do), nv.ptr(lse2), nv.ptr(delta), nv.ptr(dq_f32),
@@ -117,15 +123,42 @@ def _aligned(t: torch.Tensor) -> torch.Tensor:
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
+@functools.lru_cache(maxsize=4096)
+def _bwd_plan(B: int, Tq: int, Tk: int, Hq: int, Hkv: int, D: int, causal: bool, k_off: int, local: bool):
+    """``(pairs per CTA, floats of workspace)`` of a whole gradient."""
+    chunk, tq_pad = bwd_chunk(B, Tq, Tk, Hq, Hkv, D, causal, k_off, local), (Tq + 127) // 128 * 128
+    return chunk, B * D * (Tq * Hq + (2 * Tk * Hkv if chunk else 0)) + (2 * B * Hq + 1) * tq_pad
+
+
+def _bwd_whole(q: int, k: int, v: int, o, do, lse, dq: int, dk: int, dv: int, dims, strides, dq_st: int, dkv_st: int, scale: float, causal: bool,
+               k_off: int, q_pos) -> None:
+    """Preparation, kernel and cast behind one call of the library; ``q`` .. ``dv`` are addresses, ``strides`` those of q and of k/v."""
+    chunk, floats = _bwd_plan(*dims, bool(causal), k_off, q_pos is None)
+    dev = o.device
+    ws = torch.empty(floats, dtype=torch.float32, device=dev)
+    nv.LAUNCHES[0] += 2                                              # three kernels
+    nv.call("flash_attn_bwd", q, k, v, o.data_ptr(), do.data_ptr(), lse.data_ptr(), ws.data_ptr(), dq, dk, dv, *dims, *strides, dq_st, dkv_st,
+            scale, int(causal), k_off, nv.ptr(q_pos), chunk, nv.status_for(dev).ptr(), nv.stream_ptr(dev))
+
+
 def flash_bwd_cuda(q, k, v, o, lse, do, scale, causal=True, q_pos=None, k_off=0,
                    dq=None, dk=None, dv=None, dkv_accumulate=False):
     B, Tq, Hq, D = q.shape
     Tk, Hkv = k.shape[1], k.shape[2]
     q, k, v = _launch_ready(q, k, v)
     do, o = _aligned(do), _aligned(o)
+    pos32 = None if q_pos is None else q_pos.to(torch.int32).contiguous()
+    # a launch timer (nv.profile_start) wants the launches one by one
+    if dq is None and not dkv_accumulate and nv._PROFILE is None and not (D == 64 and _USE_GENERAL_D64):
+        dq = torch.empty((B, Tq, Hq, D), dtype=torch.bfloat16, device=q.device)
+        dk = torch.empty((B, Tk, Hkv, D), dtype=torch.bfloat16, device=q.device)
+        dv = torch.empty_like(dk)
+        _bwd_whole(q.data_ptr(), k.data_ptr(), v.data_ptr(), o, do, lse, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), (B, Tq, Tk, Hq, Hkv, D),
+                   (*_strides(q), *_strides(k)), Hq * D, Hkv * D, scale, causal, k_off, pos32)
+        return dq, dk, dv
     dq_f32 = torch.empty((B, Tq, Hq, D), dtype=torch.float32, device=q.device) if dq is None else dq
     qpos_pad = torch.empty((Tq + 127) // 128 * 128, dtype=torch.int32, device=q.device)
-    delta, lse2 = flash_bwd_prep(o, do, lse, dq_f32 if dq is None else None, None if q_pos is None else q_pos.to(torch.int32).contiguous(), qpos_pad)
+    delta, lse2 = flash_bwd_prep(o, do, lse, dq_f32 if dq is None else None, pos32, qpos_pad)
     if dkv_accumulate:
         assert dk is not None and dv is not None and dk.dtype == torch.float32
     else:
@@ -138,23 +171,18 @@ def flash_bwd_cuda(q, k, v, o, lse, do, scale, causal=True, q_pos=None, k_off=0,
 
 
 def flash_bwd_packed(qkv: torch.Tensor, Hq: int, Hkv: int, o, lse, do, scale: float, causal: bool = True) -> torch.Tensor:
-    """Gradient of packed projections ``qkv [B,T,Hq+2·Hkv,D]`` (query heads, then key heads, then value heads), every part
-    written where it belongs: three separate gradients cost autograd a zero-filled full-size tensor and a copy each, and
-    two full-size additions."""
-    B, T, H, D = qkv.shape
-    q, k, v = qkv[:, :, :Hq], qkv[:, :, Hq:Hq + Hkv], qkv[:, :, Hq + Hkv:]
-    dqkv = torch.empty((B, T, H, D), dtype=torch.bfloat16, device=qkv.device)
-    if D == 64 and _USE_GENERAL_D64:
-        for part, g in zip((dqkv[:, :, :Hq], dqkv[:, :, Hq:Hq + Hkv], dqkv[:, :, Hq + Hkv:]),
-                           flash_bwd_cuda(q, k, v, o, lse, do, scale, causal)):
-            part.copy_(g)
+    """Gradient of packed projections ``qkv`` (``[B,T,Hq+2·Hkv,D]`` or ``[B,T,(Hq+2·Hkv)·D]``: query heads, then key heads, then value
+    heads), every part written where it belongs: three separate gradients cost autograd a zero-filled full-size tensor and a copy
+    each, and two full-size additions."""
+    B, T, H = qkv.shape[0], qkv.shape[1], Hq + 2 * Hkv
+    W = qkv.shape[2] * (qkv.shape[3] if qkv.dim() == 4 else 1)
+    D = W // H
+    if nv._PROFILE is None and not (D == 64 and _USE_GENERAL_D64) and qkv.is_contiguous() and qkv.data_ptr() % 16 == 0:
+        dqkv = torch.empty_like(qkv)
+        x, g, k_at, v_at = qkv.data_ptr(), dqkv.data_ptr(), 2 * Hq * D, 2 * (Hq + Hkv) * D
+        _bwd_whole(x, x + k_at, x + v_at, _aligned(o), _aligned(do), lse, g, g + k_at, g + v_at, (B, T, T, Hq, Hkv, D),
+                   (D, W, T * W, D, W, T * W), W, W, scale, causal, 0, None)
         return dqkv
-    q, k, v = _launch_ready(q, k, v)
-    do, o = _aligned(do), _aligned(o)
-    dq_f32 = torch.empty((B, T, Hq, D), dtype=torch.float32, device=qkv.device)
-    qpos_pad = torch.empty((T + 127) // 128 * 128, dtype=torch.int32, device=qkv.device)
-    delta, lse2 = flash_bwd_prep(o, do, lse, dq_f32, None, qpos_pad)
-    flash_bwd_core(q, k, v, do, lse2, delta, qpos_pad, scale, causal, 0, dq_f32, dqkv[:, :, Hq:Hq + Hkv], dqkv[:, :, Hq + Hkv:], False,
-                   dkv_st=H * D)
-    nv.call("cast_f32_bf16_rows", nv.ptr(dq_f32), nv.ptr(dqkv), nv.l(B * T), nv.i(Hq * D), nv.l(H * D), nv.f(1.0), nv.stream_ptr(qkv.device))
-    return dqkv
+    x, heads = qkv.view(B, T, H, D), (B, T, Hq, D)
+    grads = flash_bwd_cuda(x[:, :, :Hq], x[:, :, Hq:Hq + Hkv], x[:, :, Hq + Hkv:], o.reshape(heads), lse, do.reshape(heads), scale, causal)
+    return torch.cat(grads, 2).view(qkv.shape)

@@ -30,6 +30,9 @@
 #include "common.cuh"
 #include <type_traits>
 #include "host_utils.h"
+#include <functional>
+#include <queue>
+#include <vector>
 
 #include <stdlib.h>
 
@@ -452,17 +455,18 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
 // delta[b,h,t] = sum_d dO*O ; lse2 = lse*log2(e) ; padding rows get delta 0 / lse2 +inf.  Rows are taken in the order of o and
 // dout, D / 8 lanes with one 16-byte load each per row, so a warp reads 512 contiguous bytes of both.  The same pass
-// clears the fp32 dQ accumulator and pads the query positions, which were four launches of their own.
+// clears the fp32 accumulators and pads the query positions, which were four launches of their own.
 template <int D>
 __global__ void bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
                                 const float* __restrict__ lse, float* __restrict__ delta, float* __restrict__ lse2,
-                                float* __restrict__ dq, const int* __restrict__ q_pos, int* __restrict__ q_pos_pad,
+                                float4* __restrict__ acc, size_t acc4, const int* __restrict__ q_pos, int* __restrict__ q_pos_pad,
                                 int B, int Tq, int Hq, int Tq_pad) {
   constexpr int LPR = D / 8;                                 // lanes per row
   const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (q_pos_pad != nullptr)
     for (size_t t = tid; t < (size_t)Tq_pad; t += (size_t)gridDim.x * blockDim.x)
       q_pos_pad[t] = t < (size_t)Tq ? (q_pos != nullptr ? q_pos[t] : (int)t) : 0x7fffffff;
+  for (size_t i = tid; i < acc4; i += (size_t)gridDim.x * blockDim.x) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   const int sub = threadIdx.x % LPR;
   const size_t nrow = (size_t)B * Hq * Tq_pad;
   for (size_t w = tid / LPR; w < nrow; w += (size_t)gridDim.x * blockDim.x / LPR) {   // LPR lanes share a row
@@ -490,10 +494,6 @@ __global__ void bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, const __nv_
       const float l = lse[((size_t)b * Hq + h) * Tq + t];
       lse2[out] = (l == -INFINITY) ? INFINITY : l * 1.4426950408889634f;
     }
-    if (dq) {
-      *(float4*)(dq + off) = make_float4(0.f, 0.f, 0.f, 0.f);
-      *(float4*)(dq + off + 4) = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
   }
 }
 
@@ -510,12 +510,12 @@ using namespace cpb;
 
 // o and dout are contiguous [B,Tq,Hq,D]; delta/lse2 are [B,Hq,Tq_pad] with Tq_pad = ceil(Tq/128)*128.
 // Either output may be null (then its inputs are not read): the Ulysses backward computes delta where the
-// tokens live and lse2 where the heads live.  dq (fp32, shaped like o), when given, is set to zero; q_pos_pad [Tq_pad], when
+// tokens live and lse2 where the heads live.  acc (fp32, acc_n elements, a multiple of four), when given, is set to zero; q_pos_pad [Tq_pad], when
 // given, receives q_pos (int32 [Tq], or 0 .. Tq-1 when null) followed by INT_MAX.
-extern "C" int cpb_flash_bwd_prep(const void* o, const void* dout, const float* lse, float* delta, float* lse2, float* dq,
+extern "C" int cpb_flash_bwd_prep(const void* o, const void* dout, const float* lse, float* delta, float* lse2, float* acc, long acc_n,
                                   const int* q_pos, int* q_pos_pad, int B, int Tq, int Hq, int D, int Tq_pad, cudaStream_t stream) {
   if (D != 64 && D != 128) return set_error(CPB_ERR_ARG, "flash_bwd_prep: head_dim %d not in {64,128}", D);
-  if ((delta != nullptr && (((uintptr_t)o | (uintptr_t)dout) & 15)) || ((uintptr_t)dq & 15))
+  if ((delta != nullptr && (((uintptr_t)o | (uintptr_t)dout) & 15)) || ((uintptr_t)acc & 15) || (acc_n & 3))
     return set_error(CPB_ERR_ARG, "flash_bwd_prep: tensors must be 16-byte aligned");
   const size_t rows_per_block = 256 / (D / 8);
   const size_t nrow = (size_t)B * Hq * Tq_pad;
@@ -523,7 +523,8 @@ extern "C" int cpb_flash_bwd_prep(const void* o, const void* dout, const float* 
   const size_t cap = (size_t)sm_count() * 32;
   if (g > cap) g = cap;
   auto kern = D == 64 ? bwd_prep_kernel<64> : bwd_prep_kernel<128>;
-  kern<<<(int)g, 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, lse, delta, lse2, dq, q_pos, q_pos_pad, B, Tq, Hq, Tq_pad);
+  kern<<<(int)g, 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, lse, delta, lse2, (float4*)acc, acc != nullptr ? (size_t)acc_n / 4 : 0, q_pos, q_pos_pad,
+                                 B, Tq, Hq, Tq_pad);
   return check_launch("flash_bwd_prep");
 }
 
@@ -575,4 +576,77 @@ extern "C" int cpb_flash_bwd(const void* q, const void* k, const void* v, const 
   if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem::TOTAL)); cfg = true; }
   flash_bwd_kernel<<<grid, FB_THREADS, BwdSmem::TOTAL, stream>>>(tq, tk, tv, tdo, tdq, p);
   return check_launch("flash_bwd");
+}
+
+extern "C" int cpb_flash_bwd64(const void* q, const void* k, const void* v, const void* dout, const float* lse2, const float* delta, float* dq, void* dk,
+                               void* dv, int B, int Tq, int Tk, int Hq, int Hkv, int Tq_pad, long q_sh, long q_st, long q_sb, long k_sh, long k_st,
+                               long k_sb, float scale, int causal, int k_off, const int* q_pos, int dkv_mode, long dkv_st, const uint64_t* route_k,
+                               const uint64_t* route_v, int route_rows, int route_tl, int it_chunk, int local, int* status, cudaStream_t stream);
+extern "C" int cpb_flash_bwd128(const void* q, const void* k, const void* v, const void* dout, const float* lse2, const float* delta, float* dq, void* dk,
+                                void* dv, int B, int Tq, int Tk, int Hq, int Hkv, int Tq_pad, long q_sh, long q_st, long q_sb, long k_sh, long k_st,
+                                long k_sb, float scale, int causal, int k_off, const int* q_pos, int dkv_mode, long dkv_st, const uint64_t* route_k,
+                                const uint64_t* route_v, int route_rows, int route_tl, int it_chunk, int local, int* status, cudaStream_t stream);
+extern "C" int cpb_cast_f32_bf16_rows(const float* in, void* out_q, long rows_q, int cols_q, long q_stride, void* out_k, void* out_v, long rows_k,
+                                      int cols_k, long kv_stride, float scale, cudaStream_t stream);
+
+// The three launches of a whole gradient (preparation, kernel, cast) behind one call: what the host did between them cost more than
+// the kernels of a short sequence.  o, dout dense; dq, dk, dv bf16, tokens dq_st / dkv_st elements apart, batches dense.  ws:
+// B Tq Hq D floats for dQ, twice B Tk Hkv D for dK and dV if chunk > 0 (see cpb_flash_bwd_chunk), 2 B Hq Tq_pad and Tq_pad, in this
+// order, with Tq_pad = Tq rounded up to 128.  q_pos: int32 [Tq], or null for 0 .. Tq-1.
+extern "C" int cpb_flash_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* lse, float* ws, void* dq,
+                                  void* dk, void* dv, int B, int Tq, int Tk, int Hq, int Hkv, int D, long q_sh, long q_st, long q_sb, long k_sh,
+                                  long k_st, long k_sb, long dq_st, long dkv_st, float scale, int causal, int k_off, const int* q_pos, int chunk,
+                                  int* status, cudaStream_t stream) {
+  if (D != 64 && D != 128) return set_error(CPB_ERR_ARG, "flash_attn_bwd: head_dim %d not in {64,128}", D);
+  if ((uintptr_t)ws & 15) return set_error(CPB_ERR_ARG, "flash_attn_bwd: the workspace must be 16-byte aligned");
+  const int Tq_pad = (Tq + 127) / 128 * 128;
+  const long nq = (long)B * Tq * Hq * D, nk = chunk ? (long)B * Tk * Hkv * D : 0;
+  float *delta = ws + nq + 2 * nk, *lse2 = delta + (long)B * Hq * Tq_pad;
+  int* pos = (int*)(lse2 + (long)B * Hq * Tq_pad);
+  int rc = cpb_flash_bwd_prep(o, dout, lse, delta, lse2, ws, nq + 2 * nk, q_pos, pos, B, Tq, Hq, D, Tq_pad, stream);
+  if (rc != CPB_OK) return rc;
+  rc = (D == 64 ? cpb_flash_bwd64 : cpb_flash_bwd128)(q, k, v, dout, lse2, delta, ws, chunk ? (void*)(ws + nq) : dk, chunk ? (void*)(ws + nq + nk) : dv, B, Tq,
+                                                      Tk, Hq, Hkv, Tq_pad, q_sh, q_st, q_sb, k_sh, k_st, k_sb, scale, causal, k_off, pos,
+                                                      chunk ? 3 : 0, chunk ? (long)Hkv * D : dkv_st, nullptr, nullptr, 0, 0, chunk, q_pos == nullptr,
+                                                      status, stream);
+  if (rc != CPB_OK) return rc;
+  return cpb_cast_f32_bf16_rows(ws, dq, (long)B * Tq, Hq * D, dq_st, dk, dv, chunk ? (long)B * Tk : 0, Hkv * D, dkv_st, 1.f, stream);
+}
+
+// How many (query head, query tile) pairs a CTA of the head_dim-64 / 128 kernels should take at most, 0 for whole sweeps.  Whole sweeps
+// are uneven under the causal mask (the first K/V tile meets every query, the last one tile of them) and few when there are few
+// heads; parts even out, but each costs the CTA's start and end and an fp32 addition of its dK / dV, and the sums have to be
+// cleared and cast.  So both ways of handing out the CTAs to the SMs are followed here, with the times that they take.
+extern "C" int cpb_flash_bwd_chunk(int B, int Tq, int Tk, int Hq, int Hkv, int D, int causal, int k_off, int local) {
+  const int nq = (Tq + 127) / 128, n_kt = (Tk + 127) / 128, G = Hq / (Hkv > 0 ? Hkv : 1), hb = Hkv * B, sms = sm_count();
+  if (nq <= 0 || n_kt <= 0 || G <= 0 || hb <= 0 || (D != 64 && D != 128) || (long)n_kt * hb > 16L * sms) return 0;
+  const double tile = D == 64 ? 1.55 : 2.4, start_end = D == 64 ? 4.0 : 5.5;            // us
+  std::vector<int> len(n_kt);
+  for (int k = 0; k < n_kt; ++k) {
+    // positions that are not 0 .. Tq - 1 (a ring rank's): the share that sees the tile falls evenly, near enough
+    long hidden = !causal ? 0 : local ? ((long)k_off + (long)k * 128) / 128 : (long)nq * k / n_kt;
+    len[k] = G * (int)(nq - (hidden < 0 ? 0 : hidden > nq ? nq : hidden));
+  }
+  const auto finish = [&](int chunk) {
+    std::priority_queue<double, std::vector<double>, std::greater<double>> sm;
+    for (int i = 0; i < sms; ++i) sm.push(0.0);
+    double end = 0.0;
+    const auto run = [&](int pairs) { const double t = sm.top() + start_end + pairs * tile; sm.pop(); sm.push(t); end = t > end ? t : end; };
+    if (chunk == 0) {
+      for (int h = 0; h < hb; ++h) for (int k = 0; k < n_kt; ++k) run(len[k]);
+    } else {
+      for (int c = 0; c < G * nq; c += chunk) for (int k = 0; k < n_kt; ++k) if (len[k] > c) for (int h = 0; h < hb; ++h) run(len[k] - c < chunk ? len[k] - c : chunk);
+    }
+    return end;
+  };
+  const double whole = finish(0), extra = 0.5 + (double)B * Tk * Hkv * D * 2 * 14 / 4e6;     // cleared, read and cast at 4 TB/s
+  double best = whole * 0.95;
+  int chunk = 0;
+  for (int parts = 2; parts <= 24; ++parts) {
+    const int c = (G * nq + parts - 1) / parts;
+    if (c < 2) break;
+    const double t = finish(c) + extra;
+    if (t < best) { best = t; chunk = c; }
+  }
+  return chunk;
 }

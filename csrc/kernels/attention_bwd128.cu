@@ -36,6 +36,7 @@
 //
 // Warp roles (768 threads): 0 = TMA loader, 1 = MMA issuer, 2, 3 idle, 4..19 = softmax-gradient warps (thread = key row, 32
 // queries), 20..23 = dQ drain warps (thread = query row).
+#include "attention_bwd.cuh"
 #include "common.cuh"
 #include "host_utils.h"
 
@@ -60,7 +61,9 @@ struct Bwd128Params {
   const int* q_pos;             // [Tq_pad] global positions, INT_MAX in the padding
   void* dk; void* dv;           // [B,Tk,Hkv,D] bf16 (store) or fp32 (accumulate)
   long dkv_st;                  // elements from one token of dk / dv to the next (heads adjacent, batches dense)
-  int dkv_mode;                 // 0 bf16 store, 1 fp32 accumulate, 2 routed red.add (fused ring)
+  int dkv_mode;                 // 0 bf16 store, 1 fp32 accumulate, 2 routed red.add (fused ring), 3 red.add (several CTAs per tile)
+  int it_chunk;                 // pairs of (query head, query tile) per CTA, 0: all (see BwdWork)
+  int local;                    // q_pos is 0 .. Tq - 1: the first visible query tile needs no search
   const uint64_t* route_k;      // mode 2: per chunk of route_rows K/V rows the address of its owner's fp32 accumulator
   const uint64_t* route_v;
   int route_rows, route_tl;
@@ -110,10 +113,12 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   int* qt_start_s = (int*)(tmem_slot + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kt = blockIdx.x, hkv = blockIdx.y, b = blockIdx.z;
+  const BwdWork work = bwd_work(p.it_chunk, (p.Tk + B128_T - 1) / B128_T, p.Hkv, p.B);
+  const int kt = work.kt, hkv = work.hkv, b = work.b;
   const int G = p.Hq / p.Hkv;
   const int k0 = kt * B128_T;
   const int num_q_tiles = p.Tq_pad / B128_T;
+  if (p.it_chunk && p.local && work.it0 >= (num_q_tiles - (p.causal ? min(num_q_tiles, max(0, p.k_off + k0) / B128_T) : 0)) * G) return;
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
@@ -144,7 +149,8 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   __syncthreads();
   const int qt_start = *qt_start_s;
   const int n_qt = num_q_tiles - qt_start;
-  const int n_it = n_qt * G;
+  const int n_it = max(0, min(p.it_chunk ? p.it_chunk : n_qt * G, n_qt * G - work.it0));      // this CTA's pairs
+  const int hq0 = hkv * G + (n_it ? work.it0 / n_qt : 0), t0 = n_it ? work.it0 % n_qt : 0;    // the first of them
 
   if (warp < 4) {
   regs_give<B128_REGS_ISSUE>();
@@ -158,10 +164,10 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         tma_load_4d(smem + L::K_OFF + h * L::HALF, &tmK, kv_full, h * 64, hkv, k0, b);
         tma_load_4d(smem + L::V_OFF + h * L::HALF, &tmV, kv_full, h * 64, hkv, k0, b);
       }
+      int hq = hq0, t = t0;
       for (int i = 0; i < n_it; ++i) {
         const int st = i & 1;
-        const int hq = hkv * G + i / n_qt;
-        const int q0 = (qt_start + i % n_qt) * B128_T;
+        const int q0 = (qt_start + t) * B128_T;
         if (!mbar_wait_lean(&q_empty[st], ((i >> 1) & 1) ^ 1, abort_flag, 800)) break;
         mbar_expect_tx(&q_full[st], L::TILE + 1024);
 #pragma unroll
@@ -173,6 +179,7 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         mbar_expect_tx(do_full, L::TILE);
 #pragma unroll
         for (int h = 0; h < 2; ++h) tma_load_4d(smem + L::DO_OFF + h * L::HALF, &tmDO, do_full, h * 64, hq, q0, b);
+        if (++t == n_qt) { t = 0; ++hq; }
       }
     }
   } else if (warp == 1) {
@@ -268,11 +275,14 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const int chunk0 = (cbase % 64) / 8;
     bool alive = true;
     // first query position of a tile decides whether it needs masking; read one tile ahead, straight from global memory
-    int qmin_next = n_it > 0 ? ld_ahead_s32(p.q_pos + qt_start * B128_T) : 0;
+    int qmin_next = n_it > 0 ? ld_ahead_s32(p.q_pos + (qt_start + t0) * B128_T) : 0;
+    int t = t0;
     for (int i = 0; i < n_it && alive; ++i) {
       const int st = i & 1;
       const int qmin = qmin_next;
-      if (i + 1 < n_it) qmin_next = ld_ahead_s32(p.q_pos + (qt_start + (i + 1) % n_qt) * B128_T);
+      const int t_cur = t;
+      if (++t == n_qt) t = 0;
+      if (i + 1 < n_it) qmin_next = ld_ahead_s32(p.q_pos + (qt_start + t) * B128_T);
       // slow path only for tiles that touch the causal diagonal or the end of the key sequence
       const bool need_mask = (k0 + B128_T > p.Tk) || (p.causal && (p.k_off + k0 + B128_T - 1 > qmin));
       const float* vec = (const float*)(smem + L::VEC_OFF + st * 1024) + cbase;
@@ -296,7 +306,7 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
       } else {
         const int lim = (p.causal ? kpos : -0x7fffffff - 1);               // visible: lim <= q position
-        const int4* qp = (const int4*)(p.q_pos + (qt_start + i % n_qt) * B128_T + cbase);
+        const int4* qp = (const int4*)(p.q_pos + (qt_start + t_cur) * B128_T + cbase);
 #pragma unroll
         for (int j = 0; j < CW; j += 4) {
           const float4 l = *(const float4*)(vec + j);
@@ -380,6 +390,10 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll
               for (int j = 0; j < 32; j += 4)
                 red_add_v4(dst + j, __uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+            } else if (p.dkv_mode == 3) {
+#pragma unroll
+              for (int j = 0; j < 32; j += 4)
+                red_add_v4((float*)base + off + c + j, __uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
             } else if (p.dkv_mode == 1) {
               float* dst = (float*)base + off + c;
 #pragma unroll
@@ -416,13 +430,13 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     uint8_t* stage = smem + L::DQS_OFF + quarter * 8192;      // [2 boxes][32 rows][128 B]
     const bool issuer = (lane == 0);
     if (issuer) tma_prefetch_desc(&tmDQ);
+    int hq = hq0, t = t0;
     for (int i = 0; i < n_it; ++i) {
       bool ok = mbar_wait_lean(dq_full, i & 1, abort_flag, 1100);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      const int hq = hkv * G + i / n_qt;
-      const int q0 = (qt_start + i % n_qt) * B128_T;
+      const int q0 = (qt_start + t) * B128_T;
       uint32_t v[4][32];
 #pragma unroll
       for (int h = 0; h < 4; ++h) tmem_ld32(t_lane + 32 * h, v[h]);
@@ -453,6 +467,7 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
       }
+      if (++t == n_qt) { t = 0; ++hq; }
     }
     if (issuer) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
@@ -482,7 +497,7 @@ extern "C" int cpb_flash_bwd128(const void* q, const void* k, const void* v, con
                                 int B, int Tq, int Tk, int Hq, int Hkv, int Tq_pad,
                                 long q_sh, long q_st, long q_sb, long k_sh, long k_st, long k_sb,
                                 float scale, int causal, int k_off, const int* q_pos, int dkv_mode, long dkv_st,
-                                const uint64_t* route_k, const uint64_t* route_v, int route_rows, int route_tl,
+                                const uint64_t* route_k, const uint64_t* route_v, int route_rows, int route_tl, int it_chunk, int local,
                                 int* status, cudaStream_t stream) {
   if (Hq % Hkv) return set_error(CPB_ERR_ARG, "flash_bwd128: Hq %% Hkv != 0");
   if (Tq_pad % B128_T || Tq_pad < Tq) return set_error(CPB_ERR_ARG, "flash_bwd128: bad Tq_pad");
@@ -509,6 +524,8 @@ extern "C" int cpb_flash_bwd128(const void* q, const void* k, const void* v, con
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   p.lse2 = lse2; p.delta = delta; p.q_pos = q_pos; p.dk = dk; p.dv = dv; p.dkv_mode = dkv_mode; p.dkv_st = dkv_st; p.status = status;
   p.route_k = route_k; p.route_v = route_v; p.route_rows = route_rows; p.route_tl = route_tl;
+  if (it_chunk < 0 || (it_chunk > 0) != (dkv_mode == 3)) return set_error(CPB_ERR_ARG, "flash_bwd128: several CTAs per K/V tile add their dK/dV in fp32 (dkv_mode 3)");
+  p.it_chunk = it_chunk; p.local = local;
   static const bool skip_dq = [] {
     const char* e = getenv("CPB_BWD_SKIP_DQ");
     const bool on = e != nullptr && e[0] == '1';
@@ -516,7 +533,8 @@ extern "C" int cpb_flash_bwd128(const void* q, const void* k, const void* v, con
     return on;
   }();
   p.debug_skip_dq = skip_dq;
-  dim3 grid((Tk + B128_T - 1) / B128_T, Hkv, B);
+  const int n_kt = (Tk + B128_T - 1) / B128_T, pairs = Hq / Hkv * (Tq_pad / B128_T);
+  const dim3 grid = it_chunk ? dim3((unsigned)n_kt * ((pairs + it_chunk - 1) / it_chunk) * Hkv * B) : dim3(n_kt, Hkv, B);
   static bool cfg = false;
   if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_bwd128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Bwd128Smem::TOTAL)); cfg = true; }
   flash_bwd128_kernel<<<grid, B128_THREADS, Bwd128Smem::TOTAL, stream>>>(tq, tk, tv, tdo, tdq, p);

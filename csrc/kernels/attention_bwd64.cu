@@ -36,6 +36,7 @@
 //
 // Warp roles (768 threads): 0 = TMA loader, 1 = MMA issuer, 2, 3 idle, 4..11 = softmax-gradient warps of half A, 12..19 of
 // half B (thread = key row, 32 queries), 20..23 = dQ drain warps (thread = query row).
+#include "attention_bwd.cuh"
 #include "common.cuh"
 #include "host_utils.h"
 
@@ -63,7 +64,9 @@ struct Bwd64Params {
   const int* q_pos;             // [Tq_pad] global positions, INT_MAX in the padding
   void* dk; void* dv;           // [B,Tk,Hkv,D] bf16 (store) or fp32 (accumulate)
   long dkv_st;                  // elements from one token of dk / dv to the next (heads adjacent, batches dense)
-  int dkv_mode;                 // 0 bf16 store, 1 fp32 accumulate, 2 routed red.add (fused ring)
+  int dkv_mode;                 // 0 bf16 store, 1 fp32 accumulate, 2 routed red.add (fused ring), 3 red.add (several CTAs per tile)
+  int it_chunk;                 // pairs of (query head, query tile) per CTA, 0: all (see BwdWork)
+  int local;                    // q_pos is 0 .. Tq - 1: the first visible query tile needs no search
   const uint64_t* route_k;      // mode 2: per chunk of route_rows K/V rows the address of its owner's fp32 accumulator
   const uint64_t* route_v;
   int route_rows, route_tl;
@@ -112,10 +115,12 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   int* qt_start_s = (int*)(tmem_slot + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kt = blockIdx.x, hkv = blockIdx.y, b = blockIdx.z;
+  const BwdWork work = bwd_work(p.it_chunk, (p.Tk + B64_T - 1) / B64_T, p.Hkv, p.B);
+  const int kt = work.kt, hkv = work.hkv, b = work.b;
   const int G = p.Hq / p.Hkv;
   const int k0 = kt * B64_T;
   const int num_q_tiles = p.Tq_pad / B64_T;
+  if (p.it_chunk && p.local && work.it0 >= (num_q_tiles - (p.causal ? min(num_q_tiles, max(0, p.k_off + k0) / B64_T) : 0)) * G) return;
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
@@ -159,7 +164,8 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   const int qt_start = *qt_start_s;
   const int n_qt = num_q_tiles - qt_start;
-  const int n_it = n_qt * G;
+  const int n_it = max(0, min(p.it_chunk ? p.it_chunk : n_qt * G, n_qt * G - work.it0));      // this CTA's pairs
+  const int hq0 = hkv * G + (n_it ? work.it0 / n_qt : 0), t0 = n_it ? work.it0 % n_qt : 0;    // the first of them
 
   if (warp < 4) {
   regs_give<B64_REGS_ISSUE>();
@@ -169,7 +175,7 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmDO);
       mbar_expect_tx(kv_full, L::TILE);
       tma_load_4d(smem + L::K_OFF, &tmK, kv_full, 0, hkv, k0, b);
-      int st = 0, ph = 1, hq = hkv * G, t = 0;
+      int st = 0, ph = 1, hq = hq0, t = t0;
       for (int i = 0; i < n_it; ++i) {
         const int q0 = (qt_start + t) * B64_T;
         if (!mbar_wait_lean(&q_empty[st], ph, abort_flag, 800)) break;
@@ -288,8 +294,8 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     bool alive = true;
     // first query position of a half tile decides whether it needs masking; read one tile ahead, straight from global memory
     const int* qp0 = p.q_pos + qt_start * B64_T + 64 * half;
-    int qmin_next = n_it > 0 ? ld_ahead_s32(qp0) : 0;
-    int st = 0, ph = 0, t = 0;
+    int qmin_next = n_it > 0 ? ld_ahead_s32(qp0 + t0 * B64_T) : 0;
+    int st = 0, ph = 0, t = t0;
     for (int i = 0; i < n_it && alive; ++i) {
       const int qmin = qmin_next;
       const int t_cur = t;
@@ -405,6 +411,10 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
               for (int j = 0; j < 32; j += 4)
                 red_add_v4(dst + j, __uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+            } else if (p.dkv_mode == 3) {
+#pragma unroll
+              for (int j = 0; j < 32; j += 4)
+                red_add_v4((float*)base + off + c + j, __uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
             } else if (p.dkv_mode == 1) {
               float* dst = (float*)base + off + c;
 #pragma unroll
@@ -441,7 +451,7 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     uint8_t* stage = smem + L::DQS_OFF + quarter * 8192;      // [2 boxes][32 rows][128 B]
     const bool issuer = (lane == 0);
     if (issuer) tma_prefetch_desc(&tmDQ);
-    int hq = hkv * G, t = 0;
+    int hq = hq0, t = t0;
     for (int i = 0; i < n_it; ++i) {
       bool ok = mbar_wait_lean(dq_full, i & 1, abort_flag, 1100);
       ok = __all_sync(0xffffffffu, ok);
@@ -504,7 +514,7 @@ extern "C" int cpb_flash_bwd64(const void* q, const void* k, const void* v, cons
                                 int B, int Tq, int Tk, int Hq, int Hkv, int Tq_pad,
                                 long q_sh, long q_st, long q_sb, long k_sh, long k_st, long k_sb,
                                 float scale, int causal, int k_off, const int* q_pos, int dkv_mode, long dkv_st,
-                                const uint64_t* route_k, const uint64_t* route_v, int route_rows, int route_tl,
+                                const uint64_t* route_k, const uint64_t* route_v, int route_rows, int route_tl, int it_chunk, int local,
                                 int* status, cudaStream_t stream) {
   if (Hq % Hkv) return set_error(CPB_ERR_ARG, "flash_bwd64: Hq %% Hkv != 0");
   if (Tq_pad % B64_T || Tq_pad < Tq) return set_error(CPB_ERR_ARG, "flash_bwd64: bad Tq_pad");
@@ -532,6 +542,8 @@ extern "C" int cpb_flash_bwd64(const void* q, const void* k, const void* v, cons
   p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v; p.k_sh = k_sh; p.k_st = k_st; p.k_sb = k_sb;
   p.lse2 = lse2; p.delta = delta; p.q_pos = q_pos; p.dk = dk; p.dv = dv; p.dkv_mode = dkv_mode; p.dkv_st = dkv_st; p.status = status;
   p.route_k = route_k; p.route_v = route_v; p.route_rows = route_rows; p.route_tl = route_tl;
+  if (it_chunk < 0 || (it_chunk > 0) != (dkv_mode == 3)) return set_error(CPB_ERR_ARG, "flash_bwd64: several CTAs per K/V tile add their dK/dV in fp32 (dkv_mode 3)");
+  p.it_chunk = it_chunk; p.local = local;
   static const bool skip_dq = [] {
     const char* e = getenv("CPB_BWD_SKIP_DQ");
     const bool on = e != nullptr && e[0] == '1';
@@ -539,7 +551,8 @@ extern "C" int cpb_flash_bwd64(const void* q, const void* k, const void* v, cons
     return on;
   }();
   p.debug_skip_dq = skip_dq;
-  dim3 grid((Tk + B64_T - 1) / B64_T, Hkv, B);
+  const int n_kt = (Tk + B64_T - 1) / B64_T, pairs = Hq / Hkv * (Tq_pad / B64_T);
+  const dim3 grid = it_chunk ? dim3((unsigned)n_kt * ((pairs + it_chunk - 1) / it_chunk) * Hkv * B) : dim3(n_kt, Hkv, B);
   static bool cfg = false;
   if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_bwd64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Bwd64Smem::TOTAL)); cfg = true; }
   flash_bwd64_kernel<<<grid, B64_THREADS, Bwd64Smem::TOTAL, stream>>>(tq, tk, tdo, tdq, p);

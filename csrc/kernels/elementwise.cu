@@ -783,13 +783,25 @@ __global__ void cast_f32_bf16_kernel(const float* __restrict__ in, __nv_bfloat16
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     out[i] = __float2bfloat16(in[i] * scale);
 }
-// rows x (8 c8) fp32, dense, into bf16 rows `out_stride` elements apart; eight elements per thread (32 bytes in, 16 out).
-__global__ void cast_f32_bf16_rows_kernel(const float* __restrict__ in, __nv_bfloat16* __restrict__ out, size_t n8, int c8, long out_stride, float scale) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n8; i += (size_t)gridDim.x * blockDim.x) {
-    const size_t r = i / c8;
-    const float4 a = *(const float4*)(in + i * 8), b = *(const float4*)(in + i * 8 + 4);
-    *(uint4*)(out + r * out_stride + (i - r * c8) * 8) =
-        make_uint4(pack_bf16(a.x * scale, a.y * scale), pack_bf16(a.z * scale, a.w * scale), pack_bf16(b.x * scale, b.y * scale), pack_bf16(b.z * scale, b.w * scale));
+// Up to three dense fp32 matrices that follow one another in memory -> bf16 rows at a place and a distance of their own; eight
+// elements per thread (32 bytes in, 16 out).
+struct CastPiece {
+  __nv_bfloat16* out;
+  size_t n8;               // sixteen-byte groups of the result
+  int c8;                  // of one row
+  long stride;             // elements from row to row
+};
+__global__ void cast_f32_bf16_rows_kernel(const float* __restrict__ in, CastPiece a, CastPiece b, CastPiece c, float scale) {
+  const size_t total = a.n8 + b.n8 + c.n8;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+    const bool in_a = i < a.n8, in_b = !in_a && i < a.n8 + b.n8;
+    __nv_bfloat16* out = in_a ? a.out : in_b ? b.out : c.out;
+    const int c8 = in_a ? a.c8 : in_b ? b.c8 : c.c8;
+    const long stride = in_a ? a.stride : in_b ? b.stride : c.stride;
+    const size_t k = in_a ? i : in_b ? i - a.n8 : i - a.n8 - b.n8, r = k / c8;
+    const float4 x = *(const float4*)(in + i * 8), y = *(const float4*)(in + i * 8 + 4);
+    *(uint4*)(out + r * stride + (k - r * c8) * 8) = make_uint4(pack_bf16(x.x * scale, x.y * scale), pack_bf16(x.z * scale, x.w * scale),
+                                                                pack_bf16(y.x * scale, y.y * scale), pack_bf16(y.z * scale, y.w * scale));
   }
 }
 __global__ void cast_bf16_f32_kernel(const __nv_bfloat16* __restrict__ in, float* __restrict__ out, size_t n, float scale, int accumulate) {
@@ -999,18 +1011,24 @@ extern "C" int cpb_adamw(float* p, const float* g, float* m, float* v, void* p16
   adamw_kernel<<<grid_for((size_t)n, 256), 256, 0, stream>>>(p, g, m, v, (__nv_bfloat16*)p16, (size_t)n, lr, b1, b2, eps, wd, bc1, bc2, grad_prescale, clip, sumsq, flag);
   return check_launch("adamw");
 }
-extern "C" int cpb_cast_f32_bf16_rows(const float* in, void* out, long rows, int cols, long out_stride, float scale, cudaStream_t stream) {
-  if (rows <= 0 || cols <= 0) return CPB_OK;
-  if (cols % 8 || out_stride % 8 || (((uintptr_t)in | (uintptr_t)out) & 15))
-    return set_error(CPB_ERR_ARG, "cast_f32_bf16_rows: rows must be 16-byte aligned multiples of eight elements");
-  const size_t n8 = (size_t)rows * (cols / 8);
-  cast_f32_bf16_rows_kernel<<<grid_for(n8, 256, 32), 256, 0, stream>>>(in, (__nv_bfloat16*)out, n8, cols / 8, out_stride, scale);
-  return check_launch("cast_f32_bf16_rows");
+// in: fp32, rows_q x cols_q values and then twice rows_k x cols_k (rows_k 0: none); each goes to bf16 rows q_stride / kv_stride elements apart.
+extern "C" int cpb_cast_f32_bf16_rows(const float* in, void* out_q, long rows_q, int cols_q, long q_stride, void* out_k, void* out_v, long rows_k,
+                                      int cols_k, long kv_stride, float scale, cudaStream_t stream) {
+  if ((cols_q % 8) || (q_stride % 8) || ((uintptr_t)in & 15) || ((uintptr_t)out_q & 15)) return set_error(CPB_ERR_ARG, "cast_rows: columns, stride and pointers must be multiples of 16 bytes");
+  if (rows_k > 0 && ((cols_k % 8) || (kv_stride % 8) || (((uintptr_t)out_k | (uintptr_t)out_v) & 15)))
+    return set_error(CPB_ERR_ARG, "cast_rows: columns, stride and pointers must be multiples of 16 bytes");
+  const CastPiece q{(__nv_bfloat16*)out_q, (size_t)(rows_q > 0 ? rows_q : 0) * (cols_q / 8), cols_q > 0 ? cols_q / 8 : 1, q_stride};
+  const size_t nk = (size_t)(rows_k > 0 ? rows_k : 0) * (cols_k / 8);
+  const CastPiece k{(__nv_bfloat16*)out_k, nk, cols_k > 0 ? cols_k / 8 : 1, kv_stride}, v{(__nv_bfloat16*)out_v, nk, k.c8, kv_stride};
+  const size_t total = q.n8 + 2 * nk;
+  if (total == 0) return CPB_OK;
+  cast_f32_bf16_rows_kernel<<<grid_for(total, 256, 32), 256, 0, stream>>>(in, q, k, v, scale);
+  return check_launch("cast_rows");
 }
 extern "C" int cpb_cast_f32_bf16(const float* in, void* out, long n, float scale, cudaStream_t stream) {
   if (n <= 0) return CPB_OK;
   if (n % 8 == 0 && (((uintptr_t)in | (uintptr_t)out) & 15) == 0)
-    return cpb_cast_f32_bf16_rows(in, out, n / 8, 8, 8, scale, stream);
+    return cpb_cast_f32_bf16_rows(in, out, n / 8, 8, 8, nullptr, nullptr, 0, 0, 0, scale, stream);
   cast_f32_bf16_kernel<<<grid_for((size_t)n, 256), 256, 0, stream>>>(in, (__nv_bfloat16*)out, (size_t)n, scale);
   return check_launch("cast_f32_bf16");
 }
