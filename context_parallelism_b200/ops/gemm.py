@@ -34,9 +34,9 @@ def _rowmajor2d(t: torch.Tensor) -> torch.Tensor:
 
 
 @functools.lru_cache(maxsize=4096)
-def acc_splits(M: int, N: int, K: int) -> int:
-    """Into how many ranges of K the kernel's plan splits an accumulating GEMM of this shape."""
-    return nv.lib().cpb_gemm_splits(M, N, K)
+def acc_splits(M: int, N: int, K: int, epi: int = EPI_F32_ACC) -> int:
+    """Into how many ranges of K the kernel's plan splits a GEMM of this shape (accumulating and bf16 epilogues)."""
+    return nv.lib().cpb_gemm_plan(M, N, K, epi, 0) & 0xffff
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
@@ -67,10 +67,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         bias = bias.float().contiguous()
         if bias.data_ptr() % 16:
             bias = bias.clone()
-    # A split accumulation adds its partial tiles in a fixed order in a launch of its own, from a workspace of this call.
-    splits, part = (acc_splits(M, N, K) if epi == EPI_F32_ACC else 1), None
+    # A GEMM split along K adds its partial tiles in a fixed order in a launch of its own, from a workspace of this call.
+    splits, part = (acc_splits(M, N, K, epi) if epi in (EPI_F32_ACC, EPI_BF16) else 1), None
     if splits > 1:
-        part = torch.empty((splits - 1) * M * N, dtype=torch.float32, device=a.device)
+        part = torch.empty((splits if epi == EPI_BF16 else splits - 1) * M * N, dtype=torch.float32, device=a.device)
         nv.LAUNCHES[0] += 1
     nv.call("gemm_bf16", nv.ptr(a), nv.ptr(b), nv.ptr(out), nv.ptr(aux), nv.ptr(bias),
             nv.i(M), nv.i(N), nv.i(K), nv.i(a.stride(0)), nv.i(b.stride(0)), nv.i(out.stride(0)),

@@ -32,10 +32,12 @@ namespace cpb {
 
 template <int BN>
 struct GemmSmem {
-  static constexpr int STAGES = BN == 256 ? 6 : 8;               // 192 KB of operands in flight
+  static constexpr int STAGES = BN > 128 ? 6 : 8;                // up to 192 KB of operands in flight
   static constexpr int A_BYTES = GEMM_BM * GEMM_BK * 2;          // 128 rows of A
-  static constexpr int B_BYTES = (BN / 2) * GEMM_BK * 2;         // this CTA's half of B's columns
+  static constexpr int B_GROUPS = (BN / 2 + 63) / 64;            // this CTA's half of B's columns, in groups of 64 (N-major: 96 columns
+  static constexpr int B_BYTES = B_GROUPS * 64 * GEMM_BK * 2;    // take two groups, the last 32 columns are loaded and not used)
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int ACC_COLS = BN > 128 ? 256 : 128;          // tensor-memory columns of an accumulator (a power of two)
   static constexpr int STORE_OFFSET = STAGES * STAGE_BYTES;      // 4 epilogue warps x 2 buffers x 4 KB
   static constexpr int BAR_OFFSET = STORE_OFFSET + 32768;
   static constexpr int TOTAL = BAR_OFFSET + 256 + 1024;
@@ -141,7 +143,7 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     fence_mbar_init();
   }
   if (warp == 1) {
-    tmem_alloc_pair(tmem_slot, 2 * BN);
+    tmem_alloc_pair(tmem_slot, 2 * L::ACC_COLS);
     tmem_relinquish_pair();
   }
   tc_fence_before();
@@ -167,7 +169,7 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           uint8_t* sa = smem + stage * L::STAGE_BYTES;
           uint8_t* sb = sa + L::A_BYTES;
           const uint32_t full_even = map_to_cta(smem_u32(&full_bar[stage]), 0);
-          if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * L::STAGE_BYTES);              // the bytes of both CTAs
+          if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * (L::A_BYTES + (B_MN ? L::B_BYTES : BN * GEMM_BK)));    // the bytes of both CTAs
           const int k0 = kb * GEMM_BK;
           if (A_MN) {
 #pragma unroll
@@ -182,7 +184,7 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           } else if (B_MN) {
             const int n0 = nb * BN + (int)rank * (BN / 2);
 #pragma unroll
-            for (int g = 0; g < BN / 2 / 64; ++g) tma_load_2d_pair(sb + g * 8192, &tmB, full_even, n0 + g * 64, k0);
+            for (int g = 0; g < L::B_GROUPS; ++g) tma_load_2d_pair(sb + g * 8192, &tmB, full_even, n0 + g * 64, k0);
           } else {
             tma_load_2d_pair(sb, &tmB, full_even, k0, nb * BN + (int)rank * (BN / 2));
           }
@@ -208,7 +210,7 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         const uint32_t acc_phase = (it >> 1) & 1;
         if (!__all_sync(0xffffffffu, mbar_wait(&tempty_bar[acc], acc_phase ^ 1, abort_flag, p.status, 210))) break;
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
+        const uint32_t d_tmem = tmem_base + acc * L::ACC_COLS;
         const int split = item / num_tiles;
         const int kb0 = split * p.k_per_split, kb1 = min(p.num_k_blocks, kb0 + p.k_per_split);
         for (int kb = kb0; kb < kb1; ++kb) {
@@ -247,7 +249,7 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
+      const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * L::ACC_COLS;
       const auto release = [&] {
         tc_fence_before();
         __syncwarp();
@@ -267,7 +269,7 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   cluster_sync_all();          // the even CTA's MMAs have finished reading the odd CTA's operands; no remote arrival is in flight
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc_pair(tmem_base, 2 * BN);
+    tmem_dealloc_pair(tmem_base, 2 * L::ACC_COLS);
   }
 }
 
@@ -314,6 +316,29 @@ gemm_add_partials_kernel(float* __restrict__ C, const float4* __restrict__ parti
   }
 }
 
+// C (bf16) = partials[0] + partials[1] + ... (+ bias), in that order.
+__global__ void __launch_bounds__(256)
+gemm_sum_partials_kernel(__nv_bfloat16* __restrict__ C, const float4* __restrict__ partials, const float* __restrict__ bias, unsigned n8,
+                         unsigned total8, long ldc, int count) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total8; i += gridDim.x * blockDim.x) {
+    const unsigned r = i / n8, c = i - r * n8;
+    float4 a = partials[2 * (size_t)i], b = partials[2 * (size_t)i + 1];
+#pragma unroll 4
+    for (int s = 1; s < count; ++s) {
+      const float4 u = partials[2 * ((size_t)s * total8 + i)], v = partials[2 * ((size_t)s * total8 + i) + 1];
+      a.x += u.x; a.y += u.y; a.z += u.z; a.w += u.w;
+      b.x += v.x; b.y += v.y; b.z += v.z; b.w += v.w;
+    }
+    if (bias != nullptr) {
+      const float4 u = __ldg((const float4*)bias + 2 * c), v = __ldg((const float4*)bias + 2 * c + 1);
+      a.x += u.x; a.y += u.y; a.z += u.z; a.w += u.w;
+      b.x += v.x; b.y += v.y; b.z += v.z; b.w += v.w;
+    }
+    *(uint4*)(C + r * ldc + 8 * (long)c) = make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
+  }
+}
+
 // Tile width and K split.  The work items of a launch (tiles x splits) run on 74 pairs, so the time is that of the pair
 // with the most items: items / 74 rounded up, each the longer of its main loop and its epilogue, plus one epilogue at the
 // end.  Nanoseconds, measured: main loop per 64 of K 370 at 256 columns (8192^3: 694 us) and 240 at 128 columns (892 us),
@@ -334,19 +359,24 @@ static void plan_tiles(int M, int N, int K, int epi, int has_aux, int want, int&
   const long m_tiles = (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM), pairs = sm_count() > 1 ? sm_count() / 2 : 1;
   const long pass = (long)M * N * 8 / 16000;
   long best = -1;
-  for (int cand = 256; cand >= 128; cand -= 128) {
+  const bool sums = epi == EPI_F32_ACC || epi == EPI_BF16;
+  for (int cand = 256; cand >= 128; cand -= 64) {
+    if (cand == 192 && epi == EPI_BF16_SWIGLU) continue;
     const int per_tile = epi == EPI_BF16_SWIGLU ? cand / 2 : cand;
     const long tiles = m_tiles * ((N + per_tile - 1) / per_tile);
     long ce = epi == EPI_F32 || epi == EPI_F32_ACC ? 1200 : epi == EPI_BF16_GELU ? (has_aux ? 1600 : 1400) : epi == EPI_BF16_SWIGLU ? (has_aux ? 1300 : 1000) : 650;
-    if (cand == 128) ce = ce / 2 + 50;
-    const long max_split = want > 0 ? want : epi == EPI_F32_ACC ? (nk + 3) / 4 : 1;     // at least four K blocks per item
-    for (long s = want > 0 ? want : 1; s <= max_split && (s == 1 || want > 0 || (s - 1) * (long)M * N <= (32L << 20)); ++s) {
+    if (cand < 256) ce = ce * cand / 256 + 50;
+    const long max_split = want > 0 ? want : sums ? (nk + 3) / 4 : 1;                   // at least four K blocks per item
+    for (long s = want > 0 ? want : 1; s <= max_split; ++s) {
+      const bool sum16 = epi == EPI_BF16 && s > 1;
+      if (s > 1 && want == 0 && (sum16 ? s : s - 1) * (long)M * N > (32L << 20)) break;        // the workspace
       const long kps = (nk + s - 1) / s;
       if ((nk + kps - 1) / kps != s) continue;                       // the same items as a smaller split
       const long waves = (tiles * s + pairs - 1) / pairs, busy = tiles * s < pairs ? tiles * s : pairs;
-      const long main = kps * (cand == 256 ? 370 : epi == EPI_F32_ACC ? 240 + 50 * busy / pairs : 240);
-      long t = waves * (main > ce ? main : ce) + (main > ce ? ce : main);
-      if (s > 1) t += 8000 + (s + 1) * pass;                         // 1.4 us and what a split has to save
+      const long main = kps * (cand == 256 ? 370 : cand == 192 ? 300 : epi == EPI_F32_ACC || sum16 ? 240 + 50 * busy / pairs : 240);
+      const long out = !sum16 ? ce : cand == 256 ? 1200 : 1200 * cand / 256 + 50;
+      long t = waves * (main > out ? main : out) + (main > out ? out : main);
+      if (s > 1) t += 8000 + (sum16 ? 2 * s + 1 : s + 1) * pass;     // 1.4 us and what a split has to save
       if (best < 0 || t < best) { best = t; bn = cand; splits = (int)s; }
     }
   }
@@ -376,8 +406,8 @@ using namespace cpb;
 // A: bf16, [M,K] row stride lda (a_mn=0) or [K,M] row stride lda (a_mn=1).
 // B: bf16, [N,K] row stride ldb (b_mn=0) or [K,N] row stride ldb (b_mn=1).
 // epi: see EPI_* above.  For EPI_BF16_SWIGLU B is the fused [2F, K] weight, N = F output features.
-// splits > 1 (accumulating epilogue only, see cpb_gemm_splits): K is split that often; partials is a workspace of
-// (splits - 1) * M * N floats, 16-byte aligned, and a second launch adds it to C.
+// splits > 1 (accumulating and bf16 epilogues, see cpb_gemm_plan): K is split that often; partials is a 16-byte aligned workspace of
+// splits - 1 (bf16: splits) matrices of M x N floats, and a second launch adds them to C (bf16: sums them, adds the bias and rounds once).
 extern "C" int cpb_gemm_bf16(const void* A, const void* B, void* C, void* aux, const float* bias,
                              int M, int N, int K, int lda, int ldb, int ldc, int ld_aux,
                              int a_mn, int b_mn, int epi, float* partials, int splits, int* status, cudaStream_t stream) {
@@ -392,9 +422,9 @@ extern "C" int cpb_gemm_bf16(const void* A, const void* B, void* C, void* aux, c
   if (splits < 1) splits = 1;
   {
     const int nk = (K + GEMM_BK - 1) / GEMM_BK, kps = (nk + splits - 1) / splits;
-    if (splits > 1 && (epi != EPI_F32_ACC || partials == nullptr || ((uintptr_t)partials & 15) || (nk + kps - 1) / kps != splits))
-      return set_error(CPB_ERR_ARG, "gemm: %d splits of K=%d need the accumulating epilogue and a 16-byte aligned workspace", splits, K);
-    if (splits > 1 && (((uintptr_t)C & 15) || (ldc & 3) || (long)M * N >= (1L << 32)))
+    if (splits > 1 && ((epi != EPI_F32_ACC && epi != EPI_BF16) || partials == nullptr || ((uintptr_t)partials & 15) || (nk + kps - 1) / kps != splits))
+      return set_error(CPB_ERR_ARG, "gemm: %d splits of K=%d need the accumulating or the bf16 epilogue and a 16-byte aligned workspace", splits, K);
+    if (splits > 1 && (((uintptr_t)C & 15) || (ldc & (epi == EPI_BF16 ? 7 : 3)) || (long)M * N >= (1L << 32)))
       return set_error(CPB_ERR_ARG, "gemm: a split C must have 16-byte aligned rows and less than 2^32 elements");
   }
   int bn = 256;
@@ -410,6 +440,8 @@ extern "C" int cpb_gemm_bf16(const void* A, const void* B, void* C, void* aux, c
   const int per_tile = epi == EPI_BF16_SWIGLU ? bn / 2 : bn;
   p.num_n_blocks = (N + per_tile - 1) / per_tile;
   p.has_aux = aux != nullptr; p.bias = bias; p.status = status;
+  const bool sum16 = splits > 1 && epi == EPI_BF16;      // every split goes to the workspace, the sum kernel writes C
+  if (sum16) { p.epi = EPI_F32; p.bias = nullptr; }
 
   CUtensorMap tm[4];
   int rc;
@@ -434,21 +466,21 @@ extern "C" int cpb_gemm_bf16(const void* A, const void* B, void* C, void* aux, c
     if ((rc = encode_tmap(&tm[3], aux, 2, 2, dims, strides, box, 1)) != CPB_OK) return rc;
   }
   if (splits > 1) {
-    uint64_t dims[3] = {(uint64_t)N, (uint64_t)M, (uint64_t)(splits - 1)}, strides[3] = {0, (uint64_t)N * 4, (uint64_t)M * N * 4};
+    uint64_t dims[3] = {(uint64_t)N, (uint64_t)M, (uint64_t)(sum16 ? splits : splits - 1)}, strides[3] = {0, (uint64_t)N * 4, (uint64_t)M * N * 4};
     uint32_t box[3] = {32, 32, 1};
     if ((rc = encode_tmap(&tm[3], partials, 4, 3, dims, strides, box, 1)) != CPB_OK) return rc;
   }
-  rc = bn == 256 ? dispatch_pair<256>(tm, p, a_mn, b_mn, stream) : dispatch_pair<128>(tm, p, a_mn, b_mn, stream);
+  rc = bn == 256 ? dispatch_pair<256>(tm, p, a_mn, b_mn, stream) : bn == 192 ? dispatch_pair<192>(tm, p, a_mn, b_mn, stream) : dispatch_pair<128>(tm, p, a_mn, b_mn, stream);
   if (rc != CPB_OK || splits == 1) return rc;
-  const unsigned total4 = (unsigned)((long)M * N / 4);
-  const unsigned blocks = (total4 + 255) / 256, cap = (unsigned)sm_count() * 8;
+  const unsigned total = (unsigned)((long)M * N / (sum16 ? 8 : 4)), blocks = (total + 255) / 256, cap = (unsigned)sm_count() * 8;
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(blocks < cap ? blocks : cap); lc.blockDim = dim3(256); lc.stream = stream;
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   lc.attrs = &at; lc.numAttrs = 1;
-  CPB_CUDA_OK(cudaLaunchKernelEx(&lc, gemm_add_partials_kernel, (float*)C, (const float4*)partials, (unsigned)N / 4, total4, (long)ldc, splits - 1));
+  if (sum16) CPB_CUDA_OK(cudaLaunchKernelEx(&lc, gemm_sum_partials_kernel, (__nv_bfloat16*)C, (const float4*)partials, bias, (unsigned)N / 8, total, (long)ldc, splits));
+  else CPB_CUDA_OK(cudaLaunchKernelEx(&lc, gemm_add_partials_kernel, (float*)C, (const float4*)partials, (unsigned)N / 4, total, (long)ldc, splits - 1));
   return check_launch("gemm_add_partials");
 }
 
@@ -489,9 +521,10 @@ extern "C" int cpb_gemm_head(const void* x, const void* w, void* dlogits, const 
   return launch_pair<256, false, false>(tm, p, stream);
 }
 
-// How often the accumulating GEMM of this shape should split K (at least 1): the caller brings the workspace.
-extern "C" int cpb_gemm_splits(int M, int N, int K) {
+// The plan of a GEMM of this shape and epilogue: tile width << 16 | how often K is split (at least 1).  For a split the caller brings the
+// workspace, splits - 1 matrices of M x N floats for the accumulating epilogue, splits for the bf16 one.
+extern "C" int cpb_gemm_plan(int M, int N, int K, int epi, int has_aux) {
   int bn = 256, splits = 1;
-  if (M > 0 && N > 0 && K > 0) plan_tiles(M, N, K, EPI_F32_ACC, 0, 0, bn, splits);
-  return splits;
+  if (M > 0 && N > 0 && K > 0) plan_tiles(M, N, K, epi, has_aux, 0, bn, splits);
+  return bn << 16 | splits;
 }

@@ -40,8 +40,9 @@ struct GemmParams {
   int M, N, K;
   int epi;
   int num_m_tiles, num_n_blocks, num_k_blocks;
-  int splits, k_per_split;   // split-K (accumulating epilogue only): 64-wide K blocks per work item.  The first split
-                             // adds to C, the others go to a workspace [splits - 1][M][N] for gemm_add_partials_kernel
+  int splits, k_per_split;   // split-K: 64-wide K blocks per work item.  EPI_F32_ACC: the first split adds to C, the others go to a
+                             // workspace [splits - 1][M][N] for gemm_add_partials_kernel.  EPI_F32 (a bf16 result): all splits go to
+                             // a workspace [splits][M][N] for gemm_sum_partials_kernel
   int swiglu_half;     // number of output features F when epi == SWIGLU (B has 2F rows)
   int band;            // pair-rows per band of the tile order (1 = rows of tiles, columns fastest)
   int has_aux;
@@ -274,7 +275,8 @@ __device__ __forceinline__ void gemm_epilogue(const GemmParams& p, const CUtenso
           }
       }
       ws.fill(ws.row_ptr(lane), lane, v);
-      if (split > 0) ws.store3(tmX, col, row0, split - 1);
+      if (p.splits > 1 && p.epi == EPI_F32) ws.store3(tmX, col, row0, split);
+      else if (split > 0) ws.store3(tmX, col, row0, split - 1);
       else if (p.epi == EPI_F32_ACC) ws.add(tmC, col, row0);
       else ws.store(tmC, col, row0);
     }
