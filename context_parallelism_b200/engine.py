@@ -15,6 +15,7 @@ from typing import Optional
 import torch
 import torch.distributed as dist
 
+from . import graphs
 from .config import Config
 from .ops import permute
 from .ops.optim import AdamW, FlatParams
@@ -113,6 +114,8 @@ class TrainEngine:
 
     # ------------------------------------------------------------------ one optimiser step
     def forward_backward(self, tokens, targets, accum: int = 1, last: bool = True) -> torch.Tensor:
+        if self._recordable(targets):
+            return self._recorded_micro_batch(tokens, targets, accum)
         idx, tgt, pos = self.shard_batch(tokens, targets)
         n_local = idx.numel()
         scale = 1.0 / (n_local * accum)
@@ -120,10 +123,27 @@ class TrainEngine:
         ctx = self.reducer.no_sync() if not last else _null()
         with ctx:
             loss_sum = self.model.loss_sum(idx, tgt, pos, scale)
-            loss_sum.backward(torch.tensor(scale, device=loss_sum.device, dtype=loss_sum.dtype))
+            # filled on the device: a host scalar copied there would wait for everything issued so far
+            loss_sum.backward(torch.full_like(loss_sum, scale))
         if last:
             self.reducer.finish()
         return loss_sum.detach() / n_local
+
+    def _recordable(self, targets) -> bool:
+        """One GPU and nothing but this package's own forward and backward pass in the micro-batch."""
+        return (self.device.type == "cuda" and not self.reducer.enabled and torch.is_grad_enabled() and isinstance(targets, torch.Tensor)
+                and not torch.is_inference_mode_enabled() and self.model.recordable())
+
+    def _recorded_micro_batch(self, tokens, targets, accum: int) -> torch.Tensor:
+        scale = 1.0 / (tokens.numel() * accum)
+
+        def micro_batch(idx, tgt, pos, *extra):
+            loss_sum = self.model.loss_with(idx, tgt, pos, *extra, scale)
+            loss_sum.backward(torch.full_like(loss_sum, scale))
+            return (loss_sum.detach() / idx.numel(),)
+        return self.model.graphs.run(f"micro-batch/{accum}", self.model, micro_batch,
+                                     (tokens, targets, self.local_pos(tokens.shape[1]), *self.model.recorded_inputs()), self.device,
+                                     graphs.model_flops(self.cfg, *tokens.shape, True), train=True)[0]
 
     def optimizer_step(self) -> torch.Tensor:
         lr = self.lr_at(self.step_idx)
@@ -167,6 +187,7 @@ class TrainEngine:
             nv.status_for(self.device).check("train step")
 
     def close(self) -> None:
+        self.model.graphs.clear()
         if self.native_pg is not None:
             from .parallel import rotators
             torch.cuda.synchronize(self.device)

@@ -1,0 +1,227 @@
+"""CUDA graphs of launch-bound calls: a micro-batch of training, the hidden states or the per-token NLL of a window.
+
+A small model's forward and backward pass is some hundred kernels of 3 to 30 us each, and issuing one costs 13 to 25 us of
+Python, autograd and ``ctypes``.  :class:`GraphCache` runs a call eagerly the first times that it sees its shapes, then records it
+once and replays the record.  Nothing depends on the caller's buffers: inputs are copied into the record's own, results are
+returned as new tensors.  What the record does read by address (weights, gradient buffers) is compared at every call, and a
+record whose weights have moved is dropped.
+"""
+from __future__ import annotations
+
+import threading
+import weakref
+from collections import OrderedDict
+from typing import Callable, Optional, Sequence, Tuple
+
+import torch
+
+from . import _native as nv
+
+MAX_RECORDS = 4                  # per model; the one used longest ago makes room
+EAGER_CALLS = 2                  # calls with new shapes that run as they always did: a shape met only once records nothing
+MAX_POOL_BYTES = 8 << 30         # a record whose buffers take more than this is not kept
+MIN_FREE_SHARE = 0.25            # share of the GPU's memory that has to be free before a record is made
+# A call is recorded while the GPU needs less time for it than the host: a launch costs the host about 25 us (forward and backward;
+# 13 us without autograd), the kernels of such models reach about 400 TFLOP/s.
+HOST_US_PER_LAUNCH = 25.0
+GPU_TFLOPS = 400.0
+
+
+def model_flops(cfg, batch: int, T: int, train: bool) -> float:
+    """Matrix products of one pass over ``batch`` x ``T`` tokens (causal attention; the head at every token)."""
+    d, qw = cfg.n_embd, cfg.n_head * cfg.head_dim
+    layer = d * (cfg.n_head + 2 * cfg.n_kv_head) * cfg.head_dim + qw * d + (3 if cfg.family == "llama" else 2) * d * cfg.ffn_hidden
+    tokens = batch * T
+    fwd = 2.0 * tokens * (cfg.n_layer * layer + d * cfg.vocab_size) + 2.0 * batch * T * T * qw * cfg.n_layer
+    return (3.3 if train else 1.0) * fwd
+
+
+def as_written(obj, cls, *names: str) -> bool:
+    """Whether the methods ``names`` of ``obj`` are those of ``cls``: neither overridden by a subclass nor replaced on the object."""
+    return all(getattr(type(obj), n) is getattr(cls, n) and n not in obj.__dict__ for n in names)
+
+
+def _plain_call() -> bool:
+    """Whether nothing is listening that a replay would pass by: a capture, a mode, a tracer, saved-tensor hooks, a launch timer."""
+    return not (torch.cuda.is_current_stream_capturing() or nv._PROFILE is not None or torch.is_anomaly_enabled()
+                or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack()
+                or torch._C._functorch.peek_interpreter_stack() is not None or torch.jit.is_tracing()
+                or torch._C._autograd._top_saved_tensors_default_hooks(True) is not None
+                or torch.autograd.forward_ad._current_level >= 0)
+
+
+def _main_grad(p) -> int:
+    mg = getattr(p, "main_grad", None)
+    return 0 if mg is None else mg.data_ptr()
+
+
+def _quiet(p) -> bool:
+    """Whether nobody is to be told about the gradient of ``p``."""
+    return getattr(p, "_grad_ready", None) is None and not p._backward_hooks and not p._post_accumulate_grad_hooks
+
+
+class Weights:
+    """The modules and parameters of a model as a record read them (weak references: a record does not keep its model alive)."""
+
+    def __init__(self, model: torch.nn.Module, train: bool):
+        self.train = train
+        self.mods = []
+        for m in model.modules():
+            parts = [(n, weakref.ref(c)) for n, c in m._modules.items() if c is not None]
+            attrs = [(n, m.__dict__[n]) for n in ("cfg", "attn") if n in m.__dict__]
+            params = [(n, weakref.ref(p), p.data_ptr(), _main_grad(p)) for n, p in m._parameters.items() if p is not None]
+            self.mods.append((weakref.ref(m), parts, attrs, params))
+
+    @staticmethod
+    def recordable(model: torch.nn.Module) -> bool:
+        """A training record needs every gradient in its ``main_grad``."""
+        return all(p.requires_grad and _main_grad(p) and _quiet(p) for p in model.parameters())
+
+    def hold(self) -> bool:
+        for ref, parts, attrs, params in self.mods:
+            m = ref()
+            if m is None:
+                return False
+            for n, c in parts:
+                if m._modules.get(n) is not c():
+                    return False
+            for n, v in attrs:
+                if m.__dict__.get(n) is not v:
+                    return False
+            for n, r, at, grad in params:
+                p = m._parameters.get(n)
+                if p is not r() or p is None or p.data_ptr() != at:
+                    return False
+                if self.train and not (p.requires_grad and _main_grad(p) == grad and _quiet(p)):
+                    return False
+        return True
+
+
+class _Record:
+    def __init__(self, fn: Callable, inputs: Sequence[torch.Tensor], weights: Weights, device: torch.device):
+        """Records ``fn(*inputs)``; nothing is executed.  Raises what ``fn`` or the capture raises."""
+        self.weights = weights
+        self.outputs = None
+        self.graph = torch.cuda.CUDAGraph()
+        self.done = torch.cuda.Event()
+        with torch.inference_mode(False):
+            self.inputs = [torch.empty(t.shape, dtype=t.dtype, device=device) for t in inputs]
+        side = torch.cuda.Stream(device=device)
+        side.wait_stream(torch.cuda.current_stream(device))
+        before = torch.cuda.memory_reserved(device)
+        launches = nv.LAUNCHES[0]
+        with torch.cuda.stream(side):
+            # thread_local: other threads may allocate and synchronise while this one records
+            self.graph.capture_begin(capture_error_mode="thread_local")
+            try:
+                outs = fn(*self.inputs)
+            except BaseException:
+                try:
+                    self.graph.capture_end()
+                except RuntimeError:
+                    pass                                             # the capture was invalidated by what fn raised
+                raise
+            finally:
+                self.launches = nv.LAUNCHES[0] - launches
+                nv.LAUNCHES[0] = launches
+            self.graph.capture_end()
+        self.pool_bytes = torch.cuda.memory_reserved(device) - before
+        self.done.record(torch.cuda.current_stream(device))
+        self.outputs = [o.detach() for o in outs]
+
+    def replay(self, inputs: Sequence[torch.Tensor], stream: torch.cuda.Stream) -> Tuple[torch.Tensor, ...]:
+        stream.wait_event(self.done)                                 # the last replay may have run on another stream
+        for s, t in zip(self.inputs, inputs):
+            s.copy_(t, non_blocking=True)
+        self.graph.replay()
+        nv.LAUNCHES[0] += self.launches
+        outs = tuple(o.clone() for o in self.outputs)
+        self.done.record(stream)
+        return outs
+
+    def close(self) -> None:
+        self.done.synchronize()                                      # the buffers may not be given back under a running replay
+        self.outputs = None
+        self.graph.reset()
+
+    def __del__(self):
+        try:
+            if self.outputs is not None:
+                self.close()
+        except Exception:                                            # the end of the process
+            pass
+
+
+class GraphCache:
+    """The records of one model, by name, input shapes and modes.  Safe with several threads and streams: a lock covers the copies in,
+    the replay and the copies out, and an event orders replays of different streams."""
+
+    def __init__(self):
+        self._lock = threading.Lock()
+        self._records: "OrderedDict[tuple, Optional[_Record]]" = OrderedDict()
+        self._seen: "OrderedDict[tuple, int]" = OrderedDict()
+
+    def __reduce__(self):                                            # a copied or unpickled model starts without records
+        return GraphCache, ()
+
+    def __deepcopy__(self, memo):
+        return GraphCache()
+
+    def run(self, name: str, model: torch.nn.Module, fn: Callable, inputs: Sequence[torch.Tensor], device: torch.device,
+            flops: float, train: bool = False) -> Tuple[torch.Tensor, ...]:
+        """``fn(*inputs)`` with the inputs on ``device``: a tuple of tensors."""
+        if device.type != "cuda" or not _plain_call() or any(t.requires_grad for t in inputs):
+            return self._eager(fn, inputs, device)
+        from .ops import attention
+        key = (name, device.index, train, torch.is_inference_mode_enabled(), attention.FP32_ACCURATE,
+               *((t.dtype, tuple(t.shape)) for t in inputs))
+        with self._lock:
+            rec = self._records.get(key)
+            if rec is not None:
+                if rec.weights.hold():
+                    self._records.move_to_end(key)
+                    return rec.replay(inputs, torch.cuda.current_stream(device))
+                self._drop(key)
+        launches = nv.LAUNCHES[0]
+        outs = self._eager(fn, inputs, device)
+        launches = nv.LAUNCHES[0] - launches
+        with self._lock:
+            if key not in self._records:
+                n = self._seen[key] = self._seen.pop(key, 0) + 1
+                while len(self._seen) > 64:
+                    self._seen.popitem(last=False)
+                if n >= EAGER_CALLS:
+                    self._seen.pop(key, None)
+                    self._record(key, model, fn, inputs, device, flops < GPU_TFLOPS * 1e6 * HOST_US_PER_LAUNCH * launches, train)
+        return outs
+
+    @staticmethod
+    def _eager(fn, inputs, device):
+        return tuple(fn(*(t if t.device == device else t.to(device, non_blocking=True) for t in inputs)))
+
+    def _record(self, key, model, fn, inputs, device, launch_bound: bool, train: bool) -> None:
+        free, total = torch.cuda.mem_get_info(device) if launch_bound else (0, 1)
+        rec = None
+        if free > MIN_FREE_SHARE * total and (not train or Weights.recordable(model)):
+            try:
+                rec = _Record(fn, inputs, Weights(model, train), device)
+            except (RuntimeError, nv.NativeError):                   # out of memory, or something in fn that cannot be recorded
+                nv.lib().cpb_clear_error()                           # the call itself has run; its like stay eager from now on
+            if rec is not None and rec.pool_bytes > MAX_POOL_BYTES:
+                rec.close()
+                rec = None
+        self._records[key] = rec                                     # None: not to be tried again
+        while len(self._records) > 64 or sum(r is not None for r in self._records.values()) > MAX_RECORDS:
+            self._drop(next((k for k, r in self._records.items() if r is not None), next(iter(self._records))))
+
+    def _drop(self, key) -> None:
+        rec = self._records.pop(key)
+        if rec is not None:
+            rec.close()
+
+    def clear(self) -> None:
+        """Give back every record and its memory."""
+        with self._lock:
+            while self._records:
+                self._drop(next(iter(self._records)))
+            self._seen.clear()

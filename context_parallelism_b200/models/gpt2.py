@@ -13,6 +13,7 @@ import torch
 import torch.nn as nn
 from torch.utils.checkpoint import checkpoint
 
+from .. import graphs
 from ..config import Config
 from ..ops import elementwise as E
 from ..ops import gemm as G
@@ -70,6 +71,7 @@ class GPT2(nn.Module):
             _padded_normal(cfg.vocab_size, cfg.vocab_padded, d, gen))
         self.to(device)
         self.attn = CPAttention(cfg, self.cp)
+        self.graphs = graphs.GraphCache()
 
     def named_tensors(self) -> Dict[str, torch.Tensor]:
         """Parameters under the names of the named-init files: each block's first LayerNorm lives inside its
@@ -90,6 +92,19 @@ class GPT2(nn.Module):
         return out
 
     def hidden(self, idx_local: torch.Tensor, pos: torch.Tensor) -> torch.Tensor:
+        if torch.is_grad_enabled() or self.cp.cp_size > 1:
+            return self._hidden(idx_local, pos)
+        return self.graphs.run("hidden", self, lambda i, p: (self._hidden(i, p),), (idx_local, pos), self.wte.device,
+                               graphs.model_flops(self.cfg, *idx_local.shape, False))[0]
+
+    def recorded_inputs(self) -> tuple:
+        """What ``loss_with`` reads beside its tokens, targets and positions and the weights."""
+        return ()
+
+    def recordable(self) -> bool:
+        return self.cp.cp_size == 1 and graphs.as_written(self, GPT2, "hidden", "loss_sum", "per_token_nll")
+
+    def _hidden(self, idx_local: torch.Tensor, pos: torch.Tensor) -> torch.Tensor:
         cfg = self.cfg
         x = E.embedding(idx_local, self.wte, pos, self.wpe)
         pending = None
@@ -97,11 +112,11 @@ class GPT2(nn.Module):
         full = cfg.recompute == "full" and torch.is_grad_enabled()
         for blk in self.blocks:
             if full:
-                x, pending = checkpoint(self._block, blk, x, pending, pos, use_reentrant=False)
+                x, pending = checkpoint(self._block, blk, x, pending, pos, use_reentrant=False, preserve_rng_state=False)
             elif use_ckpt:
-                x, qkv = checkpoint(blk.pre_attention, x, pending, use_reentrant=False)
+                x, qkv = checkpoint(blk.pre_attention, x, pending, use_reentrant=False, preserve_rng_state=False)
                 o = self.attn(qkv, pos)
-                x, pending = checkpoint(blk.post_attention, x, o, use_reentrant=False)
+                x, pending = checkpoint(blk.post_attention, x, o, use_reentrant=False, preserve_rng_state=False)
             else:
                 x, qkv = blk.pre_attention(x, pending)
                 o = self.attn(qkv, pos)
@@ -118,11 +133,19 @@ class GPT2(nn.Module):
     def head_weight(self) -> torch.Tensor:
         return self.wte if self.lm_head is None else self.lm_head
 
+    def loss_with(self, idx_local, targets_local, pos, grad_scale: float) -> torch.Tensor:
+        return xent.linear_cross_entropy(self._hidden(idx_local, pos), self.head_weight(), targets_local, grad_scale, self.cfg.vocab_size)
+
     def loss_sum(self, idx_local, targets_local, pos, grad_scale: float = 1.0) -> torch.Tensor:
         h = self.hidden(idx_local, pos)
         return xent.linear_cross_entropy(h, self.head_weight(), targets_local, grad_scale, self.cfg.vocab_size)
 
     def per_token_nll(self, idx_local, targets_local, pos) -> torch.Tensor:
+        def nll(idx, targets, pos):
+            return (xent.per_token_nll(self._hidden(idx, pos), self.head_weight(), targets, self.cfg.vocab_size).view(idx.shape),)
         with torch.no_grad():
-            h = self.hidden(idx_local, pos)
-            return xent.per_token_nll(h, self.head_weight(), targets_local, self.cfg.vocab_size).view(idx_local.shape)
+            if not self.recordable():
+                h = self.hidden(idx_local, pos)
+                return xent.per_token_nll(h, self.head_weight(), targets_local, self.cfg.vocab_size).view(idx_local.shape)
+            return self.graphs.run("nll", self, nll, (idx_local, targets_local, pos), self.wte.device,
+                                   graphs.model_flops(self.cfg, *idx_local.shape, False))[0]

@@ -20,6 +20,7 @@ import torch
 import torch.nn as nn
 from torch.utils.checkpoint import checkpoint
 
+from .. import graphs
 from ..config import Config
 from ..ops import elementwise as E
 from ..ops import gemm as G
@@ -90,6 +91,7 @@ class Llama(nn.Module):
         self.attn = CPAttention(cfg, self.cp)
         self.rope_cache = R.build_rope_cache(cfg.T, cfg.head_dim, cfg.rope_theta, device, cfg.yarn)
         self.rope_pos_override: Optional[torch.Tensor] = None
+        self.graphs = graphs.GraphCache()
 
     # ------------------------------------------------------------------ RoPE cache control
     def set_rope_cache(self, cache: torch.Tensor) -> None:
@@ -125,35 +127,54 @@ class Llama(nn.Module):
     # ------------------------------------------------------------------ forward
     def hidden(self, idx_local: torch.Tensor, pos: torch.Tensor) -> torch.Tensor:
         """Final-norm hidden states ``[B, T_local, d]`` for local tokens at global positions ``pos``."""
+        if torch.is_grad_enabled() or self.cp.cp_size > 1:
+            return self._hidden(idx_local, pos, *self.recorded_inputs())
+        return self.graphs.run("hidden", self, lambda *a: (self._hidden(*a),), (idx_local, pos, *self.recorded_inputs()),
+                               self.wte.device, graphs.model_flops(self.cfg, *idx_local.shape, False))[0]
+
+    def recorded_inputs(self) -> tuple:
+        """What ``loss_with`` reads beside its tokens, targets and positions and the weights: these are swapped between calls."""
+        return (self.rope_cache,) if self.rope_pos_override is None else (self.rope_cache, self.rope_pos_override)
+
+    def recordable(self) -> bool:
+        return self.cp.cp_size == 1 and graphs.as_written(self, Llama, "hidden", "loss_sum", "per_token_nll")
+
+    def _hidden(self, idx_local: torch.Tensor, pos: torch.Tensor, rope_cache: torch.Tensor,
+                rope_pos: Optional[torch.Tensor] = None) -> torch.Tensor:
         cfg = self.cfg
         x = E.embedding(idx_local, self.wte)
         pending = None
-        rpos = pos if self.rope_pos_override is None else self.rope_pos_override
+        rpos = pos if rope_pos is None else rope_pos
         use_ckpt = cfg.recompute in ("selective", "full") and torch.is_grad_enabled()
         full = cfg.recompute == "full" and torch.is_grad_enabled()
         for blk in self.blocks:
             if full:
                 # full activation recompute: only the block's input survives the forward pass; backward re-runs the
                 # whole block, context-parallel attention (and its communication) included, on every rank alike
-                x, pending = checkpoint(self._block, blk, x, pending, rpos, pos, use_reentrant=False)
+                x, pending = checkpoint(self._block, blk, x, pending, rope_cache, rpos, pos, use_reentrant=False, preserve_rng_state=False)
             elif use_ckpt:
-                x, qkv = checkpoint(blk.pre_attention, x, pending, self.rope_cache, rpos, use_reentrant=False)
+                x, qkv = checkpoint(blk.pre_attention, x, pending, rope_cache, rpos, use_reentrant=False, preserve_rng_state=False)
                 o = self.attn(qkv, pos)
-                x, pending = checkpoint(blk.post_attention, x, o, use_reentrant=False)
+                x, pending = checkpoint(blk.post_attention, x, o, use_reentrant=False, preserve_rng_state=False)
             else:
-                x, qkv = blk.pre_attention(x, pending, self.rope_cache, rpos)
+                x, qkv = blk.pre_attention(x, pending, rope_cache, rpos)
                 o = self.attn(qkv, pos)
                 x, pending = blk.post_attention(x, o)
         h, _ = E.rmsnorm(x, self.norm_f, cfg.rms_eps, pending)
         return h
 
-    def _block(self, blk, x, pending, rpos, pos):
-        x, qkv = blk.pre_attention(x, pending, self.rope_cache, rpos)
+    def _block(self, blk, x, pending, rope_cache, rpos, pos):
+        x, qkv = blk.pre_attention(x, pending, rope_cache, rpos)
         o = self.attn(qkv, pos)
         return blk.post_attention(x, o)
 
     def head_weight(self) -> torch.Tensor:
         return self.wte if self.lm_head is None else self.lm_head
+
+    def loss_with(self, idx_local, targets_local, pos, *rope_and_scale) -> torch.Tensor:
+        *rope, grad_scale = rope_and_scale
+        h = self._hidden(idx_local, pos, *rope)
+        return xent.linear_cross_entropy(h, self.head_weight(), targets_local, grad_scale, self.cfg.vocab_size)
 
     def loss_sum(self, idx_local, targets_local, pos, grad_scale: float = 1.0) -> torch.Tensor:
         """Sum of token NLLs over the local shard (fp32 scalar)."""
@@ -161,6 +182,11 @@ class Llama(nn.Module):
         return xent.linear_cross_entropy(h, self.head_weight(), targets_local, grad_scale, self.cfg.vocab_size)
 
     def per_token_nll(self, idx_local, targets_local, pos) -> torch.Tensor:
+        def nll(idx, targets, pos, *rope):
+            return (xent.per_token_nll(self._hidden(idx, pos, *rope), self.head_weight(), targets, self.cfg.vocab_size).view(idx.shape),)
         with torch.no_grad():
-            h = self.hidden(idx_local, pos)
-            return xent.per_token_nll(h, self.head_weight(), targets_local, self.cfg.vocab_size).view(idx_local.shape)
+            if not self.recordable():
+                h = self.hidden(idx_local, pos)
+                return xent.per_token_nll(h, self.head_weight(), targets_local, self.cfg.vocab_size).view(idx_local.shape)
+            return self.graphs.run("nll", self, nll, (idx_local, targets_local, pos, *self.recorded_inputs()), self.wte.device,
+                                   graphs.model_flops(self.cfg, *idx_local.shape, False))[0]

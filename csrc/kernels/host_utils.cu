@@ -81,3 +81,9 @@ int encode_tmap(CUtensorMap* out, const void* base, int elem_bytes, int rank, co
 }  // namespace cpb
 
 extern "C" const char* cpb_last_error() { return cpb::last_error_buf(); }
+
+// Forget the error that a failed stream capture left behind: the next launch would report it as its own.
+extern "C" int cpb_clear_error() {
+  (void)cudaGetLastError();
+  return cpb::CPB_OK;
+}
