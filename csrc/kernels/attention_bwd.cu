@@ -461,6 +461,8 @@ __global__ void bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, const __nv_
                                 const float* __restrict__ lse, float* __restrict__ delta, float* __restrict__ lse2,
                                 float4* __restrict__ acc, size_t acc4, const int* __restrict__ q_pos, int* __restrict__ q_pos_pad,
                                 int B, int Tq, int Hq, int Tq_pad) {
+  pdl_release();
+  pdl_wait();
   constexpr int LPR = D / 8;                                 // lanes per row
   const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (q_pos_pad != nullptr)
@@ -523,8 +525,8 @@ extern "C" int cpb_flash_bwd_prep(const void* o, const void* dout, const float* 
   const size_t cap = (size_t)sm_count() * 32;
   if (g > cap) g = cap;
   auto kern = D == 64 ? bwd_prep_kernel<64> : bwd_prep_kernel<128>;
-  kern<<<(int)g, 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, lse, delta, lse2, (float4*)acc, acc != nullptr ? (size_t)acc_n / 4 : 0, q_pos, q_pos_pad,
-                                 B, Tq, Hq, Tq_pad);
+  CPB_CUDA_OK(launch_pdl(kern, (int)g, 256, 0, stream, (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, lse, delta, lse2, (float4*)acc, acc != nullptr ? (size_t)acc_n / 4 : 0, q_pos, q_pos_pad,
+                                 B, Tq, Hq, Tq_pad));
   return check_launch("flash_bwd_prep");
 }
 

@@ -94,7 +94,7 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   constexpr int D = B128_D, CW = B128_CW;
   constexpr uint32_t ST_COL = 0, DPT_COL = 128, DV_COL = 256, DK_COL = 384;
   extern __shared__ __align__(1024) uint8_t smem[];
-  if (smem_u32(smem) & 1023) { report(p.status, ST_BAD_INDEX, 870, (int)smem_u32(smem)); return; }
+  if (smem_u32(smem) & 1023) { pdl_wait(); report(p.status, ST_BAD_INDEX, 870, (int)smem_u32(smem)); return; }
   uint64_t* bars = (uint64_t*)(smem + L::BAR_OFF);
   uint64_t* kv_full = bars + 0;
   uint64_t* q_full = bars + 1;        // [2]
@@ -118,7 +118,10 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const int G = p.Hq / p.Hkv;
   const int k0 = kt * B128_T;
   const int num_q_tiles = p.Tq_pad / B128_T;
-  if (p.it_chunk && p.local && work.it0 >= (num_q_tiles - (p.causal ? min(num_q_tiles, max(0, p.k_off + k0) / B128_T) : 0)) * G) return;
+  if (p.it_chunk && p.local && work.it0 >= (num_q_tiles - (p.causal ? min(num_q_tiles, max(0, p.k_off + k0) / B128_T) : 0)) * G) {
+    pdl_wait();
+    return;
+  }
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
@@ -134,6 +137,8 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_release();
+  pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
 
   // first query tile that can see this K/V tile (q_pos is non-decreasing)
@@ -537,6 +542,6 @@ extern "C" int cpb_flash_bwd128(const void* q, const void* k, const void* v, con
   const dim3 grid = it_chunk ? dim3((unsigned)n_kt * ((pairs + it_chunk - 1) / it_chunk) * Hkv * B) : dim3(n_kt, Hkv, B);
   static bool cfg = false;
   if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_bwd128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Bwd128Smem::TOTAL)); cfg = true; }
-  flash_bwd128_kernel<<<grid, B128_THREADS, Bwd128Smem::TOTAL, stream>>>(tq, tk, tv, tdo, tdq, p);
+  CPB_CUDA_OK(launch_pdl(flash_bwd128_kernel, grid, B128_THREADS, Bwd128Smem::TOTAL, stream, tq, tk, tv, tdo, tdq, p));
   return check_launch("flash_bwd128");
 }

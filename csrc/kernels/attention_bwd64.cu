@@ -96,7 +96,7 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   constexpr int D = B64_D, CW = B64_CW, NST = L::NST;
   constexpr uint32_t ST_COL = 0, DPT_COL = 128, DV_COL = 256, DK_COL = 320, DQ_COL = 384, K_COL = 448, V_COL = 480;
   extern __shared__ __align__(1024) uint8_t smem[];
-  if (smem_u32(smem) & 1023) { report(p.status, ST_BAD_INDEX, 870, (int)smem_u32(smem)); return; }
+  if (smem_u32(smem) & 1023) { pdl_wait(); report(p.status, ST_BAD_INDEX, 870, (int)smem_u32(smem)); return; }
   uint64_t* bars = (uint64_t*)(smem + L::BAR_OFF);
   uint64_t* kv_full = bars + 0;
   uint64_t* q_full = bars + 1;        // [NST]
@@ -120,7 +120,10 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const int G = p.Hq / p.Hkv;
   const int k0 = kt * B64_T;
   const int num_q_tiles = p.Tq_pad / B64_T;
-  if (p.it_chunk && p.local && work.it0 >= (num_q_tiles - (p.causal ? min(num_q_tiles, max(0, p.k_off + k0) / B64_T) : 0)) * G) return;
+  if (p.it_chunk && p.local && work.it0 >= (num_q_tiles - (p.causal ? min(num_q_tiles, max(0, p.k_off + k0) / B64_T) : 0)) * G) {
+    pdl_wait();
+    return;
+  }
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
@@ -135,6 +138,8 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_release();
+  pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
 
   // first query tile that can see this K/V tile (q_pos is non-decreasing)
@@ -555,6 +560,6 @@ extern "C" int cpb_flash_bwd64(const void* q, const void* k, const void* v, cons
   const dim3 grid = it_chunk ? dim3((unsigned)n_kt * ((pairs + it_chunk - 1) / it_chunk) * Hkv * B) : dim3(n_kt, Hkv, B);
   static bool cfg = false;
   if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_bwd64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Bwd64Smem::TOTAL)); cfg = true; }
-  flash_bwd64_kernel<<<grid, B64_THREADS, Bwd64Smem::TOTAL, stream>>>(tq, tk, tdo, tdq, p);
+  CPB_CUDA_OK(launch_pdl(flash_bwd64_kernel, grid, B64_THREADS, Bwd64Smem::TOTAL, stream, tq, tk, tdo, tdq, p));
   return check_launch("flash_bwd64");
 }

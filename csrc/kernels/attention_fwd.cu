@@ -60,6 +60,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                  const __grid_constant__ CUtensorMap tmV, FwdParams p) {
   using L = FwdSmem<D>;
   if (p.n_copy > 0 && blockIdx.x < (unsigned)p.n_copy) {
+    pdl_wait();
     if (blockIdx.y == 0 && blockIdx.z == 0) ring_copy_cta(p.segs, p.n_segs, p.n_copy, blockIdx.x, p.ready);
     return;
   }
@@ -95,23 +96,6 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const int b = blockIdx.z;
   const int q0 = qt * FA_BQ;
 
-  // Range of K/V tiles this query tile attends to.
-  const int q_last = min(q0 + FA_BQ, p.Tq) - 1;
-  const int qpos_min = p.q_pos ? p.q_pos[q0] : q0;
-  const int qpos_max = p.q_pos ? p.q_pos[q_last] : q_last;
-  int n_kv = (p.Tk + FA_BK - 1) / FA_BK;
-  if (p.causal) {
-    const int last_idx = qpos_max - p.k_off;                  // last visible K index
-    n_kv = last_idx < 0 ? 0 : min(n_kv, last_idx / FA_BK + 1);
-  }
-  // Order of the K/V sweep: tile (j + j_start) % n_kv.  With readiness flags the sweep starts at the chunk
-  // that contains this tile's own positions (resident locally), so remote chunks have time to arrive.
-  int j_start = 0;
-  if (p.ready != nullptr && n_kv > 0 && (p.block_rows % FA_BK) == 0) {
-    const int c = max(qpos_min - p.k_off, 0) / p.block_rows;
-    j_start = min(c * (p.block_rows / FA_BK), n_kv - 1);
-  }
-
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int s = 0; s < FA_KSTAGES; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
@@ -129,6 +113,25 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (p.ready == nullptr) pdl_release();
+  pdl_wait();
+
+  // Range of K/V tiles this query tile attends to.
+  const int q_last = min(q0 + FA_BQ, p.Tq) - 1;
+  const int qpos_min = p.q_pos ? p.q_pos[q0] : q0;
+  const int qpos_max = p.q_pos ? p.q_pos[q_last] : q_last;
+  int n_kv = (p.Tk + FA_BK - 1) / FA_BK;
+  if (p.causal) {
+    const int last_idx = qpos_max - p.k_off;                  // last visible K index
+    n_kv = last_idx < 0 ? 0 : min(n_kv, last_idx / FA_BK + 1);
+  }
+  // Order of the K/V sweep: tile (j + j_start) % n_kv.  With readiness flags the sweep starts at the chunk
+  // that contains this tile's own positions (resident locally), so remote chunks have time to arrive.
+  int j_start = 0;
+  if (p.ready != nullptr && n_kv > 0 && (p.block_rows % FA_BK) == 0) {
+    const int c = max(qpos_min - p.k_off, 0) / p.block_rows;
+    j_start = min(c * (p.block_rows / FA_BK), n_kv - 1);
+  }
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA loader
@@ -476,7 +479,7 @@ extern "C" int cpb_flash_fwd(const void* q, const void* k, const void* v, void* 
   do {                                                                                                                 \
     static bool cfg = false;                                                                                           \
     if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_fwd_kernel<DD, PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdSmem<DD>::TOTAL)); cfg = true; } \
-    flash_fwd_kernel<DD, PP><<<grid, FA_THREADS, FwdSmem<DD>::TOTAL, stream>>>(tq, tk, tv, p);                         \
+    CPB_CUDA_OK(launch_pdl(flash_fwd_kernel<DD, PP>, grid, FA_THREADS, FwdSmem<DD>::TOTAL, stream, tq, tk, tv, p));    \
   } while (0)
   if (D == 64) {
     switch (poly) {

@@ -40,6 +40,7 @@ flash_fwd128_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   using L = FpSmem;
   constexpr int D = L::D;
   if (p.n_copy > 0 && blockIdx.x < (unsigned)p.n_copy) {
+    pdl_wait();
     if (blockIdx.y == 0 && blockIdx.z == 0) ring_copy_cta(p.segs, p.n_segs, p.n_copy, blockIdx.x, p.ready);
     return;
   }
@@ -69,6 +70,22 @@ flash_fwd128_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   const int b = blockIdx.z;
   const int q0 = qt * 2 * FA_BQ;
 
+  if (threadIdx.x == 0) {
+    for (int t = 0; t < 2; ++t) { mbar_init(&q_full[t], 1); mbar_init(&s_full[t], 1); mbar_init(&p_full[t], 4); }
+    for (int s = 0; s < L::KST; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
+    for (int s = 0; s < L::VST; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
+    mbar_init(o_done, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  if (p.ready == nullptr) pdl_release();
+  pdl_wait();
+
   // K/V tiles that each of the two query tiles attends to: 0 .. n_t - 1
   const int qpos_min0 = p.q_pos ? p.q_pos[q0] : q0;
   int n0 = (p.Tk + FA_BK - 1) / FA_BK, n1 = n0;
@@ -90,20 +107,6 @@ flash_fwd128_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   // a wrapped sweep visits every tile for both query tiles (what a tile cannot see is masked)
   const int cnt0 = n0 == 0 || j_start == 0 ? n0 : n_kv, cnt1 = n1 == 0 || j_start == 0 ? n1 : n_kv;
   auto kv_tile = [&](int j) { const int jj = j + j_start; return jj >= n_kv ? jj - n_kv : jj; };
-
-  if (threadIdx.x == 0) {
-    for (int t = 0; t < 2; ++t) { mbar_init(&q_full[t], 1); mbar_init(&s_full[t], 1); mbar_init(&p_full[t], 4); }
-    for (int s = 0; s < L::KST; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
-    for (int s = 0; s < L::VST; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
-    mbar_init(o_done, 1);
-    *abort_flag = 0;
-    fence_mbar_init();
-  }
-  if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
 
   if (warp < 4) {
     regs_give<FP_REGS_ISSUE>();
@@ -391,7 +394,7 @@ static int launch_pair(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
   static bool cfg = false;
   if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_fwd128_pair_kernel<POLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, FpSmem::TOTAL)); cfg = true; }
   const dim3 grid(p.n_copy + (p.Tq + 2 * FA_BQ - 1) / (2 * FA_BQ) * (p.Hq / p.Hkv), p.Hkv, p.B);
-  flash_fwd128_pair_kernel<POLY><<<grid, FP_THREADS, FpSmem::TOTAL, stream>>>(tq, tk, tv, p);
+  CPB_CUDA_OK(launch_pdl(flash_fwd128_pair_kernel<POLY>, grid, FP_THREADS, FpSmem::TOTAL, stream, tq, tk, tv, p));
   return check_launch("flash_fwd");
 }
 

@@ -48,6 +48,17 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// ------------------------------------------------------------------ programmatic dependent launch
+// A kernel started with launch_pdl (host_utils.h) may begin while the one before it on the stream still runs: its blocks set up
+// barriers, tensor memory and descriptors, and pdl_wait() returns once every earlier kernel has finished and its writes are
+// visible.  So pdl_wait() comes before the first access to global memory, weights included (the optimiser may be what runs before),
+// and every block gets there: a grid that ended without it could end before its predecessor.
+// pdl_release() lets the next kernel's blocks in as soon as every block of this one has got that far: after the block has its
+// tensor memory, or a waiting block on the same SM could hold the columns that a running one still wants, and never in a kernel
+// that waits for other GPUs, whose SMs the blocks let in would keep from the kernels of other streams.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ------------------------------------------------------------------ mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");

@@ -51,6 +51,8 @@ __global__ void norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_
                                 const float* __restrict__ w, const float* __restrict__ b,
                                 __nv_bfloat16* __restrict__ xout, __nv_bfloat16* __restrict__ y,
                                 float* __restrict__ stats, int rows, int d, float eps) {
+  pdl_release();
+  pdl_wait();
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31;
@@ -126,6 +128,8 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
                 const __nv_bfloat16* __restrict__ dres, const float* __restrict__ w,
                 const float* __restrict__ stats, __nv_bfloat16* __restrict__ dx,
                 float* __restrict__ dw, float* __restrict__ db, int rows, int d) {
+  pdl_release();
+  pdl_wait();
   constexpr int TB = G > 256 ? 512 : 256, NG = TB / G, W = G / 32, R = 4;
   __shared__ float4 red[2][NG][W][LAYER ? 2 : 1];            // per warp: four rows' sums; two buffers, one barrier per turn
   __shared__ float part[NG > 1 ? TB * 8 : 1];                // used only when a block holds several groups
@@ -239,6 +243,8 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 // gu: [rows, 2F] = [gate | up]; dact: [rows, F]; dgu: [rows, 2F]
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dact,
                                   __nv_bfloat16* __restrict__ dgu, size_t rows, int F) {
+  pdl_release();
+  pdl_wait();
   const size_t nvec = rows * (size_t)(F >> 3);
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nvec; i += (size_t)gridDim.x * blockDim.x) {
     const size_t row = i / (F >> 3);
@@ -262,6 +268,8 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __
 
 // forward (standalone, used when the GEMM epilogue fusion is not): act = silu(g)*u
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ act, size_t rows, int F) {
+  pdl_release();
+  pdl_wait();
   const size_t nvec = rows * (size_t)(F >> 3);
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nvec; i += (size_t)gridDim.x * blockDim.x) {
     const size_t row = i / (F >> 3);
@@ -294,6 +302,8 @@ __device__ __forceinline__ float gelu_tanh_val(float x) {
 // mode 0: y = gelu(x) ; mode 1: y = dy * gelu'(x)
 __global__ void gelu_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
                             __nv_bfloat16* __restrict__ y, size_t n8, int mode) {
+  pdl_release();
+  pdl_wait();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n8; i += (size_t)gridDim.x * blockDim.x) {
     float xv[8], o[8];
     uint4 ux = ((const uint4*)x)[i];
@@ -327,6 +337,8 @@ __global__ void add_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloa
 
 // db[n] += sum_rows dy[row, n]; grid (ceil(N/64), row_blocks); block 256 = 8 row-lanes x 32 col-pairs
 __global__ void bias_grad_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ db, int rows, int N, int rows_per_block) {
+  pdl_release();
+  pdl_wait();
   __shared__ float red[8][64];
   const int cp = threadIdx.x & 31, rl = threadIdx.x >> 5;
   const int col = blockIdx.x * 64 + cp * 2;
@@ -354,6 +366,8 @@ __global__ void bias_grad_kernel(const __nv_bfloat16* __restrict__ dy, float* __
 __global__ void embedding_fwd_kernel(const int64_t* __restrict__ idx, const int64_t* __restrict__ pos,
                                      const __nv_bfloat16* __restrict__ wte, const __nv_bfloat16* __restrict__ wpe,
                                      __nv_bfloat16* __restrict__ out, size_t rows, int d, int pos_period) {
+  pdl_release();
+  pdl_wait();
   const int nvec = d >> 3;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < rows * nvec; i += (size_t)gridDim.x * blockDim.x) {
     const size_t row = i / nvec;
@@ -374,6 +388,8 @@ __global__ void embedding_fwd_kernel(const int64_t* __restrict__ idx, const int6
 __global__ void embedding_bwd_kernel(const int64_t* __restrict__ idx, const int64_t* __restrict__ pos,
                                      const __nv_bfloat16* __restrict__ dout, float* __restrict__ dwte,
                                      float* __restrict__ dwpe, size_t rows, int d, int pos_period) {
+  pdl_release();
+  pdl_wait();
   const int nvec = d >> 3;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < rows * nvec; i += (size_t)gridDim.x * blockDim.x) {
     const size_t row = i / nvec;
@@ -420,6 +436,8 @@ __global__ void __launch_bounds__(256, 3) qk_norm_rope_fwd_kernel(const __nv_bfl
                                         const float* __restrict__ cache, const int64_t* __restrict__ pos,
                                         float* __restrict__ rstd, size_t rows, int T, int Hq, int Hkv, float eps,
                                         int cache_len, int* status) {
+  pdl_release();
+  pdl_wait();
   constexpr int GL = D / 8, VPW = 32 / GL, half = D / 2, U = 4;
   const int H = Hq + 2 * Hkv;
   const int lane = threadIdx.x & 31;
@@ -491,6 +509,8 @@ __global__ void __launch_bounds__(256, 2) qk_norm_rope_bwd_kernel(const __nv_bfl
                                         const float* __restrict__ gk, const float* __restrict__ cache,
                                         const int64_t* __restrict__ pos, float* __restrict__ dgq, float* __restrict__ dgk,
                                         size_t rows, int T, int Hq, int Hkv, float eps, int cache_len) {
+  pdl_release();
+  pdl_wait();
   constexpr int GL = D / 8, VPW = 32 / GL, half = D / 2, U = 2;
   __shared__ float sg[2][D];
   for (int i = threadIdx.x; i < 2 * D; i += blockDim.x) (&sg[0][0])[i] = 0.f;
@@ -780,6 +800,8 @@ __global__ void adamw_sharded_kernel(float* __restrict__ p, const float* __restr
 }
 
 __global__ void cast_f32_bf16_kernel(const float* __restrict__ in, __nv_bfloat16* __restrict__ out, size_t n, float scale) {
+  pdl_release();
+  pdl_wait();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     out[i] = __float2bfloat16(in[i] * scale);
 }
@@ -792,6 +814,8 @@ struct CastPiece {
   long stride;             // elements from row to row
 };
 __global__ void cast_f32_bf16_rows_kernel(const float* __restrict__ in, CastPiece a, CastPiece b, CastPiece c, float scale) {
+  pdl_release();
+  pdl_wait();
   const size_t total = a.n8 + b.n8 + c.n8;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const bool in_a = i < a.n8, in_b = !in_a && i < a.n8 + b.n8;
@@ -821,14 +845,14 @@ static inline int grid_for(size_t work, int block, int per_sm = 8) {
 
 using namespace cpb;
 
-#define NORM_DISPATCH(KERN, LAYER, ...)                                              \
+#define NORM_DISPATCH(KERN, LAYER)                                                   \
   do {                                                                               \
     const int nv = (d / 8 + 31) / 32;                                                \
-    if (nv <= 1) KERN<LAYER, 1> __VA_ARGS__;                                         \
-    else if (nv <= 2) KERN<LAYER, 2> __VA_ARGS__;                                    \
-    else if (nv <= 4) KERN<LAYER, 4> __VA_ARGS__;                                    \
-    else if (nv <= 8) KERN<LAYER, 8> __VA_ARGS__;                                    \
-    else if (nv <= 16) KERN<LAYER, 16> __VA_ARGS__;                                  \
+    if (nv <= 1) kern = KERN<LAYER, 1>;                                              \
+    else if (nv <= 2) kern = KERN<LAYER, 2>;                                         \
+    else if (nv <= 4) kern = KERN<LAYER, 4>;                                         \
+    else if (nv <= 8) kern = KERN<LAYER, 8>;                                         \
+    else if (nv <= 16) kern = KERN<LAYER, 16>;                                       \
     else return set_error(CPB_ERR_LIMIT, "norm: d=%d exceeds 4096", d);              \
   } while (0)
 
@@ -838,9 +862,10 @@ extern "C" int cpb_norm_fwd(const void* x, const void* res, const float* w, cons
   if (d % 8) return set_error(CPB_ERR_ARG, "norm: d=%d must be a multiple of 8", d);
   if (rows <= 0) return CPB_OK;
   const int wpb = 8;
-  dim3 grid((rows + wpb - 1) / wpb), block(wpb * 32);
-  if (layer) NORM_DISPATCH(norm_fwd_kernel, true, <<<grid, block, 0, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)res, w, b, (__nv_bfloat16*)xout, (__nv_bfloat16*)y, stats, rows, d, eps));
-  else NORM_DISPATCH(norm_fwd_kernel, false, <<<grid, block, 0, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)res, w, b, (__nv_bfloat16*)xout, (__nv_bfloat16*)y, stats, rows, d, eps));
+  decltype(&norm_fwd_kernel<true, 1>) kern;
+  if (layer) NORM_DISPATCH(norm_fwd_kernel, true);
+  else NORM_DISPATCH(norm_fwd_kernel, false);
+  CPB_CUDA_OK(launch_pdl(kern, (rows + wpb - 1) / wpb, wpb * 32, 0, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res, w, b, (__nv_bfloat16*)xout, (__nv_bfloat16*)y, stats, rows, d, eps));
   return check_launch("norm_fwd");
 }
 
@@ -856,8 +881,8 @@ extern "C" int cpb_norm_bwd(const void* x, const void* dy, const void* dres, con
     const int tb = G > 256 ? 512 : 256, per_block = 4 * (tb / G);                                                               \
     const int cap = sm_count() * (G > 256 ? 1 : 2), need = (rows + per_block - 1) / per_block, blocks = need < cap ? need : cap; \
     auto kern = layer ? norm_bwd_kernel<true, G> : norm_bwd_kernel<false, G>;                                                   \
-    kern<<<blocks, tb, 0, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)dres, w, stats,    \
-                                    (__nv_bfloat16*)dx, dw, db, rows, d);                                                       \
+    CPB_CUDA_OK(launch_pdl(kern, blocks, tb, 0, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)dres, w, stats,    \
+                                    (__nv_bfloat16*)dx, dw, db, rows, d));                                                       \
   } while (0)
   if (nvec <= 32) NORM_BWD(32);
   else if (nvec <= 64) NORM_BWD(64);
@@ -871,19 +896,19 @@ extern "C" int cpb_norm_bwd(const void* x, const void* dy, const void* dres, con
 extern "C" int cpb_swiglu_fwd(const void* gu, void* act, long rows, int F, cudaStream_t stream) {
   if (F % 8) return set_error(CPB_ERR_ARG, "swiglu: F must be a multiple of 8");
   if (rows <= 0) return CPB_OK;
-  swiglu_fwd_kernel<<<grid_for((size_t)rows * (F / 8), 256), 256, 0, stream>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)act, (size_t)rows, F);
+  CPB_CUDA_OK(launch_pdl(swiglu_fwd_kernel, grid_for((size_t)rows * (F / 8), 256), 256, 0, stream, (const __nv_bfloat16*)gu, (__nv_bfloat16*)act, (size_t)rows, F));
   return check_launch("swiglu_fwd");
 }
 extern "C" int cpb_swiglu_bwd(const void* gu, const void* dact, void* dgu, long rows, int F, cudaStream_t stream) {
   if (F % 8) return set_error(CPB_ERR_ARG, "swiglu: F must be a multiple of 8");
   if (rows <= 0) return CPB_OK;
-  swiglu_bwd_kernel<<<grid_for((size_t)rows * (F / 8), 256), 256, 0, stream>>>((const __nv_bfloat16*)gu, (const __nv_bfloat16*)dact, (__nv_bfloat16*)dgu, (size_t)rows, F);
+  CPB_CUDA_OK(launch_pdl(swiglu_bwd_kernel, grid_for((size_t)rows * (F / 8), 256), 256, 0, stream, (const __nv_bfloat16*)gu, (const __nv_bfloat16*)dact, (__nv_bfloat16*)dgu, (size_t)rows, F));
   return check_launch("swiglu_bwd");
 }
 extern "C" int cpb_gelu(const void* x, const void* dy, void* y, long n, int mode, cudaStream_t stream) {
   if (n % 8) return set_error(CPB_ERR_ARG, "gelu: n must be a multiple of 8");
   if (n <= 0) return CPB_OK;
-  gelu_kernel<<<grid_for((size_t)n / 8, 256), 256, 0, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, (__nv_bfloat16*)y, (size_t)n / 8, mode);
+  CPB_CUDA_OK(launch_pdl(gelu_kernel, grid_for((size_t)n / 8, 256), 256, 0, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, (__nv_bfloat16*)y, (size_t)n / 8, mode));
   return check_launch("gelu");
 }
 extern "C" int cpb_add_bf16(const void* a, const void* b, void* y, long n, cudaStream_t stream) {
@@ -900,21 +925,21 @@ extern "C" int cpb_bias_grad(const void* dy, float* db, int rows, int N, cudaStr
   int rpb = (rows + rb - 1) / rb;
   if (rpb < 64) rpb = 64;
   rb = (rows + rpb - 1) / rpb;
-  bias_grad_kernel<<<dim3((N + 63) / 64, rb), 256, 0, stream>>>((const __nv_bfloat16*)dy, db, rows, N, rpb);
+  CPB_CUDA_OK(launch_pdl(bias_grad_kernel, dim3((N + 63) / 64, rb), 256, 0, stream, (const __nv_bfloat16*)dy, db, rows, N, rpb));
   return check_launch("bias_grad");
 }
 extern "C" int cpb_embedding_fwd(const int64_t* idx, const int64_t* pos, const void* wte, const void* wpe, void* out,
                                  long rows, int d, int pos_period, cudaStream_t stream) {
   if (d % 8) return set_error(CPB_ERR_ARG, "embedding: d must be a multiple of 8");
   if (rows <= 0) return CPB_OK;
-  embedding_fwd_kernel<<<grid_for((size_t)rows * (d / 8), 256), 256, 0, stream>>>(idx, pos, (const __nv_bfloat16*)wte, (const __nv_bfloat16*)wpe, (__nv_bfloat16*)out, (size_t)rows, d, pos_period);
+  CPB_CUDA_OK(launch_pdl(embedding_fwd_kernel, grid_for((size_t)rows * (d / 8), 256), 256, 0, stream, idx, pos, (const __nv_bfloat16*)wte, (const __nv_bfloat16*)wpe, (__nv_bfloat16*)out, (size_t)rows, d, pos_period));
   return check_launch("embedding_fwd");
 }
 extern "C" int cpb_embedding_bwd(const int64_t* idx, const int64_t* pos, const void* dout, float* dwte, float* dwpe,
                                  long rows, int d, int pos_period, cudaStream_t stream) {
   if (d % 8) return set_error(CPB_ERR_ARG, "embedding: d must be a multiple of 8");
   if (rows <= 0) return CPB_OK;
-  embedding_bwd_kernel<<<grid_for((size_t)rows * (d / 8), 256), 256, 0, stream>>>(idx, pos, (const __nv_bfloat16*)dout, dwte, dwpe, (size_t)rows, d, pos_period);
+  CPB_CUDA_OK(launch_pdl(embedding_bwd_kernel, grid_for((size_t)rows * (d / 8), 256), 256, 0, stream, idx, pos, (const __nv_bfloat16*)dout, dwte, dwpe, (size_t)rows, d, pos_period));
   return check_launch("embedding_bwd");
 }
 
@@ -923,8 +948,8 @@ extern "C" int cpb_qk_norm_rope_fwd(const void* in, void* out, const float* gq, 
                                     float eps, int cache_len, int* status, cudaStream_t stream) {
   if (rows <= 0) return CPB_OK;
   const int grid = grid_for((size_t)rows, 8);      // one warp per token row, eight warps per block
-  if (D == 64) qk_norm_rope_fwd_kernel<64><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)in, (__nv_bfloat16*)out, gq, gk, cache, pos, rstd, (size_t)rows, T, Hq, Hkv, eps, cache_len, status);
-  else if (D == 128) qk_norm_rope_fwd_kernel<128><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)in, (__nv_bfloat16*)out, gq, gk, cache, pos, rstd, (size_t)rows, T, Hq, Hkv, eps, cache_len, status);
+  if (D == 64) CPB_CUDA_OK(launch_pdl(qk_norm_rope_fwd_kernel<64>, grid, 256, 0, stream, (const __nv_bfloat16*)in, (__nv_bfloat16*)out, gq, gk, cache, pos, rstd, (size_t)rows, T, Hq, Hkv, eps, cache_len, status));
+  else if (D == 128) CPB_CUDA_OK(launch_pdl(qk_norm_rope_fwd_kernel<128>, grid, 256, 0, stream, (const __nv_bfloat16*)in, (__nv_bfloat16*)out, gq, gk, cache, pos, rstd, (size_t)rows, T, Hq, Hkv, eps, cache_len, status));
   else return set_error(CPB_ERR_ARG, "qk_norm_rope: head_dim %d not in {64,128}", D);
   return check_launch("qk_norm_rope_fwd");
 }
@@ -933,8 +958,8 @@ extern "C" int cpb_qk_norm_rope_bwd(const void* in, const void* dout, void* din,
                                     int Hq, int Hkv, int D, float eps, int cache_len, cudaStream_t stream) {
   if (rows <= 0) return CPB_OK;
   const int grid = grid_for((size_t)rows, 8, 4);
-  if (D == 64) qk_norm_rope_bwd_kernel<64><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)in, (const __nv_bfloat16*)dout, (__nv_bfloat16*)din, gq, gk, cache, pos, dgq, dgk, (size_t)rows, T, Hq, Hkv, eps, cache_len);
-  else if (D == 128) qk_norm_rope_bwd_kernel<128><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)in, (const __nv_bfloat16*)dout, (__nv_bfloat16*)din, gq, gk, cache, pos, dgq, dgk, (size_t)rows, T, Hq, Hkv, eps, cache_len);
+  if (D == 64) CPB_CUDA_OK(launch_pdl(qk_norm_rope_bwd_kernel<64>, grid, 256, 0, stream, (const __nv_bfloat16*)in, (const __nv_bfloat16*)dout, (__nv_bfloat16*)din, gq, gk, cache, pos, dgq, dgk, (size_t)rows, T, Hq, Hkv, eps, cache_len));
+  else if (D == 128) CPB_CUDA_OK(launch_pdl(qk_norm_rope_bwd_kernel<128>, grid, 256, 0, stream, (const __nv_bfloat16*)in, (const __nv_bfloat16*)dout, (__nv_bfloat16*)din, gq, gk, cache, pos, dgq, dgk, (size_t)rows, T, Hq, Hkv, eps, cache_len));
   else return set_error(CPB_ERR_ARG, "qk_norm_rope: head_dim %d not in {64,128}", D);
   return check_launch("qk_norm_rope_bwd");
 }
@@ -1022,14 +1047,14 @@ extern "C" int cpb_cast_f32_bf16_rows(const float* in, void* out_q, long rows_q,
   const CastPiece k{(__nv_bfloat16*)out_k, nk, cols_k > 0 ? cols_k / 8 : 1, kv_stride}, v{(__nv_bfloat16*)out_v, nk, k.c8, kv_stride};
   const size_t total = q.n8 + 2 * nk;
   if (total == 0) return CPB_OK;
-  cast_f32_bf16_rows_kernel<<<grid_for(total, 256, 32), 256, 0, stream>>>(in, q, k, v, scale);
+  CPB_CUDA_OK(launch_pdl(cast_f32_bf16_rows_kernel, grid_for(total, 256, 32), 256, 0, stream, in, q, k, v, scale));
   return check_launch("cast_rows");
 }
 extern "C" int cpb_cast_f32_bf16(const float* in, void* out, long n, float scale, cudaStream_t stream) {
   if (n <= 0) return CPB_OK;
   if (n % 8 == 0 && (((uintptr_t)in | (uintptr_t)out) & 15) == 0)
     return cpb_cast_f32_bf16_rows(in, out, n / 8, 8, 8, nullptr, nullptr, 0, 0, 0, scale, stream);
-  cast_f32_bf16_kernel<<<grid_for((size_t)n, 256), 256, 0, stream>>>(in, (__nv_bfloat16*)out, (size_t)n, scale);
+  CPB_CUDA_OK(launch_pdl(cast_f32_bf16_kernel, grid_for((size_t)n, 256), 256, 0, stream, in, (__nv_bfloat16*)out, (size_t)n, scale));
   return check_launch("cast_f32_bf16");
 }
 extern "C" int cpb_cast_bf16_f32(const void* in, float* out, long n, float scale, int accumulate, cudaStream_t stream) {

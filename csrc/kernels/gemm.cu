@@ -150,6 +150,8 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   __syncthreads();
   cluster_sync_all();                           // both CTAs' barriers exist before anything arrives on them remotely
   tc_fence_after();
+  pdl_release();
+  pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
@@ -284,7 +286,7 @@ static int launch_pair(const CUtensorMap (&tm)[4], const GemmParams& p, cudaStre
   const int items = p.num_m_tiles * p.num_n_blocks * p.splits;
   const int max_pairs = sm_count() / 2;
   const int pairs = items < max_pairs ? items : max_pairs;
-  kern<<<2 * pairs, GEMM_THREADS, GemmSmem<BN>::TOTAL, stream>>>(tm[0], tm[1], tm[2], tm[3], p);
+  CPB_CUDA_OK(launch_pdl(kern, 2 * pairs, GEMM_THREADS, GemmSmem<BN>::TOTAL, stream, tm[0], tm[1], tm[2], tm[3], p));
   return check_launch("gemm_pair_bf16");
 }
 
@@ -297,11 +299,11 @@ static int dispatch_pair(const CUtensorMap (&tm)[4], const GemmParams& p, int a_
 }
 
 // C += partials[0] + partials[1] + ..., always in that order and after the first split has been added, so that a weight gradient
-// repeats bit for bit (all splits adding to C in L2 as they finish, in one launch, do not).  Launched while the GEMM drains
-// (programmatic dependent launch); griddepcontrol.wait returns once the GEMM is complete and its writes are visible.
+// repeats bit for bit (all splits adding to C in L2 as they finish, in one launch, do not).  
 __global__ void __launch_bounds__(256)
 gemm_add_partials_kernel(float* __restrict__ C, const float4* __restrict__ partials, unsigned n4, unsigned total4, long ldc, int count) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_release();
+  pdl_wait();
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total4; i += gridDim.x * blockDim.x) {
     const unsigned r = i / n4;
     float4* dst = (float4*)(C + r * ldc) + (i - r * n4);
@@ -320,7 +322,8 @@ gemm_add_partials_kernel(float* __restrict__ C, const float4* __restrict__ parti
 __global__ void __launch_bounds__(256)
 gemm_sum_partials_kernel(__nv_bfloat16* __restrict__ C, const float4* __restrict__ partials, const float* __restrict__ bias, unsigned n8,
                          unsigned total8, long ldc, int count) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_release();
+  pdl_wait();
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total8; i += gridDim.x * blockDim.x) {
     const unsigned r = i / n8, c = i - r * n8;
     float4 a = partials[2 * (size_t)i], b = partials[2 * (size_t)i + 1];
@@ -473,14 +476,9 @@ extern "C" int cpb_gemm_bf16(const void* A, const void* B, void* C, void* aux, c
   rc = bn == 256 ? dispatch_pair<256>(tm, p, a_mn, b_mn, stream) : bn == 192 ? dispatch_pair<192>(tm, p, a_mn, b_mn, stream) : dispatch_pair<128>(tm, p, a_mn, b_mn, stream);
   if (rc != CPB_OK || splits == 1) return rc;
   const unsigned total = (unsigned)((long)M * N / (sum16 ? 8 : 4)), blocks = (total + 255) / 256, cap = (unsigned)sm_count() * 8;
-  cudaLaunchConfig_t lc = {};
-  lc.gridDim = dim3(blocks < cap ? blocks : cap); lc.blockDim = dim3(256); lc.stream = stream;
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  lc.attrs = &at; lc.numAttrs = 1;
-  if (sum16) CPB_CUDA_OK(cudaLaunchKernelEx(&lc, gemm_sum_partials_kernel, (__nv_bfloat16*)C, (const float4*)partials, bias, (unsigned)N / 8, total, (long)ldc, splits));
-  else CPB_CUDA_OK(cudaLaunchKernelEx(&lc, gemm_add_partials_kernel, (float*)C, (const float4*)partials, (unsigned)N / 4, total, (long)ldc, splits - 1));
+  const unsigned grid = blocks < cap ? blocks : cap;
+  if (sum16) CPB_CUDA_OK(launch_pdl(gemm_sum_partials_kernel, grid, 256, 0, stream, (__nv_bfloat16*)C, (const float4*)partials, bias, (unsigned)N / 8, total, (long)ldc, splits));
+  else CPB_CUDA_OK(launch_pdl(gemm_add_partials_kernel, grid, 256, 0, stream, (float*)C, (const float4*)partials, (unsigned)N / 4, total, (long)ldc, splits - 1));
   return check_launch("gemm_add_partials");
 }
 

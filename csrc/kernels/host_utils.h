@@ -23,6 +23,18 @@ int check_launch(const char* what);         // cudaGetLastError -> code
 int encode_tmap(CUtensorMap* out, const void* base, int elem_bytes, int rank, const uint64_t* dims,
                 const uint64_t* strides_bytes, const uint32_t* box, int swizzle128);
 
+// Launch a kernel that calls pdl_wait() (common.cuh): it may start while its predecessor on the stream still runs.
+template <class... P, class... A>
+cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, int block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = grid; lc.blockDim = dim3(block); lc.dynamicSmemBytes = smem; lc.stream = stream;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = &at; lc.numAttrs = 1;
+  return cudaLaunchKernelEx(&lc, kern, P(args)...);
+}
+
 #define CPB_CUDA_OK(expr)                                                              \
   do {                                                                                 \
     cudaError_t _e = (expr);                                                           \

@@ -19,6 +19,8 @@ __global__ void __launch_bounds__(512)
 xent_kernel(const float* __restrict__ logits, const int64_t* __restrict__ targets, __nv_bfloat16* __restrict__ dlogits,
             float* __restrict__ loss_sum, float* __restrict__ row_loss, int rows, int V, int Vcols, long ld_logits, long ld_dlogits,
             float grad_scale, int* status) {
+  pdl_release();
+  pdl_wait();
   __shared__ float red_m[16], red_s[16];
   __shared__ float s_max, s_sum;
   const int row = blockIdx.x;
@@ -112,6 +114,8 @@ __global__ void __launch_bounds__(XE_THREADS)
 xent_smem_kernel(const float* __restrict__ logits, const int64_t* __restrict__ targets, __nv_bfloat16* __restrict__ dlogits,
                  float* __restrict__ loss_sum, float* __restrict__ row_loss, int V, int Vcols, int seg, int ranks,
                  long ld_logits, long ld_dlogits, float grad_scale, int* status) {
+  pdl_release();
+  pdl_wait();
   extern __shared__ __align__(16) float xs[];
   __shared__ __align__(8) uint64_t bars[XE_PARTS];
   __shared__ float red_m[XE_THREADS / 32], red_s[XE_THREADS / 32];
@@ -211,6 +215,8 @@ __global__ void __launch_bounds__(XR_WARPS * 32)
 xent_rows_kernel(const float2* __restrict__ stats, const float* __restrict__ target_logit, const int64_t* __restrict__ targets,
                  float2* __restrict__ row_coef, float* __restrict__ row_loss, float* __restrict__ loss_sum, int rows, int tiles, int V,
                  float grad_scale, int* status) {
+  pdl_release();
+  pdl_wait();
   __shared__ float2 part[XR_WARPS][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row = blockIdx.x * 32 + lane;
@@ -261,8 +267,8 @@ using namespace cpb;
 extern "C" int cpb_xent_rows(const float* stats, const float* target_logit, const int64_t* targets, float* row_coef, float* row_loss,
                              float* loss_sum, int rows, int tiles, int V, float grad_scale, int* status, cudaStream_t stream) {
   if (rows <= 0) return CPB_OK;
-  xent_rows_kernel<<<(rows + 31) / 32, XR_WARPS * 32, 0, stream>>>((const float2*)stats, target_logit, targets, (float2*)row_coef, row_loss,
-                                                                    loss_sum, rows, tiles, V, grad_scale, status);
+  CPB_CUDA_OK(launch_pdl(xent_rows_kernel, (rows + 31) / 32, XR_WARPS * 32, 0, stream, (const float2*)stats, target_logit, targets, (float2*)row_coef, row_loss,
+                                                                    loss_sum, rows, tiles, V, grad_scale, status));
   return check_launch("xent_rows");
 }
 
@@ -286,15 +292,17 @@ extern "C" int cpb_xent(const float* logits, const int64_t* targets, void* dlogi
       if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(xent_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, XE_SEG_BYTES + 64)); cfg = true; }
       cudaLaunchConfig_t lc = {};
       lc.gridDim = dim3((unsigned)(rows * ranks)); lc.blockDim = dim3(XE_THREADS); lc.dynamicSmemBytes = (size_t)seg * 4; lc.stream = stream;
-      cudaLaunchAttribute at;
-      at.id = cudaLaunchAttributeClusterDimension;
-      at.val.clusterDim.x = ranks; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
-      lc.attrs = &at; lc.numAttrs = 1;
+      cudaLaunchAttribute at[2];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = ranks; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+      at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at[1].val.programmaticStreamSerializationAllowed = 1;
+      lc.attrs = at; lc.numAttrs = 2;
       CPB_CUDA_OK(cudaLaunchKernelEx(&lc, xent_smem_kernel, logits, targets, (__nv_bfloat16*)dlogits, loss_sum, row_loss, V, Vcols, seg, ranks,
                                      ld_logits, ld_dlogits, grad_scale, status));
       return check_launch("xent");
     }
   }
-  xent_kernel<<<rows, 512, 0, stream>>>(logits, targets, (__nv_bfloat16*)dlogits, loss_sum, row_loss, rows, V, Vcols, ld_logits, ld_dlogits, grad_scale, status);
+  CPB_CUDA_OK(launch_pdl(xent_kernel, rows, 512, 0, stream, logits, targets, (__nv_bfloat16*)dlogits, loss_sum, row_loss, rows, V, Vcols, ld_logits, ld_dlogits, grad_scale, status));
   return check_launch("xent");
 }
