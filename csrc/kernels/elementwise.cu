@@ -390,6 +390,7 @@ __global__ void embedding_bwd_kernel(const int64_t* __restrict__ idx, const int6
                                      float* __restrict__ dwpe, size_t rows, int d, int pos_period) {
   pdl_release();
   pdl_wait();
+  const bool wide = (((uintptr_t)dwte | (uintptr_t)dwpe) & 15) == 0;       // d is a multiple of eight
   const int nvec = d >> 3;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < rows * nvec; i += (size_t)gridDim.x * blockDim.x) {
     const size_t row = i / nvec;
@@ -397,14 +398,17 @@ __global__ void embedding_bwd_kernel(const int64_t* __restrict__ idx, const int6
     float g[8];
     uint4 u = *(const uint4*)(dout + row * d + c);
     unpack8(u, g);
-    float* wt = dwte + (size_t)idx[row] * d + c;
+    const auto add = [&](float* dst) {
+      if (wide) {
+        red_add_v4(dst, g[0], g[1], g[2], g[3]);
+        red_add_v4(dst + 4, g[4], g[5], g[6], g[7]);
+      } else {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) atomicAdd(wt + j, g[j]);
-    if (dwpe) {
-      float* wp = dwpe + (size_t)pos[row % pos_period] * d + c;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) atomicAdd(wp + j, g[j]);
-    }
+        for (int j = 0; j < 8; ++j) atomicAdd(dst + j, g[j]);
+      }
+    };
+    add(dwte + (size_t)idx[row] * d + c);
+    if (dwpe) add(dwpe + (size_t)pos[row % pos_period] * d + c);
   }
 }
 
@@ -739,6 +743,7 @@ __global__ void sumsq_kernel(const float* __restrict__ g, size_t n, float* __res
 // AdamW on flat fp32 master / moment buffers, writing the bf16 compute copy in the same pass.
 //   gscale = grad_prescale * min(1, clip / (sqrt(sumsq)*grad_prescale + 1e-6))   (sumsq read on device, no host sync)
 // If sumsq is not finite the step is skipped (NaN/Inf guard) and flag[0] is set.
+// Bound by memory: 30 bytes per parameter, four parameters per thread and turn.
 __global__ void adamw_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
                              float* __restrict__ v, __nv_bfloat16* __restrict__ p16, size_t n, float lr, float b1,
                              float b2, float eps, float wd, float bc1, float bc2, float grad_prescale, float clip,
@@ -751,14 +756,28 @@ __global__ void adamw_kernel(float* __restrict__ p, const float* __restrict__ g,
     if (clip > 0.f) gs *= fminf(1.f, clip / (norm + 1e-6f));
   }
   const float inv_bc2_sqrt = rsqrtf(bc2);
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const float gi = g[i] * gs;
-    float pi = p[i] * (1.f - lr * wd);
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
+  const auto step = [&](float gr, float& pi, float& mi, float& vi) {
+    const float gi = gr * gs;
+    pi *= 1.f - lr * wd;
+    mi = b1 * mi + (1.f - b1) * gi;
+    vi = b2 * vi + (1.f - b2) * gi * gi;
     pi -= (lr / bc1) * mi / (sqrtf(vi) * inv_bc2_sqrt + eps);
-    p[i] = pi; m[i] = mi; v[i] = vi;
-    if (p16) p16[i] = __float2bfloat16(pi);
+  };
+  const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, nt = (size_t)gridDim.x * blockDim.x;
+  const bool wide = ((((uintptr_t)p | (uintptr_t)g | (uintptr_t)m | (uintptr_t)v) & 15) | ((uintptr_t)p16 & 7)) == 0;
+  const size_t n4 = wide ? n >> 2 : 0;
+  for (size_t i = tid; i < n4; i += nt) {
+    const float4 gr = ((const float4*)g)[i];
+    float4 a = ((const float4*)p)[i], b = ((const float4*)m)[i], c = ((const float4*)v)[i];
+    step(gr.x, a.x, b.x, c.x); step(gr.y, a.y, b.y, c.y); step(gr.z, a.z, b.z, c.z); step(gr.w, a.w, b.w, c.w);
+    ((float4*)p)[i] = a; ((float4*)m)[i] = b; ((float4*)v)[i] = c;
+    if (p16) ((uint2*)p16)[i] = make_uint2(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w));
+  }
+  for (size_t i = 4 * n4 + tid; i < n; i += nt) {
+    float a = p[i], b = m[i], c = v[i];
+    step(g[i], a, b, c);
+    p[i] = a; m[i] = b; v[i] = c;
+    if (p16) p16[i] = __float2bfloat16(a);
   }
 }
 
