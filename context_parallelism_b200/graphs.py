@@ -22,9 +22,9 @@ EAGER_CALLS = 2                  # calls with new shapes that run as they always
 MAX_POOL_BYTES = 8 << 30         # a record whose buffers take more than this is not kept
 MIN_FREE_SHARE = 0.25            # share of the GPU's memory that has to be free before a record is made
 # A call is recorded while the GPU needs less time for it than the host: a launch costs the host about 25 us (forward and backward;
-# 13 us without autograd), the kernels of such models reach about 400 TFLOP/s.
+# 13 us without autograd), the kernels of such models reach about 600 TFLOP/s.
 HOST_US_PER_LAUNCH = 25.0
-GPU_TFLOPS = 400.0
+GPU_TFLOPS = 600.0
 
 
 def model_flops(cfg, batch: int, T: int, train: bool) -> float:

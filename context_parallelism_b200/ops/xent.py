@@ -39,25 +39,32 @@ HEAD_TILE = 256          # columns per tile of the head's GEMM
 
 
 def _head_rows(xc: torch.Tensor, w: torch.Tensor, tg: torch.Tensor, n_valid: int, grad_scale: float, loss_sum: Optional[torch.Tensor],
-               row_loss: Optional[torch.Tensor], want_coef: bool) -> Optional[torch.Tensor]:
-    """Loss of the rows ``xc`` without their logits (``loss_sum`` += , ``row_loss`` =); returns the rows' gradient coefficients."""
+               row_loss: Optional[torch.Tensor], want_coef: bool, logits: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
+    """Loss of the rows ``xc`` (``loss_sum`` += , ``row_loss`` =); returns the rows' gradient coefficients.  ``logits`` (fp32) are stored only
+    when given."""
     rows, V = xc.shape[0], w.shape[0]
     tiles = (V + HEAD_TILE - 1) // HEAD_TILE
     stats = torch.empty((tiles, rows, 2), dtype=torch.float32, device=xc.device)
     tlogit = torch.empty(rows, dtype=torch.float32, device=xc.device)
     coef = torch.empty((rows, 2), dtype=torch.float32, device=xc.device) if want_coef else None
     st, stream = nv.status_for(xc.device).ptr(), nv.stream_ptr(xc.device)
-    nv.call("gemm_head", xc.data_ptr(), w.data_ptr(), 0, tg.data_ptr(), stats.data_ptr(), tlogit.data_ptr(), 0, rows, V, xc.shape[1],
-            xc.stride(0), w.stride(0), 0, n_valid, grad_scale, st, stream)
+    nv.call("gemm_head", xc.data_ptr(), w.data_ptr(), nv.ptr(logits), tg.data_ptr(), stats.data_ptr(), tlogit.data_ptr(), 0, rows, V, xc.shape[1],
+            xc.stride(0), w.stride(0), 0 if logits is None else logits.stride(0), n_valid, 0, grad_scale, st, stream)
     nv.call("xent_rows", stats.data_ptr(), tlogit.data_ptr(), tg.data_ptr(), nv.ptr(coef), nv.ptr(row_loss), nv.ptr(loss_sum), rows, tiles,
             n_valid, grad_scale, st, stream)
     return coef
 
 
-def _head_dlogits(xc: torch.Tensor, w: torch.Tensor, tg: torch.Tensor, coef: torch.Tensor, n_valid: int, grad_scale: float) -> torch.Tensor:
+def _head_dlogits(xc: torch.Tensor, w: torch.Tensor, tg: torch.Tensor, coef: torch.Tensor, n_valid: int, grad_scale: float,
+                  logits: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """bf16 gradient of the logits, which are computed again unless they were stored."""
     dlog = torch.empty((xc.shape[0], w.shape[0]), dtype=torch.bfloat16, device=xc.device)
+    if logits is not None:
+        nv.call("xent_dlogits", logits.data_ptr(), tg.data_ptr(), coef.data_ptr(), dlog.data_ptr(), xc.shape[0], n_valid, w.shape[0],
+                logits.stride(0), dlog.stride(0), grad_scale, nv.stream_ptr(xc.device))
+        return dlog
     nv.call("gemm_head", xc.data_ptr(), w.data_ptr(), dlog.data_ptr(), tg.data_ptr(), 0, 0, coef.data_ptr(), xc.shape[0], w.shape[0], xc.shape[1],
-            xc.stride(0), w.stride(0), dlog.stride(0), n_valid, grad_scale, nv.status_for(xc.device).ptr(), nv.stream_ptr(xc.device))
+            xc.stride(0), w.stride(0), dlog.stride(0), n_valid, 1, grad_scale, nv.status_for(xc.device).ptr(), nv.stream_ptr(xc.device))
     return dlog
 
 
@@ -81,14 +88,10 @@ class _LinearCEFn(torch.autograd.Function):
         for r0 in range(0, N, CHUNK_ROWS):
             r1 = min(N, r0 + CHUNK_ROWS)
             xc, tc = x2[r0:r1], tg[r0:r1]
-            if stored:
-                lg = logits[: r1 - r0]
-                gemm(xc, wm, out=lg, epi=1)
-                dlog = xent_chunk(lg, tc, loss_sum, grad_scale, True, None, n_valid)
-            else:
-                coef = _head_rows(xc, wm, tc, n_valid or V, grad_scale, loss_sum, None, need_grad)
-                dlog = _head_dlogits(xc, wm, tc, coef, n_valid or V, grad_scale) if need_grad else None
+            lg = logits[: r1 - r0] if stored else None
+            coef = _head_rows(xc, wm, tc, n_valid or V, grad_scale, loss_sum, None, need_grad, lg)
             if need_grad:
+                dlog = _head_dlogits(xc, wm, tc, coef, n_valid or V, grad_scale, lg)
                 gemm(dlog, wm, b_mn=True, out=dx[r0:r1])
                 gemm(dlog, xc, a_mn=True, b_mn=True, out=(mg if mg is not None else dw_own).view(V, d), accumulate=True)
         if need_grad and mg is not None:
@@ -152,8 +155,4 @@ def logits_last(x_last: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """fp32 logits for a few rows (generation)."""
     if not x_last.is_cuda:
         return F.linear(x_last.float(), w.float())
-    x2 = x_last.reshape(-1, x_last.shape[-1])
-    pad = (-x2.shape[0]) % 8
-    if pad:
-        x2 = torch.cat([x2, x2.new_zeros(pad, x2.shape[1])])
-    return gemm(x2.contiguous(), w, out_dtype=torch.float32)[: x_last.reshape(-1, x_last.shape[-1]).shape[0]]
+    return gemm(x_last.reshape(-1, x_last.shape[-1]), w, out_dtype=torch.float32)

@@ -482,22 +482,22 @@ extern "C" int cpb_gemm_bf16(const void* A, const void* B, void* C, void* aux, c
   return check_launch("gemm_add_partials");
 }
 
-// Cross entropy of the language-model head without its logits: logits = x w^T (x [M,K], w [N,K], both K-major) stay in tensor memory.
-// dlogits == null: per row and 256-wide tile (max, sum of exponentials) to stats [ceil(N / 256)][M] and the target's logit; otherwise
-// dlogits (bf16 [M,N], row stride ldc) = (softmax - onehot) * grad_scale from row_coef (cpb_xent_rows).
+// Cross entropy of the language-model head, logits = x w^T (x [M,K], w [N,K], both K-major).  out == null or fp32 (grad == 0): per row and
+// 256-wide tile (max, sum of exponentials) to stats [ceil(N / 256)][M] and the target's logit; out, if given, gets the logits as well.
+// grad == 1: out (bf16) = (softmax - onehot) * grad_scale from row_coef (cpb_xent_rows).  out: [M,N], row stride ldc.
 //
-// The second pass computes the logits again, 2 K operations for each, where storing them in fp32 moves 4 bytes for the GEMM and 4
-// more for the kernel that turns them into dlogits.
-extern "C" int cpb_gemm_head(const void* x, const void* w, void* dlogits, const int64_t* targets, float* stats, float* target_logit,
-                             const float* row_coef, int M, int N, int K, int ldx, int ldw, int ldc, int n_valid, float grad_scale,
+// The gradient pass computes the logits again, 2 K operations for each, where storing them in fp32 moves 4 bytes for the GEMM and 4
+// more for the kernel that turns them into dlogits; beyond a K of about a thousand storing them is cheaper (cpb_xent_dlogits).
+extern "C" int cpb_gemm_head(const void* x, const void* w, void* out, const int64_t* targets, float* stats, float* target_logit,
+                             const float* row_coef, int M, int N, int K, int ldx, int ldw, int ldc, int n_valid, int grad, float grad_scale,
                              int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return set_error(CPB_ERR_ARG, "gemm_head: empty problem %dx%dx%d", M, N, K);
-  if ((N % 8) || (K % 8) || (ldx % 8) || (ldw % 8) || (dlogits && (ldc % 8)))
+  if ((N % 8) || (K % 8) || (ldx % 8) || (ldw % 8) || (out && (ldc % 8)))
     return set_error(CPB_ERR_ARG, "gemm_head: N,K,ldx,ldw,ldc must be multiples of 8 (got N=%d K=%d ldx=%d ldw=%d ldc=%d)", N, K, ldx, ldw, ldc);
   if (n_valid <= 0 || n_valid > N) return set_error(CPB_ERR_ARG, "gemm_head: n_valid=%d outside 1..%d", n_valid, N);
-  if (dlogits ? row_coef == nullptr : (stats == nullptr || target_logit == nullptr)) return set_error(CPB_ERR_ARG, "gemm_head: missing buffers");
+  if (grad ? (out == nullptr || row_coef == nullptr) : (stats == nullptr || target_logit == nullptr)) return set_error(CPB_ERR_ARG, "gemm_head: missing buffers");
   GemmParams p{};
-  p.M = M; p.N = N; p.K = K; p.epi = dlogits ? EPI_HEAD_GRAD : EPI_HEAD_STATS;
+  p.M = M; p.N = N; p.K = K; p.epi = grad ? EPI_HEAD_GRAD : out ? EPI_HEAD_STORE : EPI_HEAD_STATS;
   p.num_m_tiles = (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM);
   p.num_n_blocks = (N + 255) / 256;
   p.num_k_blocks = p.k_per_split = (K + GEMM_BK - 1) / GEMM_BK;
@@ -510,10 +510,11 @@ extern "C" int cpb_gemm_head(const void* x, const void* w, void* dlogits, const 
   if ((rc = kmajor_tmap(&tm[0], x, M, K, ldx, GEMM_BM)) != CPB_OK) return rc;
   if ((rc = kmajor_tmap(&tm[1], w, N, K, ldw, 128)) != CPB_OK) return rc;
   tm[2] = tm[0];
-  if (dlogits) {
-    uint64_t dims[2] = {(uint64_t)N, (uint64_t)M}, strides[2] = {0, (uint64_t)ldc * 2};
-    uint32_t box[2] = {64, 32};
-    if ((rc = encode_tmap(&tm[2], dlogits, 2, 2, dims, strides, box, 1)) != CPB_OK) return rc;
+  if (out) {
+    const int eb = grad ? 2 : 4;
+    uint64_t dims[2] = {(uint64_t)N, (uint64_t)M}, strides[2] = {0, (uint64_t)ldc * eb};
+    uint32_t box[2] = {(uint32_t)(128 / eb), 32};
+    if ((rc = encode_tmap(&tm[2], out, eb, 2, dims, strides, box, 1)) != CPB_OK) return rc;
   }
   tm[3] = tm[2];
   return launch_pair<256, false, false>(tm, p, stream);

@@ -23,7 +23,8 @@ enum : int {
   EPI_BF16_GELU = 3,   // C(bf16) = gelu_tanh(acc + bias); aux(bf16) = acc + bias (pre-activation) when aux != null
   EPI_BF16_SWIGLU = 4, // B tile = [gate rows | up rows]; C(bf16)[:, n] = silu(g)*u ; aux gets [g | u] when aux != null
   EPI_HEAD_STATS = 5,  // language-model head: (max, sum of exponentials) of the tile's columns per row, no C
-  EPI_HEAD_GRAD = 6,   // C(bf16) = (softmax - onehot(target)) * grad_scale from the rows' (max, grad_scale / sum)
+  EPI_HEAD_STORE = 6,  // both: EPI_HEAD_STATS, and C(f32) = acc
+  EPI_HEAD_GRAD = 7,   // C(bf16) = (softmax - onehot(target)) * grad_scale from the rows' (max, grad_scale / sum)
 };
 
 // Cross entropy in the epilogue of the head's GEMM (xent.cu has the kernel between the two passes).
@@ -161,7 +162,15 @@ __device__ __forceinline__ void head_epilogue(const GemmParams& p, const CUtenso
     if (!live || col >= p.N) continue;
     const int at = h.target - col;
     const bool hit = at >= 0 && at < 64;
-    if (p.epi == EPI_HEAD_STATS) {
+    if (p.epi != EPI_HEAD_GRAD) {
+      if (p.epi == EPI_HEAD_STORE) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (col + 32 * h >= p.N) break;
+          ws.fill(ws.row_ptr(lane), lane, *(uint32_t(*)[32])&f[32 * h]);
+          ws.store(tmC, col + 32 * h, row0);
+        }
+      }
       if (col >= p.head.n_valid) continue;
       if (hit) p.head.target_logit[row] = pick64(f, at);
       if (col + 64 > p.head.n_valid) {
@@ -213,7 +222,7 @@ __device__ __forceinline__ void head_epilogue(const GemmParams& p, const CUtenso
       ws.store(tmC, col, row0);
     }
   }
-  if (p.epi == EPI_HEAD_STATS && row < p.M) p.head.stats[(size_t)nb * p.M + row] = make_float2(m, s);
+  if (p.epi != EPI_HEAD_GRAD && row < p.M) p.head.stats[(size_t)nb * p.M + row] = make_float2(m, s);
 }
 
 // Epilogue of one 32-row slice of a 128 x BN accumulator tile: `t_row` is the tensor-memory address of this warp's lanes at

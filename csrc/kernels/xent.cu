@@ -258,9 +258,49 @@ xent_rows_kernel(const float2* __restrict__ stats, const float* __restrict__ tar
   }
 }
 
+// dlogits = (softmax - onehot) * grad_scale from stored logits and the rows' (max, grad_scale / sum).  Bound by memory: 4 bytes in and 2
+// out per logit; four 16-byte loads per thread before the first use.
+constexpr int XD_COLS = 256 * 16;
+__global__ void __launch_bounds__(256)
+xent_dlogits_kernel(const float* __restrict__ logits, const int64_t* __restrict__ targets, const float2* __restrict__ row_coef,
+                    __nv_bfloat16* __restrict__ dlogits, int V, int Vcols, long ld_logits, long ld_dlogits, float grad_scale) {
+  pdl_release();
+  pdl_wait();
+  const int row = blockIdx.y, c0 = blockIdx.x * XD_COLS + 4 * threadIdx.x;
+  const float4* x = (const float4*)(logits + (size_t)row * ld_logits);
+  const float2 coef = row_coef[row];
+  const int64_t tgt = targets[row];
+  float4 v[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) if (c0 + 1024 * k < Vcols) v[k] = x[(c0 + 1024 * k) >> 2];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int c = c0 + 1024 * k;
+    if (c >= Vcols) break;
+    float p[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      p[e] = c + e < V ? __expf(p[e] - coef.x) * coef.y : 0.f;
+      if (tgt == c + e && c + e < V) p[e] -= grad_scale;
+    }
+    *(uint2*)(dlogits + (size_t)row * ld_dlogits + c) = make_uint2(pack_bf16(p[0], p[1]), pack_bf16(p[2], p[3]));
+  }
+}
+
 }  // namespace cpb
 
 using namespace cpb;
+
+// logits fp32 [rows, Vcols] and row_coef as written by cpb_gemm_head and cpb_xent_rows; dlogits bf16 [rows, Vcols], zero from column V on.
+extern "C" int cpb_xent_dlogits(const float* logits, const int64_t* targets, const float* row_coef, void* dlogits, int rows, int V, int Vcols,
+                                long ld_logits, long ld_dlogits, float grad_scale, cudaStream_t stream) {
+  if (rows <= 0) return CPB_OK;
+  if (Vcols < V || (Vcols % 4) || (ld_logits % 4) || (ld_dlogits % 4) || ((uintptr_t)logits & 15) || ((uintptr_t)dlogits & 7) || rows > 65535)
+    return set_error(CPB_ERR_ARG, "xent_dlogits: columns and strides must be multiples of 4, rows at most 65535");
+  CPB_CUDA_OK(launch_pdl(xent_dlogits_kernel, dim3((Vcols + XD_COLS - 1) / XD_COLS, rows), 256, 0, stream, logits, targets, (const float2*)row_coef,
+                         (__nv_bfloat16*)dlogits, V, Vcols, ld_logits, ld_dlogits, grad_scale));
+  return check_launch("xent_dlogits");
+}
 
 // stats [tiles][rows] (max, sum) pairs and target_logit [rows] of cpb_gemm_head; row_coef [rows] pairs, row_loss [rows] and
 // loss_sum (fp32 scalar, +=) are optional.  V: columns that are real vocabulary.

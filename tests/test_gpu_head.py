@@ -40,6 +40,12 @@ def test_loss_and_dlogits(rows, d, V, n_valid, spread):
     err = (dlog[:, :n_valid].double() - p).abs()
     assert bool((err <= 2 ** -8 * p.abs() + tol * scale).all())            # one rounding to bf16 (2^-9) beside the fp32 error
     assert not bool(dlog[:, n_valid:].any())
+    logits32 = torch.full((rows, V + 8), 3.0, device="cuda")[:, :V]
+    stored = xent._head_rows(x, w, tg, n_valid, scale, None, row2 := torch.empty_like(row), True, logits32)
+    assert torch.equal(row, row2) and torch.equal(coef, stored)
+    assert float((logits32[:, :n_valid].double() - logits).abs().max()) <= tol
+    other = xent._head_dlogits(x, w, tg, stored, n_valid, scale, logits32)
+    assert bool(((other[:, :n_valid].double() - p).abs() <= 2 ** -8 * p.abs() + tol * scale).all()) and not bool(other[:, n_valid:].any())
     again = xent._head_rows(x, w, tg, n_valid, scale, None, row2 := torch.empty_like(row), True)
     assert torch.equal(row, row2) and torch.equal(coef, again)
 
