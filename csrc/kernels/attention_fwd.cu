@@ -452,8 +452,10 @@ extern "C" int cpb_flash_fwd(const void* q, const void* k, const void* v, void* 
   CUtensorMap tq, tk, tv;
   int rc;
   if ((rc = make_qkv_tmap(&tq, q, D, Hq, Tq, B, q_sh, q_st, q_sb, FA_BQ)) != CPB_OK) return rc;
-  if ((rc = make_qkv_tmap(&tk, k, D, Hkv, Tk, B, k_sh, k_st, k_sb, FA_BK)) != CPB_OK) return rc;
-  if ((rc = make_qkv_tmap(&tv, v, D, Hkv, Tk, B, k_sh, k_st, k_sb, FA_BK)) != CPB_OK) return rc;
+  static const bool new64 = getenv("CPB_F64") != nullptr && getenv("CPB_F64")[0] == '1';
+  const int kv_rows = D == 64 && new64 ? 64 : FA_BK;
+  if ((rc = make_qkv_tmap(&tk, k, D, Hkv, Tk, B, k_sh, k_st, k_sb, kv_rows)) != CPB_OK) return rc;
+  if ((rc = make_qkv_tmap(&tv, v, D, Hkv, Tk, B, k_sh, k_st, k_sb, kv_rows)) != CPB_OK) return rc;
   FwdParams p;
   p.B = B; p.Tq = Tq; p.Tk = Tk; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal; p.k_off = k_off;
   p.scale_log2 = scale * 1.4426950408889634f;
@@ -473,6 +475,7 @@ extern "C" int cpb_flash_fwd(const void* q, const void* k, const void* v, void* 
   // 236; 8192, 224 CTAs 154 and 153; 8192, 256 CTAs 163 and 153; 32768 keys, 256 CTAs 528 and 507).
   const long pairs = (long)((Tq + 2 * FA_BQ - 1) / (2 * FA_BQ)) * Hq * B;
   if (D == 128 && Tk >= 8192 && Tq > FA_BQ && 5 * pairs >= 8 * sm_count()) return launch_flash_fwd128_pair(poly, tq, tk, tv, p, stream);
+  if (D == 64 && new64) return launch_flash_fwd64(poly, tq, tk, tv, p, stream);
   const int G = Hq / Hkv;
   dim3 grid(p.n_copy + ((Tq + FA_BQ - 1) / FA_BQ) * G, Hkv, B);
 #define CPB_FWD_LAUNCH(DD, PP)                                                                                         \

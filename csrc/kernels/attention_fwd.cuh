@@ -54,4 +54,7 @@ __device__ __forceinline__ bool wait_flag_ge(const int* flag, int value, volatil
 // attention_fwd128.cu: head_dim 128, two query tiles per CTA; poly = share (of 8) of polynomial exponentials, 0 to 4
 int launch_flash_fwd128_pair(int poly, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p, cudaStream_t stream);
 
+// attention_fwd64.cu: head_dim 64, tk and tv with boxes of 64 keys; poly as above, 0 to 5
+int launch_flash_fwd64(int poly, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p, cudaStream_t stream);
+
 }  // namespace cpb
