@@ -127,7 +127,8 @@ def _aligned(t: torch.Tensor) -> torch.Tensor:
 def _bwd_plan(B: int, Tq: int, Tk: int, Hq: int, Hkv: int, D: int, causal: bool, k_off: int, local: bool):
     """``(pairs per CTA, floats of workspace)`` of a whole gradient."""
     chunk, tq_pad = bwd_chunk(B, Tq, Tk, Hq, Hkv, D, causal, k_off, local), (Tq + 127) // 128 * 128
-    return chunk, B * D * (Tq * Hq + (2 * Tk * Hkv if chunk else 0)) + (2 * B * Hq + 1) * tq_pad
+    parts = -(-(Hq // Hkv * tq_pad // 128) // chunk) if chunk else 0
+    return chunk, B * D * (Tq * Hq + 2 * parts * Tk * Hkv) + (2 * B * Hq + 1) * tq_pad
 
 
 def _bwd_whole(q: int, k: int, v: int, o, do, lse, dq: int, dk: int, dv: int, dims, strides, dq_st: int, dkv_st: int, scale: float, causal: bool,

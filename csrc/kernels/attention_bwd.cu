@@ -589,36 +589,38 @@ extern "C" int cpb_flash_bwd128(const void* q, const void* k, const void* v, con
                                 long k_sb, float scale, int causal, int k_off, const int* q_pos, int dkv_mode, long dkv_st, const uint64_t* route_k,
                                 const uint64_t* route_v, int route_rows, int route_tl, int it_chunk, int local, int* status, cudaStream_t stream);
 extern "C" int cpb_cast_f32_bf16_rows(const float* in, void* out_q, long rows_q, int cols_q, long q_stride, void* out_k, void* out_v, long rows_k,
-                                      int cols_k, long kv_stride, float scale, cudaStream_t stream);
+                                      int cols_k, long kv_stride, int parts, int Tk, int k_off, int nq, int G, int chunk, int local, float scale,
+                                      cudaStream_t stream);
 
 // The three launches of a whole gradient (preparation, kernel, cast) behind one call: what the host did between them cost more than
 // the kernels of a short sequence.  o, dout dense; dq, dk, dv bf16, tokens dq_st / dkv_st elements apart, batches dense.  ws:
-// B Tq Hq D floats for dQ, twice B Tk Hkv D for dK and dV if chunk > 0 (see cpb_flash_bwd_chunk), 2 B Hq Tq_pad and Tq_pad, in this
-// order, with Tq_pad = Tq rounded up to 128.  q_pos: int32 [Tq], or null for 0 .. Tq-1.
+// B Tq Hq D floats for dQ, twice parts B Tk Hkv D for dK and dV, 2 B Hq Tq_pad and Tq_pad, in this order, with Tq_pad = Tq rounded up
+// to 128 and parts = (pairs of a whole sweep) / chunk, rounded up, or 0 for chunk 0 (see cpb_flash_bwd_chunk).  q_pos: int32 [Tq], or null for 0 .. Tq-1.
 extern "C" int cpb_flash_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* lse, float* ws, void* dq,
                                   void* dk, void* dv, int B, int Tq, int Tk, int Hq, int Hkv, int D, long q_sh, long q_st, long q_sb, long k_sh,
                                   long k_st, long k_sb, long dq_st, long dkv_st, float scale, int causal, int k_off, const int* q_pos, int chunk,
                                   int* status, cudaStream_t stream) {
   if (D != 64 && D != 128) return set_error(CPB_ERR_ARG, "flash_attn_bwd: head_dim %d not in {64,128}", D);
   if ((uintptr_t)ws & 15) return set_error(CPB_ERR_ARG, "flash_attn_bwd: the workspace must be 16-byte aligned");
-  const int Tq_pad = (Tq + 127) / 128 * 128;
-  const long nq = (long)B * Tq * Hq * D, nk = chunk ? (long)B * Tk * Hkv * D : 0;
+  const int Tq_pad = (Tq + 127) / 128 * 128, pairs = Hq / Hkv * (Tq_pad / 128), parts = chunk > 0 ? (pairs + chunk - 1) / chunk : 0;
+  const long nq = (long)B * Tq * Hq * D, nk = (long)B * Tk * Hkv * D * parts;
   float *delta = ws + nq + 2 * nk, *lse2 = delta + (long)B * Hq * Tq_pad;
   int* pos = (int*)(lse2 + (long)B * Hq * Tq_pad);
-  int rc = cpb_flash_bwd_prep(o, dout, lse, delta, lse2, ws, nq + 2 * nk, q_pos, pos, B, Tq, Hq, D, Tq_pad, stream);
+  int rc = cpb_flash_bwd_prep(o, dout, lse, delta, lse2, ws, nq, q_pos, pos, B, Tq, Hq, D, Tq_pad, stream);
   if (rc != CPB_OK) return rc;
-  rc = (D == 64 ? cpb_flash_bwd64 : cpb_flash_bwd128)(q, k, v, dout, lse2, delta, ws, chunk ? (void*)(ws + nq) : dk, chunk ? (void*)(ws + nq + nk) : dv, B, Tq,
+  rc = (D == 64 ? cpb_flash_bwd64 : cpb_flash_bwd128)(q, k, v, dout, lse2, delta, ws, parts ? (void*)(ws + nq) : dk, parts ? (void*)(ws + nq + nk) : dv, B, Tq,
                                                       Tk, Hq, Hkv, Tq_pad, q_sh, q_st, q_sb, k_sh, k_st, k_sb, scale, causal, k_off, pos,
-                                                      chunk ? 3 : 0, chunk ? (long)Hkv * D : dkv_st, nullptr, nullptr, 0, 0, chunk, q_pos == nullptr,
+                                                      parts ? 3 : 0, parts ? (long)Hkv * D : dkv_st, nullptr, nullptr, 0, 0, chunk, q_pos == nullptr,
                                                       status, stream);
   if (rc != CPB_OK) return rc;
-  return cpb_cast_f32_bf16_rows(ws, dq, (long)B * Tq, Hq * D, dq_st, dk, dv, chunk ? (long)B * Tk : 0, Hkv * D, dkv_st, 1.f, stream);
+  return cpb_cast_f32_bf16_rows(ws, dq, (long)B * Tq, Hq * D, dq_st, dk, dv, (long)B * Tk, Hkv * D, dkv_st, parts, Tk, k_off, Tq_pad / 128, Hq / Hkv, chunk,
+                                causal && q_pos == nullptr, 1.f, stream);
 }
 
 // How many (query head, query tile) pairs a CTA of the head_dim-64 / 128 kernels should take at most, 0 for whole sweeps.  Whole sweeps
 // are uneven under the causal mask (the first K/V tile meets every query, the last one tile of them) and few when there are few
-// heads; parts even out, but each costs the CTA's start and end and an fp32 addition of its dK / dV, and the sums have to be
-// cleared and cast.  So both ways of handing out the CTAs to the SMs are followed here, with the times that they take.
+// heads; parts even out, but each costs the CTA's start and end, and a part of dK / dV is written and read in fp32 (added in a
+// fixed order, so that dK and dV repeat bit for bit).  So both ways of handing out the CTAs to the SMs are followed here, with the times that they take.
 extern "C" int cpb_flash_bwd_chunk(int B, int Tq, int Tk, int Hq, int Hkv, int D, int causal, int k_off, int local) {
   const int nq = (Tq + 127) / 128, n_kt = (Tk + 127) / 128, G = Hq / (Hkv > 0 ? Hkv : 1), hb = Hkv * B, sms = sm_count();
   if (nq <= 0 || n_kt <= 0 || G <= 0 || hb <= 0 || (D != 64 && D != 128) || (long)n_kt * hb > 16L * sms) return 0;
@@ -641,13 +643,14 @@ extern "C" int cpb_flash_bwd_chunk(int B, int Tq, int Tk, int Hq, int Hkv, int D
     }
     return end;
   };
-  const double whole = finish(0), extra = 0.5 + (double)B * Tk * Hkv * D * 2 * 14 / 4e6;     // cleared, read and cast at 4 TB/s
-  double best = whole * 0.95;
+  double best = finish(0) * 0.95;
   int chunk = 0;
   for (int parts = 2; parts <= 24; ++parts) {
     const int c = (G * nq + parts - 1) / parts;
     if (c < 2) break;
-    const double t = finish(c) + extra;
+    long written = 0;                                                // K/V tiles times parts
+    for (int k = 0; k < n_kt; ++k) written += local ? (len[k] + c - 1) / c : parts;
+    const double t = finish(c) + 0.5 + (double)written * hb * 128 * D * 2 * 8 / 4e6;       // written and read at 4 TB/s
     if (t < best) { best = t; chunk = c; }
   }
   return chunk;

@@ -5,7 +5,7 @@
 namespace cpb {
 
 // A CTA owns a K/V tile and sweeps the (query head, query tile) pairs that see it: `it_chunk` of them at most when that is not 0, and
-// then several CTAs share a tile and add their parts of dK / dV in fp32 (dkv_mode 3).
+// then several CTAs share a tile and each writes a part of dK / dV in fp32 (dkv_mode 3).
 struct BwdWork {
   int kt, hkv, b;
   int it0;                 // first pair of the sweep

@@ -61,8 +61,9 @@ struct Bwd128Params {
   const int* q_pos;             // [Tq_pad] global positions, INT_MAX in the padding
   void* dk; void* dv;           // [B,Tk,Hkv,D] bf16 (store) or fp32 (accumulate)
   long dkv_st;                  // elements from one token of dk / dv to the next (heads adjacent, batches dense)
-  int dkv_mode;                 // 0 bf16 store, 1 fp32 accumulate, 2 routed red.add (fused ring), 3 red.add (several CTAs per tile)
+  int dkv_mode;                 // 0 bf16 store, 1 fp32 accumulate, 2 routed red.add (fused ring), 3 fp32 store to the part of this CTA (several per tile)
   int it_chunk;                 // pairs of (query head, query tile) per CTA, 0: all (see BwdWork)
+  long part_st;                 // mode 3: floats from one part of dk / dv to the next
   int local;                    // q_pos is 0 .. Tq - 1: the first visible query tile needs no search
   const uint64_t* route_k;      // mode 2: per chunk of route_rows K/V rows the address of its owner's fp32 accumulator
   const uint64_t* route_v;
@@ -365,6 +366,13 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
     // final: dK, dV -> global
     if (n_it == 0) {
+      if (p.dkv_mode == 3 && k_valid && grp == 0) {
+        const size_t at = work.it0 / p.it_chunk * p.part_st + ((size_t)b * p.Tk + kidx) * p.dkv_st + hkv * D;
+        for (int c = 0; c < D; c += 4) {
+          *(float4*)((float*)p.dk + at + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+          *(float4*)((float*)p.dv + at + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+      }
       if (p.dkv_mode == 0 && k_valid && grp == 0) {
         __nv_bfloat16* dkr = (__nv_bfloat16*)p.dk + ((size_t)b * p.Tk + kidx) * p.dkv_st + hkv * D;
         __nv_bfloat16* dvr = (__nv_bfloat16*)p.dv + ((size_t)b * p.Tk + kidx) * p.dkv_st + hkv * D;
@@ -396,9 +404,9 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
               for (int j = 0; j < 32; j += 4)
                 red_add_v4(dst + j, __uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
             } else if (p.dkv_mode == 3) {
+              uint4* dst = (uint4*)((float*)base + work.it0 / p.it_chunk * p.part_st + off + c);
 #pragma unroll
-              for (int j = 0; j < 32; j += 4)
-                red_add_v4((float*)base + off + c + j, __uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+              for (int j = 0; j < 32; j += 4) dst[j >> 2] = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
             } else if (p.dkv_mode == 1) {
               float* dst = (float*)base + off + c;
 #pragma unroll
@@ -529,8 +537,8 @@ extern "C" int cpb_flash_bwd128(const void* q, const void* k, const void* v, con
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   p.lse2 = lse2; p.delta = delta; p.q_pos = q_pos; p.dk = dk; p.dv = dv; p.dkv_mode = dkv_mode; p.dkv_st = dkv_st; p.status = status;
   p.route_k = route_k; p.route_v = route_v; p.route_rows = route_rows; p.route_tl = route_tl;
-  if (it_chunk < 0 || (it_chunk > 0) != (dkv_mode == 3)) return set_error(CPB_ERR_ARG, "flash_bwd128: several CTAs per K/V tile add their dK/dV in fp32 (dkv_mode 3)");
-  p.it_chunk = it_chunk; p.local = local;
+  if (it_chunk < 0 || (it_chunk > 0) != (dkv_mode == 3)) return set_error(CPB_ERR_ARG, "flash_bwd128: several CTAs per K/V tile write parts of dK/dV (dkv_mode 3)");
+  p.it_chunk = it_chunk; p.local = local; p.part_st = (long)B * Tk * dkv_st;
   static const bool skip_dq = [] {
     const char* e = getenv("CPB_BWD_SKIP_DQ");
     const bool on = e != nullptr && e[0] == '1';

@@ -824,15 +824,26 @@ __global__ void cast_f32_bf16_kernel(const float* __restrict__ in, __nv_bfloat16
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     out[i] = __float2bfloat16(in[i] * scale);
 }
-// Up to three dense fp32 matrices that follow one another in memory -> bf16 rows at a place and a distance of their own; eight
-// elements per thread (32 bytes in, 16 out).
+// fp32 -> bf16 rows `stride` elements apart; eight elements per thread (32 bytes in, 16 out).
 struct CastPiece {
   __nv_bfloat16* out;
   size_t n8;               // sixteen-byte groups of the result
   int c8;                  // of one row
   long stride;             // elements from row to row
 };
-__global__ void cast_f32_bf16_rows_kernel(const float* __restrict__ in, CastPiece a, CastPiece b, CastPiece c, float scale) {
+// The parts of dK and dV that several CTAs of the attention backward wrote for one K/V tile of 128 rows (see cpb_flash_attn_bwd): part j
+// of a matrix starts j * n8 groups after it.
+struct CastParts {
+  int count;               // parts of every tile; with `local` a tile has ceil(G (nq - first visible query tile) / chunk) of them
+  int local, Tk, k_off, nq, G, chunk;
+};
+__device__ __forceinline__ int tile_parts(const CastParts& q, size_t row) {
+  if (!q.local) return q.count;
+  const int seen = q.nq - max(0, q.k_off + (int)(row % q.Tk) / 128 * 128) / 128;
+  return seen <= 0 ? 0 : (q.G * seen + q.chunk - 1) / q.chunk;
+}
+// in: the rows of `a`, then the parts of `b`, then those of `c`, added in their order.
+__global__ void cast_f32_bf16_rows_kernel(const float* __restrict__ in, CastPiece a, CastPiece b, CastPiece c, CastParts q, float scale) {
   pdl_release();
   pdl_wait();
   const size_t total = a.n8 + b.n8 + c.n8;
@@ -842,7 +853,15 @@ __global__ void cast_f32_bf16_rows_kernel(const float* __restrict__ in, CastPiec
     const int c8 = in_a ? a.c8 : in_b ? b.c8 : c.c8;
     const long stride = in_a ? a.stride : in_b ? b.stride : c.stride;
     const size_t k = in_a ? i : in_b ? i - a.n8 : i - a.n8 - b.n8, r = k / c8;
-    const float4 x = *(const float4*)(in + i * 8), y = *(const float4*)(in + i * 8 + 4);
+    const float4* src = (const float4*)in + 2 * (in_a ? i : a.n8 + (in_b ? 0 : b.n8 * q.count) + k);
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+    const int parts = in_a ? 1 : tile_parts(q, r);
+    if (parts > 0) { x = src[0]; y = src[1]; }
+    for (int j = 1; j < parts; ++j) {
+      const float4 u = src[2 * j * b.n8], v = src[2 * j * b.n8 + 1];
+      x.x += u.x; x.y += u.y; x.z += u.z; x.w += u.w;
+      y.x += v.x; y.y += v.y; y.z += v.z; y.w += v.w;
+    }
     *(uint4*)(out + r * stride + (k - r * c8) * 8) = make_uint4(pack_bf16(x.x * scale, x.y * scale), pack_bf16(x.z * scale, x.w * scale),
                                                                 pack_bf16(y.x * scale, y.y * scale), pack_bf16(y.z * scale, y.w * scale));
   }
@@ -1055,24 +1074,26 @@ extern "C" int cpb_adamw(float* p, const float* g, float* m, float* v, void* p16
   adamw_kernel<<<grid_for((size_t)n, 256), 256, 0, stream>>>(p, g, m, v, (__nv_bfloat16*)p16, (size_t)n, lr, b1, b2, eps, wd, bc1, bc2, grad_prescale, clip, sumsq, flag);
   return check_launch("adamw");
 }
-// in: fp32, rows_q x cols_q values and then twice rows_k x cols_k (rows_k 0: none); each goes to bf16 rows q_stride / kv_stride elements apart.
+// in: fp32, rows_q x cols_q values and then twice `parts` matrices of rows_k x cols_k (parts 0: none), the parts to be added; each result goes
+// to bf16 rows q_stride / kv_stride elements apart.  Tk, k_off, nq, G, chunk, local: see CastParts.
 extern "C" int cpb_cast_f32_bf16_rows(const float* in, void* out_q, long rows_q, int cols_q, long q_stride, void* out_k, void* out_v, long rows_k,
-                                      int cols_k, long kv_stride, float scale, cudaStream_t stream) {
+                                      int cols_k, long kv_stride, int parts, int Tk, int k_off, int nq, int G, int chunk, int local, float scale,
+                                      cudaStream_t stream) {
   if ((cols_q % 8) || (q_stride % 8) || ((uintptr_t)in & 15) || ((uintptr_t)out_q & 15)) return set_error(CPB_ERR_ARG, "cast_rows: columns, stride and pointers must be multiples of 16 bytes");
-  if (rows_k > 0 && ((cols_k % 8) || (kv_stride % 8) || (((uintptr_t)out_k | (uintptr_t)out_v) & 15)))
+  if (parts > 0 && ((cols_k % 8) || (kv_stride % 8) || (((uintptr_t)out_k | (uintptr_t)out_v) & 15) || Tk <= 0 || chunk <= 0))
     return set_error(CPB_ERR_ARG, "cast_rows: columns, stride and pointers must be multiples of 16 bytes");
   const CastPiece q{(__nv_bfloat16*)out_q, (size_t)(rows_q > 0 ? rows_q : 0) * (cols_q / 8), cols_q > 0 ? cols_q / 8 : 1, q_stride};
-  const size_t nk = (size_t)(rows_k > 0 ? rows_k : 0) * (cols_k / 8);
+  const size_t nk = parts > 0 ? (size_t)rows_k * (cols_k / 8) : 0;
   const CastPiece k{(__nv_bfloat16*)out_k, nk, cols_k > 0 ? cols_k / 8 : 1, kv_stride}, v{(__nv_bfloat16*)out_v, nk, k.c8, kv_stride};
   const size_t total = q.n8 + 2 * nk;
   if (total == 0) return CPB_OK;
-  CPB_CUDA_OK(launch_pdl(cast_f32_bf16_rows_kernel, grid_for(total, 256, 32), 256, 0, stream, in, q, k, v, scale));
+  CPB_CUDA_OK(launch_pdl(cast_f32_bf16_rows_kernel, grid_for(total, 256, 32), 256, 0, stream, in, q, k, v, CastParts{parts, local, Tk, k_off, nq, G, chunk}, scale));
   return check_launch("cast_rows");
 }
 extern "C" int cpb_cast_f32_bf16(const float* in, void* out, long n, float scale, cudaStream_t stream) {
   if (n <= 0) return CPB_OK;
   if (n % 8 == 0 && (((uintptr_t)in | (uintptr_t)out) & 15) == 0)
-    return cpb_cast_f32_bf16_rows(in, out, n / 8, 8, 8, nullptr, nullptr, 0, 0, 0, scale, stream);
+    return cpb_cast_f32_bf16_rows(in, out, n / 8, 8, 8, nullptr, nullptr, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, scale, stream);
   CPB_CUDA_OK(launch_pdl(cast_f32_bf16_kernel, grid_for((size_t)n, 256), 256, 0, stream, in, (__nv_bfloat16*)out, (size_t)n, scale));
   return check_launch("cast_f32_bf16");
 }

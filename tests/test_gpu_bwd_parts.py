@@ -47,6 +47,7 @@ def test_parts(monkeypatch, B, Tq, Tk, Hq, Hkv, causal, k_off, ring, D, chunk):
     for a, b in zip(got, _dense(q, k, v, do, scale, pos, k_off, causal)):
         # P and dS are rounded to bf16 (2^-9 each) before products whose terms partly cancel: 2.5e-3 is what whole sweeps have
         assert a.shape == b.shape and a.is_contiguous() and _rel(a, b) < 5e-3
+    assert all(torch.equal(a, b) for a, b in zip(got[1:], AB.flash_bwd_cuda(q, k, v, o, lse, do, scale, causal, qp, k_off)[1:]))      # dK, dV repeat
     if not ring and Tq == Tk and k_off == 0:
         packed = torch.cat([q, k, v], 2)
         for x in (packed, packed.transpose(0, 1).contiguous().transpose(0, 1)):      # dense, and a layout that takes three gradients
