@@ -452,8 +452,11 @@ extern "C" int cpb_flash_fwd(const void* q, const void* k, const void* v, void* 
   CUtensorMap tq, tk, tv;
   int rc;
   if ((rc = make_qkv_tmap(&tq, q, D, Hq, Tq, B, q_sh, q_st, q_sb, FA_BQ)) != CPB_OK) return rc;
-  static const bool new64 = getenv("CPB_F64") != nullptr && getenv("CPB_F64")[0] == '1';
-  const int kv_rows = D == 64 && new64 ? 64 : FA_BK;
+  // head_dim 64: four CTAs per SM with steps of 64 keys (attention_fwd64.cu) pay when the SMs stay full of them, because each is slower
+  // than one of two: us with two and with four, 32/8 heads, keys 8192 (2048 CTAs) 427 and 453, 16384 (4096) 1446 and 1466, 32768 (8192)
+  // 5712 and 5272, 65536 (16384) 23345 and 22326; 4096 queries of 32768 keys, 8/8 heads (256) 472 and 573.
+  const bool four = D == 64 && (long)((Tq + FA_BQ - 1) / FA_BQ) * Hq * B >= 32L * sm_count();
+  const int kv_rows = four ? 64 : FA_BK;
   if ((rc = make_qkv_tmap(&tk, k, D, Hkv, Tk, B, k_sh, k_st, k_sb, kv_rows)) != CPB_OK) return rc;
   if ((rc = make_qkv_tmap(&tv, v, D, Hkv, Tk, B, k_sh, k_st, k_sb, kv_rows)) != CPB_OK) return rc;
   FwdParams p;
@@ -475,7 +478,7 @@ extern "C" int cpb_flash_fwd(const void* q, const void* k, const void* v, void* 
   // 236; 8192, 224 CTAs 154 and 153; 8192, 256 CTAs 163 and 153; 32768 keys, 256 CTAs 528 and 507).
   const long pairs = (long)((Tq + 2 * FA_BQ - 1) / (2 * FA_BQ)) * Hq * B;
   if (D == 128 && Tk >= 8192 && Tq > FA_BQ && 5 * pairs >= 8 * sm_count()) return launch_flash_fwd128_pair(poly, tq, tk, tv, p, stream);
-  if (D == 64 && new64) return launch_flash_fwd64(poly, tq, tk, tv, p, stream);
+  if (four) return launch_flash_fwd64(poly, tq, tk, tv, p, stream);
   const int G = Hq / Hkv;
   dim3 grid(p.n_copy + ((Tq + FA_BQ - 1) / FA_BQ) * G, Hkv, B);
 #define CPB_FWD_LAUNCH(DD, PP)                                                                                         \
