@@ -32,12 +32,13 @@ namespace cpb {
 
 template <int BN>
 struct GemmSmem {
-  static constexpr int STAGES = BN > 128 ? 6 : 8;                // up to 192 KB of operands in flight
+  static constexpr int STAGES = BN == 384 ? 4 : BN > 128 ? 6 : 8;       // 160 to 192 KB of operands in flight
   static constexpr int A_BYTES = GEMM_BM * GEMM_BK * 2;          // 128 rows of A
   static constexpr int B_GROUPS = (BN / 2 + 63) / 64;            // this CTA's half of B's columns, in groups of 64 (N-major: 96 columns
   static constexpr int B_BYTES = B_GROUPS * 64 * GEMM_BK * 2;    // take two groups, the last 32 columns are loaded and not used)
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int ACC_COLS = BN > 128 ? 256 : 128;          // tensor-memory columns of an accumulator (a power of two)
+  static constexpr int ACCS = BN == 384 ? 1 : 2;                 // accumulators
+  static constexpr int ACC_COLS = BN == 384 ? 512 : BN > 128 ? 256 : 128;      // tensor-memory columns of one (a power of two)
   static constexpr int STORE_OFFSET = STAGES * STAGE_BYTES;      // 4 epilogue warps x 2 buffers x 4 KB
   static constexpr int BAR_OFFSET = STORE_OFFSET + 32768;
   static constexpr int TOTAL = BAR_OFFSET + 256 + 1024;
@@ -143,14 +144,16 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     fence_mbar_init();
   }
   if (warp == 1) {
-    tmem_alloc_pair(tmem_slot, 2 * L::ACC_COLS);
+    tmem_alloc_pair(tmem_slot, L::ACCS * L::ACC_COLS);
     tmem_relinquish_pair();
   }
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();                           // both CTAs' barriers exist before anything arrives on them remotely
   tc_fence_after();
-  pdl_release();
+  // not before a launch that adds the splits' parts: its waiting blocks made the pair of launches slower (us with and without:
+  // 136 x 768 x 3072 in twelve 14.4 and 9.1, 1152 x 384 x 4096 in seven 17.3 and 15.2, 384 x 384 x 4096 in eleven 10.6 and 9.4)
+  if (p.splits == 1) pdl_release();
   pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
 
@@ -183,6 +186,14 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             // the even CTA stages the gate rows of features nb*BN/2.., the odd CTA the matching up rows
             const int f0 = nb * (BN / 2);
             tma_load_2d_pair(sb, &tmB, full_even, k0, (rank == 0 ? 0 : p.swiglu_half) + f0);
+          } else if (BN == 384) {
+            // columns of the 256-wide product, 128 per CTA, then those of the 128-wide one, 64 per CTA
+            const int n0 = nb * BN + (int)rank * 128, n2 = nb * BN + 256 + (int)rank * 64;
+#pragma unroll
+            for (int g = 0; g < 3; ++g) {
+              const int n = g < 2 ? n0 + g * 64 : n2;
+              tma_load_2d_pair(sb + g * 8192, &tmB, full_even, B_MN ? n : k0, B_MN ? k0 : n);
+            }
           } else if (B_MN) {
             const int n0 = nb * BN + (int)rank * (BN / 2);
 #pragma unroll
@@ -199,7 +210,8 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     // ------------------------------------------------------------------ MMA issuer (even CTA only; convergent warp, elected lane)
     if (rank == 0) {
       const uint32_t leader = elect_one() ? 1u : 0u;
-      constexpr uint32_t idesc = make_idesc_bf16(2 * GEMM_BM, BN, A_MN, B_MN);
+      constexpr uint32_t idesc = make_idesc_bf16(2 * GEMM_BM, BN == 384 ? 256 : BN, A_MN, B_MN);
+      constexpr uint32_t idesc2 = make_idesc_bf16(2 * GEMM_BM, 128, A_MN, B_MN);       // the last 128 of 384 columns
       const uint32_t s0 = smem_u32(smem);
       const SDesc da0 = sdesc_split(A_MN ? make_sdesc(s0, 8192, 1024) : sdesc_kmajor(s0));
       const SDesc db0 = sdesc_split(B_MN ? make_sdesc(s0 + L::A_BYTES, 8192, 1024) : sdesc_kmajor(s0 + L::A_BYTES));
@@ -208,8 +220,8 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       int it = 0;
       bool alive = true;
       for (int item = pair; item < num_items && alive; item += num_pairs, ++it) {
-        const int acc = it & 1;
-        const uint32_t acc_phase = (it >> 1) & 1;
+        const int acc = L::ACCS == 2 ? it & 1 : 0;
+        const uint32_t acc_phase = (L::ACCS == 2 ? it >> 1 : it) & 1;
         if (!__all_sync(0xffffffffu, mbar_wait(&tempty_bar[acc], acc_phase ^ 1, abort_flag, p.status, 210))) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * L::ACC_COLS;
@@ -221,9 +233,12 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           const uint32_t so = (uint32_t)stage * (L::STAGE_BYTES >> 4);
           const SDesc da = SDesc{da0.lo + so, da0.hi}, db = SDesc{db0.lo + so, db0.hi};
           umma_pair_ss_p(leader, d_tmem, sdesc_at(da, 0), sdesc_at(db, 0), idesc, kb != kb0);
+          if (BN == 384) umma_pair_ss_p(leader, d_tmem + 256, sdesc_at(da, 0), sdesc_at(db, 16384), idesc2, kb != kb0);
 #pragma unroll
-          for (int k = 1; k < GEMM_BK / 16; ++k)
+          for (int k = 1; k < GEMM_BK / 16; ++k) {
             umma_pair_ss_cp<true>(leader, d_tmem, sdesc_at(da, k * A_STEP), sdesc_at(db, k * B_STEP), idesc);
+            if (BN == 384) umma_pair_ss_cp<true>(leader, d_tmem + 256, sdesc_at(da, k * A_STEP), sdesc_at(db, 16384 + k * B_STEP), idesc2);
+          }
           // the stage is free in both CTAs once these MMAs have read it
           const uint32_t e_own = smem_u32(&empty_bar[stage]);
           umma_pair_commit_p(leader, e_own);
@@ -241,8 +256,8 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     WarpStore ws{smem + L::STORE_OFFSET + quarter * 8192, 0u, lane == 0};
     int it = 0;
     for (int item = pair; item < num_items; item += num_pairs, ++it) {
-      const int acc = it & 1;
-      const uint32_t acc_phase = (it >> 1) & 1;
+      const int acc = L::ACCS == 2 ? it & 1 : 0;
+      const uint32_t acc_phase = (L::ACCS == 2 ? it >> 1 : it) & 1;
       int mt, nb;
       pair_tile_coords(item % num_tiles, p.num_m_tiles, p.num_n_blocks, p.band, mt, nb);
       const int row0 = mt * (2 * GEMM_BM) + (int)rank * GEMM_BM + quarter * 32;
@@ -271,7 +286,7 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   cluster_sync_all();          // the even CTA's MMAs have finished reading the odd CTA's operands; no remote arrival is in flight
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc_pair(tmem_base, 2 * L::ACC_COLS);
+    tmem_dealloc_pair(tmem_base, L::ACCS * L::ACC_COLS);
   }
 }
 
@@ -344,18 +359,19 @@ gemm_sum_partials_kernel(__nv_bfloat16* __restrict__ C, const float4* __restrict
 
 // Tile width and K split.  The work items of a launch (tiles x splits) run on 74 pairs, so the time is that of the pair
 // with the most items: items / 74 rounded up, each the longer of its main loop and its epilogue, plus one epilogue at the
-// end.  Nanoseconds, measured: main loop per 64 of K 370 at 256 columns (8192^3: 694 us) and 240 at 128 columns (892 us),
-// so narrow tiles pay only where they fill a wave (M 4096, N 384, K 50304: 238 us at 256 columns, 182 at 128).
+// end.  Nanoseconds, measured: main loop per 64 of K 370 at 256 columns (8192^3: 694 us), 300 at 192 and 240 at 128 columns (892 us),
+// so narrow tiles pay only where they fill a wave (M 4096, N 384, K 50304: 238 us at 256 columns, 182 at 128; M 4096, K 3072, N 768: 19.4
+// at 256 and 15.4 at 192; M 8192, N 384, K 1024 10.4 at 128 and 8.3 at 192).
 //
-// Only the accumulating epilogue is split: all splits but the first go through a workspace of at most 128 MB, and a second
-// launch adds them in a fixed order.  On the GPU that costs 1.4 us and, per split, a write and a read of the fp32 matrix in L2 at
+// The accumulating and the bf16 epilogue may be split: all splits but the first (bf16: all) go through a workspace of at most 128 MB,
+// and a second launch adds them in a fixed order.  On the GPU that costs 1.4 us and, per split, a write and a read of the fp32 matrix in L2 at
 // about 16 TB/s (M 3072, N 2048, K 8192: 106 us unsplit, 86 in two; M 384, N 384, K 8192: 36.6 unsplit, 22.6 in two, 11.7 in
 // twelve; M 2048, N 2048, K 8192: 50 unsplit, 57 in two); the host pays 4 us for the launch and the workspace.  So a split has to
 // save 8 us: with 1.4 us as the bar the small training steps, which wait for the host, were 1 to 3 % slower, and without any
 // split 1 to 2 %.  All splits adding to C in L2 from one launch took 9.0 us in twelve and 75.7 in two, but in the order in
 // which they finished: weight gradients did not repeat.
-// With all pairs on narrow tiles their operands come to 15 TB/s out of L2 and 64 of K takes 290 instead of 240 (M 3072, N 768,
-// K 4096: 24 us, against 22 in two splits of wide tiles).
+// With all pairs on narrow tiles their operands come to 15 TB/s out of L2 and 64 of K takes 290 instead of 240, 400 instead of 300 (M 3072,
+// N 768, K 4096: 24 us, against 22 in two splits of wide tiles).  bf16 in splits: M 136, N 768, K 3072 14.6 us unsplit, 9.1 in twelve.
 // `want` > 0 asks for the best width at that many splits, 0 for the best of both.
 static void plan_tiles(int M, int N, int K, int epi, int has_aux, int want, int& bn, int& splits) {
   const long nk = (K + GEMM_BK - 1) / GEMM_BK;
@@ -363,12 +379,17 @@ static void plan_tiles(int M, int N, int K, int epi, int has_aux, int want, int&
   const long pass = (long)M * N * 8 / 16000;
   long best = -1;
   const bool sums = epi == EPI_F32_ACC || epi == EPI_BF16;
-  for (int cand = 256; cand >= 128; cand -= 64) {
-    if (cand == 192 && epi == EPI_BF16_SWIGLU) continue;
+  // N = 384 and an A that L2 does not hold: one column of tiles reads A once (us with narrower tiles and with this one: 4096 x 384 x 50304
+  // 150 and 122, 50304 x 384 x 4096 155 and 135).  With two and more columns of tiles its single accumulator costs more than it
+  // saves (4096 x 768 x 50304 217 to 234 and 233 to 255, 50304 x 768 x 4096 238 and 267).
+  const bool one_column = sums && N == 384 && (long)M * K * 2 >= (64L << 20);
+  static const int widths[] = {256, 192, 128, 384};
+  for (const int cand : widths) {
+    if ((cand == 192 && epi == EPI_BF16_SWIGLU) || (cand == 384) != one_column) continue;
     const int per_tile = epi == EPI_BF16_SWIGLU ? cand / 2 : cand;
     const long tiles = m_tiles * ((N + per_tile - 1) / per_tile);
     long ce = epi == EPI_F32 || epi == EPI_F32_ACC ? 1200 : epi == EPI_BF16_GELU ? (has_aux ? 1600 : 1400) : epi == EPI_BF16_SWIGLU ? (has_aux ? 1300 : 1000) : 650;
-    if (cand < 256) ce = ce * cand / 256 + 50;
+    if (cand != 256) ce = ce * cand / 256 + 50;
     const long max_split = want > 0 ? want : sums ? (nk + 3) / 4 : 1;                   // at least four K blocks per item
     for (long s = want > 0 ? want : 1; s <= max_split; ++s) {
       const bool sum16 = epi == EPI_BF16 && s > 1;
@@ -376,10 +397,11 @@ static void plan_tiles(int M, int N, int K, int epi, int has_aux, int want, int&
       const long kps = (nk + s - 1) / s;
       if ((nk + kps - 1) / kps != s) continue;                       // the same items as a smaller split
       const long waves = (tiles * s + pairs - 1) / pairs, busy = tiles * s < pairs ? tiles * s : pairs;
-      const long main = kps * (cand == 256 ? 370 : cand == 192 ? 300 : epi == EPI_F32_ACC || sum16 ? 240 + 50 * busy / pairs : 240);
+      const long main = kps * (cand == 384 ? 620 : cand == 256 ? 370 : cand == 192 ? (epi == EPI_F32_ACC || sum16 ? 300 + 100 * busy / pairs : 300) : epi == EPI_F32_ACC || sum16 ? 240 + 50 * busy / pairs : 240);
       const long out = !sum16 ? ce : cand == 256 ? 1200 : 1200 * cand / 256 + 50;
-      long t = waves * (main > out ? main : out) + (main > out ? out : main);
-      if (s > 1) t += 8000 + (sum16 ? 2 * s + 1 : s + 1) * pass;     // 1.4 us and what a split has to save
+      // with one accumulator the epilogue is not hidden behind the next item's main loop
+      long t = cand == 384 ? waves * (main + out) : waves * (main > out ? main : out) + (main > out ? out : main);
+      if (s > 1) t += 8000 + (sum16 ? 3 * s + 1 : s + 1) * pass;     // 1.4 us and what a split has to save
       if (best < 0 || t < best) { best = t; bn = cand; splits = (int)s; }
     }
   }
@@ -450,7 +472,7 @@ extern "C" int cpb_gemm_bf16(const void* A, const void* B, void* C, void* aux, c
   int rc;
   const int b_rows = epi == EPI_BF16_SWIGLU ? 2 * N : N;
   if ((rc = a_mn ? mnmajor_tmap(&tm[0], A, M, K, lda) : kmajor_tmap(&tm[0], A, M, K, lda, GEMM_BM)) != CPB_OK) return rc;
-  if ((rc = b_mn ? mnmajor_tmap(&tm[1], B, b_rows, K, ldb) : kmajor_tmap(&tm[1], B, b_rows, K, ldb, bn / 2)) != CPB_OK) return rc;
+  if ((rc = b_mn ? mnmajor_tmap(&tm[1], B, b_rows, K, ldb) : kmajor_tmap(&tm[1], B, b_rows, K, ldb, bn == 384 ? 64 : bn / 2)) != CPB_OK) return rc;
   {
     // one store box = 32 rows x 128 bytes; the map's extents clip the edges of C
     const int eb = (epi == EPI_F32 || epi == EPI_F32_ACC) ? 4 : 2;
@@ -473,7 +495,7 @@ extern "C" int cpb_gemm_bf16(const void* A, const void* B, void* C, void* aux, c
     uint32_t box[3] = {32, 32, 1};
     if ((rc = encode_tmap(&tm[3], partials, 4, 3, dims, strides, box, 1)) != CPB_OK) return rc;
   }
-  rc = bn == 256 ? dispatch_pair<256>(tm, p, a_mn, b_mn, stream) : bn == 192 ? dispatch_pair<192>(tm, p, a_mn, b_mn, stream) : dispatch_pair<128>(tm, p, a_mn, b_mn, stream);
+  rc = bn == 384 ? dispatch_pair<384>(tm, p, a_mn, b_mn, stream) : bn == 256 ? dispatch_pair<256>(tm, p, a_mn, b_mn, stream) : bn == 192 ? dispatch_pair<192>(tm, p, a_mn, b_mn, stream) : dispatch_pair<128>(tm, p, a_mn, b_mn, stream);
   if (rc != CPB_OK || splits == 1) return rc;
   const unsigned total = (unsigned)((long)M * N / (sum16 ? 8 : 4)), blocks = (total + 255) / 256, cap = (unsigned)sm_count() * 8;
   const unsigned grid = blocks < cap ? blocks : cap;

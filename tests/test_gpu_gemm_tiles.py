@@ -11,19 +11,23 @@ pytestmark = pytest.mark.gpu
 SHAPES = [(256 * 74, 192, 64), (256 * 74, 384, 72), (256 * 37, 376, 520), (4096, 768, 3072), (256 * 74 - 120, 184, 328)]
 
 
+# 384 columns: two products of 256 and 128 columns per step, one accumulator; M and K with remainders, one and several items per pair
+WIDE = [(256 * 74, 384, 2048), (256 * 80 - 120, 384, 2056), (4096, 384, 12008)]
+
+
 def _operands(M, N, K):
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     a, b = (torch.randn(r, K, device="cuda", generator=g).bfloat16() for r in (M, N))
     return a, b, torch.randn(N, device="cuda", generator=g), (a.double() @ b.double().t()).float()
 
 
-@pytest.mark.parametrize("M,N,K", SHAPES)
+@pytest.mark.parametrize("M,N,K", SHAPES + WIDE)
 def test_every_epilogue_and_order(M, N, K):
     from context_parallelism_b200 import _native as nv
     from context_parallelism_b200.ops import gemm as G
     a, b, bias, ref = _operands(M, N, K)
     plans = {e: nv.lib().cpb_gemm_plan(M, N, K, e, 0) >> 16 for e in (G.EPI_BF16, G.EPI_F32, G.EPI_F32_ACC, G.EPI_BF16_GELU)}
-    assert 192 in plans.values(), plans
+    assert (384 if (M, N, K) in WIDE else 192) in plans.values(), plans
     at, bt = a.t().contiguous(), b.t().contiguous()
     fp32 = 1e-4 * K ** 0.5                       # two orders of K products of unit normals, see the other GEMM tests
     for x, xm in ((a, False), (at, True)):
