@@ -17,9 +17,9 @@ import torch
 
 from . import _native as nv
 
-MAX_RECORDS = 4                  # per model; the one used longest ago makes room
-EAGER_CALLS = 2                  # calls with new shapes that run as they always did: a shape met only once records nothing
-MAX_POOL_BYTES = 8 << 30         # a record whose buffers take more than this is not kept
+MAX_RECORDS = 8                  # per model; the one used longest ago makes room
+EAGER_CALLS = 2                  # calls with new shapes that run as they always did; twice as many each time that the record was lost
+MAX_POOL_BYTES = 8 << 30         # buffers of all records of a model
 MIN_FREE_SHARE = 0.25            # share of the GPU's memory that has to be free before a record is made
 # A call is recorded while the GPU needs less time for it than the host: a launch costs the host about 25 us (forward and backward;
 # 13 us without autograd), the kernels of such models reach about 600 TFLOP/s.
@@ -159,7 +159,8 @@ class GraphCache:
     def __init__(self):
         self._lock = threading.Lock()
         self._records: "OrderedDict[tuple, Optional[_Record]]" = OrderedDict()
-        self._seen: "OrderedDict[tuple, int]" = OrderedDict()
+        self._seen: "OrderedDict[tuple, int]" = OrderedDict()        # eager calls since the record was lost, or at all
+        self._lost: "OrderedDict[tuple, int]" = OrderedDict()        # how often it was
 
     def __reduce__(self):                                            # a copied or unpickled model starts without records
         return GraphCache, ()
@@ -190,7 +191,7 @@ class GraphCache:
                 n = self._seen[key] = self._seen.pop(key, 0) + 1
                 while len(self._seen) > 64:
                     self._seen.popitem(last=False)
-                if n >= EAGER_CALLS:
+                if n >= EAGER_CALLS << min(self._lost.get(key, 0), 8):
                     self._seen.pop(key, None)
                     self._record(key, model, fn, inputs, device, flops < GPU_TFLOPS * 1e6 * HOST_US_PER_LAUNCH * launches, train)
         return outs
@@ -211,13 +212,22 @@ class GraphCache:
                 rec.close()
                 rec = None
         self._records[key] = rec                                     # None: not to be tried again
-        while len(self._records) > 64 or sum(r is not None for r in self._records.values()) > MAX_RECORDS:
-            self._drop(next((k for k, r in self._records.items() if r is not None), next(iter(self._records))))
+        while True:
+            held = [(k, r.pool_bytes) for k, r in self._records.items() if r is not None]
+            if len(held) > MAX_RECORDS or sum(b for _, b in held) > MAX_POOL_BYTES:
+                self._drop(held[0][0])
+            elif len(self._records) > 64:
+                self._drop(next(iter(self._records)))
+            else:
+                break
 
     def _drop(self, key) -> None:
         rec = self._records.pop(key)
         if rec is not None:
             rec.close()
+            self._lost[key] = self._lost.pop(key, 0) + 1
+            while len(self._lost) > 64:
+                self._lost.popitem(last=False)
 
     def clear(self) -> None:
         """Give back every record and its memory."""
@@ -225,3 +235,4 @@ class GraphCache:
             while self._records:
                 self._drop(next(iter(self._records)))
             self._seen.clear()
+            self._lost.clear()

@@ -114,6 +114,22 @@ def test_what_is_not_recorded():
 
 
 @torch.no_grad()
+def test_more_shapes_than_records(monkeypatch):
+    """Shapes met in turn, one more than there is room for: results stay right, and the records lost are made ever less often."""
+    from context_parallelism_b200 import graphs
+    monkeypatch.setattr(graphs, "MAX_RECORDS", 2)
+    eng, made = _engine(), []
+    init = graphs._Record.__init__
+    monkeypatch.setattr(graphs._Record, "__init__", lambda self, *a: (made.append(1), init(self, *a))[1])
+    batches = [eng.shard_batch(*_batch(eng, i, T=104 + 8 * i)) for i in range(3)]
+    want = [eng.model._hidden(x, p, *eng.model.recorded_inputs()) for x, _, p in batches]
+    for _ in range(16):
+        for (x, _, p), w in zip(batches, want):
+            assert torch.equal(eng.model.hidden(x, p), w)
+    assert len(_records(eng)) <= 2 and len(made) <= 9
+
+
+@torch.no_grad()
 def test_threads_and_streams():
     from context_parallelism_b200.ops import xent
     eng = _engine()
