@@ -620,11 +620,13 @@ extern "C" int cpb_flash_attn_bwd(const void* q, const void* k, const void* v, c
 // How many (query head, query tile) pairs a CTA of the head_dim-64 / 128 kernels should take at most, 0 for whole sweeps.  Whole sweeps
 // are uneven under the causal mask (the first K/V tile meets every query, the last one tile of them) and few when there are few
 // heads; parts even out, but each costs the CTA's start and end, and a part of dK / dV is written and read in fp32 (added in a
-// fixed order, so that dK and dV repeat bit for bit).  So both ways of handing out the CTAs to the SMs are followed here, with the times that they take.
+// fixed order, so that dK and dV repeat bit for bit).  Whole gradient, us, whole sweeps and parts: 2 x 1000, 6/2 heads of 64 50 and 26
+// (six), 2 x 4096, 6/2 163 and 99 (two), 16384, 4/1 794 and 422 (two); heads of 128: 1200, 4/1 98 and 32 (eight), 4000, 8/2 302 and 112
+// (four), 32749, 4/1 2904 and 2644 (four); longest first alone: 8192, 32/8 of 64 955 and 834, of 128 1539 and 1378.  So both ways of handing out the CTAs to the SMs are followed here, with the times that they take.
 extern "C" int cpb_flash_bwd_chunk(int B, int Tq, int Tk, int Hq, int Hkv, int D, int causal, int k_off, int local) {
   const int nq = (Tq + 127) / 128, n_kt = (Tk + 127) / 128, G = Hq / (Hkv > 0 ? Hkv : 1), hb = Hkv * B, sms = sm_count();
   if (nq <= 0 || n_kt <= 0 || G <= 0 || hb <= 0 || (D != 64 && D != 128) || (long)n_kt * hb > 16L * sms) return 0;
-  const double tile = D == 64 ? 1.55 : 2.4, start_end = D == 64 ? 4.0 : 5.5;            // us
+  const double tile = D == 64 ? 1.25 : 1.9, start_end = D == 64 ? 11.0 : 13.0;          // us, a chip that is not full
   std::vector<int> len(n_kt);
   for (int k = 0; k < n_kt; ++k) {
     // positions that are not 0 .. Tq - 1 (a ring rank's): the share that sees the tile falls evenly, near enough
@@ -643,11 +645,11 @@ extern "C" int cpb_flash_bwd_chunk(int B, int Tq, int Tk, int Hq, int Hkv, int D
     }
     return end;
   };
-  double best = finish(0) * 0.95;
+  double best = finish(0) * 0.97;
   int chunk = 0;
-  for (int parts = 2; parts <= 24; ++parts) {
+  for (int parts = 1; parts <= 24; ++parts) {                      // one part: whole sweeps, the longest first over all heads
     const int c = (G * nq + parts - 1) / parts;
-    if (c < 2) break;
+    if (parts > 1 && c < 2) break;
     long written = 0;                                                // K/V tiles times parts
     for (int k = 0; k < n_kt; ++k) written += local ? (len[k] + c - 1) / c : parts;
     const double t = finish(c) + 0.5 + (double)written * hb * 128 * D * 2 * 8 / 4e6;       // written and read at 4 TB/s

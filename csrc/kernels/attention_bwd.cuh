@@ -10,11 +10,21 @@ struct BwdWork {
   int kt, hkv, b;
   int it0;                 // first pair of the sweep
 };
-__device__ __forceinline__ BwdWork bwd_work(int it_chunk, int n_kt, int Hkv, int B) {
+// K/V tiles that have a part number c: under a causal mask over positions 0 .. Tq - 1 (`local`) those with more than c chunk visible pairs.
+__host__ __device__ __forceinline__ int bwd_tiles(int c, int it_chunk, int n_kt, int nq, int G, int k_off, int local) {
+  if (!local) return n_kt;
+  const int last = nq - 1 - (int)((long)c * it_chunk / G);             // last first-visible query tile
+  const long end = 128L * last + 127 - k_off;
+  return last < 0 || end < 0 ? 0 : (int)(end / 128 + 1 < n_kt ? end / 128 + 1 : n_kt);
+}
+// `local` here: causal and local
+__device__ __forceinline__ BwdWork bwd_work(int it_chunk, int n_kt, int nq, int G, int Hkv, int B, int k_off, int local) {
   if (it_chunk == 0) return BwdWork{(int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, 0};
-  // longest first over all heads and batches: the parts of a tile are numbered last
-  const int i = (int)blockIdx.x, hb = Hkv * B, kc = i / hb;
-  return BwdWork{kc % n_kt, i % Hkv, (i / Hkv) % B, kc / n_kt * it_chunk};
+  // longest first over all heads and batches, part 0 of every tile, then part 1 of those that have one, ...
+  int i = (int)blockIdx.x, c = 0;
+  const int hb = Hkv * B;
+  for (int n; i >= (n = bwd_tiles(c, it_chunk, n_kt, nq, G, k_off, local) * hb); ++c) i -= n;
+  return BwdWork{i / hb, i % Hkv, (i / Hkv) % B, c * it_chunk};
 }
 
 }  // namespace cpb

@@ -114,15 +114,10 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   int* qt_start_s = (int*)(tmem_slot + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const BwdWork work = bwd_work(p.it_chunk, (p.Tk + B128_T - 1) / B128_T, p.Hkv, p.B);
+  const int G = p.Hq / p.Hkv, num_q_tiles = p.Tq_pad / B128_T;
+  const BwdWork work = bwd_work(p.it_chunk, (p.Tk + B128_T - 1) / B128_T, num_q_tiles, G, p.Hkv, p.B, p.k_off, p.causal && p.local);
   const int kt = work.kt, hkv = work.hkv, b = work.b;
-  const int G = p.Hq / p.Hkv;
   const int k0 = kt * B128_T;
-  const int num_q_tiles = p.Tq_pad / B128_T;
-  if (p.it_chunk && p.local && work.it0 >= (num_q_tiles - (p.causal ? min(num_q_tiles, max(0, p.k_off + k0) / B128_T) : 0)) * G) {
-    pdl_wait();
-    return;
-  }
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
@@ -143,7 +138,9 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const uint32_t tmem_base = *tmem_slot;
 
   // first query tile that can see this K/V tile (q_pos is non-decreasing)
-  if (p.causal) {
+  if (p.causal && p.local) {
+    if (threadIdx.x == 0 && p.k_off + k0 < p.Tq) *qt_start_s = max(0, p.k_off + k0) / B128_T;
+  } else if (p.causal) {
     const int kpos_min = p.k_off + k0;
     for (int t = threadIdx.x; t < num_q_tiles; t += blockDim.x) {
       const int last = min(t * B128_T + B128_T, p.Tq) - 1;
@@ -546,8 +543,14 @@ extern "C" int cpb_flash_bwd128(const void* q, const void* k, const void* v, con
     return on;
   }();
   p.debug_skip_dq = skip_dq;
-  const int n_kt = (Tk + B128_T - 1) / B128_T, pairs = Hq / Hkv * (Tq_pad / B128_T);
-  const dim3 grid = it_chunk ? dim3((unsigned)n_kt * ((pairs + it_chunk - 1) / it_chunk) * Hkv * B) : dim3(n_kt, Hkv, B);
+  const int n_kt = (Tk + B128_T - 1) / B128_T, G = Hq / Hkv, nq = Tq_pad / B128_T;
+  dim3 grid(n_kt, Hkv, B);
+  if (it_chunk) {
+    long ctas = 0;
+    for (int c = 0; (long)c * it_chunk < (long)G * nq; ++c) ctas += (long)bwd_tiles(c, it_chunk, n_kt, nq, G, k_off, causal && local) * Hkv * B;
+    if (ctas == 0) return CPB_OK;                        // no query sees a key: the cast reads no part
+    grid = dim3((unsigned)ctas);
+  }
   static bool cfg = false;
   if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_bwd128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Bwd128Smem::TOTAL)); cfg = true; }
   CPB_CUDA_OK(launch_pdl(flash_bwd128_kernel, grid, B128_THREADS, Bwd128Smem::TOTAL, stream, tq, tk, tv, tdo, tdq, p));
