@@ -19,7 +19,10 @@ from .. import _native as nv
 from .gemm import _rowmajor2d, gemm
 
 CHUNK_ROWS = 4096
-# Up to this width of the hidden states the gradient pass computes the logits a second time instead of reading them back.
+# Up to this width of the hidden states the gradient pass computes the logits a second time instead of reading them back.  Whole call, 4096
+# rows, us, stored and computed again: width 384, 50304 columns 793 and 654; 768 954 and 911; 1024 1150 and 1161 (128256 columns 3027 and
+# 3080); 1280 1582 and 1751; 2048, 128256 columns 5724 and 6338.  Before either, with a cross entropy of its own that kept each row in
+# a cluster's shared memory: 384 873, 768 1037, 1280 1900, 2048 5900; losses alone 383, 425, 599, 1984, now 174, 218, 472, 1650.
 RECOMPUTE_WIDTH = 1024
 
 
