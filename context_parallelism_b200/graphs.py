@@ -4,7 +4,9 @@ A small model's forward and backward pass is some hundred kernels of 3 to 30 us 
 Python, autograd and ``ctypes``.  :class:`GraphCache` runs a call eagerly the first times that it sees its shapes, then records it
 once and replays the record.  Nothing depends on the caller's buffers: inputs are copied into the record's own, results are
 returned as new tensors.  What the record does read by address (weights, gradient buffers) is compared at every call, and a
-record whose weights have moved is dropped.
+record whose weights have moved is dropped.  Measured on one B200, ms without and with records (and without the host's wait for every
+micro-batch): next-token logits of 136 tokens, GPT-2 124M 2.69 and 0.71; NLL of 4096 tokens, 48M 1.48 and 0.77; a step of GPT-2 44M, 16
+micro-batches of 4 x 1024 tokens 47.7 and 22.6; of GPT-2 124M, two micro-batches 17.6 and 14.9.
 """
 from __future__ import annotations
 
