@@ -621,8 +621,9 @@ extern "C" int cpb_flash_attn_bwd(const void* q, const void* k, const void* v, c
 // are uneven under the causal mask (the first K/V tile meets every query, the last one tile of them) and few when there are few
 // heads; parts even out, but each costs the CTA's start and end, and a part of dK / dV is written and read in fp32 (added in a
 // fixed order, so that dK and dV repeat bit for bit).  Whole gradient, us, whole sweeps and parts: 2 x 1000, 6/2 heads of 64 50 and 26
-// (six), 2 x 4096, 6/2 163 and 99 (two), 16384, 4/1 794 and 422 (two); heads of 128: 1200, 4/1 98 and 32 (eight), 4000, 8/2 302 and 112
-// (four); longest first alone: 8192, 32/8 of 64 956 and 828, of 128 1528 and 1354.  So both ways of handing out the CTAs to the SMs are followed here, with the times that they take.
+// (eight), 2 x 4096, 6/2 163 and 99 (two), 16384, 4/1 794 and 422 (two); heads of 128: 1200, 4/1 98 and 32 (eight), 4000, 8/2 302 and 112
+// (four); longest first alone: 8192, 32/8 of 64 956 and 828, of 128 1528 and 1354.  So both ways of
+// handing out the CTAs to the SMs are followed here, with the times that they take.
 extern "C" int cpb_flash_bwd_chunk(int B, int Tq, int Tk, int Hq, int Hkv, int D, int causal, int k_off, int local) {
   const int nq = (Tq + 127) / 128, n_kt = (Tk + 127) / 128, G = Hq / (Hkv > 0 ? Hkv : 1), hb = Hkv * B, sms = sm_count();
   if (nq <= 0 || n_kt <= 0 || G <= 0 || hb <= 0 || (D != 64 && D != 128) || (long)n_kt * hb > 16L * sms) return 0;
