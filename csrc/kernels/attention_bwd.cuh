@@ -18,8 +18,9 @@ __host__ __device__ __forceinline__ int bwd_tiles(int c, int it_chunk, int n_kt,
   return last < 0 || end < 0 ? 0 : (int)(end / 128 + 1 < n_kt ? end / 128 + 1 : n_kt);
 }
 // `local` here: causal and local
+template <bool PARTS>
 __device__ __forceinline__ BwdWork bwd_work(int it_chunk, int n_kt, int nq, int G, int Hkv, int B, int k_off, int local) {
-  if (it_chunk == 0) return BwdWork{(int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, 0};
+  if (!PARTS) return BwdWork{(int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, 0};
   // longest first over all heads and batches, part 0 of every tile, then part 1 of those that have one, ...
   int i = (int)blockIdx.x, c = 0;
   const int hb = Hkv * B;

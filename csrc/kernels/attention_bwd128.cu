@@ -87,6 +87,9 @@ struct Bwd128Smem {
 };
 
 
+// PARTS (several CTAs per tile) is an instance of its own: its state in the whole sweep's softmax warps raised the spilled loads from 24
+// to 144 bytes, and 32749 tokens of 4/1 heads took 2590 us instead of 2455.
+template <bool PARTS>
 __global__ void __launch_bounds__(B128_THREADS, 1)
 flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -115,7 +118,7 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = p.Hq / p.Hkv, num_q_tiles = p.Tq_pad / B128_T;
-  const BwdWork work = bwd_work(p.it_chunk, (p.Tk + B128_T - 1) / B128_T, num_q_tiles, G, p.Hkv, p.B, p.k_off, p.causal && p.local);
+  const BwdWork work = bwd_work<PARTS>(p.it_chunk, (p.Tk + B128_T - 1) / B128_T, num_q_tiles, G, p.Hkv, p.B, p.k_off, p.causal && p.local);
   const int kt = work.kt, hkv = work.hkv, b = work.b;
   const int k0 = kt * B128_T;
 
@@ -127,6 +130,7 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     mbar_init(dq_full, 1); mbar_init(dq_empty, 4); mbar_init(acc_done, 1);
     *abort_flag = 0;
     *qt_start_s = num_q_tiles;
+    if (PARTS) qt_start_s[1] = work.it0 / p.it_chunk;
     fence_mbar_init();
   }
   if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
@@ -152,8 +156,8 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   __syncthreads();
   const int qt_start = *qt_start_s;
   const int n_qt = num_q_tiles - qt_start;
-  const int n_it = max(0, min(p.it_chunk ? p.it_chunk : n_qt * G, n_qt * G - work.it0));      // this CTA's pairs
-  const int hq0 = hkv * G + (n_it ? work.it0 / n_qt : 0), t0 = n_it ? work.it0 % n_qt : 0;    // the first of them
+  const int n_it = PARTS ? max(0, min(p.it_chunk, n_qt * G - work.it0)) : n_qt * G;          // this CTA's pairs
+  const int hq0 = hkv * G + (PARTS && n_it ? work.it0 / n_qt : 0), t0 = PARTS && n_it ? work.it0 % n_qt : 0;       // the first of them
 
   if (warp < 4) {
   regs_give<B128_REGS_ISSUE>();
@@ -279,13 +283,10 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     bool alive = true;
     // first query position of a tile decides whether it needs masking; read one tile ahead, straight from global memory
     int qmin_next = n_it > 0 ? ld_ahead_s32(p.q_pos + (qt_start + t0) * B128_T) : 0;
-    int t = t0;
     for (int i = 0; i < n_it && alive; ++i) {
       const int st = i & 1;
       const int qmin = qmin_next;
-      const int t_cur = t;
-      if (++t == n_qt) t = 0;
-      if (i + 1 < n_it) qmin_next = ld_ahead_s32(p.q_pos + (qt_start + t) * B128_T);
+      if (i + 1 < n_it) qmin_next = ld_ahead_s32(p.q_pos + (qt_start + (t0 + i + 1) % n_qt) * B128_T);
       // slow path only for tiles that touch the causal diagonal or the end of the key sequence
       const bool need_mask = (k0 + B128_T > p.Tk) || (p.causal && (p.k_off + k0 + B128_T - 1 > qmin));
       const float* vec = (const float*)(smem + L::VEC_OFF + st * 1024) + cbase;
@@ -309,7 +310,7 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
       } else {
         const int lim = (p.causal ? kpos : -0x7fffffff - 1);               // visible: lim <= q position
-        const int4* qp = (const int4*)(p.q_pos + (qt_start + t_cur) * B128_T + cbase);
+        const int4* qp = (const int4*)(p.q_pos + (qt_start + (t0 + i) % n_qt) * B128_T + cbase);
 #pragma unroll
         for (int j = 0; j < CW; j += 4) {
           const float4 l = *(const float4*)(vec + j);
@@ -363,14 +364,14 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
     // final: dK, dV -> global
     if (n_it == 0) {
-      if (p.dkv_mode == 3 && k_valid && grp == 0) {
-        const size_t at = work.it0 / p.it_chunk * p.part_st + ((size_t)b * p.Tk + kidx) * p.dkv_st + hkv * D;
+      if (PARTS && k_valid && grp == 0) {
+        const size_t at = qt_start_s[1] * p.part_st + ((size_t)b * p.Tk + kidx) * p.dkv_st + hkv * D;
         for (int c = 0; c < D; c += 4) {
           *(float4*)((float*)p.dk + at + c) = make_float4(0.f, 0.f, 0.f, 0.f);
           *(float4*)((float*)p.dv + at + c) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
       }
-      if (p.dkv_mode == 0 && k_valid && grp == 0) {
+      if (!PARTS && p.dkv_mode == 0 && k_valid && grp == 0) {
         __nv_bfloat16* dkr = (__nv_bfloat16*)p.dk + ((size_t)b * p.Tk + kidx) * p.dkv_st + hkv * D;
         __nv_bfloat16* dvr = (__nv_bfloat16*)p.dv + ((size_t)b * p.Tk + kidx) * p.dkv_st + hkv * D;
 #pragma unroll
@@ -394,14 +395,14 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * osc);
           if (k_valid) {
-            if (p.dkv_mode == 2) {
+            if (!PARTS && p.dkv_mode == 2) {
               const int ch = kidx / p.route_rows, lrow = kidx % p.route_rows;
               float* dst = (float*)(which ? p.route_v[ch] : p.route_k[ch]) + (((size_t)b * p.route_tl + lrow) * p.Hkv + hkv) * D + c;
 #pragma unroll
               for (int j = 0; j < 32; j += 4)
                 red_add_v4(dst + j, __uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
-            } else if (p.dkv_mode == 3) {
-              uint4* dst = (uint4*)((float*)base + work.it0 / p.it_chunk * p.part_st + off + c);
+            } else if (PARTS) {
+              uint4* dst = (uint4*)((float*)base + qt_start_s[1] * p.part_st + off + c);
 #pragma unroll
               for (int j = 0; j < 32; j += 4) dst[j >> 2] = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
             } else if (p.dkv_mode == 1) {
@@ -440,13 +441,13 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     uint8_t* stage = smem + L::DQS_OFF + quarter * 8192;      // [2 boxes][32 rows][128 B]
     const bool issuer = (lane == 0);
     if (issuer) tma_prefetch_desc(&tmDQ);
-    int hq = hq0, t = t0;
     for (int i = 0; i < n_it; ++i) {
       bool ok = mbar_wait_lean(dq_full, i & 1, abort_flag, 1100);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      const int q0 = (qt_start + t) * B128_T;
+      const int hq = hq0 + (t0 + i) / n_qt;
+      const int q0 = (qt_start + (t0 + i) % n_qt) * B128_T;
       uint32_t v[4][32];
 #pragma unroll
       for (int h = 0; h < 4; ++h) tmem_ld32(t_lane + 32 * h, v[h]);
@@ -477,7 +478,6 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
       }
-      if (++t == n_qt) { t = 0; ++hq; }
     }
     if (issuer) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
@@ -551,8 +551,9 @@ extern "C" int cpb_flash_bwd128(const void* q, const void* k, const void* v, con
     if (ctas == 0) return CPB_OK;                        // no query sees a key: the cast reads no part
     grid = dim3((unsigned)ctas);
   }
-  static bool cfg = false;
-  if (!cfg) { CPB_CUDA_OK(cudaFuncSetAttribute(flash_bwd128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Bwd128Smem::TOTAL)); cfg = true; }
-  CPB_CUDA_OK(launch_pdl(flash_bwd128_kernel, grid, B128_THREADS, Bwd128Smem::TOTAL, stream, tq, tk, tv, tdo, tdq, p));
+  const auto kernel = it_chunk ? flash_bwd128_kernel<true> : flash_bwd128_kernel<false>;
+  static bool cfg[2] = {false, false};
+  if (!cfg[it_chunk > 0]) { CPB_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Bwd128Smem::TOTAL)); cfg[it_chunk > 0] = true; }
+  CPB_CUDA_OK(launch_pdl(kernel, grid, B128_THREADS, Bwd128Smem::TOTAL, stream, tq, tk, tv, tdo, tdq, p));
   return check_launch("flash_bwd128");
 }
