@@ -20,7 +20,7 @@ import torch
 from . import _native as nv
 
 MAX_RECORDS = 8                  # per model; the one used longest ago makes room
-EAGER_CALLS = 2                  # calls with new shapes that run as they always did; twice as many each time that the record was lost
+EAGER_CALLS = 3                  # calls with new shapes that run as they always did; twice as many each time that the record was lost
 MAX_POOL_BYTES = 8 << 30         # buffers of all records of a model
 MIN_FREE_SHARE = 0.25            # share of the GPU's memory that has to be free before a record is made
 # A call is recorded while the GPU needs less time for it than the host: a launch costs the host about 25 us (forward and backward;
