@@ -41,6 +41,16 @@ def xent_chunk(logits: torch.Tensor, targets: torch.Tensor, loss_sum: torch.Tens
 HEAD_TILE = 256          # columns per tile of the head's GEMM
 
 
+def _head_operands(x: torch.Tensor, w: torch.Tensor, targets: torch.Tensor):
+    """``x`` and ``w`` as the head's GEMM takes them, and 64-bit targets: the launchers get addresses and know neither types nor widths."""
+    assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16, f"the head computes in bf16 (got {x.dtype} and {w.dtype})"
+    assert w.device == x.device and targets.device == x.device, f"operands on {x.device}, {w.device} and {targets.device}"
+    x2, w2, tg = _rowmajor2d(x), _rowmajor2d(w), targets.reshape(-1).contiguous().long()
+    assert x2.shape[1] == w2.shape[1], f"hidden states of width {x2.shape[1]}, weights of width {w2.shape[1]}"
+    assert tg.numel() >= x2.shape[0], f"{tg.numel()} targets for {x2.shape[0]} rows"
+    return x2, w2, tg
+
+
 def _head_rows(xc: torch.Tensor, w: torch.Tensor, tg: torch.Tensor, n_valid: int, grad_scale: float, loss_sum: Optional[torch.Tensor],
                row_loss: Optional[torch.Tensor], want_coef: bool, logits: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
     """Loss of the rows ``xc`` (``loss_sum`` += , ``row_loss`` =); returns the rows' gradient coefficients.  ``logits`` (fp32) are stored only
@@ -74,8 +84,7 @@ def _head_dlogits(xc: torch.Tensor, w: torch.Tensor, tg: torch.Tensor, coef: tor
 class _LinearCEFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, targets, grad_scale, n_valid):
-        x2 = x.reshape(-1, x.shape[-1])
-        tg = targets.reshape(-1).contiguous().long()
+        x2, wm, tg = _head_operands(x, w, targets)
         N, d = x2.shape
         V = w.shape[0]
         loss_sum = torch.zeros(1, dtype=torch.float32, device=x.device)
@@ -85,7 +94,6 @@ class _LinearCEFn(torch.autograd.Function):
         dw_own = None
         if need_grad and mg is None:
             dw_own = torch.zeros((V, d), dtype=torch.float32, device=x.device)
-        x2, wm = _rowmajor2d(x2), _rowmajor2d(w)
         stored = need_grad and d > RECOMPUTE_WIDTH
         logits = torch.empty((min(CHUNK_ROWS, N), V), dtype=torch.float32, device=x.device) if stored else None
         for r0 in range(0, N, CHUNK_ROWS):
@@ -138,16 +146,14 @@ def linear_cross_entropy(x: torch.Tensor, w: torch.Tensor, targets: torch.Tensor
 
 def per_token_nll(x: torch.Tensor, w: torch.Tensor, targets: torch.Tensor, n_valid: int = 0) -> torch.Tensor:
     """Forward-only per-token NLL ``[tokens]`` (per-position perplexity evaluation)."""
-    x2 = x.reshape(-1, x.shape[-1])
-    tg = targets.reshape(-1).contiguous().long()
     if not x.is_cuda:
-        logits = F.linear(x2.float(), w.float())
+        logits = F.linear(x.reshape(-1, x.shape[-1]).float(), w.float())
         if n_valid:
             logits = logits[:, :n_valid]
-        return F.cross_entropy(logits, tg, reduction="none")
+        return F.cross_entropy(logits, targets.reshape(-1).long(), reduction="none")
+    x2, wm, tg = _head_operands(x, w, targets)
     N, V = x2.shape[0], w.shape[0]
     out = torch.empty(N, dtype=torch.float32, device=x.device)
-    x2, wm = _rowmajor2d(x2), _rowmajor2d(w)
     for r0 in range(0, N, CHUNK_ROWS):
         r1 = min(N, r0 + CHUNK_ROWS)
         _head_rows(x2[r0:r1], wm, tg[r0:r1], n_valid or V, 1.0, None, out[r0:r1], False)
