@@ -28,7 +28,8 @@ EPI_BF16, EPI_F32, EPI_F32_ACC, EPI_BF16_GELU, EPI_BF16_SWIGLU = 0, 1, 2, 3, 4
 def _rowmajor2d(t: torch.Tensor) -> torch.Tensor:
     if t.dim() != 2:
         t = t.reshape(-1, t.shape[-1])
-    if t.stride(1) != 1 or (t.stride(0) % 8) or (t.data_ptr() % 16):
+    # a tensor map takes no stride of zero (one row expanded)
+    if t.stride(1) != 1 or (t.stride(0) % 8) or (t.data_ptr() % 16) or not t.stride(0):
         t = t.contiguous()
     return t
 

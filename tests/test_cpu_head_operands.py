@@ -3,6 +3,7 @@ import pytest
 import torch
 
 from context_parallelism_b200 import _native as nv
+from context_parallelism_b200.ops import gemm as G
 from context_parallelism_b200.ops import xent
 
 
@@ -55,3 +56,10 @@ def test_refused_on_another_device(calls):
 def test_accepted(calls, tdtype):
     assert xent.per_token_nll(_t(2, 3, 64), _t(16, 64), torch.zeros(2, 3, dtype=tdtype)).shape == (6,)
     assert calls == ["gemm_head", "xent_rows"]
+
+
+def test_rows_at_one_address():
+    """Rows that are one row expanded are copied out: a tensor map takes no stride of zero."""
+    assert G._rowmajor2d(torch.zeros(1, 64).expand(4, 64)).stride() == (64, 1)
+    for keep in (torch.zeros(4, 64), torch.zeros(4, 72)[:, :64], torch.zeros(1, 64)):
+        assert G._rowmajor2d(keep).data_ptr() == keep.data_ptr()
