@@ -30,8 +30,8 @@
 #include "common.cuh"
 #include <type_traits>
 #include "host_utils.h"
-#include <functional>
-#include <queue>
+#include <algorithm>
+#include <new>
 #include <vector>
 
 #include <stdlib.h>
@@ -624,37 +624,58 @@ extern "C" int cpb_flash_attn_bwd(const void* q, const void* k, const void* v, c
 // (eight), 2 x 4096, 6/2 163 and 99 (two), 16384, 4/1 794 and 422 (two); heads of 128: 1200, 4/1 98 and 32 (eight), 4000, 8/2 302 and 112
 // (four); longest first alone: 8192, 32/8 of 64 956 and 828, of 128 1528 and 1354.  So both ways of
 // handing out the CTAs to the SMs are followed here, with the times that they take.
+// A hand-out that could not win even if it came out even is not followed: 32768 tokens, 32/8 heads took the host 15 ms for 25 of them.
 extern "C" int cpb_flash_bwd_chunk(int B, int Tq, int Tk, int Hq, int Hkv, int D, int causal, int k_off, int local) {
   const int nq = (Tq + 127) / 128, n_kt = (Tk + 127) / 128, G = Hq / (Hkv > 0 ? Hkv : 1), hb = Hkv * B, sms = sm_count();
   if (nq <= 0 || n_kt <= 0 || G <= 0 || hb <= 0 || (D != 64 && D != 128) || (long)n_kt * hb > 16L * sms) return 0;
   const double tile = D == 64 ? 1.25 : 1.9, start_end = D == 64 ? 11.0 : 13.0;          // us, a chip that is not full
-  std::vector<int> len(n_kt);
-  for (int k = 0; k < n_kt; ++k) {
-    // positions that are not 0 .. Tq - 1 (a ring rank's): the share that sees the tile falls evenly, near enough
-    long hidden = !causal ? 0 : local ? ((long)k_off + (long)k * 128) / 128 : (long)nq * k / n_kt;
-    len[k] = G * (int)(nq - (hidden < 0 ? 0 : hidden > nq ? nq : hidden));
-  }
-  const auto finish = [&](int chunk) {
-    std::priority_queue<double, std::vector<double>, std::greater<double>> sm;
-    for (int i = 0; i < sms; ++i) sm.push(0.0);
-    double end = 0.0;
-    const auto run = [&](int pairs) { const double t = sm.top() + start_end + pairs * tile; sm.pop(); sm.push(t); end = t > end ? t : end; };
-    if (chunk == 0) {
-      for (int h = 0; h < hb; ++h) for (int k = 0; k < n_kt; ++k) run(len[k]);
-    } else {
-      for (int c = 0; c < G * nq; c += chunk) for (int k = 0; k < n_kt; ++k) if (len[k] > c) for (int h = 0; h < hb; ++h) run(len[k] - c < chunk ? len[k] - c : chunk);
+  try {
+    std::vector<int> len(n_kt);
+    for (int k = 0; k < n_kt; ++k) {
+      // positions that are not 0 .. Tq - 1 (a ring rank's): the share that sees the tile falls evenly, near enough
+      long hidden = !causal ? 0 : local ? ((long)k_off + (long)k * 128) / 128 : (long)nq * k / n_kt;
+      len[k] = G * (int)(nq - (hidden < 0 ? 0 : hidden > nq ? nq : hidden));
     }
-    return end;
-  };
-  double best = finish(0) * 0.97;
-  int chunk = 0;
-  for (int parts = 1; parts <= 24; ++parts) {                      // one part: whole sweeps, the longest first over all heads
-    const int c = (G * nq + parts - 1) / parts;
-    if (parts > 1 && c < 2) break;
-    long written = 0;                                                // K/V tiles times parts
-    for (int k = 0; k < n_kt; ++k) written += local ? (len[k] + c - 1) / c : parts;
-    const double t = finish(c) + 0.5 + (double)written * hb * 128 * D * 2 * 8 / 4e6;       // written and read at 4 TB/s
-    if (t < best) { best = t; chunk = c; }
+    std::vector<double> sm(sms);                                     // a heap: when each SM is done, the earliest first
+    const auto finish = [&](int chunk) {
+      std::fill(sm.begin(), sm.end(), 0.0);
+      double end = 0.0;
+      const auto run = [&](int pairs) {
+        const double t = sm[0] + start_end + pairs * tile;
+        int at = 0;
+        for (int child; (child = 2 * at + 1) < sms; at = child) {
+          if (child + 1 < sms && sm[child + 1] < sm[child]) ++child;
+          if (sm[child] >= t) break;
+          sm[at] = sm[child];
+        }
+        sm[at] = t;
+        end = t > end ? t : end;
+      };
+      if (chunk == 0) {
+        for (int h = 0; h < hb; ++h) for (int k = 0; k < n_kt; ++k) run(len[k]);
+      } else {
+        for (int c = 0; c < G * nq; c += chunk) for (int k = 0; k < n_kt; ++k) if (len[k] > c) for (int h = 0; h < hb; ++h) run(len[k] - c < chunk ? len[k] - c : chunk);
+      }
+      return end;
+    };
+    double best = finish(0) * 0.97;
+    int chunk = 0;
+    for (int parts = 1; parts <= 24; ++parts) {                      // one part: whole sweeps, the longest first over all heads
+      const int c = (G * nq + parts - 1) / parts;
+      if (parts > 1 && c < 2) break;
+      long written = 0, ctas = 0, pairs = 0;                         // K/V tiles times parts; what there is to do
+      for (int k = 0; k < n_kt; ++k) {
+        written += local ? (len[k] + c - 1) / c : parts;
+        ctas += (len[k] + c - 1) / c;
+        pairs += len[k];
+      }
+      const double rest = 0.5 + (double)written * hb * 128 * D * 2 * 8 / 4e6;                // written and read at 4 TB/s
+      if ((ctas * start_end + pairs * tile) * hb / sms * (1 - 1e-9) + rest >= best) continue;
+      const double t = finish(c) + rest;
+      if (t < best) { best = t; chunk = c; }
+    }
+    return chunk;
+  } catch (const std::bad_alloc&) {
+    return 0;
   }
-  return chunk;
 }
