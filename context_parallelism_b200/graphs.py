@@ -38,9 +38,29 @@ def model_flops(cfg, batch: int, T: int, train: bool) -> float:
     return (3.3 if train else 1.0) * fwd
 
 
-def as_written(obj, cls, *names: str) -> bool:
-    """Whether the methods ``names`` of ``obj`` are those of ``cls``: neither overridden by a subclass nor replaced on the object."""
-    return all(getattr(type(obj), n) is getattr(cls, n) and n not in obj.__dict__ for n in names)
+class Written:
+    """The methods of a model, its blocks and its attention as this package wrote them.  A record runs no Python, so one that holds for
+    anything else (a subclass's method, one replaced on a class or an object, another attention) would leave out what that does."""
+
+    def __init__(self, model_cls, block_cls, attn_cls):
+        self.attn_cls, self.methods = attn_cls, {}
+        for cls, names in ((model_cls, ("hidden", "_hidden", "_block", "head_weight", "loss_with", "loss_sum", "per_token_nll", "recorded_inputs")),
+                           (block_cls, ("pre_attention", "post_attention")), (attn_cls, ("__call__",))):
+            self.methods[cls] = {n: cls.__dict__[n] for n in names}
+        self.model_cls, self.block_cls = model_cls, block_cls
+
+    def _is(self, obj, cls) -> bool:
+        return all(getattr(type(obj), n) is f and n not in obj.__dict__ for n, f in self.methods[cls].items())
+
+    def holds(self, model) -> bool:
+        attn = model.__dict__.get("attn")
+        return (self._is(model, self.model_cls) and type(attn) is self.attn_cls and self._is(attn, self.attn_cls) and attn.ctx.cp_size == 1
+                and all(isinstance(b, self.block_cls) and self._is(b, self.block_cls) for b in model.blocks))
+
+
+def _read(attr):
+    """What a record has read of a module's ``cfg`` or ``attn``: configurations do not change, an attention object has one and a scale."""
+    return attr if not hasattr(attr, "scale") else (attr.cfg, attr.scale, attr.ctx.cp_size)
 
 
 def _plain_call() -> bool:
@@ -62,6 +82,10 @@ def _quiet(p) -> bool:
     return getattr(p, "_grad_ready", None) is None and not p._backward_hooks and not p._post_accumulate_grad_hooks
 
 
+def _same(a, b) -> bool:
+    return a is b or (isinstance(a, tuple) and isinstance(b, tuple) and a[0] is b[0] and a[1:] == b[1:])
+
+
 class Weights:
     """The modules and parameters of a model as a record read them (weak references: a record does not keep its model alive)."""
 
@@ -70,7 +94,7 @@ class Weights:
         self.mods = []
         for m in model.modules():
             parts = [(n, weakref.ref(c)) for n, c in m._modules.items() if c is not None]
-            attrs = [(n, m.__dict__[n]) for n in ("cfg", "attn") if n in m.__dict__]
+            attrs = [(n, _read(m.__dict__[n])) for n in ("cfg", "attn") if n in m.__dict__]
             params = [(n, weakref.ref(p), p.data_ptr(), _main_grad(p)) for n, p in m._parameters.items() if p is not None]
             self.mods.append((weakref.ref(m), parts, attrs, params))
 
@@ -88,7 +112,7 @@ class Weights:
                 if m._modules.get(n) is not c():
                     return False
             for n, v in attrs:
-                if m.__dict__.get(n) is not v:
+                if n not in m.__dict__ or not _same(_read(m.__dict__[n]), v):
                     return False
             for n, r, at, grad in params:
                 p = m._parameters.get(n)

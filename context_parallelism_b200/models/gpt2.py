@@ -92,7 +92,7 @@ class GPT2(nn.Module):
         return out
 
     def hidden(self, idx_local: torch.Tensor, pos: torch.Tensor) -> torch.Tensor:
-        if torch.is_grad_enabled() or self.cp.cp_size > 1:
+        if torch.is_grad_enabled() or not self.recordable():
             return self._hidden(idx_local, pos)
         return self.graphs.run("hidden", self, lambda i, p: (self._hidden(i, p),), (idx_local, pos), self.wte.device,
                                graphs.model_flops(self.cfg, *idx_local.shape, False))[0]
@@ -102,7 +102,8 @@ class GPT2(nn.Module):
         return ()
 
     def recordable(self) -> bool:
-        return self.cp.cp_size == 1 and graphs.as_written(self, GPT2, "hidden", "loss_sum", "per_token_nll")
+        """One GPU, and nothing in a call but what this package wrote."""
+        return self.cp.cp_size == 1 and _WRITTEN.holds(self)
 
     def _hidden(self, idx_local: torch.Tensor, pos: torch.Tensor) -> torch.Tensor:
         cfg = self.cfg
@@ -149,3 +150,6 @@ class GPT2(nn.Module):
                 return xent.per_token_nll(h, self.head_weight(), targets_local, self.cfg.vocab_size).view(idx_local.shape)
             return self.graphs.run("nll", self, nll, (idx_local, targets_local, pos), self.wte.device,
                                    graphs.model_flops(self.cfg, *idx_local.shape, False))[0]
+
+
+_WRITTEN = graphs.Written(GPT2, GPT2Block, CPAttention)

@@ -127,7 +127,7 @@ class Llama(nn.Module):
     # ------------------------------------------------------------------ forward
     def hidden(self, idx_local: torch.Tensor, pos: torch.Tensor) -> torch.Tensor:
         """Final-norm hidden states ``[B, T_local, d]`` for local tokens at global positions ``pos``."""
-        if torch.is_grad_enabled() or self.cp.cp_size > 1:
+        if torch.is_grad_enabled() or not self.recordable():
             return self._hidden(idx_local, pos, *self.recorded_inputs())
         return self.graphs.run("hidden", self, lambda *a: (self._hidden(*a),), (idx_local, pos, *self.recorded_inputs()),
                                self.wte.device, graphs.model_flops(self.cfg, *idx_local.shape, False))[0]
@@ -137,7 +137,8 @@ class Llama(nn.Module):
         return (self.rope_cache,) if self.rope_pos_override is None else (self.rope_cache, self.rope_pos_override)
 
     def recordable(self) -> bool:
-        return self.cp.cp_size == 1 and graphs.as_written(self, Llama, "hidden", "loss_sum", "per_token_nll")
+        """One GPU, and nothing in a call but what this package wrote."""
+        return self.cp.cp_size == 1 and _WRITTEN.holds(self)
 
     def _hidden(self, idx_local: torch.Tensor, pos: torch.Tensor, rope_cache: torch.Tensor,
                 rope_pos: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -190,3 +191,6 @@ class Llama(nn.Module):
                 return xent.per_token_nll(h, self.head_weight(), targets_local, self.cfg.vocab_size).view(idx_local.shape)
             return self.graphs.run("nll", self, nll, (idx_local, targets_local, pos, *self.recorded_inputs()), self.wte.device,
                                    graphs.model_flops(self.cfg, *idx_local.shape, False))[0]
+
+
+_WRITTEN = graphs.Written(Llama, LlamaBlock, CPAttention)

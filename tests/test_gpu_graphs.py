@@ -113,6 +113,51 @@ def test_what_is_not_recorded():
         gc.enable()
 
 
+def _replace(eng, what, seen, monkeypatch):
+    """Put something that counts its calls in the place of a part of the model; returns how often one forward pass calls it."""
+    m = eng.model
+    count = lambda f: lambda *a, **k: (seen.append(1), f(*a, **k))[1]          # noqa: E731
+    if what == "attention":
+        m.attn = count(m.attn)
+        return len(m.blocks)
+    if what == "subclass":
+        m.__class__ = type("Own", (type(m),), {"_hidden": count(type(m)._hidden)})
+        return 1
+    if what == "block":
+        m.blocks[1].pre_attention = count(m.blocks[1].pre_attention)
+        return 1
+    monkeypatch.setattr(type(m.blocks[0]), "post_attention", count(type(m.blocks[0]).post_attention))
+    return len(m.blocks)
+
+
+@pytest.mark.parametrize("what", ["attention", "subclass", "block", "block class"])
+@pytest.mark.parametrize("family", ["llama", "gpt2"])
+def test_what_the_caller_put_into_the_model_runs_every_time(family, what, monkeypatch):
+    eng, seen = _engine(family), []
+    x, y, pos = eng.shard_batch(*_batch(eng, 1))
+    per_pass = _replace(eng, what, seen, monkeypatch)
+    for grad, call in ((False, lambda: eng.model.hidden(x, pos)), (False, lambda: eng.model.per_token_nll(x, y, pos)),
+                       (True, lambda: eng.forward_backward(x, y))):
+        del seen[:]
+        for _ in range(6):
+            with torch.set_grad_enabled(grad):
+                call()
+        assert len(seen) == 6 * per_pass
+    assert not _records(eng)
+
+
+@torch.no_grad()
+def test_another_attention_scale():
+    eng = _engine()
+    x, _, pos = eng.shard_batch(*_batch(eng, 1))
+    first = [eng.model.hidden(x, pos) for _ in range(4)][-1]
+    eng.model.attn.scale *= 2
+    assert torch.equal(eng.model.hidden(x, pos), eng.model._hidden(x, pos, eng.model.rope_cache))
+    eng.model.attn.scale /= 2
+    eng.model.attn = type(eng.model.attn)(eng.cfg, eng.cp)           # another object, the same attention
+    assert torch.equal(eng.model.hidden(x, pos), first)
+
+
 @torch.no_grad()
 def test_more_shapes_than_records(monkeypatch):
     """Shapes met in turn, one more than there is room for: results stay right, and the records lost are made ever less often."""
