@@ -10,6 +10,7 @@ micro-batches of 4 x 1024 tokens 47.7 and 22.6; of GPT-2 124M, two micro-batches
 """
 from __future__ import annotations
 
+import ctypes
 import threading
 import weakref
 from collections import OrderedDict
@@ -123,57 +124,66 @@ class Weights:
         return True
 
 
-class _Record:
-    def __init__(self, fn: Callable, inputs: Sequence[torch.Tensor], weights: Weights, device: torch.device):
-        """Records ``fn(*inputs)``; nothing is executed.  Raises what ``fn`` or the capture raises."""
-        self.weights = weights
-        self.outputs = None
-        self.graph = torch.cuda.CUDAGraph()
+class _Room:
+    """Where the records of a model are made and run: a stream for captures, a private pool of memory, and the end of the last replay."""
+
+    def __init__(self, device: torch.device):
+        self.device = device
+        self.stream = torch.cuda.Stream(device=device)
+        self.pool = torch.cuda.MemPool()
         self.done = torch.cuda.Event()
+
+    def bytes(self) -> int:
+        return sum(seg["total_size"] for seg in self.pool.snapshot())
+
+
+class _Record:
+    def __init__(self, fn: Callable, inputs: Sequence[torch.Tensor], weights: Weights, room: _Room):
+        """Records ``fn(*inputs)``; nothing is executed.  Raises what ``fn`` or the capture raises."""
+        self.weights, self.room = weights, room
+        self.exec = ctypes.c_void_p()
+        stream = torch.cuda.current_stream(room.device)
+        stream.wait_event(room.done)
         with torch.inference_mode(False):
-            self.inputs = [torch.empty(t.shape, dtype=t.dtype, device=device) for t in inputs]
-        side = torch.cuda.Stream(device=device)
-        side.wait_stream(torch.cuda.current_stream(device))
-        before = torch.cuda.memory_reserved(device)
-        launches = nv.LAUNCHES[0]
-        with torch.cuda.stream(side):
-            # thread_local: other threads may allocate and synchronise while this one records
-            self.graph.capture_begin(capture_error_mode="thread_local")
+            self.inputs = [torch.zeros(t.shape, dtype=t.dtype, device=room.device) for t in inputs]
+        room.done.record(stream)
+        lib, launches = nv.lib(), nv.LAUNCHES[0]
+        # the backward pass runs in this thread: the pool and the capture are this thread's
+        with torch.cuda.stream(room.stream), torch.cuda.use_mem_pool(room.pool), torch.autograd.set_multithreading_enabled(False):
+            nv.check(lib.cpb_graph_begin(room.stream.cuda_stream), "graph_begin")
             try:
                 outs = fn(*self.inputs)
             except BaseException:
-                try:
-                    self.graph.capture_end()
-                except RuntimeError:
-                    pass                                             # the capture was invalidated by what fn raised
+                lib.cpb_graph_end(room.stream.cuda_stream, None)
                 raise
             finally:
                 self.launches = nv.LAUNCHES[0] - launches
                 nv.LAUNCHES[0] = launches
-            self.graph.capture_end()
-        self.pool_bytes = torch.cuda.memory_reserved(device) - before
-        self.done.record(torch.cuda.current_stream(device))
+            nv.check(lib.cpb_graph_end(room.stream.cuda_stream, ctypes.byref(self.exec)), "graph_end")
         self.outputs = [o.detach() for o in outs]
+        self.pool_bytes = room.bytes()
 
     def replay(self, inputs: Sequence[torch.Tensor], stream: torch.cuda.Stream) -> Tuple[torch.Tensor, ...]:
-        stream.wait_event(self.done)                                 # the last replay may have run on another stream
+        stream.wait_event(self.room.done)                            # the last replay may have run on another stream
         for s, t in zip(self.inputs, inputs):
             s.copy_(t, non_blocking=True)
-        self.graph.replay()
+        with torch.cuda.device(stream.device_index):
+            nv.check(nv.lib().cpb_graph_launch(self.exec, stream.cuda_stream), "graph_launch")
         nv.LAUNCHES[0] += self.launches
         outs = tuple(o.clone() for o in self.outputs)
-        self.done.record(stream)
+        self.room.done.record(stream)
         return outs
 
     def close(self) -> None:
-        self.done.synchronize()                                      # the buffers may not be given back under a running replay
-        self.outputs = None
-        self.graph.reset()
+        if self.exec:
+            self.room.done.synchronize()                             # the buffers may not be given back under a running replay
+            self.outputs = None
+            nv.lib().cpb_graph_free(self.exec)
+            self.exec = None
 
     def __del__(self):
         try:
-            if self.outputs is not None:
-                self.close()
+            self.close()
         except Exception:                                            # the end of the process
             pass
 
@@ -231,7 +241,7 @@ class GraphCache:
         rec = None
         if free > MIN_FREE_SHARE * total and (not train or Weights.recordable(model)):
             try:
-                rec = _Record(fn, inputs, Weights(model, train), device)
+                rec = _Record(fn, inputs, Weights(model, train), _Room(device))
             except (RuntimeError, nv.NativeError):                   # out of memory, or something in fn that cannot be recorded
                 nv.lib().cpb_clear_error()                           # the call itself has run; its like stay eager from now on
             if rec is not None and rec.pool_bytes > MAX_POOL_BYTES:

@@ -196,3 +196,43 @@ def test_threads_and_streams():
     [t.join(60) for t in ts]
     assert not any(t.is_alive() for t in ts) and not bad and len(_records(eng)) == 1
     eng.check_kernels()
+
+
+@torch.no_grad()
+def test_another_thread_draws_random_numbers_while_one_records():
+    eng, stop, raised = _engine(), threading.Event(), []
+
+    def draw():
+        with torch.cuda.stream(torch.cuda.Stream()):
+            while not stop.is_set():
+                try:
+                    torch.randn(100, device="cuda")
+                except RuntimeError as e:
+                    raised.append(str(e))
+    t = threading.Thread(target=draw, daemon=True)
+    t.start()
+    for T in range(64, 128, 8):
+        x, _, pos = eng.shard_batch(*_batch(eng, T, T=T))
+        want = eng.model._hidden(x, pos, *eng.model.recorded_inputs())
+        assert all(torch.equal(eng.model.hidden(x, pos), want) for _ in range(5))
+    stop.set()
+    t.join(60)
+    assert len(_records(eng)) == 8 and not raised and not t.is_alive()
+
+
+@torch.no_grad()
+def test_a_call_that_cannot_be_recorded():
+    """A capture that fails leaves the call as it was: eager from then on, its like and everything else usable."""
+    from context_parallelism_b200.graphs import GraphCache
+    eng, cache = _engine(), GraphCache()
+    x, _, pos = eng.shard_batch(*_batch(eng, 1))
+
+    def waits(idx):
+        torch.cuda.current_stream().synchronize()                    # not allowed while a stream records
+        return (eng.model._hidden(idx, pos, eng.model.rope_cache),)
+    want = waits(x)[0]
+    for _ in range(5):
+        assert torch.equal(cache.run("waits", eng.model, waits, (x,), eng.device, 0.0)[0], want)
+        assert torch.equal(eng.model.hidden(x, pos), want)
+    assert list(cache._records.values()) == [None] and len(_records(eng)) == 1
+    eng.check_kernels()
