@@ -138,8 +138,7 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  pdl_release();
-  pdl_wait();
+  pdl_wait();                               // and no pdl_release(), see common.cuh
   const uint32_t tmem_base = *tmem_slot;
 
   // first query tile that can see this K/V tile (q_pos is non-decreasing)

@@ -113,8 +113,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (p.ready == nullptr) pdl_release();
-  pdl_wait();
+  pdl_wait();                               // and no pdl_release(), see common.cuh
 
   // Range of K/V tiles this query tile attends to.
   const int q_last = min(q0 + FA_BQ, p.Tq) - 1;

@@ -83,8 +83,7 @@ flash_fwd128_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (p.ready == nullptr) pdl_release();
-  pdl_wait();
+  pdl_wait();                               // and no pdl_release(), see common.cuh
 
   // K/V tiles that each of the two query tiles attends to: 0 .. n_t - 1
   const int qpos_min0 = p.q_pos ? p.q_pos[q0] : q0;
