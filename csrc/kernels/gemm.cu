@@ -372,38 +372,62 @@ gemm_sum_partials_kernel(__nv_bfloat16* __restrict__ C, const float4* __restrict
 // which they finished: weight gradients did not repeat.
 // With all pairs on narrow tiles their operands come to 15 TB/s out of L2 and 64 of K takes 290 instead of 240, 400 instead of 300 (M 3072,
 // N 768, K 4096: 24 us, against 22 in two splits of wide tiles).  bf16 in splits: M 136, N 768, K 3072 14.6 us unsplit, 9.1 in twelve.
-// `want` > 0 asks for the best width at that many splits, 0 for the best of both.
-static void plan_tiles(int M, int N, int K, int epi, int has_aux, int want, int& bn, int& splits) {
+// `want` > 0 asks for the time at that many splits, 0 for the best number of them; -1: no such split.
+static long plan_width(int cand, int M, int N, int K, int epi, int has_aux, int want, int& splits) {
   const long nk = (K + GEMM_BK - 1) / GEMM_BK;
   const long m_tiles = (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM), pairs = sm_count() > 1 ? sm_count() / 2 : 1;
   const long pass = (long)M * N * 8 / 16000;
-  long best = -1;
   const bool sums = epi == EPI_F32_ACC || epi == EPI_BF16;
-  // N = 384 and an A that L2 does not hold: one column of tiles reads A once (us with narrower tiles and with this one: 4096 x 384 x 50304
-  // 150 and 122, 50304 x 384 x 4096 155 and 135).  With two and more columns of tiles its single accumulator costs more than it
-  // saves (4096 x 768 x 50304 217 to 234 and 233 to 255, 50304 x 768 x 4096 238 and 267).
-  const bool one_column = sums && N == 384 && (long)M * K * 2 >= (64L << 20);
-  static const int widths[] = {256, 192, 128, 384};
-  for (const int cand : widths) {
-    if ((cand == 192 && epi == EPI_BF16_SWIGLU) || (cand == 384) != one_column) continue;
-    const int per_tile = epi == EPI_BF16_SWIGLU ? cand / 2 : cand;
-    const long tiles = m_tiles * ((N + per_tile - 1) / per_tile);
-    long ce = epi == EPI_F32 || epi == EPI_F32_ACC ? 1200 : epi == EPI_BF16_GELU ? (has_aux ? 1600 : 1400) : epi == EPI_BF16_SWIGLU ? (has_aux ? 1300 : 1000) : 650;
-    if (cand != 256) ce = ce * cand / 256 + 50;
-    const long max_split = want > 0 ? want : sums ? (nk + 3) / 4 : 1;                   // at least four K blocks per item
-    for (long s = want > 0 ? want : 1; s <= max_split; ++s) {
-      const bool sum16 = epi == EPI_BF16 && s > 1;
-      if (s > 1 && want == 0 && (sum16 ? s : s - 1) * (long)M * N > (32L << 20)) break;        // the workspace
-      const long kps = (nk + s - 1) / s;
-      if ((nk + kps - 1) / kps != s) continue;                       // the same items as a smaller split
-      const long waves = (tiles * s + pairs - 1) / pairs, busy = tiles * s < pairs ? tiles * s : pairs;
-      const long main = kps * (cand == 384 ? 620 : cand == 256 ? 370 : cand == 192 ? (epi == EPI_F32_ACC || sum16 ? 300 + 100 * busy / pairs : 300) : epi == EPI_F32_ACC || sum16 ? 240 + 50 * busy / pairs : 240);
-      const long out = !sum16 ? ce : cand == 256 ? 1200 : 1200 * cand / 256 + 50;
-      // with one accumulator the epilogue is not hidden behind the next item's main loop
-      long t = cand == 384 ? waves * (main + out) : waves * (main > out ? main : out) + (main > out ? out : main);
-      if (s > 1) t += 8000 + (sum16 ? 3 * s + 1 : s + 1) * pass;     // 1.4 us and what a split has to save
-      if (best < 0 || t < best) { best = t; bn = cand; splits = (int)s; }
-    }
+  const int per_tile = epi == EPI_BF16_SWIGLU ? cand / 2 : cand;
+  const long tiles = m_tiles * ((N + per_tile - 1) / per_tile);
+  long ce = epi == EPI_F32 || epi == EPI_F32_ACC ? 1200 : epi == EPI_BF16_GELU ? (has_aux ? 1600 : 1400) : epi == EPI_BF16_SWIGLU ? (has_aux ? 1300 : 1000) : 650;
+  if (cand != 256) ce = ce * cand / 256 + 50;
+  const long max_split = want > 0 ? want : sums ? (nk + 3) / 4 : 1;                     // at least four K blocks per item
+  long best = -1;
+  for (long s = want > 0 ? want : 1; s <= max_split; ++s) {
+    const bool sum16 = epi == EPI_BF16 && s > 1;
+    if (s > 1 && want == 0 && (sum16 ? s : s - 1) * (long)M * N > (32L << 20)) break;          // the workspace
+    const long kps = (nk + s - 1) / s;
+    if ((nk + kps - 1) / kps != s) continue;                         // the same items as a smaller split
+    const long waves = (tiles * s + pairs - 1) / pairs, busy = tiles * s < pairs ? tiles * s : pairs;
+    const long main = kps * (cand == 384 ? 620 : cand == 256 ? 370 : cand == 192 ? (epi == EPI_F32_ACC || sum16 ? 300 + 100 * busy / pairs : 300) : epi == EPI_F32_ACC || sum16 ? 240 + 50 * busy / pairs : 240);
+    const long out = !sum16 ? ce : cand == 256 ? 1200 : 1200 * cand / 256 + 50;
+    // with one accumulator the epilogue is not hidden behind the next item's main loop
+    long t = cand == 384 ? waves * (main + out) : waves * (main > out ? main : out) + (main > out ? out : main);
+    if (s > 1) t += 8000 + (sum16 ? 3 * s + 1 : s + 1) * pass;       // 1.4 us and what a split has to save
+    if (best < 0 || t < best) { best = t; splits = (int)s; }
+  }
+  return best;
+}
+
+// Tiles of 384 columns where N is one column of them and two of the others, and L2 does not hold A: it is read once.  us, the best of
+// the other widths and this one: bf16 4096 x 264 x 50304 144 and 124, x 384 144 and 134; accumulating 50304 x 320 x 4096 151 and 132, x 384
+// 155 and 136; bf16 16384 x 264 x 2048 33.9 and 31.7.  Its one accumulator leaves the epilogue bare, so it wants many K blocks or a single
+// wave (65536 x 384 x 1024 54.3 and 56.4, accumulating 64.5 and 72; 65536 x 384 x 2048 87 and 91), and few large items want full waves (12000
+// x 384 x 4096, 47 items for 74 pairs, 46.1 and 50.2; 20360 x 384 x 2056, 80 items, 50.2 and 54.3) without a split that the others can do
+// without (8192 x 384 x 4096 in two 33.8 and 35.8, 8192 x 384 x 8192 54.3 and 56.3; 4096 x 384 x 8192 in four 39.8 and 37.7).  With two
+// and more columns of tiles it costs more than it saves (4096 x 768 x 50304 217 to 234 and 233 to 255, 50304 x 768 x 4096 238 and 267).
+static bool one_column(int M, int N, int K, int epi) {
+  if ((epi != EPI_F32_ACC && epi != EPI_BF16) || N <= 256 || N > 384 || (long)M * K * 2 < (64L << 20)) return false;
+  const long m_tiles = (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM), pairs = sm_count() > 1 ? sm_count() / 2 : 1;
+  int s = 1;
+  plan_width(384, M, N, K, epi, 0, 0, s);
+  const long waves = (m_tiles * s + pairs - 1) / pairs;
+  return 5 * m_tiles * s >= 4 * pairs * waves && K >= (waves > 1 ? 4096 : 2048) && (s == 1 || 10 * m_tiles < 4 * pairs);
+}
+
+// `want` > 0 asks for the best width at that many splits, 0 for the best of both.
+static void plan_tiles(int M, int N, int K, int epi, int has_aux, int want, int& bn, int& splits) {
+  if (one_column(M, N, K, epi)) {
+    plan_width(bn = 384, M, N, K, epi, has_aux, want, splits);
+    return;
+  }
+  long best = -1;
+  for (const int cand : {256, 192, 128}) {
+    if (cand == 192 && epi == EPI_BF16_SWIGLU) continue;
+    int s = 1;
+    const long t = plan_width(cand, M, N, K, epi, has_aux, want, s);
+    if (t >= 0 && (best < 0 || t < best)) { best = t; bn = cand; splits = s; }
   }
 }
 
