@@ -50,18 +50,32 @@ class Written:
             self.methods[cls] = {n: cls.__dict__[n] for n in names}
         self.model_cls, self.block_cls = model_cls, block_cls
 
-    def _is(self, obj, cls) -> bool:
-        return all(getattr(type(obj), n) is f and n not in obj.__dict__ for n, f in self.methods[cls].items())
+    def _is(self, cls, objects) -> bool:
+        """Whether the methods that count are those of ``cls``, on the objects' types and on the objects."""
+        methods = self.methods[cls]
+        for t in set(map(type, objects)):
+            for n, f in methods.items():
+                if getattr(t, n, None) is not f:
+                    return False
+        names = methods.keys()
+        for o in objects:
+            if not names.isdisjoint(o.__dict__):
+                return False
+        return True
 
     def holds(self, model) -> bool:
         attn = model.__dict__.get("attn")
-        return (self._is(model, self.model_cls) and type(attn) is self.attn_cls and self._is(attn, self.attn_cls) and attn.ctx.cp_size == 1
-                and all(isinstance(b, self.block_cls) and self._is(b, self.block_cls) for b in model.blocks))
+        return (type(attn) is self.attn_cls and attn.ctx.cp_size == 1 and self._is(self.attn_cls, (attn,)) and self._is(self.model_cls, (model,))
+                and self._is(self.block_cls, [*model.blocks]))
 
 
-def _read(attr):
-    """What a record has read of a module's ``cfg`` or ``attn``: configurations do not change, an attention object has one and a scale."""
-    return attr if not hasattr(attr, "scale") else (attr.cfg, attr.scale, attr.ctx.cp_size)
+def _read(module) -> tuple:
+    """What a record reads of a module beside its parameters: a configuration, which does not change, and an attention's, with its scale."""
+    d = module.__dict__
+    if "attn" not in d:
+        return (d.get("cfg"),)
+    attn = d["attn"]
+    return d.get("cfg"), getattr(attn, "cfg", attn), getattr(attn, "scale", None), getattr(getattr(attn, "ctx", None), "cp_size", 1)
 
 
 def _plain_call() -> bool:
@@ -83,8 +97,8 @@ def _quiet(p) -> bool:
     return getattr(p, "_grad_ready", None) is None and not p._backward_hooks and not p._post_accumulate_grad_hooks
 
 
-def _same(a, b) -> bool:
-    return a is b or (isinstance(a, tuple) and isinstance(b, tuple) and a[0] is b[0] and a[1:] == b[1:])
+def _unchanged(a: tuple, b: tuple) -> bool:
+    return a[0] is b[0] and len(a) == len(b) and (len(a) == 1 or (a[1] is b[1] and a[2:] == b[2:]))
 
 
 class Weights:
@@ -95,9 +109,8 @@ class Weights:
         self.mods = []
         for m in model.modules():
             parts = [(n, weakref.ref(c)) for n, c in m._modules.items() if c is not None]
-            attrs = [(n, _read(m.__dict__[n])) for n in ("cfg", "attn") if n in m.__dict__]
             params = [(n, weakref.ref(p), p.data_ptr(), _main_grad(p)) for n, p in m._parameters.items() if p is not None]
-            self.mods.append((weakref.ref(m), parts, attrs, params))
+            self.mods.append((weakref.ref(m), parts, _read(m), params))
 
     @staticmethod
     def recordable(model: torch.nn.Module) -> bool:
@@ -105,21 +118,21 @@ class Weights:
         return all(p.requires_grad and _main_grad(p) and _quiet(p) for p in model.parameters())
 
     def hold(self) -> bool:
-        for ref, parts, attrs, params in self.mods:
+        train = self.train
+        for ref, parts, read, params in self.mods:
             m = ref()
-            if m is None:
+            if m is None or not _unchanged(_read(m), read):
                 return False
+            d = m._modules
             for n, c in parts:
-                if m._modules.get(n) is not c():
+                if d.get(n) is not c():
                     return False
-            for n, v in attrs:
-                if n not in m.__dict__ or not _same(_read(m.__dict__[n]), v):
-                    return False
+            d = m._parameters
             for n, r, at, grad in params:
-                p = m._parameters.get(n)
-                if p is not r() or p is None or p.data_ptr() != at:
+                p = d.get(n)
+                if p is None or p is not r() or p.data_ptr() != at:
                     return False
-                if self.train and not (p.requires_grad and _main_grad(p) == grad and _quiet(p)):
+                if train and not (p.requires_grad and _main_grad(p) == grad and _quiet(p)):
                     return False
         return True
 
@@ -167,8 +180,7 @@ class _Record:
         stream.wait_event(self.room.done)                            # the last replay may have run on another stream
         for s, t in zip(self.inputs, inputs):
             s.copy_(t, non_blocking=True)
-        with torch.cuda.device(stream.device_index):
-            nv.check(nv.lib().cpb_graph_launch(self.exec, stream.cuda_stream), "graph_launch")
+        nv.check(nv.lib().cpb_graph_launch(self.exec, stream.cuda_stream, stream.device_index), "graph_launch")
         nv.LAUNCHES[0] += self.launches
         outs = tuple(o.clone() for o in self.outputs)
         self.room.done.record(stream)

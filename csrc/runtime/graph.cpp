@@ -28,8 +28,13 @@ extern "C" int cpb_graph_end(cudaStream_t stream, void** exec_out) {
   return CPB_OK;
 }
 
-extern "C" int cpb_graph_launch(void* exec, cudaStream_t stream) {
-  CPB_CUDA_OK(cudaGraphLaunch((cudaGraphExec_t)exec, stream));
+extern "C" int cpb_graph_launch(void* exec, cudaStream_t stream, int device) {
+  int current = 0;
+  CPB_CUDA_OK(cudaGetDevice(&current));
+  if (current != device) CPB_CUDA_OK(cudaSetDevice(device));
+  const cudaError_t e = cudaGraphLaunch((cudaGraphExec_t)exec, stream);
+  if (current != device) (void)cudaSetDevice(current);
+  if (e != cudaSuccess) return set_error(CPB_ERR_CUDA, "graph launch: %s", cudaGetErrorString(e));
   return CPB_OK;
 }
 
