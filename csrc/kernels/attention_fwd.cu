@@ -431,9 +431,32 @@ static int make_qkv_tmap(CUtensorMap* m, const void* ptr, int D, int H, int T, i
   return encode_tmap(m, ptr, 2, 4, dims, strides, box, 1);
 }
 
+// Which kernel a forward pass takes: 0 one query tile per CTA (flash_fwd_kernel), 1 two of them (head_dim 128, attention_fwd128.cu), 2 four
+// CTAs per SM with steps of 64 keys (head_dim 64, attention_fwd64.cu).
+//
+// Two query tiles per CTA pay when the sweep over the keys is long (one CTA per SM: its start and end are not hidden; 4096
+// keys, 32/8 heads: 187 us with one tile, 189 to 205 with two; 8192 keys: 615 and 552) and when there are enough CTAs for
+// their unequal lengths to even out (us with one tile and with two: 12000 keys, 188 CTAs 191 and 228; 14336, 224 CTAs 231 and
+// 236; 8192, 224 CTAs 154 and 153; 8192, 256 CTAs 163 and 153; 32768 keys, 256 CTAs 528 and 507).
+//
+// Four CTAs per SM pay when the SMs stay full of them, because each is slower than one of two.  us with two and with four CTAs per SM, 32/8
+// heads: 64 x 300 tokens (41 CTAs for an SM in all) 176 and 111, 40 x 1024 (69) 449 and 331, 5 x 4096 (35) 580 and 511, 3 x 8192 (42) 1193 and 1129,
+// 2 x 12288 (42) 1748 and 1687; one sequence of 8192 (14) 427 and 453, 16384 (28) 1446 and 1466, 32768 (55) 5712 and 5272, 65536 23345 and 22326; 4096
+// queries of 32768 keys, 8/8 heads (2) 472 and 573.
+static int fwd_kernel(int B, int Tq, int Tk, int Hq, int D) {
+  const long tiles = (Tq + FA_BQ - 1) / FA_BQ, ctas = tiles * Hq * B, sms = sm_count();
+  if (D == 128) return Tk >= 8192 && Tq > FA_BQ && 5 * ((tiles + 1) / 2 * Hq * B) >= 8 * sms ? 1 : 0;
+  return ctas >= 32 * sms ? 2 : 0;
+}
+
 }  // namespace cpb
 
 using namespace cpb;
+
+// The kernel that cpb_flash_fwd takes for these sizes (see fwd_kernel); q_positions: it is given q_pos.
+extern "C" int cpb_flash_fwd_plan(int B, int Tq, int Tk, int Hq, int Hkv, int D, int causal, int q_positions) {
+  return fwd_kernel(B, Tq, Tk, Hq, D);
+}
 
 // strides are in elements: (head, token, batch) for q and for k/v (k and v share strides).
 extern "C" int cpb_flash_fwd(const void* q, const void* k, const void* v, void* o, float* lse,
@@ -451,11 +474,8 @@ extern "C" int cpb_flash_fwd(const void* q, const void* k, const void* v, void* 
   CUtensorMap tq, tk, tv;
   int rc;
   if ((rc = make_qkv_tmap(&tq, q, D, Hq, Tq, B, q_sh, q_st, q_sb, FA_BQ)) != CPB_OK) return rc;
-  // head_dim 64: four CTAs per SM with steps of 64 keys (attention_fwd64.cu) pay when the SMs stay full of them, because each is slower
-  // than one of two: us with two and with four, 32/8 heads, keys 8192 (2048 CTAs) 427 and 453, 16384 (4096) 1446 and 1466, 32768 (8192)
-  // 5712 and 5272, 65536 (16384) 23345 and 22326; 4096 queries of 32768 keys, 8/8 heads (256) 472 and 573.
-  const bool four = D == 64 && (long)((Tq + FA_BQ - 1) / FA_BQ) * Hq * B >= 32L * sm_count();
-  const int kv_rows = four ? 64 : FA_BK;
+  const int kernel = fwd_kernel(B, Tq, Tk, Hq, D);
+  const int kv_rows = kernel == 2 ? 64 : FA_BK;
   if ((rc = make_qkv_tmap(&tk, k, D, Hkv, Tk, B, k_sh, k_st, k_sb, kv_rows)) != CPB_OK) return rc;
   if ((rc = make_qkv_tmap(&tv, v, D, Hkv, Tk, B, k_sh, k_st, k_sb, kv_rows)) != CPB_OK) return rc;
   FwdParams p;
@@ -471,13 +491,8 @@ extern "C" int cpb_flash_fwd(const void* q, const void* k, const void* v, void* 
   // default and is read once.
   static const int poly_env = [] { const char* e = getenv("CPB_FWD_POLY"); return e ? atoi(e) : -1; }();
   const int poly = poly_env < 0 ? (D == 64 ? FA_POLY_D64 : FA_POLY_D128) : poly_env;
-  // Two query tiles per CTA pay when the sweep over the keys is long (one CTA per SM: its start and end are not hidden; 4096
-  // keys, 32/8 heads: 187 us with one tile, 189 to 205 with two; 8192 keys: 615 and 552) and when there are enough CTAs for
-  // their unequal lengths to even out (us with one tile and with two: 12000 keys, 188 CTAs 191 and 228; 14336, 224 CTAs 231 and
-  // 236; 8192, 224 CTAs 154 and 153; 8192, 256 CTAs 163 and 153; 32768 keys, 256 CTAs 528 and 507).
-  const long pairs = (long)((Tq + 2 * FA_BQ - 1) / (2 * FA_BQ)) * Hq * B;
-  if (D == 128 && Tk >= 8192 && Tq > FA_BQ && 5 * pairs >= 8 * sm_count()) return launch_flash_fwd128_pair(poly, tq, tk, tv, p, stream);
-  if (four) return launch_flash_fwd64(poly, tq, tk, tv, p, stream);
+  if (kernel == 1) return launch_flash_fwd128_pair(poly, tq, tk, tv, p, stream);
+  if (kernel == 2) return launch_flash_fwd64(poly, tq, tk, tv, p, stream);
   const int G = Hq / Hkv;
   dim3 grid(p.n_copy + ((Tq + FA_BQ - 1) / FA_BQ) * G, Hkv, B);
 #define CPB_FWD_LAUNCH(DD, PP)                                                                                         \

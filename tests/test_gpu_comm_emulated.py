@@ -224,6 +224,61 @@ def test_fused_ulysses_emulated_two_query_tiles(B, T, hq, hkv):
         assert_close(lse[:, h:h + 1], wlse, cos=0.99999, rel=1e-3, name=f"ulysses lse head {h}")
 
 
+# ------------------------------------------------------------------- many CTAs: four per SM, steps of 64 keys (head_dim 64)
+@pytest.mark.parametrize("n,chunk,hq,hkv,B", [(4, 328, 32, 2, 25), (2, 512, 32, 4, 19)])
+def test_fused_ring_emulated_four_ctas_per_sm(n, chunk, hq, hkv, B):
+    """Copy CTAs, flags and the wrapped sweep where ``cpb_flash_fwd`` takes the kernel with four CTAs per SM: chunks of 5 1/8 steps (one
+    straddles the chunks' border, and the sweep starts at the first key) and of eight (it starts at the tile's own chunk)."""
+    from context_parallelism_b200 import _native as nv
+    from context_parallelism_b200.ops import reference as R
+    from context_parallelism_b200.parallel import fused as F
+    from context_parallelism_b200.parallel import shard
+    torch.manual_seed(n + chunk)
+    T, D = 2 * n * chunk, 64
+    Tl, scale = T // n, D ** -0.5
+    assert nv.lib().cpb_flash_fwd_plan(B, Tl, T, hq, hkv, D, 1, 1) == 2
+    cfg, fcs = make_comms(n, "ring", heap_mb=128)
+    q, k, v = (torch.randn(B, T, h, D, device=dev()).bfloat16() for h in (hq, hkv, hkv))
+    pos = [shard.local_positions(T, n, r, True).to(dev()) for r in range(n)]
+    loc = lambda t, r: t.index_select(1, pos[r]).contiguous()        # noqa: E731
+    st = [F.ring_fwd_publish(fcs[r], loc(k, r), loc(v, r)) for r in range(n)]
+    for r in (0, n - 1):
+        o, lse = F.ring_fwd_compute(fcs[r], st[r][0], st[r][1], loc(q, r), pos[r].int(), scale)
+        status_ok()
+        assert torch.equal(st[r][0].gathered[0].view_as(k), k) and torch.equal(st[r][0].gathered[1].view_as(v), v)
+        o2, lse2 = F.ring_fwd_settled(fcs[r], st[r][0], loc(q, r), pos[r].int(), scale)
+        assert torch.equal(o, o2) and torch.equal(lse, lse2)
+        for h in range(0, hq, 8):                                     # the dense result a few heads at a time
+            kv = slice(h * hkv // hq, h * hkv // hq + 1)
+            want, wlse = R.attention_dense(loc(q, r)[:, :, h:h + 1].float(), k[:, :, kv].float(), v[:, :, kv].float(), scale, q_pos=pos[r], causal=True)
+            assert_close(o[:, :, h:h + 1].float(), want, cos=0.9995, rel=3e-2, name=f"ring out rank {r} head {h}")
+            assert_close(lse[:, h:h + 1], wlse, cos=0.99999, rel=1e-3, name=f"ring lse rank {r} head {h}")
+
+
+def test_fused_ulysses_emulated_four_ctas_per_sm():
+    """The scatter epilogue of the kernel with four CTAs per SM: a batch, and rows of one tile in two owners' arenas."""
+    from context_parallelism_b200 import _native as nv
+    from context_parallelism_b200.ops import reference as R
+    from context_parallelism_b200.parallel import fused as F
+    torch.manual_seed(3)
+    n, B, T, hq, hkv, D = 2, 33, 1032, 32, 4, 64
+    Tl, scale = T // n, D ** -0.5
+    assert nv.lib().cpb_flash_fwd_plan(B, T, T, hq // n, hkv // n, D, 1, 0) == 2
+    cfg, fcs = make_comms(n, "ulysses", heap_mb=1024)
+    q, k, v = (torch.randn(B, T, h, D, device=dev()).bfloat16() for h in (hq, hkv, hkv))
+    loc = lambda t, r: t[:, r * Tl:(r + 1) * Tl].clone(memory_format=torch.contiguous_format)        # noqa: E731
+    st = [F.uly_fwd_push(fcs[r], loc(q, r), loc(k, r), loc(v, r)) for r in range(n)]
+    lses = [F.uly_fwd_compute(fcs[r], st[r][0], st[r][1], scale) for r in range(n)]
+    status_ok()
+    out = torch.cat([st[r][0].o_view(fcs[r], st[r][1]) for r in range(n)], 1)
+    lse = torch.cat(lses, 1)
+    for h in range(0, hq, 5):
+        kv = slice(h * hkv // hq, h * hkv // hq + 1)
+        want, wlse = R.attention_dense(q[:, :, h:h + 1].float(), k[:, :, kv].float(), v[:, :, kv].float(), scale, causal=True)
+        assert_close(out[:, :, h:h + 1].float(), want, cos=0.9995, rel=3e-2, name=f"ulysses out head {h}")
+        assert_close(lse[:, h:h + 1], wlse, cos=0.99999, rel=1e-3, name=f"ulysses lse head {h}")
+
+
 # ----------------------------------------------------------------------------------------------------- gradient transport
 def _tiny_params(seed):
     g = torch.Generator().manual_seed(seed)
