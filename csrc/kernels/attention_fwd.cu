@@ -442,11 +442,15 @@ static int make_qkv_tmap(CUtensorMap* m, const void* ptr, int D, int H, int T, i
 // Four CTAs per SM pay when the SMs stay full of them, because each is slower than one of two.  us with two and with four CTAs per SM, 32/8
 // heads: 64 x 300 tokens (41 CTAs for an SM in all) 176 and 111, 40 x 1024 (69) 449 and 331, 5 x 4096 (35) 580 and 511, 3 x 8192 (42) 1193 and 1129,
 // 2 x 12288 (42) 1748 and 1687; one sequence of 8192 (14) 427 and 453, 16384 (28) 1446 and 1466, 32768 (55) 5712 and 5272, 65536 23345 and 22326; 4096
-// queries of 32768 keys, 8/8 heads (2) 472 and 573.
-static int fwd_kernel(int B, int Tq, int Tk, int Hq, int D) {
+// queries of 32768 keys, 8/8 heads (2) 472 and 573.  A long causal sequence with few K/V heads ends with the CTAs of its last one: 18944 (32) 1912
+// and 1964, 20480 (35) 2315 and 2356, 22000 (37) 2671 and 2690, 23000 (39) 2914 and 2913, 24576 (42) 3334 and 3305, 28672 (48) 4511 and 4409;
+// not with more of them, without the mask or at a ring rank's positions (4 x 20480, 8/8 (35) 2473 and 2407; 20480 without the mask 4626 and 4510;
+// 20000 of 40000 keys in two chunks (34) 4223 and 4083).
+static int fwd_kernel(int B, int Tq, int Tk, int Hq, int Hkv, int D, int causal, bool q_pos) {
   const long tiles = (Tq + FA_BQ - 1) / FA_BQ, ctas = tiles * Hq * B, sms = sm_count();
   if (D == 128) return Tk >= 8192 && Tq > FA_BQ && 5 * ((tiles + 1) / 2 * Hq * B) >= 8 * sms ? 1 : 0;
-  return ctas >= 32 * sms ? 2 : 0;
+  const bool uneven = causal && !q_pos && Tk > 16384 && Hkv * B < 16;
+  return ctas >= (uneven ? 40 : 32) * sms ? 2 : 0;
 }
 
 }  // namespace cpb
@@ -455,7 +459,7 @@ using namespace cpb;
 
 // The kernel that cpb_flash_fwd takes for these sizes (see fwd_kernel); q_positions: it is given q_pos.
 extern "C" int cpb_flash_fwd_plan(int B, int Tq, int Tk, int Hq, int Hkv, int D, int causal, int q_positions) {
-  return fwd_kernel(B, Tq, Tk, Hq, D);
+  return fwd_kernel(B, Tq, Tk, Hq, Hkv, D, causal, q_positions != 0);
 }
 
 // strides are in elements: (head, token, batch) for q and for k/v (k and v share strides).
@@ -474,7 +478,7 @@ extern "C" int cpb_flash_fwd(const void* q, const void* k, const void* v, void* 
   CUtensorMap tq, tk, tv;
   int rc;
   if ((rc = make_qkv_tmap(&tq, q, D, Hq, Tq, B, q_sh, q_st, q_sb, FA_BQ)) != CPB_OK) return rc;
-  const int kernel = fwd_kernel(B, Tq, Tk, Hq, D);
+  const int kernel = fwd_kernel(B, Tq, Tk, Hq, Hkv, D, causal, q_pos != nullptr);
   const int kv_rows = kernel == 2 ? 64 : FA_BK;
   if ((rc = make_qkv_tmap(&tk, k, D, Hkv, Tk, B, k_sh, k_st, k_sb, kv_rows)) != CPB_OK) return rc;
   if ((rc = make_qkv_tmap(&tv, v, D, Hkv, Tk, B, k_sh, k_st, k_sb, kv_rows)) != CPB_OK) return rc;
