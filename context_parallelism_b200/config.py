@@ -74,6 +74,7 @@ KNOWN_ENV = {
     "CP_RING_SIZE", "CP_HYBRID_GQA",
     # this framework's additions
     "CP_FUSED", "CP_WATCHDOG_S", "CP_NVLS", "CP_GRAD_BUCKET_MB", "CP_DKV_MODE", "CP_SHARD_OPTIM", "CP_AR_CTAS",
+    "CP_GRAPH_POOL_MB",
     "CP_FUSED_HYBRID_ULYSSES", "CP_LOAD_BALANCE", "CP_INIT_DEVICE", "CP_TEST_LOG_DIR", "CP_NATIVE_PG",
 }
 
@@ -205,6 +206,7 @@ class Config:
     shard_optim: bool = True            # fused transport: reduce-scatter -> AdamW on the owned slice -> all-gather
     load_balance_ring: bool = True      # HeadTail sharding on the ring axis; False = contiguous shards
     grad_bucket_mb: int = 25
+    graph_pool_mb: int = 4096           # memory that a model's recorded calls may keep; 0: nothing is recorded
     nvls: bool = False
     watchdog_s: float = 600.0
     # context extension
@@ -377,6 +379,7 @@ def _common(env, world_size):
         shard_optim=_flag(env, "CP_SHARD_OPTIM", True),
         load_balance_ring=_flag(env, "CP_LOAD_BALANCE", True),
         grad_bucket_mb=_int(env, "CP_GRAD_BUCKET_MB", 25),
+        graph_pool_mb=_int(env, "CP_GRAPH_POOL_MB", 4096),
         nvls=_flag(env, "CP_NVLS", False),
         watchdog_s=_float(env, "CP_WATCHDOG_S", 600.0),
         data_root=_str(env, "CP_DATA_ROOT", ""),

@@ -20,9 +20,9 @@ import torch
 
 from . import _native as nv
 
-MAX_RECORDS = 8                  # per model; the one used longest ago makes room
+MAX_RECORDS = 32                 # per model; the one used longest ago makes room
 EAGER_CALLS = 3                  # calls with new shapes that run as they always did; twice as many each time that the record was lost
-MAX_POOL_BYTES = 8 << 30         # buffers of all records of a model
+MAX_POOL_BYTES = 4 << 30         # buffers of all records of a model, unless its configuration says otherwise (graph_pool_mb)
 MIN_FREE_SHARE = 0.25            # share of the GPU's memory that has to be free before a record is made
 # A call is recorded while the GPU needs less time for it than the host: a launch costs the host about 25 us (forward and backward;
 # 13 us without autograd), the kernels of such models reach about 600 TFLOP/s.
@@ -138,7 +138,8 @@ class Weights:
 
 
 class _Room:
-    """Where the records of a model are made and run: a stream for captures, a private pool of memory, and the end of the last replay."""
+    """Where the records of a model are made and run: a stream for captures, a pool of memory and the end of the last replay.  Replays
+    run one after the other and their results are copied out, so all records of a model work in the same memory."""
 
     def __init__(self, device: torch.device):
         self.device = device
@@ -148,6 +149,13 @@ class _Room:
 
     def bytes(self) -> int:
         return sum(seg["total_size"] for seg in self.pool.snapshot())
+
+    def short(self) -> bool:
+        """Whether less of the GPU's memory is free, or kept by torch for the next allocation, than a record is made with."""
+        free, total = torch.cuda.mem_get_info(self.device)
+        if free < MIN_FREE_SHARE * total:
+            free += torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device) - self.bytes()
+        return free < MIN_FREE_SHARE * total
 
 
 class _Record:
@@ -174,7 +182,6 @@ class _Record:
                 nv.LAUNCHES[0] = launches
             nv.check(lib.cpb_graph_end(room.stream.cuda_stream, ctypes.byref(self.exec)), "graph_end")
         self.outputs = [o.detach() for o in outs]
-        self.pool_bytes = room.bytes()
 
     def replay(self, inputs: Sequence[torch.Tensor], stream: torch.cuda.Stream) -> Tuple[torch.Tensor, ...]:
         stream.wait_event(self.room.done)                            # the last replay may have run on another stream
@@ -202,25 +209,28 @@ class _Record:
 
 class GraphCache:
     """The records of one model, by name, input shapes and modes.  Safe with several threads and streams: a lock covers the copies in,
-    the replay and the copies out, and an event orders replays of different streams."""
+    the replay and the copies out, and an event orders replays of different streams.  ``limit``: bytes that the records' buffers may
+    take together, 0 to record nothing."""
 
-    def __init__(self):
+    def __init__(self, limit: int = MAX_POOL_BYTES):
+        self.limit = limit
         self._lock = threading.Lock()
+        self._room: Optional[_Room] = None                           # there while there are records
         self._records: "OrderedDict[tuple, Optional[_Record]]" = OrderedDict()
         self._seen: "OrderedDict[tuple, int]" = OrderedDict()        # eager calls since the record was lost, or at all
         self._lost: "OrderedDict[tuple, int]" = OrderedDict()        # how often it was
 
     def __reduce__(self):                                            # a copied or unpickled model starts without records
-        return GraphCache, ()
+        return GraphCache, (self.limit,)
 
     def __deepcopy__(self, memo):
-        return GraphCache()
+        return GraphCache(self.limit)
 
     def run(self, name: str, model: torch.nn.Module, fn: Callable, inputs: Sequence[torch.Tensor], device: torch.device,
             flops: float, train: bool = False) -> Tuple[torch.Tensor, ...]:
         """``fn(*inputs)`` with the inputs on ``device``: a tuple of tensors."""
-        if device.type != "cuda" or not _plain_call() or any(t.requires_grad for t in inputs):
-            return self._eager(fn, inputs, device)
+        if device.type != "cuda" or self.limit <= 0 or not _plain_call() or any(t.requires_grad for t in inputs):
+            return self._eager(fn, inputs, device, train)
         from .ops import attention
         key = (name, device.index, train, torch.is_inference_mode_enabled(), attention.FP32_ACCURATE,
                *((t.dtype, tuple(t.shape)) for t in inputs))
@@ -232,7 +242,7 @@ class GraphCache:
                     return rec.replay(inputs, torch.cuda.current_stream(device))
                 self._drop(key)
         launches = nv.LAUNCHES[0]
-        outs = self._eager(fn, inputs, device)
+        outs = self._eager(fn, inputs, device, train)
         launches = nv.LAUNCHES[0] - launches
         with self._lock:
             if key not in self._records:
@@ -244,30 +254,52 @@ class GraphCache:
                     self._record(key, model, fn, inputs, device, flops < GPU_TFLOPS * 1e6 * HOST_US_PER_LAUNCH * launches, train)
         return outs
 
-    @staticmethod
-    def _eager(fn, inputs, device):
-        return tuple(fn(*(t if t.device == device else t.to(device, non_blocking=True) for t in inputs)))
+    def _eager(self, fn, inputs, device, train: bool):
+        """The call without a record.  The records' memory is given back when it runs short: before a backward pass, which cannot be run
+        again once it has added to the gradients, and when a forward pass has found no memory."""
+        call = lambda: tuple(fn(*(t if t.device == device else t.to(device, non_blocking=True) for t in inputs)))      # noqa: E731
+        room = self._room
+        if room is None:
+            return call()
+        if train:
+            if room.short():
+                with self._lock:
+                    self._drop_all()
+            return call()
+        try:
+            return call()
+        except torch.OutOfMemoryError:
+            pass
+        with self._lock:
+            self._drop_all()
+        return call()
 
     def _record(self, key, model, fn, inputs, device, launch_bound: bool, train: bool) -> None:
         free, total = torch.cuda.mem_get_info(device) if launch_bound else (0, 1)
         rec = None
         if free > MIN_FREE_SHARE * total and (not train or Weights.recordable(model)):
+            if self._room is None or self._room.device != device:
+                self._drop_all()
+                self._room = _Room(device)
             try:
-                rec = _Record(fn, inputs, Weights(model, train), _Room(device))
+                rec = _Record(fn, inputs, Weights(model, train), self._room)
             except (RuntimeError, nv.NativeError):                   # out of memory, or something in fn that cannot be recorded
                 nv.lib().cpb_clear_error()                           # the call itself has run; its like stay eager from now on
-            if rec is not None and rec.pool_bytes > MAX_POOL_BYTES:
+            if rec is not None and self._room.bytes() > self.limit:
                 rec.close()
                 rec = None
+                self._drop_all()
         self._records[key] = rec                                     # None: not to be tried again
         while True:
-            held = [(k, r.pool_bytes) for k, r in self._records.items() if r is not None]
-            if len(held) > MAX_RECORDS or sum(b for _, b in held) > MAX_POOL_BYTES:
-                self._drop(held[0][0])
-            elif len(self._records) > 64:
+            held = [k for k, r in self._records.items() if r is not None]
+            if len(held) > MAX_RECORDS:
+                self._drop(held[0])
+            elif len(self._records) > 128:
                 self._drop(next(iter(self._records)))
             else:
                 break
+        if not held:
+            self._room = None
 
     def _drop(self, key) -> None:
         rec = self._records.pop(key)
@@ -276,11 +308,17 @@ class GraphCache:
             self._lost[key] = self._lost.pop(key, 0) + 1
             while len(self._lost) > 64:
                 self._lost.popitem(last=False)
+            if all(r is None for r in self._records.values()):
+                self._room = None
+
+    def _drop_all(self) -> None:
+        for key in [k for k, r in self._records.items() if r is not None]:
+            self._drop(key)
 
     def clear(self) -> None:
         """Give back every record and its memory."""
         with self._lock:
-            while self._records:
-                self._drop(next(iter(self._records)))
+            self._drop_all()
+            self._records.clear()
             self._seen.clear()
             self._lost.clear()

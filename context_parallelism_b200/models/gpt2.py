@@ -71,7 +71,7 @@ class GPT2(nn.Module):
             _padded_normal(cfg.vocab_size, cfg.vocab_padded, d, gen))
         self.to(device)
         self.attn = CPAttention(cfg, self.cp)
-        self.graphs = graphs.GraphCache()
+        self.graphs = graphs.GraphCache(cfg.graph_pool_mb << 20)
 
     def named_tensors(self) -> Dict[str, torch.Tensor]:
         """Parameters under the names of the named-init files: each block's first LayerNorm lives inside its

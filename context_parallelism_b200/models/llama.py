@@ -91,7 +91,7 @@ class Llama(nn.Module):
         self.attn = CPAttention(cfg, self.cp)
         self.rope_cache = R.build_rope_cache(cfg.T, cfg.head_dim, cfg.rope_theta, device, cfg.yarn)
         self.rope_pos_override: Optional[torch.Tensor] = None
-        self.graphs = graphs.GraphCache()
+        self.graphs = graphs.GraphCache(cfg.graph_pool_mb << 20)
 
     # ------------------------------------------------------------------ RoPE cache control
     def set_rope_cache(self, cache: torch.Tensor) -> None:

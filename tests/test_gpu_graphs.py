@@ -236,3 +236,75 @@ def test_a_call_that_cannot_be_recorded():
         assert torch.equal(eng.model.hidden(x, pos), want)
     assert list(cache._records.values()) == [None] and len(_records(eng)) == 1
     eng.check_kernels()
+
+
+@torch.no_grad()
+def test_records_share_memory_and_give_it_back():
+    """Records of different calls in one pool, replayed in turn and on two streams, keep their results apart."""
+    eng = _engine(vocab_size=8000)
+    cases = [eng.shard_batch(*_batch(eng, i, T=T)) for i, T in enumerate((200, 192, 128))]
+    want = [(eng.model._hidden(x, p, *eng.model.recorded_inputs()), eng.model.per_token_nll(x, y, p)) for x, y, p in cases]
+    before, other, sizes = torch.cuda.memory_reserved(), torch.cuda.Stream(), []
+    torch.cuda.synchronize()
+    for i in range(12):
+        with torch.cuda.stream(other if i % 2 else torch.cuda.current_stream()):
+            got = [(eng.model.hidden(x, p), eng.model.per_token_nll(x, y, p)) for x, y, p in cases]
+        torch.cuda.synchronize()
+        assert all(torch.equal(g, w) for pair, ref in zip(got, want) for g, w in zip(pair, ref))
+        sizes += [eng.model.graphs._room.bytes()] if eng.model.graphs._room else []
+    assert len(_records(eng)) == 6 and len({id(r.room) for r in _records(eng)}) == 1
+    assert sizes[-1] <= 64 << 20                                     # in pools of their own each would have segments of 2 and 20 MB
+    eng.close()
+    assert eng.model.graphs._room is None and torch.cuda.memory_reserved() <= before + (40 << 20)
+
+
+@torch.no_grad()
+def test_limit_of_the_records_memory():
+    for mb, made in ((0, False), (1, False), (4096, True)):
+        eng = _engine(graph_pool_mb=mb)
+        x, y, pos = eng.shard_batch(*_batch(eng, 1))
+        want = eng.model._hidden(x, pos, *eng.model.recorded_inputs())
+        assert all(torch.equal(eng.model.hidden(x, pos), want) for _ in range(5))
+        assert bool(_records(eng)) == made == (eng.model.graphs._room is not None)
+
+
+def test_memory_is_given_back_when_it_runs_short(monkeypatch):
+    from context_parallelism_b200 import graphs
+    eng, left = _engine(), [1]
+    x, y, pos = eng.shard_batch(*_batch(eng, 1))
+    with torch.no_grad():
+        for _ in range(3):
+            eng.model.hidden(x, pos)
+        assert len(_records(eng)) == 1
+
+        def full(idx):
+            if left:
+                left.pop()
+                raise torch.OutOfMemoryError("full")
+            return (idx + len(_records(eng)),)
+        assert torch.equal(eng.model.graphs.run("full", eng.model, full, (x,), eng.device, 0.0)[0], x)          # run again without records
+        for _ in range(12):
+            eng.model.hidden(x, pos)
+        assert len(_records(eng)) == 1
+    eng.forward_backward(*_batch(eng, 2))
+    assert len(_records(eng)) == 1                                   # memory is plenty
+    monkeypatch.setattr(graphs, "MIN_FREE_SHARE", 2.0)
+    eng.forward_backward(*_batch(eng, 3))
+    assert not _records(eng) and eng.model.graphs._room is None
+    eng.check_kernels()
+
+
+def test_generation_keeps_its_records(monkeypatch):
+    """The trainers' generation loop meets each padded length eight times and puts an attention of its own into the model for every call."""
+    from context_parallelism_b200 import graphs
+    from context_parallelism_b200.trainers.gpt2_cp import generate
+    eng, made = _engine("gpt2"), []
+    init = graphs._Record.__init__
+    monkeypatch.setattr(graphs._Record, "__init__", lambda self, *a: (made.append(1), init(self, *a))[1])
+    prompt = torch.randint(0, 1000, (1, 20), generator=torch.Generator().manual_seed(1))
+    first, after = generate(eng, prompt, 96), len(made)
+    assert after >= 11                                               # lengths of 24 to 120; the record of one that was met twice is not made
+    for _ in range(2):
+        assert torch.equal(generate(eng, prompt, 96), first)
+    assert len(made) <= after + 1
+    eng.check_kernels()
