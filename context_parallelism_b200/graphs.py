@@ -17,6 +17,7 @@ from collections import OrderedDict
 from typing import Callable, Optional, Sequence, Tuple
 
 import torch
+from torch.autograd import forward_ad
 
 from . import _native as nv
 
@@ -78,13 +79,27 @@ def _read(module) -> tuple:
     return d.get("cfg"), getattr(attn, "cfg", attn), getattr(attn, "scale", None), getattr(getattr(attn, "ctx", None), "cp_size", 1)
 
 
+def _listeners():
+    """What only private names of torch tell about who is listening; None where one is missing, and nothing is recorded then."""
+    try:
+        forward_ad._current_level
+        return (torch._C._len_torch_dispatch_stack, torch._C._len_torch_function_stack, torch._C._functorch.peek_interpreter_stack,
+                torch._C._autograd._top_saved_tensors_default_hooks)
+    except AttributeError:
+        return None
+
+
+_LISTENERS = _listeners()
+
+
 def _plain_call() -> bool:
     """Whether nothing is listening that a replay would pass by: a capture, a mode, a tracer, saved-tensor hooks, a launch timer."""
+    if _LISTENERS is None:
+        return False
+    dispatch_modes, function_modes, transforms, saved_tensor_hooks = _LISTENERS
     return not (torch.cuda.is_current_stream_capturing() or nv._PROFILE is not None or torch.is_anomaly_enabled()
-                or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack()
-                or torch._C._functorch.peek_interpreter_stack() is not None or torch.jit.is_tracing()
-                or torch._C._autograd._top_saved_tensors_default_hooks(True) is not None
-                or torch.autograd.forward_ad._current_level >= 0)
+                or dispatch_modes() or function_modes() or transforms() is not None or torch.jit.is_tracing()
+                or saved_tensor_hooks(True) is not None or forward_ad._current_level >= 0)
 
 
 def _main_grad(p) -> int:
