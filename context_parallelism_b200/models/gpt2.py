@@ -111,13 +111,15 @@ class GPT2(nn.Module):
         pending = None
         use_ckpt = cfg.recompute in ("selective", "full") and torch.is_grad_enabled()
         full = cfg.recompute == "full" and torch.is_grad_enabled()
+        # this package's blocks draw no random numbers, and keeping the generators' states for each part costs the host more than its launches
+        draws = use_ckpt and not _WRITTEN.holds(self)
         for blk in self.blocks:
             if full:
-                x, pending = checkpoint(self._block, blk, x, pending, pos, use_reentrant=False, preserve_rng_state=False)
+                x, pending = checkpoint(self._block, blk, x, pending, pos, use_reentrant=False, preserve_rng_state=draws)
             elif use_ckpt:
-                x, qkv = checkpoint(blk.pre_attention, x, pending, use_reentrant=False, preserve_rng_state=False)
+                x, qkv = checkpoint(blk.pre_attention, x, pending, use_reentrant=False, preserve_rng_state=draws)
                 o = self.attn(qkv, pos)
-                x, pending = checkpoint(blk.post_attention, x, o, use_reentrant=False, preserve_rng_state=False)
+                x, pending = checkpoint(blk.post_attention, x, o, use_reentrant=False, preserve_rng_state=draws)
             else:
                 x, qkv = blk.pre_attention(x, pending)
                 o = self.attn(qkv, pos)

@@ -148,15 +148,17 @@ class Llama(nn.Module):
         rpos = pos if rope_pos is None else rope_pos
         use_ckpt = cfg.recompute in ("selective", "full") and torch.is_grad_enabled()
         full = cfg.recompute == "full" and torch.is_grad_enabled()
+        # this package's blocks draw no random numbers, and keeping the generators' states for each part costs the host more than its launches
+        draws = use_ckpt and not _WRITTEN.holds(self)
         for blk in self.blocks:
             if full:
                 # full activation recompute: only the block's input survives the forward pass; backward re-runs the
                 # whole block, context-parallel attention (and its communication) included, on every rank alike
-                x, pending = checkpoint(self._block, blk, x, pending, rope_cache, rpos, pos, use_reentrant=False, preserve_rng_state=False)
+                x, pending = checkpoint(self._block, blk, x, pending, rope_cache, rpos, pos, use_reentrant=False, preserve_rng_state=draws)
             elif use_ckpt:
-                x, qkv = checkpoint(blk.pre_attention, x, pending, rope_cache, rpos, use_reentrant=False, preserve_rng_state=False)
+                x, qkv = checkpoint(blk.pre_attention, x, pending, rope_cache, rpos, use_reentrant=False, preserve_rng_state=draws)
                 o = self.attn(qkv, pos)
-                x, pending = checkpoint(blk.post_attention, x, o, use_reentrant=False, preserve_rng_state=False)
+                x, pending = checkpoint(blk.post_attention, x, o, use_reentrant=False, preserve_rng_state=draws)
             else:
                 x, qkv = blk.pre_attention(x, pending, rope_cache, rpos)
                 o = self.attn(qkv, pos)
