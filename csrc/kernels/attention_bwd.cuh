@@ -21,7 +21,8 @@ __host__ __device__ __forceinline__ int bwd_tiles(int c, int it_chunk, int n_kt,
 template <bool PARTS>
 __device__ __forceinline__ BwdWork bwd_work(int it_chunk, int n_kt, int nq, int G, int Hkv, int B, int k_off, int local) {
   if (!PARTS) return BwdWork{(int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, 0};
-  // longest first over all heads and batches, part 0 of every tile, then part 1 of those that have one, ...
+  // part 0 of every tile, the longest first over all heads and batches, then part 1 of those that have one, ...: longest first within a part
+  // number, not over all of them (a second part may be longer than the first of a later tile)
   int i = (int)blockIdx.x, c = 0;
   const int hb = Hkv * B;
   for (int n; i >= (n = bwd_tiles(c, it_chunk, n_kt, nq, G, k_off, local) * hb); ++c) i -= n;

@@ -30,6 +30,7 @@ namespace cpb {
 constexpr int FA_THREADS = 320;
 constexpr int FA_KSTAGES = 3;      // K is wanted one tile ahead of V (the next score tile overlaps the softmax of this one)
 constexpr int FA_VSTAGES = 2;
+constexpr int FA_RELEASE_KEYS = 1024;  // up to here the next kernel's blocks are let in early (see common.cuh)
 constexpr int FA_POLY_D64 = 0;     // default share (of 8) of the exponentials taken off the special-function unit
 constexpr int FA_POLY_D128 = 2;
 
@@ -113,7 +114,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_wait();                               // and no pdl_release(), see common.cuh
+  if (p.ready == nullptr && p.Tk <= FA_RELEASE_KEYS) pdl_release();
+  pdl_wait();
 
   // Range of K/V tiles this query tile attends to.
   const int q_last = min(q0 + FA_BQ, p.Tq) - 1;

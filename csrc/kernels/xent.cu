@@ -1,15 +1,12 @@
-// Softmax cross-entropy over a chunk of fp32 logits, forward and backward in one launch.
+// Softmax cross-entropy.  The language-model head never materialises [tokens, vocab] for the whole sequence: the host loops over row
+// chunks, the head's GEMM leaves statistics per column tile (gemm_common.cuh), xent_rows_kernel makes losses and gradient coefficients of
+// them and xent_dlogits_kernel dlogits = (softmax - onehot) * grad_scale of logits that were stored; two more GEMMs then produce dX
+// and accumulate dW.  Replaces the reference's materialised logits + sparse_cross_entropy_loss (Scripts/Blutrain/bluscriptCP.cpp:452-459,1712).
 //
-// The language-model head never materialises [tokens, vocab] for the whole sequence: the host loops
-// over row chunks, runs the lm_head GEMM into an fp32 chunk buffer, and this kernel turns the chunk
-// into per-row losses and bf16 dlogits = (softmax - onehot) * grad_scale in place of a separate
-// backward pass; two more GEMMs then produce dX and accumulate dW.  Replaces the reference's
-// materialised logits + sparse_cross_entropy_loss (Scripts/Blutrain/bluscriptCP.cpp:452-459,1712).
-//
-// With gradients the row is read from memory once: a cluster of CTAs keeps it in shared memory between the two passes
-// (xent_smem_kernel).  Without gradients, or when a row does not fit, one CTA per row computes max and sum(exp) online and,
-// if asked to, re-reads the row for dlogits (xent_kernel).  Rows whose target is negative are ignored (zero gradient, no
-// loss).
+// cpb_xent is for fp32 logits that a caller has: loss and dlogits in one launch.  With gradients the row is read from memory once: a
+// cluster of CTAs keeps it in shared memory between the two passes (xent_smem_kernel).  Without gradients, or when a row does not fit, one
+// CTA per row computes max and sum(exp) online and, if asked to, re-reads the row for dlogits (xent_kernel).  Rows whose target is
+// negative are ignored everywhere (zero gradient, no loss).
 #include "common.cuh"
 #include "host_utils.h"
 
