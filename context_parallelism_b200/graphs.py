@@ -45,29 +45,34 @@ class Written:
     anything else (a subclass's method, one replaced on a class or an object, another attention) would leave out what that does."""
 
     def __init__(self, model_cls, block_cls, attn_cls):
-        self.attn_cls, self.methods = attn_cls, {}
-        for cls, names in ((model_cls, ("hidden", "_hidden", "_block", "head_weight", "loss_with", "loss_sum", "per_token_nll", "recorded_inputs")),
-                           (block_cls, ("pre_attention", "post_attention")), (attn_cls, ("__call__",))):
-            self.methods[cls] = {n: cls.__dict__[n] for n in names}
-        self.model_cls, self.block_cls = model_cls, block_cls
+        self.model_cls, self.block_cls, self.attn_cls = model_cls, block_cls, attn_cls
+        self.methods = {cls: {n: cls.__dict__[n] for n in names} for cls, names in (
+            (model_cls, ("hidden", "_hidden", "_block", "head_weight", "loss_with", "loss_sum", "per_token_nll", "recorded_inputs")),
+            (block_cls, ("pre_attention", "post_attention")), (attn_cls, ("__call__",)))}
 
-    def _is(self, cls, objects) -> bool:
-        """Whether the methods that count are those of ``cls``, on the objects' types and on the objects."""
+    def _holds(self, cls, obj) -> bool:
         methods = self.methods[cls]
-        for t in set(map(type, objects)):
-            for n, f in methods.items():
-                if getattr(t, n, None) is not f:
-                    return False
-        names = methods.keys()
-        for o in objects:
-            if not names.isdisjoint(o.__dict__):
-                return False
-        return True
+        return isinstance(obj, cls) and _are(type(obj), methods) and methods.keys().isdisjoint(obj.__dict__)
+
+    def model_holds(self, model) -> bool:
+        """The model's own methods alone: enough before a replay, in front of which a record looks at the rest (see Weights)."""
+        return self._holds(self.model_cls, model)
 
     def holds(self, model) -> bool:
         attn = model.__dict__.get("attn")
-        return (type(attn) is self.attn_cls and attn.ctx.cp_size == 1 and self._is(self.attn_cls, (attn,)) and self._is(self.model_cls, (model,))
-                and self._is(self.block_cls, [*model.blocks]))
+        return (type(attn) is self.attn_cls and attn.ctx.cp_size == 1 and _are(self.attn_cls, self.methods[self.attn_cls])
+                and self.model_holds(model) and all(self._holds(self.block_cls, b) for b in model.blocks))
+
+    def of(self, obj):
+        """The methods that count for one module of the model."""
+        return next((m for cls, m in self.methods.items() if isinstance(obj, cls)), {})
+
+
+def _are(cls, methods) -> bool:
+    for n, f in methods.items():
+        if getattr(cls, n, None) is not f:
+            return False
+    return True
 
 
 def _read(module) -> tuple:
@@ -76,7 +81,7 @@ def _read(module) -> tuple:
     if "attn" not in d:
         return (d.get("cfg"),)
     attn = d["attn"]
-    return d.get("cfg"), getattr(attn, "cfg", attn), getattr(attn, "scale", None), getattr(getattr(attn, "ctx", None), "cp_size", 1)
+    return d.get("cfg"), getattr(attn, "cfg", attn), type(attn), getattr(attn, "scale", None), getattr(getattr(attn, "ctx", None), "cp_size", 1)
 
 
 def _listeners():
@@ -117,15 +122,21 @@ def _unchanged(a: tuple, b: tuple) -> bool:
 
 
 class Weights:
-    """The modules and parameters of a model as a record read them (weak references: a record does not keep its model alive)."""
+    """The modules, their methods and the parameters of a model as a record has them (weak references: a record does not keep its
+    model alive)."""
 
-    def __init__(self, model: torch.nn.Module, train: bool):
+    def __init__(self, model: torch.nn.Module, train: bool, written: Optional[Written] = None):
         self.train = train
-        self.mods = []
+        self.mods, self.types = [], {}
         for m in model.modules():
+            methods = {} if written is None else written.of(m)
+            if methods:
+                self.types[type(m)] = methods
             parts = [(n, weakref.ref(c)) for n, c in m._modules.items() if c is not None]
             params = [(n, weakref.ref(p), p.data_ptr(), _main_grad(p)) for n, p in m._parameters.items() if p is not None]
-            self.mods.append((weakref.ref(m), parts, _read(m), params))
+            self.mods.append((weakref.ref(m), type(m), methods.keys(), parts, _read(m), params))
+        if written is not None:
+            self.types[written.attn_cls] = written.methods[written.attn_cls]
 
     @staticmethod
     def recordable(model: torch.nn.Module) -> bool:
@@ -134,9 +145,12 @@ class Weights:
 
     def hold(self) -> bool:
         train = self.train
-        for ref, parts, read, params in self.mods:
+        for cls, methods in self.types.items():
+            if not _are(cls, methods):
+                return False
+        for ref, cls, names, parts, read, params in self.mods:
             m = ref()
-            if m is None or not _unchanged(_read(m), read):
+            if m is None or type(m) is not cls or not names.isdisjoint(m.__dict__) or not _unchanged(_read(m), read):
                 return False
             d = m._modules
             for n, c in parts:
@@ -225,10 +239,10 @@ class _Record:
 class GraphCache:
     """The records of one model, by name, input shapes and modes.  Safe with several threads and streams: a lock covers the copies in,
     the replay and the copies out, and an event orders replays of different streams.  ``limit``: bytes that the records' buffers may
-    take together, 0 to record nothing."""
+    take together, 0 to record nothing.  ``written``: what the model has to call for a call to be recorded."""
 
-    def __init__(self, limit: int = MAX_POOL_BYTES):
-        self.limit = limit
+    def __init__(self, limit: int = MAX_POOL_BYTES, written: Optional[Written] = None):
+        self.limit, self.written = limit, written
         self._lock = threading.Lock()
         self._room: Optional[_Room] = None                           # there while there are records
         self._records: "OrderedDict[tuple, Optional[_Record]]" = OrderedDict()
@@ -236,10 +250,10 @@ class GraphCache:
         self._lost: "OrderedDict[tuple, int]" = OrderedDict()        # how often it was
 
     def __reduce__(self):                                            # a copied or unpickled model starts without records
-        return GraphCache, (self.limit,)
+        return GraphCache, (self.limit, self.written)
 
     def __deepcopy__(self, memo):
-        return GraphCache(self.limit)
+        return GraphCache(self.limit, self.written)
 
     def run(self, name: str, model: torch.nn.Module, fn: Callable, inputs: Sequence[torch.Tensor], device: torch.device,
             flops: float, train: bool = False) -> Tuple[torch.Tensor, ...]:
@@ -256,6 +270,8 @@ class GraphCache:
                     self._records.move_to_end(key)
                     return rec.replay(inputs, torch.cuda.current_stream(device))
                 self._drop(key)
+        if self.written is not None and not self.written.holds(model):
+            return self._eager(fn, inputs, device, train)
         launches = nv.LAUNCHES[0]
         outs = self._eager(fn, inputs, device, train)
         launches = nv.LAUNCHES[0] - launches
@@ -297,7 +313,7 @@ class GraphCache:
                 self._drop_all()
                 self._room = _Room(device)
             try:
-                rec = _Record(fn, inputs, Weights(model, train), self._room)
+                rec = _Record(fn, inputs, Weights(model, train, self.written), self._room)
             except (RuntimeError, nv.NativeError):                   # out of memory, or something in fn that cannot be recorded
                 nv.lib().cpb_clear_error()                           # the call itself has run; its like stay eager from now on
             if rec is not None and self._room.bytes() > self.limit:

@@ -71,7 +71,7 @@ class GPT2(nn.Module):
             _padded_normal(cfg.vocab_size, cfg.vocab_padded, d, gen))
         self.to(device)
         self.attn = CPAttention(cfg, self.cp)
-        self.graphs = graphs.GraphCache(cfg.graph_pool_mb << 20)
+        self.graphs = graphs.GraphCache(cfg.graph_pool_mb << 20, _WRITTEN)
 
     def named_tensors(self) -> Dict[str, torch.Tensor]:
         """Parameters under the names of the named-init files: each block's first LayerNorm lives inside its
@@ -102,8 +102,8 @@ class GPT2(nn.Module):
         return ()
 
     def recordable(self) -> bool:
-        """One GPU, and nothing in a call but what this package wrote."""
-        return self.cp.cp_size == 1 and _WRITTEN.holds(self)
+        """One GPU and the methods of this class (``graphs`` looks at the blocks and the attention)."""
+        return self.cp.cp_size == 1 and _WRITTEN.model_holds(self)
 
     def _hidden(self, idx_local: torch.Tensor, pos: torch.Tensor) -> torch.Tensor:
         cfg = self.cfg

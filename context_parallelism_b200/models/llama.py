@@ -91,7 +91,7 @@ class Llama(nn.Module):
         self.attn = CPAttention(cfg, self.cp)
         self.rope_cache = R.build_rope_cache(cfg.T, cfg.head_dim, cfg.rope_theta, device, cfg.yarn)
         self.rope_pos_override: Optional[torch.Tensor] = None
-        self.graphs = graphs.GraphCache(cfg.graph_pool_mb << 20)
+        self.graphs = graphs.GraphCache(cfg.graph_pool_mb << 20, _WRITTEN)
 
     # ------------------------------------------------------------------ RoPE cache control
     def set_rope_cache(self, cache: torch.Tensor) -> None:
@@ -137,8 +137,8 @@ class Llama(nn.Module):
         return (self.rope_cache,) if self.rope_pos_override is None else (self.rope_cache, self.rope_pos_override)
 
     def recordable(self) -> bool:
-        """One GPU, and nothing in a call but what this package wrote."""
-        return self.cp.cp_size == 1 and _WRITTEN.holds(self)
+        """One GPU and the methods of this class (``graphs`` looks at the blocks and the attention)."""
+        return self.cp.cp_size == 1 and _WRITTEN.model_holds(self)
 
     def _hidden(self, idx_local: torch.Tensor, pos: torch.Tensor, rope_cache: torch.Tensor,
                 rope_pos: Optional[torch.Tensor] = None) -> torch.Tensor:
