@@ -150,14 +150,18 @@ def bench_membound(tm, out, rows, d, hbm_gbs):
     dact = torch.randn(rows, F_, device=dev).bfloat16()
     ms = tm.ms(lambda: E.swiglu_bwd(gu, dact))
     rec("swiglu_bwd", ms, rows * F_ * 2 * 5)
-    # cross entropy over one fp32 logit chunk: logits in, bf16 dlogits out
+    # the head's two passes beside its GEMMs: statistics of the column tiles to losses and coefficients; stored fp32 logits to bf16 dlogits
     V = 128256
     cr = min(rows, 4096)
-    logits = torch.randn(cr, V, device=dev)
+    x, w = torch.randn(cr, 64, device=dev).bfloat16(), torch.randn(V, 64, device=dev).bfloat16()
+    logits = torch.empty(cr, V, device=dev)
     tg = torch.randint(0, V, (cr,), device=dev)
     ls = torch.zeros(1, device=dev)
-    ms = tm.kernel_ms(lambda: X.xent_chunk(logits, tg, ls, 1.0, True, None, V), "xent")
-    rec("xent (loss + bf16 dlogits)", ms, cr * V * (4 + 2), rows=cr, d=V)
+    coef = X._head_rows(x, w, tg, V, 1.0, ls, None, True, logits)
+    ms = tm.kernel_ms(lambda: X._head_rows(x, w, tg, V, 1.0, ls, None, True, logits), "xent_rows")
+    rec("xent_rows (losses, coefficients)", ms, cr * (V + 255) // 256 * 8, rows=cr, d=V)
+    ms = tm.kernel_ms(lambda: X._head_dlogits(x, w, tg, coef, V, 1.0, logits), "xent_dlogits")
+    rec("xent_dlogits (stored logits)", ms, cr * V * (4 + 2), rows=cr, d=V)
     # AdamW: p, g, m, v read; p, m, v, bf16 copy written
     n = 256 << 20
     p, gr, m, v = (torch.randn(n, device=dev) * 0.01 for _ in range(4))

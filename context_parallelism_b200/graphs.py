@@ -4,7 +4,8 @@ A small model's forward and backward pass is some hundred kernels of 3 to 30 us 
 Python, autograd and ``ctypes``.  :class:`GraphCache` runs a call eagerly the first times that it sees its shapes, then records it
 once and replays the record.  Nothing depends on the caller's buffers: inputs are copied into the record's own, results are
 returned as new tensors.  What the record does read by address (weights, gradient buffers) is compared at every call, and a
-record whose weights have moved is dropped.  Measured on one B200, ms without and with records (and without the host's wait for every
+record whose weights have moved is dropped.  A model's records share one pool of memory; ``CP_GRAPH_POOL_MB`` bounds it, 0 turns records
+off.  Measured on one B200, ms without and with records (and without the host's wait for every
 micro-batch): next-token logits of 136 tokens, GPT-2 124M 2.69 and 0.71; NLL of 4096 tokens, 48M 1.48 and 0.77; a step of GPT-2 44M, 16
 micro-batches of 4 x 1024 tokens 47.7 and 22.6; of GPT-2 124M, two micro-batches 17.6 and 14.9.
 """
@@ -22,7 +23,9 @@ from torch.autograd import forward_ad
 from . import _native as nv
 
 MAX_RECORDS = 32                 # per model; the one used longest ago makes room
-EAGER_CALLS = 3                  # calls with new shapes that run as they always did; twice as many each time that the record was lost
+# Calls with new shapes that run as they always did; twice as many each time that the record was lost.  A record costs 9 to 18 ms (98 to 178
+# launches, its memory first), what 4 to 8 replays save: at the second call a step of two micro-batches would pay for it in its first pass.
+EAGER_CALLS = 3
 MAX_POOL_BYTES = 4 << 30         # buffers of all records of a model, unless its configuration says otherwise (graph_pool_mb)
 MIN_FREE_SHARE = 0.25            # share of the GPU's memory that has to be free before a record is made
 # A call is recorded while the GPU needs less time for it than the host: a launch costs the host about 25 us (forward and backward;

@@ -1,12 +1,12 @@
 """Fused language-model head + cross-entropy that never materialises ``[tokens, vocab]``.
 
-``linear_cross_entropy(x, w, targets)`` returns the *sum* of token NLLs (fp32) and the number of
-counted tokens.  On CUDA the rows are processed in chunks: lm_head GEMM into an fp32 chunk buffer →
-``xent`` kernel (loss + bf16 dlogits in one pass) → dX chunk GEMM and dW accumulation, all inside the
-forward call (the gradient of a sum-of-NLL loss with respect to the logits does not depend on
-anything downstream except one scalar, which is applied in ``backward``).  The reference materialises
-the full logits tensor (Scripts/Blutrain/bluscriptCP.cpp:452-459), which at T = 128 K and a 128 K
-vocabulary would be 64 GB.
+``linear_cross_entropy(x, w, targets)`` returns the *sum* of token NLLs (fp32).  On CUDA the rows are processed in chunks: the lm_head
+GEMM leaves (max, sum of exponentials) of each row and column tile (``gemm_head``), ``xent_rows`` turns them into losses and the rows'
+gradient coefficients, and for gradients the bf16 dlogits come from a second GEMM with the same epilogue or, for wide hidden states,
+from logits that the first one stored (``xent_dlogits``); a dX chunk GEMM and the accumulation of dW follow.  All of it happens inside
+the forward call (the gradient of a sum-of-NLL loss with respect to the logits does not depend on anything downstream except one
+scalar, which is applied in ``backward``).  The reference materialises the full logits tensor (Scripts/Blutrain/bluscriptCP.cpp:452-459),
+which at T = 128 K and a 128 K vocabulary would be 64 GB.
 """
 from __future__ import annotations
 
@@ -28,6 +28,8 @@ RECOMPUTE_WIDTH = 1024
 
 def xent_chunk(logits: torch.Tensor, targets: torch.Tensor, loss_sum: torch.Tensor, grad_scale: float,
                want_grad: bool = True, row_loss: torch.Tensor = None, n_valid: int = 0):
+    """Cross entropy of fp32 logits that the caller has in memory: loss and bf16 dlogits in one launch.  The head does not store them whole
+    and does not come by here."""
     rows, Vc = logits.shape
     V = n_valid or Vc
     dlog = torch.empty((rows, Vc), dtype=torch.bfloat16, device=logits.device) if want_grad else None
