@@ -119,6 +119,8 @@ class TrainEngine:
         torch keeps the page-locked copy made here until the device has read it.  4 x 1024 tokens cost the host about 20 us."""
         if self.device.type != "cuda" or not isinstance(t, torch.Tensor) or t.is_cuda or not t.is_pinned():
             return t
+        if torch.cuda.is_current_stream_capturing():                 # a graph of the caller's reads the caller's buffer at every replay
+            return t
         return torch.empty(t.shape, dtype=t.dtype, pin_memory=True).copy_(t)
 
     def forward_backward(self, tokens, targets, accum: int = 1, last: bool = True) -> torch.Tensor:

@@ -33,3 +33,25 @@ def test_buffers_are_written_again_at_once(recorded, view):
         assert abs(float(la) - float(lb)) <= 1e-4 * abs(float(lb))
     assert_close(a.flat.grad, b.flat.grad, cos=0.99999, rel=1e-2, name="grad")
     a.check_kernels()
+
+
+def test_a_graph_of_the_callers_reads_the_callers_buffers():
+    """A capture of a whole micro-batch keeps the caller's page-locked buffers as its inputs."""
+    from context_parallelism_b200.config import Config
+    from context_parallelism_b200.engine import TrainEngine
+    cfg = Config.from_env("llama", 1, env={}).replace(
+        n_embd=256, n_layer=2, n_head=4, n_kv_head=2, head_dim=64, ffn_hidden=512, vocab_size=1000, T=200, B=2, checkpointing=False, dtype="bf16")
+    eng = TrainEngine(cfg, torch.device("cuda", 0))
+    batches = [torch.randint(0, 1000, (2, 201), generator=torch.Generator().manual_seed(i)) for i in range(3)]
+    x, y = (torch.zeros(2, 200, dtype=torch.int64).pin_memory() for _ in range(2))
+    want = [float(eng.forward_backward(t[:, :-1].contiguous().cuda(), t[:, 1:].contiguous().cuda())) for t in batches]
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        loss = eng.forward_backward(x, y)
+    for t, w in zip(batches, want):
+        x.copy_(t[:, :-1]), y.copy_(t[:, 1:])
+        graph.replay()
+        torch.cuda.synchronize()
+        assert abs(float(loss) - w) <= 1e-4 * abs(w)
+    eng.check_kernels()
