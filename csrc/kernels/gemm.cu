@@ -400,28 +400,8 @@ static long plan_width(int cand, int M, int N, int K, int epi, int has_aux, int 
   return best;
 }
 
-// Tiles of 384 columns where N is one column of them and two of the others, and L2 does not hold A: it is read once.  us, the best of
-// the other widths and this one: bf16 4096 x 264 x 50304 144 and 124, x 384 144 and 134; accumulating 50304 x 320 x 4096 151 and 132, x 384
-// 155 and 136; bf16 16384 x 264 x 2048 33.9 and 31.7.  Its one accumulator leaves the epilogue bare, so it wants many K blocks or a single
-// wave (65536 x 384 x 1024 54.3 and 56.4, accumulating 64.5 and 72; 65536 x 384 x 2048 87 and 91), and few large items want full waves (12000
-// x 384 x 4096, 47 items for 74 pairs, 46.1 and 50.2; 20360 x 384 x 2056, 80 items, 50.2 and 54.3) without a split that the others can do
-// without (8192 x 384 x 4096 in two 33.8 and 35.8, 8192 x 384 x 8192 54.3 and 56.3; 4096 x 384 x 8192 in four 39.8 and 37.7).  With two
-// and more columns of tiles it costs more than it saves (4096 x 768 x 50304 217 to 234 and 233 to 255, 50304 x 768 x 4096 238 and 267).
-static bool one_column(int M, int N, int K, int epi) {
-  if ((epi != EPI_F32_ACC && epi != EPI_BF16) || N <= 256 || N > 384 || (long)M * K * 2 < (64L << 20)) return false;
-  const long m_tiles = (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM), pairs = sm_count() > 1 ? sm_count() / 2 : 1;
-  int s = 1;
-  plan_width(384, M, N, K, epi, 0, 0, s);
-  const long waves = (m_tiles * s + pairs - 1) / pairs;
-  return 5 * m_tiles * s >= 4 * pairs * waves && K >= (waves > 1 ? 4096 : 2048) && (s == 1 || 10 * m_tiles < 4 * pairs);
-}
-
-// `want` > 0 asks for the best width at that many splits, 0 for the best of both.
-static void plan_tiles(int M, int N, int K, int epi, int has_aux, int want, int& bn, int& splits) {
-  if (one_column(M, N, K, epi)) {
-    plan_width(bn = 384, M, N, K, epi, has_aux, want, splits);
-    return;
-  }
+// The best of the usual widths.
+static long plan_narrow(int M, int N, int K, int epi, int has_aux, int want, int& bn, int& splits) {
   long best = -1;
   for (const int cand : {256, 192, 128}) {
     if (cand == 192 && epi == EPI_BF16_SWIGLU) continue;
@@ -429,6 +409,33 @@ static void plan_tiles(int M, int N, int K, int epi, int has_aux, int want, int&
     const long t = plan_width(cand, M, N, K, epi, has_aux, want, s);
     if (t >= 0 && (best < 0 || t < best)) { best = t; bn = cand; splits = s; }
   }
+  return best;
+}
+
+// Tiles of 384 columns where N is one column of them and two of the others, and L2 does not hold A: it is read once, which is worth a
+// tenth of the time that the plan expects of the others.  us, the best of the other widths and this one: bf16 4096 x 264 x 50304 157 and 134,
+// x 384 157 and 132, 131072 x 384 x 2056 217 and 170, 37888 x 320 x 2056 66 and 59, 55000 x 264 x 3072 100 and 95; accumulating 50304 x 320 x 4096 163
+// and 138, 33000 x 264 x 1024 53 and 43.  Left to the others: bf16 24000 x 384 x 3072 (94 tiles for 74 pairs) 60 and 68, 65536 x 384 x 1024 56 and
+// 60.  Over 224 such sizes, bf16 and accumulating, the choice is 1 % above the better of the two.
+// Splits of it: not where the others do without (8192 x 384 x 4104 in two 39 and 42), but with few tiles whatever the plan expects
+// (bf16 4096 x 384 x 8192 in four 43 and 38).  Rows of A that do not all start on a 128-byte line are dear to read twice: bf16 then takes
+// half full waves too (20360 x 384 x 4104 97 and 92, 42000 x 320 x 4104 142 and 131, 65536 x 264 x 4104 197 and 164; from a K of 2048 on above 320
+// columns: 20360 x 384 x 2056 51 and 53, 42000 78 and 78, 65536 109 and 102).  With two and more columns of tiles it costs more than it
+// saves (4096 x 768 x 50304 217 to 234 and 233 to 255, 50304 x 768 x 4096 238 and 267).
+static bool one_column(int M, int N, int K, int epi) {
+  if ((epi != EPI_F32_ACC && epi != EPI_BF16) || N <= 256 || N > 384 || K < 1024 || (long)M * K * 2 < (64L << 20)) return false;
+  const long m_tiles = (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM), pairs = sm_count() > 1 ? sm_count() / 2 : 1;
+  int bn, s = 1, narrow_s = 1;
+  const long t = plan_width(384, M, N, K, epi, 0, 0, s), narrow_t = plan_narrow(M, N, K, epi, 0, 0, bn, narrow_s);
+  if (s > 1 && 10 * m_tiles >= 4 * pairs) return false;
+  const long items = m_tiles * s, slots = (items + pairs - 1) / pairs * pairs;
+  return 10 * t <= 11 * narrow_t || (s > 1 && 5 * items >= 4 * slots) || (epi == EPI_BF16 && K % 64 != 0 && K >= (N > 320 ? 2048 : 4096) && 2 * items >= slots);
+}
+
+// `want` > 0 asks for the best width at that many splits, 0 for the best of both.
+static void plan_tiles(int M, int N, int K, int epi, int has_aux, int want, int& bn, int& splits) {
+  if (one_column(M, N, K, epi)) plan_width(bn = 384, M, N, K, epi, has_aux, want, splits);
+  else plan_narrow(M, N, K, epi, has_aux, want, bn, splits);
 }
 
 // banded tile order once B (N x K bf16) reaches 64 MB, half of L2; CPB_GEMM_BAND (read once) overrides

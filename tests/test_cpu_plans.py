@@ -13,11 +13,13 @@ def _width(M, N, K, epi):
 def test_one_column_of_384(epi):
     """Tiles of 384 columns follow sizes, not one width of the models."""
     for N in (264, 320, 344, 376, 384):                               # one such column, two of the next width
-        for M, K in ((4096, 50304), (50304, 4096), (1250, 50304), (16384, 2048), (4096, 8192), (128256, 4096)):
+        for M, K in ((4096, 50304), (50304, 4096), (1250, 50304), (16384, 2048), (4096, 8192), (128256, 4096), (30000, 2056), (33000, 1536)):
             assert _width(M, N, K, epi) == 384
         # A that L2 holds; few K blocks; items that leave a third of the pairs idle; a split that narrower tiles do without
-        for M, K in ((4096, 4096), (65536, 1024), (65536, 2048), (20360, 2056), (12000, 4096), (8192, 4096), (8192, 8192)):
+        for M, K in ((4096, 4096), (65536, 960), (20360, 2048), (24000, 3072), (12000, 3072), (8192, 4096), (8192, 8192)):
             assert _width(M, N, K, epi) < 384
+        # rows off a 128-byte line, waves half full
+        assert _width(20360, N, 2056, EPI_BF16) == (384 if N > 320 else 192) and _width(42000, N, 4104, EPI_BF16) == 384
     assert all(_width(M, N, K, epi) < 384 for N in (192, 256, 392, 768) for M, K in ((4096, 50304), (50304, 4096)))
     assert all(_width(4096, N, 50304, EPI_F32) < 384 for N in (264, 384))
 

@@ -11,9 +11,8 @@ pytestmark = pytest.mark.gpu
 SHAPES = [(256 * 74, 192, 64), (256 * 74, 384, 72), (256 * 37, 376, 520), (4096, 768, 3072), (256 * 74 - 120, 184, 328)]
 
 
-# 384 columns: two products of 256 and 128 columns per step, one accumulator; M and K with remainders, one and several items per pair, N from
-# one column of tiles of the next width on.  (80 items for 74 pairs, which stood here, are faster in narrower tiles: see one_column() in gemm.cu.)
-WIDE = [(256 * 74, 384, 2048), (256 * 148 - 120, 384, 4104), (4096, 384, 12008), (256 * 74 - 8, 264, 2056), (4096, 328, 12008)]
+# 384 columns: two products of 256 and 128 columns per step, one accumulator; M and K with remainders, one and several items per pair
+WIDE = [(256 * 74, 384, 2048), (256 * 80 - 120, 384, 2056), (4096, 384, 12008)]
 
 
 def _operands(M, N, K):
@@ -66,3 +65,13 @@ def test_bf16_split_along_k(M, N, K):
         if out is not None:
             assert bool((out[:, :8] == 7).all() and (out[:, 8 + N:] == 7).all())
     nv.status_for(a.device).check("gemm")
+
+
+# 384 columns for less than 384: one column of tiles of the next width on, with remainders in M, N and K; two full waves
+NARROWER = [(256 * 148 - 120, 384, 4104), (256 * 74 - 8, 264, 2056), (4096, 328, 12008)]
+
+
+@pytest.mark.parametrize("M,N,K", NARROWER)
+def test_one_column_of_384(M, N, K, monkeypatch):
+    monkeypatch.setitem(globals(), "WIDE", NARROWER)
+    test_every_epilogue_and_order(M, N, K)
