@@ -23,9 +23,10 @@ from torch.autograd import forward_ad
 from . import _native as nv
 
 MAX_RECORDS = 32                 # per model; the one used longest ago makes room
-# Calls with new shapes that run as they always did; twice as many each time that the record was lost.  A record costs 9 to 18 ms (98 to 178
-# launches, its memory first), what 4 to 8 replays save: at the second call a step of two micro-batches would pay for it in its first pass.
-EAGER_CALLS = 3
+# Of the calls with new shapes, the one that is recorded (those before it run as they always did); twice as late each time that the record
+# was lost.  A record costs 9 to 18 ms (98 to 178 launches, its memory first), what 4 to 8 replays save, about half of them the launches that
+# an eager call would issue as well; at the second call a step of two micro-batches would pay for it in its first pass.
+RECORD_AT = 3
 MAX_POOL_BYTES = 4 << 30         # buffers of all records of a model, unless its configuration says otherwise (graph_pool_mb)
 MIN_FREE_SHARE = 0.25            # share of the GPU's memory that has to be free before a record is made
 # A call is recorded while the GPU needs less time for it than the host: a launch costs the host about 25 us (forward and backward;
@@ -249,7 +250,7 @@ class GraphCache:
         self._lock = threading.Lock()
         self._room: Optional[_Room] = None                           # there while there are records
         self._records: "OrderedDict[tuple, Optional[_Record]]" = OrderedDict()
-        self._seen: "OrderedDict[tuple, int]" = OrderedDict()        # eager calls since the record was lost, or at all
+        self._seen: "OrderedDict[tuple, tuple]" = OrderedDict()      # eager calls since the record was lost, or at all; launches of one
         self._lost: "OrderedDict[tuple, int]" = OrderedDict()        # how often it was
 
     def __reduce__(self):                                            # a copied or unpickled model starts without records
@@ -275,17 +276,20 @@ class GraphCache:
                 self._drop(key)
         if self.written is not None and not self.written.holds(model):
             return self._eager(fn, inputs, device, train)
-        launches = nv.LAUNCHES[0]
+        with self._lock:
+            n, launches = self._seen.get(key, (0, 0))
+            if key not in self._records and n + 1 >= RECORD_AT << min(self._lost.get(key, 0), 8):
+                self._seen.pop(key, None)
+                rec = self._record(key, model, fn, inputs, device, flops < GPU_TFLOPS * 1e6 * HOST_US_PER_LAUNCH * launches, train)
+                if rec is not None:
+                    return rec.replay(inputs, torch.cuda.current_stream(device))
+        before = nv.LAUNCHES[0]
         outs = self._eager(fn, inputs, device, train)
-        launches = nv.LAUNCHES[0] - launches
         with self._lock:
             if key not in self._records:
-                n = self._seen[key] = self._seen.pop(key, 0) + 1
+                self._seen[key] = self._seen.pop(key, (0, 0))[0] + 1, nv.LAUNCHES[0] - before
                 while len(self._seen) > 64:
                     self._seen.popitem(last=False)
-                if n >= EAGER_CALLS << min(self._lost.get(key, 0), 8):
-                    self._seen.pop(key, None)
-                    self._record(key, model, fn, inputs, device, flops < GPU_TFLOPS * 1e6 * HOST_US_PER_LAUNCH * launches, train)
         return outs
 
     def _eager(self, fn, inputs, device, train: bool):
@@ -308,7 +312,7 @@ class GraphCache:
             self._drop_all()
         return call()
 
-    def _record(self, key, model, fn, inputs, device, launch_bound: bool, train: bool) -> None:
+    def _record(self, key, model, fn, inputs, device, launch_bound: bool, train: bool) -> Optional[_Record]:
         free, total = torch.cuda.mem_get_info(device) if launch_bound else (0, 1)
         rec = None
         if free > MIN_FREE_SHARE * total and (not train or Weights.recordable(model)):
@@ -318,7 +322,7 @@ class GraphCache:
             try:
                 rec = _Record(fn, inputs, Weights(model, train, self.written), self._room)
             except (RuntimeError, nv.NativeError):                   # out of memory, or something in fn that cannot be recorded
-                nv.lib().cpb_clear_error()                           # the call itself has run; its like stay eager from now on
+                nv.lib().cpb_clear_error()                           # nothing has run; this call and its like are eager
             if rec is not None and self._room.bytes() > self.limit:
                 rec.close()
                 rec = None
@@ -334,6 +338,7 @@ class GraphCache:
                 break
         if not held:
             self._room = None
+        return self._records.get(key)
 
     def _drop(self, key) -> None:
         rec = self._records.pop(key)
