@@ -106,7 +106,7 @@ class _FlashAttnPackedFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, qkv, Hq, Hkv, D, scale, causal):
-        B, T, W = qkv.shape
+        B, T, W = *qkv.shape[:2], qkv.shape[2:].numel()
         dev = qkv.device
         # allocated in the shape it is returned in: autograd refuses in-place operations on a view made in here
         out = torch.empty((B, T, Hq * D), dtype=torch.bfloat16, device=dev)

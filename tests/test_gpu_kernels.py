@@ -478,6 +478,18 @@ def test_packed_attention_output_can_be_changed_in_place():
     assert torch.equal(out.detach(), want)
 
 
+def test_packed_attention_takes_the_heads_as_a_dimension_of_their_own():
+    from context_parallelism_b200.ops import attention as A
+    torch.manual_seed(7)
+    qkv, do = torch.randn(2, 130, 8 * 64, device=dev()).bfloat16(), torch.randn(2, 130, 4 * 64, device=dev()).bfloat16()
+    a, b = qkv.clone().requires_grad_(), qkv.view(2, 130, 8, 64).clone().requires_grad_()
+    outs = [A.flash_attention_packed(x, 4, 2, 64, 0.125) for x in (a, b)]
+    [o.backward(do) for o in outs]
+    check_status()
+    assert torch.equal(*outs) and torch.equal(a.grad[..., 256:], b.grad.view(2, 130, 512)[..., 256:])
+    assert_close(a.grad.float(), b.grad.view(2, 130, 512).float(), cos=0.99999, rel=4e-3, name="dqkv")
+
+
 @pytest.mark.parametrize("B,T,H,D,with_pos", [(2, 130, 3, 64, True), (1, 128, 2, 128, False), (1, 1, 1, 64, False)])
 def test_flash_bwd_prep_outputs(B, T, H, D, with_pos):
     from context_parallelism_b200.ops import attention_bwd as AB
