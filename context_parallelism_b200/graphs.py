@@ -125,6 +125,10 @@ def _unchanged(a: tuple, b: tuple) -> bool:
     return a[0] is b[0] and len(a) == len(b) and (len(a) == 1 or (a[1] is b[1] and a[2:] == b[2:]))
 
 
+def _NONE():
+    """In the place of a weak reference to a module or parameter that is not there."""
+
+
 class Weights:
     """The modules, their methods and the parameters of a model as a record has them (weak references: a record does not keep its
     model alive)."""
@@ -136,8 +140,9 @@ class Weights:
             methods = {} if written is None else written.of(m)
             if methods:
                 self.types[type(m)] = methods
-            parts = [(n, weakref.ref(c)) for n, c in m._modules.items() if c is not None]
-            params = [(n, weakref.ref(p), p.data_ptr(), _main_grad(p)) for n, p in m._parameters.items() if p is not None]
+            parts = [(n, _NONE if c is None else weakref.ref(c)) for n, c in m._modules.items()]
+            params = [(n, weakref.ref(p), p.data_ptr(), p.shape, p.is_contiguous(), _main_grad(p)) if p is not None else (n, _NONE, 0, None, True, 0)
+                      for n, p in m._parameters.items()]
             self.mods.append((weakref.ref(m), type(m), methods.keys(), parts, _read(m), params))
         if written is not None:
             self.types[written.attn_cls] = written.methods[written.attn_cls]
@@ -156,14 +161,24 @@ class Weights:
             m = ref()
             if m is None or type(m) is not cls or not names.isdisjoint(m.__dict__) or not _unchanged(_read(m), read):
                 return False
-            d = m._modules
+            d = m._modules                                           # one more is a change as well, as is one where there was none
+            if len(d) != len(parts):
+                return False
             for n, c in parts:
-                if d.get(n) is not c():
+                if n not in d or d[n] is not c() or (d[n] is None and c is not _NONE):
                     return False
             d = m._parameters
-            for n, r, at, grad in params:
+            if len(d) != len(params):
+                return False
+            for n, r, at, shape, dense, grad in params:
                 p = d.get(n)
-                if p is None or p is not r() or p.data_ptr() != at:
+                if p is None:                                        # and was none: a weak reference to what is gone gives None, too
+                    if r is not _NONE or n not in d:
+                        return False
+                    continue
+                if p is not r():
+                    return False
+                if p.data_ptr() != at or p.shape != shape or p.is_contiguous() != dense:
                     return False
                 if train and not (p.requires_grad and _main_grad(p) == grad and _quiet(p)):
                     return False
