@@ -4,7 +4,7 @@ A small model's forward and backward pass is some hundred kernels of 3 to 30 us 
 Python, autograd and ``ctypes``.  :class:`GraphCache` runs a call eagerly the first times that it sees its shapes, then records it
 once and replays the record.  Nothing depends on the caller's buffers: inputs are copied into the record's own, results are
 returned as new tensors.  What the record does read by address (weights, gradient buffers) is compared at every call, and a
-record whose weights have moved is dropped.  A model's records share one pool of memory; ``CP_GRAPH_POOL_MB`` bounds it, 0 turns records
+record whose weights have moved or changed their shape is dropped.  A model's records share one pool of memory; ``CP_GRAPH_POOL_MB`` bounds it, 0 turns records
 off.  Measured on one B200, ms without and with records (and without the host's wait for every
 micro-batch): next-token logits of 136 tokens, GPT-2 124M 2.69 and 0.71; NLL of 4096 tokens, 48M 1.48 and 0.77; a step of GPT-2 44M, 16
 micro-batches of 4 x 1024 tokens 47.7 and 22.6; of GPT-2 124M, two micro-batches 17.6 and 14.9.
@@ -24,8 +24,8 @@ from . import _native as nv
 
 MAX_RECORDS = 32                 # per model; the one used longest ago makes room
 # Of the calls with new shapes, the one that is recorded (those before it run as they always did); twice as late each time that the record
-# was lost.  A record costs 9 to 18 ms (98 to 178 launches, its memory first), what 4 to 8 replays save, about half of them the launches that
-# an eager call would issue as well; at the second call a step of two micro-batches would pay for it in its first pass.
+# was lost.  A record costs 3 to 30 ms, its launches and 0.3 ms for each block of memory that the driver is asked for: a micro-batch of the 48M
+# model 18, 13 of them on top of an eager call, what five replays save.  At the second call a step of two would pay for it in its first pass.
 RECORD_AT = 3
 MAX_POOL_BYTES = 4 << 30         # buffers of all records of a model, unless its configuration says otherwise (graph_pool_mb)
 MIN_FREE_SHARE = 0.25            # share of the GPU's memory that has to be free before a record is made

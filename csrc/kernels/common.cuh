@@ -59,7 +59,8 @@ __device__ __forceinline__ bool elect_one() {
 // Nor in the attention kernels: their CTAs are long and uneven, and the blocks that wait on the SMs already done slow down the ones still
 // running (32749 tokens, 4/1 heads of 128, us per pass, one after the other: all releasing 3900, without the backward's 3896, without
 // the forward's either 3742, before dependent launches 3766; the backward kernel 2552 to 2680 and 2494 to 2507; the whole
-// gradient in a chain, with and without: 2 x 1000, 6/2 heads of 64 24.5 and 22.9, 4000, 8/2 of 128 105.4 and 98.5).  Up to 1024 keys the
+// gradient in a chain, with and without: 2 x 1000, 6/2 heads of 64 25.0 and 23.5, 1024, 32/8 of 128 55.6 and 53.4, 4000, 8/2 105.4 and 98.5; with
+// the forward before it 2 x 1000 39.6 and 41.7, 2 x 300 28.5 and 25.3, 1024, 32/8 of 128 78.8 and 77.3).  Up to 1024 keys the
 // forward does all the same, its CTAs are short there (one window of GPT-2 124M, us without and with: 136 tokens 633 and 624, 4 x 1024
 // tokens 1499 and 1486; of the 48M model, 1024 tokens 381 and 370; 2048 and 4096 tokens the same).
 // us per GEMM in a chain, without and with: 136 x 768 x 64 4.6 and 3.7, 136 x 2304 x 768 7.2 and 6.1, 4096 x 1536 x 384 8.7 and 8.0.
